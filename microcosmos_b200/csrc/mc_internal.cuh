@@ -20,9 +20,6 @@ constexpr int kBinTile = 16;       // binning tile edge for the deterministic re
 // kernels: 128 spreads the 1024² workload's 16,384 nodes over 128 SMs instead of 64
 // (measured: 0.1733 → 0.1720 ms per step; batch 1.990 → 1.982 ms; 64 is no better)
 constexpr int kNodeThreads = 128;
-// chain rods (one warp each) per CTA of the chain kernel: one spreads the rods over the most
-// SMs (measured per batch step: 1.963 ms with 1, 1.965 with 2, 1.973 with 4)
-constexpr int kChainWarps = 1;
 constexpr int kHeadThreads = 128;
 constexpr int kLbmTileX = 128;     // dense LBM CTA tile: 32 lanes x 4 cells
 constexpr int kStageCells = 1024;  // staged dense pass: lattice cells per item (a band of whole rows)
@@ -164,7 +161,7 @@ struct RDesc {
   int* wl_ctl;         // [0] IB list length, [1] CIC list length, [2] / [3] their cursors
   // rod components: chains (warp kernel) and general graphs (CTA kernel)
   int nchain, ngeneric;
-  const int* chain_comp;    // (nchain) component index
+  const int4* chain_info;   // (nchain) first node, nodes, first edge, first pair
   const int* generic_comp;  // (ngeneric)
   unsigned* flags;  // MC_FLAG_* for this rollout
 };
@@ -189,10 +186,12 @@ __device__ __forceinline__ int find_rollout(const int* __restrict__ off, int n, 
 // so the shortcut below returns the same bits as the fmodf route.
 __device__ __forceinline__ float fmod_floor(float x, float y) {
   if (fabsf(x) < 2.0f * y) {
-    // both signs' results are formed and one is selected (no divergent branch)
-    const float rp = (x >= y) ? x - y : x;
-    float rn = (x <= -y) ? x + y : x;
-    rn = (rn < 0.0f) ? rn + y : rn;
+    // both signs' results are formed and one is selected (no divergent branch).  For x < 0 one
+    // y is always added; the sum is below zero only where fmodf would have added it already
+    // (x < -y), and then the sign rule adds the second.
+    const float a = x + y, b = a + y, c = x - y;
+    const float rp = (x >= y) ? c : x;
+    const float rn = (a < 0.0f) ? b : a;
     return (x >= 0.0f) ? rp : rn;
   }
   float r = fmodf(x, y);
@@ -249,7 +248,7 @@ cudaError_t tiles_set_smem(size_t bytes);
 void launch_fft_rows(const Launch& L, size_t smem);
 void launch_fft_cols(const Launch& L, size_t smem);
 void launch_node(const Launch& L, const int* tdev, size_t smem, int bs);
-void launch_chain(const Launch& L, const int* tdev, int slots);
+void launch_chain(const Launch& L, const int* tdev, int longest);
 void launch_steric(const Launch& L);
 void launch_stencil(const Launch& L);
 void launch_stencil16(const Launch& L);

@@ -1,14 +1,14 @@
 // Node-side kernels of one step (src/microcosmos/simulate.py:37-84):
 //   k_predict: damping, inertial prediction, steric cloud-in-cell contributions;
 //   k_steric:  per node, the steric force added to the prediction (forces.py:41-81);
-//   k_chain:   one warp per chain rod (the topology make_edges(.., "line", F) builds),
-//              node/edge state in registers, neighbours exchanged with shuffles;
+//   k_chain:   one CTA per chain rod (the topology make_edges(.., "line", F) builds),
+//              one node per lane, neighbours exchanged with shuffles (rod.cuh);
 //   k_node:    one CTA per rod of any other topology (trees, loops), state in shared
 //              memory, scatter-adds as gather lists in the reference's order.
 //   k_stencil: per node, the velocity from positions and the IB stencil (fluid.py:40-87).
 // Both rod kernels evaluate the curvature actuation and run cycles_per_step Jacobi
 // iterations of pbd_rod_constraint (solver/pbd.py:14-91).
-#include "lbm_cell.cuh"
+#include "rod.cuh"
 
 namespace mc {
 
@@ -148,22 +148,7 @@ __device__ __forceinline__ float2 node_start(const RDesc& d, int gi) {
   return make_float2(qx, qy);
 }
 
-// Rest angle of pair gb at step t (the caller-side curvature actuation, if any).
-__device__ __forceinline__ float rest_angle(const RDesc& d, int gb, int t) {
-  if (!d.act_amp) return d.rest_ang[gb];
-  const float arg = d.act_omega[gb] * (float)(d.act_t0 + t) + d.act_phase[gb];
-  const float a = d.act_c[gb] + d.act_amp[gb] * sinf(arg);
-  d.rest_ang[gb] = a;
-  return a;
-}
-
-// One theta correction (pbd.py:35-40) and one edge force (pbd.py:60-81).
-__device__ __forceinline__ float bend_corr(float th_in, float th_out, float rest, float kb) {
-  float diff = th_out - th_in;
-  diff = fmod_floor(diff + MC_PI_F, MC_2PI_F) - MC_PI_F;
-  return ((diff - rest) * kb) * 0.5f;
-}
-
+// One edge force (pbd.py:60-81).
 __device__ __forceinline__ float2 edge_force(const RDesc& d, float th, float L0, float xs, float ys, float xt,
                                              float yt) {
   float sn, cs;
@@ -396,220 +381,16 @@ __global__ void __launch_bounds__(256) k_steric(const RDesc* __restrict__ D, con
   d.pos[2 * gi + 1] = s.y;
 }
 
-// ---------------------------------------------------------------- chains: warp per rod
-// Lane l owns nodes/edges/pairs j = l*P + q (q < P).  In a chain, edge j = (node j, node
-// j+1) and pair j = (edge j, edge j+1); the scatter-adds reduce to
-//   theta_j += ((0 + c_j) + (-c_{j-1})) / deg_j * 1.8,   x_j += ((0 + f_j) + (-f_{j-1})) / deg_j
-// with the terms that exist, in the reference's order (e_in / src updates first).
-template <int P>
-__device__ __forceinline__ void shift_next(const float (&v)[P], float (&nx)[P]) {
-  const float first_next = __shfl_down_sync(0xffffffffu, v[0], 1);
-#pragma unroll
-  for (int q = 0; q < P - 1; ++q) nx[q] = v[q + 1];
-  nx[P - 1] = first_next;
-}
-template <int P>
-__device__ __forceinline__ void shift_prev(const float (&v)[P], float (&pv)[P]) {
-  const float last_prev = __shfl_up_sync(0xffffffffu, v[P - 1], 1);
-#pragma unroll
-  for (int q = P - 1; q > 0; --q) pv[q] = v[q - 1];
-  pv[0] = last_prev;
-}
-
-// Stable-Cosserat iterations of one chain rod (solver/stable_cosserat.py:13-119), same
-// lane layout as the PBD loop below.  Phase 1: the bending pass without over-relaxation,
-// then theta += wrap(atan2(r) - theta) * 0.05 with r the segment's min-image vector.
-// Phase 2: x += (w (y0 - x) + f_j - f_{j-1}) / ((w + H_j) + H_{j-1}), f = (k_s/l)(r/l - d),
-// H = k_s/l^2, y0 the inertial prediction (the positions the kernel started from).
-template <int P>
-__device__ __forceinline__ void cosserat_chain(const RDesc& d, int lane, int nn, int ne, int nb, float (&x)[P],
-                                               float (&y)[P], float (&th)[P], const float (&l0)[P],
-                                               const float (&ra)[P], const float (&kb)[P], const float (&edg)[P]) {
-  const float W = (float)d.W, H = (float)d.H;
-  const float ks = d.k_stretch, w = d.cos_w;
-  float x0[P], y0[P];
-#pragma unroll
-  for (int q = 0; q < P; ++q) {
-    x0[q] = x[q];
-    y0[q] = y[q];
-  }
-  for (int it = 0; it < d.cycles; ++it) {
-    float nx[P], pv[P], c[P], xn[P], yn[P];
-    shift_next<P>(th, nx);
-#pragma unroll
-    for (int q = 0; q < P; ++q) c[q] = (lane * P + q < nb) ? bend_corr(th[q], nx[q], ra[q], kb[q]) : 0.0f;
-    shift_prev<P>(c, pv);
-    shift_next<P>(x, xn);
-    shift_next<P>(y, yn);
-    float fx[P], fy[P], he[P], fxp[P], fyp[P], hep[P];
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const int j = lane * P + q;
-      fx[q] = fy[q] = he[q] = 0.0f;
-      if (j < ne) {
-        float acc = 0.0f;
-        if (j < nb) acc = acc + c[q];
-        if (j >= 1 && j - 1 < nb) acc = acc + (-pv[q]);
-        const float2 r = min_image(xn[q], yn[q], x[q], y[q], W, H);
-        th[q] = cos_pull(th[q] + acc * edg[q], r.x, r.y);
-        float sn, cs;
-        sincosf(th[q], &sn, &cs);
-        const float kl = ks / l0[q];
-        fx[q] = kl * (r.x / l0[q] - cs);
-        fy[q] = kl * (r.y / l0[q] - sn);
-        he[q] = ks / (l0[q] * l0[q]);
-      }
-    }
-    shift_prev<P>(fx, fxp);
-    shift_prev<P>(fy, fyp);
-    shift_prev<P>(he, hep);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const int j = lane * P + q;
-      if (j < nn) {
-        float ax = w * (x0[q] - x[q]), ay = w * (y0[q] - y[q]), hh = w;
-        if (j < ne) {
-          ax = ax + fx[q];
-          ay = ay + fy[q];
-          hh = hh + he[q];
-        }
-        if (j >= 1) {
-          ax = ax + (-fxp[q]);
-          ay = ay + (-fyp[q]);
-          hh = hh + hep[q];
-        }
-        x[q] = x[q] + ax / hh;
-        y[q] = y[q] + ay / hh;
-      }
-    }
-  }
-}
-
-template <int P>
-__global__ void __launch_bounds__(128) k_chain(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
-                                               const int* __restrict__ tdev) {
+// ---------------------------------------------------------------- chains: CTA per rod
+// One CTA (one team) per chain rod; S: the longest chain of the plan.  At least four warps, so
+// that the sines and cosines of a short rod's iterations do not fall to a single warp.
+__global__ void __launch_bounds__(384) k_chain(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
+                                               const int* __restrict__ tdev, int S) {
+  extern __shared__ float2 chain_tab[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ci = (blockIdx.x - off[r]) * kChainWarps + warp;
-  if (ci >= d.nchain) return;  // the whole warp leaves together
-  const int comp = d.chain_comp[ci];
-  const int n0 = d.comp_n[comp], nn = d.comp_n[comp + 1] - n0;
-  const int e0 = d.comp_e[comp], ne = nn - 1;
-  const int b0 = d.comp_b[comp], nb = nn > 2 ? nn - 2 : 0;
-  const int t = *tdev;
-  float x[P], y[P], th[P], l0[P], ra[P], kb[P], edg[P], ndg[P];
-#pragma unroll
-  for (int q = 0; q < P; ++q) {
-    const int j = lane * P + q;
-    x[q] = y[q] = th[q] = l0[q] = ra[q] = kb[q] = 0.0f;
-    if (j < nn) {
-      x[q] = d.pos[2 * (n0 + j)];
-      y[q] = d.pos[2 * (n0 + j) + 1];
-    }
-    if (j < ne) {
-      th[q] = d.theta[e0 + j];
-      l0[q] = d.rest_len[e0 + j];
-    }
-    if (j < nb) {
-      ra[q] = rest_angle(d, b0 + j, t);
-      kb[q] = d.kb[b0 + j];
-    }
-    // chain degrees are 1 or 2, so x / deg == x * (1 / deg) exactly
-    edg[q] = ((j < nb) + (j >= 1 && j - 1 < nb)) == 2 ? 0.5f : 1.0f;
-    ndg[q] = ((j < ne) + (j >= 1 && j - 1 < ne)) == 2 ? 0.5f : 1.0f;
-  }
-  const int cycles = d.cycles;
-  if (d.solver == 1) {
-    cosserat_chain<P>(d, lane, nn, ne, nb, x, y, th, l0, ra, kb, edg);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const int j = lane * P + q;
-      if (j < ne) d.theta[e0 + j] = th[q];
-      if (j < nn) {
-        d.pos[2 * (n0 + j)] = x[q];
-        d.pos[2 * (n0 + j) + 1] = y[q];
-      }
-    }
-    return;
-  }
-  // descriptor values the iterations use, held in registers for the whole loop
-  const float Wf = (float)d.W, Hf = (float)d.H, ksh = d.k_shear, kst = d.k_stretch;
-  for (int it = 0; it < cycles; ++it) {
-    // The part of each edge force that depends only on the positions (min-image segment,
-    // length, stretch term: edge_force's first half) is taken before the bending pass, whose
-    // chain of shuffles and angle updates it then overlaps; the angle-dependent half follows
-    // it.  Same expressions as edge_force, so the same bits.
-    float xn[P], yn[P], sgx[P], sgy[P], stx[P], sty[P];
-    shift_next<P>(x, xn);
-    shift_next<P>(y, yn);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const float2 cur = min_image(xn[q], yn[q], x[q], y[q], Wf, Hf);
-      const float L = sqrtf(cur.x * cur.x + cur.y * cur.y);
-      const float Lc = max_prop(L, 1e-8f);
-      sgx[q] = cur.x;
-      sgy[q] = cur.y;
-      stx[q] = (cur.x / Lc) * (L - l0[q]);
-      sty[q] = (cur.y / Lc) * (L - l0[q]);
-    }
-    float nx[P], pv[P], c[P];
-    shift_next<P>(th, nx);
-#pragma unroll
-    for (int q = 0; q < P; ++q) c[q] = (lane * P + q < nb) ? bend_corr(th[q], nx[q], ra[q], kb[q]) : 0.0f;
-    shift_prev<P>(c, pv);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const int j = lane * P + q;
-      if (j < ne) {
-        float acc = 0.0f;
-        if (j < nb) acc = acc + c[q];
-        if (j >= 1 && j - 1 < nb) acc = acc + (-pv[q]);
-        th[q] = th[q] + (acc * edg[q]) * 1.8f;
-      }
-    }
-    float fx[P], fy[P], fxp[P], fyp[P];
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      fx[q] = fy[q] = 0.0f;
-      if (lane * P + q < ne) {
-        float sn, cs;
-        sincosf(th[q], &sn, &cs);
-        const float tx = cs * l0[q], ty = sn * l0[q];
-        const float shx = (sgx[q] - tx) - stx[q], shy = (sgy[q] - ty) - sty[q];
-        fx[q] = ((stx[q] + shx * ksh) * kst) * 0.5f;
-        fy[q] = ((sty[q] + shy * ksh) * kst) * 0.5f;
-      }
-    }
-    shift_prev<P>(fx, fxp);
-    shift_prev<P>(fy, fyp);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      const int j = lane * P + q;
-      if (j < nn) {
-        float ax = 0.0f, ay = 0.0f;
-        if (j < ne) {
-          ax = ax + fx[q];
-          ay = ay + fy[q];
-        }
-        if (j >= 1) {
-          ax = ax + (-fxp[q]);
-          ay = ay + (-fyp[q]);
-        }
-        x[q] = x[q] + ax * ndg[q];
-        y[q] = y[q] + ay * ndg[q];
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < P; ++q) {
-    const int j = lane * P + q;
-    if (j < ne) d.theta[e0 + j] = th[q];
-    if (j < nn) {
-      d.pos[2 * (n0 + j)] = x[q];
-      d.pos[2 * (n0 + j) + 1] = y[q];
-    }
-  }
+  const Team tm = {(int)threadIdx.x >> 5, (int)blockDim.x >> 5, 1};
+  chain_rod(d, d.chain_info[blockIdx.x - off[r]], *tdev, tm, d.pos, chain_tab, S);
 }
 
 // ---------------------------------------------------------------- general rods: CTA per rod
@@ -751,13 +532,9 @@ void launch_stencil16(const Launch& L) { k_stencil16<<<L.grid, 128, 0, L.s>>>(L.
 void launch_node(const Launch& L, const int* tdev, size_t smem, int bs) {
   k_node<<<L.grid, bs, smem, L.s>>>(L.d, L.off, L.n, tdev);
 }
-void launch_chain(const Launch& L, const int* tdev, int slots) {
-  switch (slots) {
-    case 1: k_chain<1><<<L.grid, 32 * kChainWarps, 0, L.s>>>(L.d, L.off, L.n, tdev); break;
-    case 2: k_chain<2><<<L.grid, 32 * kChainWarps, 0, L.s>>>(L.d, L.off, L.n, tdev); break;
-    case 4: k_chain<4><<<L.grid, 32 * kChainWarps, 0, L.s>>>(L.d, L.off, L.n, tdev); break;
-    default: k_chain<8><<<L.grid, 32 * kChainWarps, 0, L.s>>>(L.d, L.off, L.n, tdev); break;
-  }
+void launch_chain(const Launch& L, const int* tdev, int longest) {
+  const int warps = chain_warps(longest) < 4 ? 4 : chain_warps(longest);
+  k_chain<<<L.grid, 32 * warps, (size_t)chain_smem(longest) * sizeof(float2), L.s>>>(L.d, L.off, L.n, tdev, longest);
 }
 cudaError_t node_set_smem(size_t bytes) {
   return cudaFuncSetAttribute(k_node, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

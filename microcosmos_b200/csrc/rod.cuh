@@ -1,0 +1,384 @@
+// Chain rods (edge i = (node i, node i+1), pair i = (edge i, edge i+1)): the iterations of
+// pbd_rod_constraint (src/microcosmos/solver/pbd.py:14-91) and stable_cosserat_constraint
+// (src/microcosmos/solver/stable_cosserat.py:13-119) for one rod by a team of warps.
+//
+// One node (and edge and pair) per lane.  What bounds it is the length of one rod's chain of
+// dependent operations, not the amount of work, so the chain is cut where the equations allow:
+//  * the PBD angle pass reads no position, so all iterations' angles are advanced first (about
+//    175 cycles each) and kept in shared memory; the sines and cosines of every (iteration,
+//    edge) are then independent and spread over all threads of the team; the position pass
+//    reads the finished rest vectors.  One lane's chain per iteration no longer holds the angle
+//    update and the sincos;
+//  * rods of more than 32 nodes use several warps instead of several nodes per lane: each warp
+//    owns kSegOwn nodes and carries kSegGhost more on each side, advanced redundantly, so that
+//    warps exchange boundary values (one barrier) only every kSegGhost iterations (an angle or
+//    position depends on its direct neighbours only).
+// Measured (one B200, 20 iterations, per launch inside a rollout's graph): four 32-node rods 12.8 ->
+// 9.8 us, 256 64-node rods 22.6 -> 13.3 us, 1,032 rods of 16 to 128 nodes 56 -> 32.6 us; before: one
+// warp per rod with 1, 2 or 4 nodes per lane, all phases in one loop.
+#pragma once
+#include "lbm_cell.cuh"
+
+namespace mc {
+
+constexpr int kSegOwn = 22;
+constexpr int kSegGhost = 5;
+constexpr int kThetaChunk = 20;  // iterations whose angles are kept at a time
+
+__host__ __device__ constexpr int chain_warps(int nn) { return nn <= 32 ? 1 : (nn + kSegOwn - 1) / kSegOwn; }
+// shared memory of a team for rods of at most `S` nodes, in float2
+__host__ __device__ constexpr int chain_smem(int S) { return (kThetaChunk + 2) * S; }
+
+// The threads working on one rod.  All of them call chain_rod together; warps beyond the rod's
+// own (chain_warps) help with the sines and cosines.
+struct Team {
+  int warp, warps;  // this warp's index in the team, and the team's warps
+  int bar;          // the team's named barrier; bar + 1 is the barrier of its first warps alone
+  __device__ __forceinline__ void sync() const {
+    if (warps == 1)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(warps * 32) : "memory");
+  }
+  // sync, and whether `p` holds for any thread of the team
+  __device__ __forceinline__ bool sync_or(bool p) const {
+    if (warps == 1) return __any_sync(0xffffffffu, p) != 0;
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
+        "selp.s32 %0, 1, 0, b;\n\t}"
+        : "=r"(r)
+        : "r"((int)p), "r"(bar), "r"(warps * 32)
+        : "memory");
+    return r != 0;
+  }
+};
+
+// fmod_floor for |x| < 2 y; `bad` records an x outside (or NaN), whose result is not valid.
+__device__ __forceinline__ float fmod_near(float x, float y, bool& bad) {
+  bad = bad || !(fabsf(x) < 2.0f * y);
+  const float a = x + y, b = a + y, c = x - y;
+  const float rp = (x >= y) ? c : x;
+  const float rn = (a < 0.0f) ? b : a;
+  return (x >= 0.0f) ? rp : rn;
+}
+
+// Length L and direction v / L of a segment, each correctly rounded, without branches, by Newton
+// and residual corrections of the hardware's approximations (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): for
+// the square root, g ~ sqrt(s) and h ~ 1 / (2 sqrt(s)) are refined together and the exact
+// residual s - g g corrects g; for a quotient, with r = RN(1 / L), two corrections by the exact
+// residual v - L q.  The root equals sqrtf for every significand (all floats of [1, 4) times even
+// powers of two in 2^+-38 compared) and r equals 1 / L for all 2^23 significands.  A zero
+// component keeps its sign.  `bad` records operands outside the range where all residuals are
+// exact; there the reference's floor of the length (1e-8) could act too.
+__device__ __forceinline__ float2 unit_near(float2 v, float& L, bool& bad) {
+  const float s = v.x * v.x + v.y * v.y;
+  const float ax = fabsf(v.x), ay = fabsf(v.y);
+  const bool zx = v.x == 0.0f, zy = v.y == 0.0f;
+  bad = bad || !(s >= 0x1p-50f && s <= 0x1p70f && (zx || ax >= 0x1p-40f) && (zy || ay >= 0x1p-40f));
+  float y, r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+  float g = s * y, h = 0.5f * y;
+  const float c = __fmaf_rn(-g, h, 0.5f);
+  g = __fmaf_rn(g, c, g);
+  h = __fmaf_rn(h, c, h);
+  L = __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(L));
+  r = __fmaf_rn(__fmaf_rn(-L, r, 1.0f), r, r);
+  float qx = v.x * r, qy = v.y * r;
+  qx = __fmaf_rn(__fmaf_rn(-L, qx, v.x), r, qx);
+  qy = __fmaf_rn(__fmaf_rn(-L, qy, v.y), r, qy);
+  qx = __fmaf_rn(__fmaf_rn(-L, qx, v.x), r, qx);
+  qy = __fmaf_rn(__fmaf_rn(-L, qy, v.y), r, qy);
+  return make_float2(zx ? v.x : qx, zy ? v.y : qy);
+}
+
+// Rest angle of pair gb at step t (the caller-side curvature actuation, if any); `store` keeps
+// it in the state.
+__device__ __forceinline__ float rest_angle(const RDesc& d, int gb, int t, bool store = true) {
+  if (!d.act_amp) return d.rest_ang[gb];
+  const float arg = d.act_omega[gb] * (float)(d.act_t0 + t) + d.act_phase[gb];
+  const float a = d.act_c[gb] + d.act_amp[gb] * sinf(arg);
+  if (store) d.rest_ang[gb] = a;
+  return a;
+}
+
+// One theta correction (pbd.py:35-40).
+__device__ __forceinline__ float bend_corr(float th_in, float th_out, float rest, float kb) {
+  float diff = th_out - th_in;
+  diff = fmod_floor(diff + MC_PI_F, MC_2PI_F) - MC_PI_F;
+  return ((diff - rest) * kb) * 0.5f;
+}
+
+// Stable-Cosserat iterations of one rod.  Phase 1: the bending pass without over-relaxation,
+// then theta += wrap(atan2(r) - theta) * 0.05 with r the segment's min-image vector.
+// Phase 2: x += (w (y0 - x) + f_j - f_{j-1}) / ((w + H_j) + H_{j-1}), f = (k_s/l)(r/l - d),
+// H = k_s/l^2, y0 the inertial prediction (the positions the rod started from).  The angles
+// depend on the positions here, so the two phases alternate; values travel two nodes to the
+// right per iteration, so the warps exchange after each one.
+__device__ __forceinline__ void cosserat_iterations(const RDesc& d, const Team& rod, bool several, bool own, int j,
+                                                     int nn, int ne, int nb, float& x, float& y, float& th,
+                                                    float l0, float ra, float kb, float edg, float2* ex, float* ext,
+                                                    int S) {
+  const float W = (float)d.W, H = (float)d.H;
+  const float ks = d.k_stretch, w = d.cos_w;
+  const float x0 = x, y0 = y;
+  int buf = 0;
+  for (int it = 0; it < d.cycles; ++it) {
+    if (several && it > 0) {
+      if (own) {
+        ex[buf * S + j] = make_float2(x, y);
+        ext[buf * S + j] = th;
+      }
+      rod.sync();
+      if (!own && j >= 0 && j < nn) {
+        const float2 p = ex[buf * S + j];
+        x = p.x;
+        y = p.y;
+        th = ext[buf * S + j];
+      }
+      buf ^= 1;
+    }
+    const float nx = __shfl_down_sync(0xffffffffu, th, 1);
+    const float c = (j >= 0 && j < nb) ? bend_corr(th, nx, ra, kb) : 0.0f;
+    const float pv = __shfl_up_sync(0xffffffffu, c, 1);
+    const float xn = __shfl_down_sync(0xffffffffu, x, 1), yn = __shfl_down_sync(0xffffffffu, y, 1);
+    float fx = 0.0f, fy = 0.0f, he = 0.0f;
+    if (j >= 0 && j < ne) {
+      float acc = 0.0f;
+      if (j < nb) acc = acc + c;
+      if (j >= 1 && j - 1 < nb) acc = acc + (-pv);
+      const float2 r = min_image(xn, yn, x, y, W, H);
+      th = cos_pull(th + acc * edg, r.x, r.y);
+      float sn, cs;
+      sincosf(th, &sn, &cs);
+      const float kl = ks / l0;
+      fx = kl * (r.x / l0 - cs);
+      fy = kl * (r.y / l0 - sn);
+      he = ks / (l0 * l0);
+    }
+    const float fxp = __shfl_up_sync(0xffffffffu, fx, 1), fyp = __shfl_up_sync(0xffffffffu, fy, 1);
+    const float hep = __shfl_up_sync(0xffffffffu, he, 1);
+    if (j >= 0 && j < nn) {
+      float ax = w * (x0 - x), ay = w * (y0 - y), hh = w;
+      if (j < ne) {
+        ax = ax + fx;
+        ay = ay + fy;
+        hh = hh + he;
+      }
+      if (j >= 1) {
+        ax = ax + (-fxp);
+        ay = ay + (-fyp);
+        hh = hh + hep;
+      }
+      x = x + ax / hh;
+      y = y + ay / hh;
+    }
+  }
+}
+
+// One lane's place on its rod.
+struct RodLane {
+  int j, nn, ne, nb;  // node, edge and pair j of a rod of nn nodes (lanes off the rod: j < 0 or j >= nn)
+  bool own;           // the node is this warp's own and not a neighbour's
+};
+
+// q angle passes (pbd.py:23-49); row k of tab keeps the angles after pass k.  NEAR: without the
+// slow path of the floored modulo, `bad` telling that some lane would have needed it.
+template <bool NEAR, bool SEVERAL>
+__device__ __forceinline__ bool theta_passes(const Team& rod, const RodLane& l, int q, float& th, float ra, float kb,
+                                             float edg, float2* tab, int S) {
+  const bool pair = l.j >= 0 && l.j < l.nb, prev = l.j >= 1 && l.j - 1 < l.nb, edge = l.j >= 0 && l.j < l.ne;
+  const bool keep = l.own && edge;
+  bool bad = false;
+  int left = kSegGhost;
+  for (int k = 0; k < q; ++k) {
+    if (SEVERAL && left == 0) {
+      rod.sync();
+      if (!l.own && edge) th = tab[(k - 1) * S + l.j].x;
+      left = kSegGhost;
+    }
+    --left;
+    const float nx = __shfl_down_sync(0xffffffffu, th, 1);
+    float c;
+    if (NEAR) {
+      bool out = false;
+      const float diff = fmod_near((nx - th) + MC_PI_F, MC_2PI_F, out) - MC_PI_F;
+      c = ((diff - ra) * kb) * 0.5f;
+      bad = bad || (out && pair && l.own);
+    } else {
+      c = bend_corr(th, nx, ra, kb);
+    }
+    // the terms that do not exist are zeros: (0 + c) + (-c') as the reference scatters them
+    c = pair ? c : 0.0f;
+    float pv = __shfl_up_sync(0xffffffffu, c, 1);
+    pv = prev ? pv : 0.0f;
+    th = th + (((0.0f + c) + (-pv)) * edg) * 1.8f;
+    if (keep) tab[k * S + l.j].x = th;
+  }
+  return bad;
+}
+
+// q position passes (pbd.py:51-89) with the rest vectors in tab; first: no pass came before them.
+template <bool NEAR, bool SEVERAL>
+__device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& l, int q, bool first, float& x,
+                                                float& y, float l0, float ndg, float Wf, float Hf, float ksh,
+                                                float kst, const float2* tab, float2* ex, int& buf, int S) {
+  // (lane 31 of a warp sees no next node: with several warps its edge is a neighbour's)
+  const bool node = l.j >= 0 && l.j < l.nn, prev = l.j >= 1;
+  const bool edge = l.j >= 0 && l.j < l.ne && (threadIdx.x & 31) < 31;
+  const float hx = Wf / 2.0f, hy = Hf / 2.0f;
+  bool bad = false;
+  int left = first ? kSegGhost : 0;
+  for (int k = 0; k < q; ++k) {
+    if (SEVERAL && left == 0) {
+      if (l.own) ex[buf * S + l.j] = make_float2(x, y);
+      rod.sync();
+      if (!l.own && node) {
+        const float2 p = ex[buf * S + l.j];
+        x = p.x;
+        y = p.y;
+      }
+      buf ^= 1;
+      left = kSegGhost;
+    }
+    --left;
+    const float2 tv = edge ? tab[k * S + l.j] : make_float2(0.0f, 0.0f);
+    const float xn = __shfl_down_sync(0xffffffffu, x, 1), yn = __shfl_down_sync(0xffffffffu, y, 1);
+    float2 cur, dir;
+    float L;
+    // lanes without an edge take a unit segment: a zero length would send the whole warp
+    // through the slow paths of the square root and the reciprocal
+    if (NEAR) {
+      bool out = false;
+      cur.x = fmod_near((xn - x) + hx, Wf, out) - hx;
+      cur.y = fmod_near((yn - y) + hy, Hf, out) - hy;
+      cur = edge ? cur : make_float2(1.0f, 1.0f);
+      dir = unit_near(cur, L, out);
+      bad = bad || (out && edge && l.own);
+    } else {
+      cur = min_image(xn, yn, x, y, Wf, Hf);
+      cur = edge ? cur : make_float2(1.0f, 1.0f);
+      L = sqrtf(cur.x * cur.x + cur.y * cur.y);
+      const float Lc = max_prop(L, 1e-8f);
+      dir = make_float2(cur.x / Lc, cur.y / Lc);
+    }
+    const float stx = dir.x * (L - l0), sty = dir.y * (L - l0);
+    const float shx = (cur.x - tv.x) - stx, shy = (cur.y - tv.y) - sty;
+    const float fx = edge ? ((stx + shx * ksh) * kst) * 0.5f : 0.0f;
+    const float fy = edge ? ((sty + shy * ksh) * kst) * 0.5f : 0.0f;
+    float fxp = __shfl_up_sync(0xffffffffu, fx, 1), fyp = __shfl_up_sync(0xffffffffu, fy, 1);
+    fxp = prev ? fxp : 0.0f;
+    fyp = prev ? fyp : 0.0f;
+    x = x + ((0.0f + fx) + (-fxp)) * ndg;
+    y = y + ((0.0f + fy) + (-fyp)) * ndg;
+  }
+  return bad;
+}
+
+// All iterations of a PBD rod of rw warps.  The passes run without the slow paths of the modulo
+// and the divisions first (their branches would lie on the dependent chain); if any lane needed
+// one, the chunk is done again from its start with them.
+template <bool SEVERAL>
+__device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, int rw, const RodLane& l, int e0,
+                                               float& x, float& y, float& th, float l0, float ra, float kb, float edg,
+                                               float ndg, float2* tab, int S) {
+  const int lane = threadIdx.x & 31;
+  const bool act = tm.warp < rw, edge = l.j >= 0 && l.j < l.ne;
+  const float Wf = (float)d.W, Hf = (float)d.H, ksh = d.k_shear, kst = d.k_stretch;
+  float2* ex = tab + kThetaChunk * S;
+  const Team rod = {tm.warp, rw, tm.bar + 1};
+  const int cycles = d.cycles;
+  int buf = 0;
+  for (int it0 = 0; it0 < cycles; it0 += kThetaChunk) {
+    const int q = min(kThetaChunk, cycles - it0);
+    const float th0 = th;
+    bool bad = false;
+    if (act) bad = theta_passes<true, SEVERAL>(rod, l, q, th, ra, kb, edg, tab, S);
+    if (tm.sync_or(bad)) {
+      th = th0;
+      if (act) theta_passes<false, SEVERAL>(rod, l, q, th, ra, kb, edg, tab, S);
+      tm.sync();
+    }
+    if (SEVERAL) {
+      if (act && !l.own && edge) th = tab[(q - 1) * S + l.j].x;
+      tm.sync();
+    }
+    // rest vectors l0 (cos, sin) of every (iteration, edge): one iteration per warp at a time
+    for (int e = lane; e < l.ne; e += 32) {
+      const float le = d.rest_len[e0 + e];
+#pragma unroll 2
+      for (int k = tm.warp; k < q; k += tm.warps) {
+        float sn, cs;
+        sincosf(tab[k * S + e].x, &sn, &cs);
+        tab[k * S + e] = make_float2(cs * le, sn * le);
+      }
+    }
+    tm.sync();
+    const float x0 = x, y0 = y;
+    const int buf0 = buf;
+    bad = false;
+    if (act)
+      bad = position_passes<true, SEVERAL>(rod, l, q, it0 == 0, x, y, l0, ndg, Wf, Hf, ksh, kst, tab, ex, buf, S);
+    if (tm.sync_or(bad)) {
+      x = x0;
+      y = y0;
+      buf = buf0;
+      if (act) position_passes<false, SEVERAL>(rod, l, q, it0 == 0, x, y, l0, ndg, Wf, Hf, ksh, kst, tab, ex, buf, S);
+      tm.sync();
+    }
+  }
+}
+
+// All cycles_per_step iterations at step t of the chain info = (first node, nodes, first edge, first
+// pair).  pos: the rollout's node positions (x, y), updated in place; tab: chain_smem(S) float2 of
+// shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.
+__device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, const Team& tm, float* pos, float2* tab,
+                                          int S) {
+  const int lane = threadIdx.x & 31;
+  const int n0 = info.x, nn = info.y, e0 = info.z, b0 = info.w;
+  RodLane l;
+  l.nn = nn;
+  l.ne = nn - 1;
+  l.nb = nn > 2 ? nn - 2 : 0;
+  const int rw = chain_warps(nn);
+  const bool several = rw > 1, act = tm.warp < rw;
+  l.j = several ? tm.warp * kSegOwn + lane - kSegGhost : lane;
+  l.own = act && l.j < nn && (!several || (lane >= kSegGhost && lane < kSegGhost + kSegOwn));
+  const int j = l.j, ne = l.ne, nb = l.nb;
+  float x = 0.0f, y = 0.0f, th = 0.0f, l0 = 0.0f, ra = 0.0f, kb = 0.0f;
+  if (act && j >= 0) {
+    if (j < nn) {
+      x = pos[2 * (n0 + j)];
+      y = pos[2 * (n0 + j) + 1];
+    }
+    if (j < ne) {
+      th = d.theta[e0 + j];
+      l0 = d.rest_len[e0 + j];
+    }
+    if (j < nb) {
+      ra = rest_angle(d, b0 + j, t, l.own);
+      kb = d.kb[b0 + j];
+    }
+  }
+  // chain degrees are 1 or 2, so x / deg == x * (1 / deg) exactly
+  const float edg = ((j < nb) + (j >= 1 && j - 1 < nb)) == 2 ? 0.5f : 1.0f;
+  const float ndg = ((j < ne) + (j >= 1 && j - 1 < ne)) == 2 ? 0.5f : 1.0f;
+  if (d.solver == 1) {
+    if (act)
+      cosserat_iterations(d, Team{tm.warp, rw, tm.bar + 1}, several, l.own, j, nn, ne, nb, x, y, th, l0, ra, kb, edg,
+                          tab + kThetaChunk * S, reinterpret_cast<float*>(tab), S);
+  }
+  else if (several)
+    pbd_iterations<true>(d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
+  else
+    pbd_iterations<false>(d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
+  if (l.own) {
+    if (j < ne) d.theta[e0 + j] = th;
+    pos[2 * (n0 + j)] = x;
+    pos[2 * (n0 + j) + 1] = y;
+  }
+}
+
+}  // namespace mc

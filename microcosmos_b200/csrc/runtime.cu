@@ -74,7 +74,8 @@ struct HostRollout {
   std::vector<int> comp_n, comp_e, comp_b, ep_off, ep_idx, ne_off, ne_idx;
   std::vector<float> edeg, ndeg;
   int ncomp = 0, max_cn = 0, max_ce = 0, max_cb = 0;
-  std::vector<int> chain_comp, generic_comp;  // components by kernel
+  std::vector<int> generic_comp;  // components by kernel
+  std::vector<int4> chain_info;   // chains: first node, nodes, first edge, first pair
   int max_chain = 0;                          // longest chain (nodes)
   std::vector<int> fW, fH;
   std::vector<float2> twW, twH;
@@ -123,7 +124,7 @@ struct mc_plan {
   int any_fluid = 0, any_steric = 0, max_iters = 0;
   size_t node_smem = 0, fftr_smem = 0, fftc_smem = 0, fftr2_smem = 0, fftc2_smem = 0, sconv_smem = 0;
   int node_bs = 32;
-  int max_chain = 0, chain_slots = 1;
+  int max_chain = 0;
   int max_k = 0;  // largest IB kernel size of the plan
   int fft_e = 4;  // values per thread of the register-radix FFT kernels
   bool fuse_finalize = false;  // body force computed by the last IB spread round
@@ -390,8 +391,8 @@ mc_status build_topology(HostRollout& h) {
     h.ncomp = 1;
   }
   // chains (edge i = (n0+i, n0+i+1), pair i = (e0+i, e0+i+1), <= 256 nodes) run on the
-  // warp kernel; every other component on the CTA kernel
-  h.chain_comp.clear();
+  // chain kernel; every other component on the general one
+  h.chain_info.clear();
   h.generic_comp.clear();
   h.max_chain = 0;
   for (int c = 0; c < h.ncomp; ++c) {
@@ -404,7 +405,7 @@ mc_status build_topology(HostRollout& h) {
     for (int i = 0; chain && i < nb; ++i)
       chain = h.bpairs[2 * (b0 + i)] == e0 + i && h.bpairs[2 * (b0 + i) + 1] == e0 + i + 1;
     if (chain) {
-      h.chain_comp.push_back(c);
+      h.chain_info.push_back(make_int4(n0, nn, e0, b0));
       h.max_chain = std::max(h.max_chain, nn);
     } else {
       h.generic_comp.push_back(c);
@@ -624,9 +625,9 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.wl_ib = at<int2>(b, p->r_wl_ib);
   d.wl_cic = at<int2>(b, p->r_wl_cic);
   d.wl_ctl = at<int>(b, p->r_wl_ctl);
-  d.nchain = (int)h.chain_comp.size();
+  d.nchain = (int)h.chain_info.size();
   d.ngeneric = (int)h.generic_comp.size();
-  d.chain_comp = at<int>(b, h.r_chain);
+  d.chain_info = at<int4>(b, h.r_chain);
   d.generic_comp = at<int>(b, h.r_generic);
   d.flags = at<unsigned>(b, h.r_flags);
   p->desc[i] = d;
@@ -841,7 +842,7 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
     ++k;
   }
   if (p->grid[K_CHAIN]) {
-    timed(p, 4, s, capture, [&] { mc::launch_chain(L(p, K_CHAIN, s), tdev, p->chain_slots); });
+    timed(p, 4, s, capture, [&] { mc::launch_chain(L(p, K_CHAIN, s), tdev, p->max_chain); });
     ++k;
   }
   if (p->grid[K_COMP]) {
@@ -1430,7 +1431,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     h.r_ctc = lay.take(nt * 4);
     h.r_covf = lay.take(4 * N * 4);
     h.r_cctl = lay.take(8 * 4);
-    h.r_chain = lay.take(h.chain_comp.size() * 4);
+    h.r_chain = lay.take(h.chain_info.size() * sizeof(int4));
     h.r_generic = lay.take(h.generic_comp.size() * 4);
     h.r_pairs = lay.take(2 * E * 4);
     h.r_bpairs = lay.take(2 * B * 4);
@@ -1520,7 +1521,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     // the plan's CTAs would not all be resident)
     cnt[K_IBCOOP] = c.enable_fluid ? std::max(1, div_up(h.M, 1024)) : 0;
     cnt[K_COMP] = h.dims.N > 0 ? (int)h.generic_comp.size() : 0;
-    cnt[K_CHAIN] = h.dims.N > 0 ? div_up((long long)h.chain_comp.size(), mc::kChainWarps) : 0;
+    cnt[K_CHAIN] = h.dims.N > 0 ? (int)h.chain_info.size() : 0;
     cnt[K_IB] = div_up(h.M, mc::kHeadThreads);  // touched cells: at most M, one thread each
     cnt[K_TILES] = h.ntx * h.nty;
     cnt[K_LBM] = c.enable_fluid ? h.lbm_tx * h.lbm_ty : 0;
@@ -1553,8 +1554,6 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   recount_steric(p);
   p->coop_cap_checked = false;
   p->node_smem = (size_t)(2 * mcn + 4 * mce + 3 * mcb) * sizeof(float);
-  p->chain_slots = 1;
-  while (p->chain_slots * 32 < p->max_chain) p->chain_slots *= 2;
   if (p->node_smem > 200 * 1024) {
     delete p;
     return fail(MC_ERR_UNSUPPORTED, "rod component too large for shared memory (> ~6000 nodes)");
@@ -1717,7 +1716,7 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
     MC_CUDA(up(h.r_nei, h.ne_idx.data(), h.ne_idx.size() * 4));
     MC_CUDA(up(h.r_edeg, h.edeg.data(), h.edeg.size() * 4));
     MC_CUDA(up(h.r_ndeg, h.ndeg.data(), h.ndeg.size() * 4));
-    MC_CUDA(up(h.r_chain, h.chain_comp.data(), h.chain_comp.size() * 4));
+    MC_CUDA(up(h.r_chain, h.chain_info.data(), h.chain_info.size() * sizeof(int4)));
     MC_CUDA(up(h.r_generic, h.generic_comp.data(), h.generic_comp.size() * 4));
     MC_CUDA(up(h.r_twW, h.twW.data(), h.twW.size() * 8));
     MC_CUDA(up(h.r_twH, h.twH.data(), h.twH.size() * 8));
