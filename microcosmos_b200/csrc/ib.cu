@@ -768,11 +768,11 @@ __device__ int resize_taps(int o, int m, int n, float inv, float ks, int& i0, fl
 // is on the domain grid: a copy when the lattice is the domain grid, else the linear
 // resize of simulate.py:24-29.
 __global__ void k_record_fields(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
-                                const int* __restrict__ tdev) {
+                                const int* __restrict__ tdev, int advanced) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
   if (d.rec_every <= 0) return;
-  const int t = *tdev;
+  const int t = *tdev - advanced;  // advanced: the step counter already stands at the next step
   if ((t + 1) % d.rec_every != 0) return;
   const size_t e = (size_t)((t + 1) / d.rec_every - 1);
   const size_t HW = (size_t)d.H * d.W, LHW = (size_t)d.lH * d.lW;
@@ -871,8 +871,8 @@ void launch_ib_finalize(const Launch& L, int parity) {
 void launch_reaction(const Launch& L, const int* tdev) {
   k_reaction<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n, tdev);
 }
-void launch_record_fields(const Launch& L, const int* tdev) {
-  k_record_fields<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n, tdev);
+void launch_record_fields(const Launch& L, const int* tdev, int advanced) {
+  k_record_fields<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n, tdev, advanced);
 }
 void launch_tick(int* tdev, cudaStream_t s) { k_tick<<<1, 1, 0, s>>>(tdev); }
 

@@ -272,7 +272,7 @@ void launch_fft12_rows(const Launch& L);
 void launch_fft12_cols(const Launch& L);
 void launch_fftreg_cols(const Launch& L, int values_per_thread, int values_per_cta);
 void launch_reaction(const Launch& L, const int* tdev);
-void launch_record_fields(const Launch& L, const int* tdev);
+void launch_record_fields(const Launch& L, const int* tdev, int advanced);
 void launch_unstream(const Launch& L);
 void launch_stream_out(const Launch& L, int parity, float* dst = nullptr);
 void launch_clear_ws(const Launch& L);

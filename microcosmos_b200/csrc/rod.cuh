@@ -13,16 +13,16 @@
 //    owns kSegOwn nodes and carries kSegGhost more on each side, advanced redundantly, so that
 //    warps exchange boundary values (one barrier) only every kSegGhost iterations (an angle or
 //    position depends on its direct neighbours only).
-// Measured (one B200, 20 iterations, per launch inside a rollout's graph): four 32-node rods 12.8 ->
-// 9.8 us, 256 64-node rods 22.6 -> 13.3 us, 1,032 rods of 16 to 128 nodes 56 -> 32.6 us; before: one
-// warp per rod with 1, 2 or 4 nodes per lane, all phases in one loop.
+// Measured (one B200, 20 iterations, per launch inside a rollout's graph): 256 64-node rods 22.6 ->
+// 11.4 us, 1,032 rods of 16 to 128 nodes 56 -> 29.4 us; before: one warp per rod with 2 or 4 nodes
+// per lane, all phases in one loop.
 #pragma once
 #include "lbm_cell.cuh"
 
 namespace mc {
 
 constexpr int kSegOwn = 22;
-constexpr int kSegGhost = 5;
+constexpr int kSegGhost = 5;  // (the Cosserat passes: two nodes per iteration on the left, two iterations)
 constexpr int kThetaChunk = 20;  // iterations whose angles are kept at a time
 
 __host__ __device__ constexpr int chain_warps(int nn) { return nn <= 32 ? 1 : (nn + kSegOwn - 1) / kSegOwn; }
@@ -33,7 +33,7 @@ __host__ __device__ constexpr int chain_smem(int S) { return (kThetaChunk + 2) *
 // own (chain_warps) help with the sines and cosines.
 struct Team {
   int warp, warps;  // this warp's index in the team, and the team's warps
-  int bar;          // the team's named barrier; bar + 1 is the barrier of its first warps alone
+  int bar;          // the team's named barrier; bar + 1 is that of its first warps, when the rod has fewer
   __device__ __forceinline__ void sync() const {
     if (warps == 1)
       __syncwarp();
@@ -54,29 +54,38 @@ struct Team {
   }
 };
 
-// fmod_floor for |x| < 2 y; `bad` records an x outside (or NaN), whose result is not valid.
-__device__ __forceinline__ float fmod_near(float x, float y, bool& bad) {
-  bad = bad || !(fabsf(x) < 2.0f * y);
-  const float a = x + y, b = a + y, c = x - y;
-  const float rp = (x >= y) ? c : x;
-  const float rn = (a < 0.0f) ? b : a;
-  return (x >= 0.0f) ? rp : rn;
+// max that propagates NaN, for the range checks of the fast passes
+__device__ __forceinline__ float max_track(float m, float v) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(v)));
+  return r;
+}
+__device__ __forceinline__ float min_track(float m, float v) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(v));
+  return r;
 }
 
-// Length L and direction v / L of a segment, each correctly rounded, without branches, by Newton
-// and residual corrections of the hardware's approximations (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): for
-// the square root, g ~ sqrt(s) and h ~ 1 / (2 sqrt(s)) are refined together and the exact
-// residual s - g g corrects g; for a quotient, with r = RN(1 / L), two corrections by the exact
-// residual v - L q.  The root equals sqrtf for every significand (all floats of [1, 4) times even
-// powers of two in 2^+-38 compared) and r equals 1 / L for all 2^23 significands.  A zero
-// component keeps its sign.  `bad` records operands outside the range where all residuals are
-// exact; there the reference's floor of the length (1e-8) could act too.
-__device__ __forceinline__ float2 unit_near(float2 v, float& L, bool& bad) {
-  const float s = v.x * v.x + v.y * v.y;
-  const float ax = fabsf(v.x), ay = fabsf(v.y);
-  const bool zx = v.x == 0.0f, zy = v.y == 0.0f;
-  bad = bad || !(s >= 0x1p-50f && s <= 0x1p70f && (zx || ax >= 0x1p-40f) && (zy || ay >= 0x1p-40f));
+// fmod_floor of x = d + y / 2 where |d| < 1.49 y: x lies in (-y, 2 y), so one period at most is
+// added or taken away (exactly).
+constexpr float kNear = 1.49f;
+__device__ __forceinline__ float fmod_near(float x, float y) {
+  const float r = (x >= y) ? x - y : x;
+  return (x < 0.0f) ? x + y : r;
+}
+
+// Length L and direction v / L of a segment with squared length s, each correctly rounded, without
+// branches, by Newton and residual corrections of the hardware's approximations (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34, 1990): for the square root, g ~ sqrt(s) and h ~ 1 / (2 sqrt(s)) are refined together and
+// the exact residual s - g g corrects g; for a quotient, with r = RN(1 / L), two corrections by
+// the exact residual v - L q.  The root equals sqrtf for every significand (all floats of [1, 4)
+// times even powers of two in 2^+-38 compared) and r equals 1 / L for all 2^23 significands.
+// Valid for s >= 2^-50 (a segment's components are min-image differences, so multiples of 2^-23,
+// and below 2^35); there the reference's floor of the length (1e-8) does not act either.  A zero
+// component may lose its sign, which no later sum can show.
+constexpr float kNearLength2 = 0x1p-50f;
+__device__ __forceinline__ float2 unit_near(float2 v, float s, float& L) {
   float y, r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
   float g = s * y, h = 0.5f * y;
@@ -91,7 +100,7 @@ __device__ __forceinline__ float2 unit_near(float2 v, float& L, bool& bad) {
   qy = __fmaf_rn(__fmaf_rn(-L, qy, v.y), r, qy);
   qx = __fmaf_rn(__fmaf_rn(-L, qx, v.x), r, qx);
   qy = __fmaf_rn(__fmaf_rn(-L, qy, v.y), r, qy);
-  return make_float2(zx ? v.x : qx, zy ? v.y : qy);
+  return make_float2(qx, qy);
 }
 
 // Rest angle of pair gb at step t (the caller-side curvature actuation, if any); `store` keeps
@@ -111,73 +120,6 @@ __device__ __forceinline__ float bend_corr(float th_in, float th_out, float rest
   return ((diff - rest) * kb) * 0.5f;
 }
 
-// Stable-Cosserat iterations of one rod.  Phase 1: the bending pass without over-relaxation,
-// then theta += wrap(atan2(r) - theta) * 0.05 with r the segment's min-image vector.
-// Phase 2: x += (w (y0 - x) + f_j - f_{j-1}) / ((w + H_j) + H_{j-1}), f = (k_s/l)(r/l - d),
-// H = k_s/l^2, y0 the inertial prediction (the positions the rod started from).  The angles
-// depend on the positions here, so the two phases alternate; values travel two nodes to the
-// right per iteration, so the warps exchange after each one.
-__device__ __forceinline__ void cosserat_iterations(const RDesc& d, const Team& rod, bool several, bool own, int j,
-                                                     int nn, int ne, int nb, float& x, float& y, float& th,
-                                                    float l0, float ra, float kb, float edg, float2* ex, float* ext,
-                                                    int S) {
-  const float W = (float)d.W, H = (float)d.H;
-  const float ks = d.k_stretch, w = d.cos_w;
-  const float x0 = x, y0 = y;
-  int buf = 0;
-  for (int it = 0; it < d.cycles; ++it) {
-    if (several && it > 0) {
-      if (own) {
-        ex[buf * S + j] = make_float2(x, y);
-        ext[buf * S + j] = th;
-      }
-      rod.sync();
-      if (!own && j >= 0 && j < nn) {
-        const float2 p = ex[buf * S + j];
-        x = p.x;
-        y = p.y;
-        th = ext[buf * S + j];
-      }
-      buf ^= 1;
-    }
-    const float nx = __shfl_down_sync(0xffffffffu, th, 1);
-    const float c = (j >= 0 && j < nb) ? bend_corr(th, nx, ra, kb) : 0.0f;
-    const float pv = __shfl_up_sync(0xffffffffu, c, 1);
-    const float xn = __shfl_down_sync(0xffffffffu, x, 1), yn = __shfl_down_sync(0xffffffffu, y, 1);
-    float fx = 0.0f, fy = 0.0f, he = 0.0f;
-    if (j >= 0 && j < ne) {
-      float acc = 0.0f;
-      if (j < nb) acc = acc + c;
-      if (j >= 1 && j - 1 < nb) acc = acc + (-pv);
-      const float2 r = min_image(xn, yn, x, y, W, H);
-      th = cos_pull(th + acc * edg, r.x, r.y);
-      float sn, cs;
-      sincosf(th, &sn, &cs);
-      const float kl = ks / l0;
-      fx = kl * (r.x / l0 - cs);
-      fy = kl * (r.y / l0 - sn);
-      he = ks / (l0 * l0);
-    }
-    const float fxp = __shfl_up_sync(0xffffffffu, fx, 1), fyp = __shfl_up_sync(0xffffffffu, fy, 1);
-    const float hep = __shfl_up_sync(0xffffffffu, he, 1);
-    if (j >= 0 && j < nn) {
-      float ax = w * (x0 - x), ay = w * (y0 - y), hh = w;
-      if (j < ne) {
-        ax = ax + fx;
-        ay = ay + fy;
-        hh = hh + he;
-      }
-      if (j >= 1) {
-        ax = ax + (-fxp);
-        ay = ay + (-fyp);
-        hh = hh + hep;
-      }
-      x = x + ax / hh;
-      y = y + ay / hh;
-    }
-  }
-}
-
 // One lane's place on its rod.
 struct RodLane {
   int j, nn, ne, nb;  // node, edge and pair j of a rod of nn nodes (lanes off the rod: j < 0 or j >= nn)
@@ -185,42 +127,45 @@ struct RodLane {
 };
 
 // q angle passes (pbd.py:23-49); row k of tab keeps the angles after pass k.  NEAR: without the
-// slow path of the floored modulo, `bad` telling that some lane would have needed it.
+// slow path of the floored modulo; returns whether this lane would have needed it.
 template <bool NEAR, bool SEVERAL>
 __device__ __forceinline__ bool theta_passes(const Team& rod, const RodLane& l, int q, float& th, float ra, float kb,
                                              float edg, float2* tab, int S) {
   const bool pair = l.j >= 0 && l.j < l.nb, prev = l.j >= 1 && l.j - 1 < l.nb, edge = l.j >= 0 && l.j < l.ne;
   const bool keep = l.own && edge;
-  bool bad = false;
+  float far = 0.0f;
   int left = kSegGhost;
-  for (int k = 0; k < q; ++k) {
-    if (SEVERAL && left == 0) {
-      rod.sync();
-      if (!l.own && edge) th = tab[(k - 1) * S + l.j].x;
-      left = kSegGhost;
+  float2* row = tab + max(l.j, 0);
+  for (int k = 0; k < q; ++k, row += S) {
+    if (SEVERAL) {
+      if (left == 0) {
+        rod.sync();
+        if (!l.own && edge) th = (row - S)->x;
+        left = kSegGhost;
+      }
+      --left;
     }
-    --left;
     const float nx = __shfl_down_sync(0xffffffffu, th, 1);
     float c;
     if (NEAR) {
-      bool out = false;
-      const float diff = fmod_near((nx - th) + MC_PI_F, MC_2PI_F, out) - MC_PI_F;
-      c = ((diff - ra) * kb) * 0.5f;
-      bad = bad || (out && pair && l.own);
+      const float d = nx - th;
+      far = max_track(far, d);
+      c = (((fmod_near(d + MC_PI_F, MC_2PI_F) - MC_PI_F) - ra) * kb) * 0.5f;
     } else {
       c = bend_corr(th, nx, ra, kb);
     }
-    // the terms that do not exist are zeros: (0 + c) + (-c') as the reference scatters them
+    // the terms that do not exist are zeros
     c = pair ? c : 0.0f;
     float pv = __shfl_up_sync(0xffffffffu, c, 1);
     pv = prev ? pv : 0.0f;
-    th = th + (((0.0f + c) + (-pv)) * edg) * 1.8f;
-    if (keep) tab[k * S + l.j].x = th;
+    th = th + ((c - pv) * edg) * 1.8f;
+    if (keep) row->x = th;
   }
-  return bad;
+  return NEAR && pair && l.own && !(far < kNear * MC_2PI_F);
 }
 
 // q position passes (pbd.py:51-89) with the rest vectors in tab; first: no pass came before them.
+// NEAR: without the slow paths of the modulo, the square root and the divisions.
 template <bool NEAR, bool SEVERAL>
 __device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& l, int q, bool first, float& x,
                                                 float& y, float l0, float ndg, float Wf, float Hf, float ksh,
@@ -229,37 +174,39 @@ __device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& 
   const bool node = l.j >= 0 && l.j < l.nn, prev = l.j >= 1;
   const bool edge = l.j >= 0 && l.j < l.ne && (threadIdx.x & 31) < 31;
   const float hx = Wf / 2.0f, hy = Hf / 2.0f;
-  bool bad = false;
+  float far_x = 0.0f, far_y = 0.0f, s_min = 1.0f;
   int left = first ? kSegGhost : 0;
-  for (int k = 0; k < q; ++k) {
-    if (SEVERAL && left == 0) {
-      if (l.own) ex[buf * S + l.j] = make_float2(x, y);
-      rod.sync();
-      if (!l.own && node) {
-        const float2 p = ex[buf * S + l.j];
-        x = p.x;
-        y = p.y;
+  const float2* row = tab + min(max(l.j, 0), max(l.ne - 1, 0));
+  for (int k = 0; k < q; ++k, row += S) {
+    if (SEVERAL) {
+      if (left == 0) {
+        if (l.own) ex[buf * S + l.j] = make_float2(x, y);
+        rod.sync();
+        if (!l.own && node) {
+          const float2 p = ex[buf * S + l.j];
+          x = p.x;
+          y = p.y;
+        }
+        buf ^= 1;
+        left = kSegGhost;
       }
-      buf ^= 1;
-      left = kSegGhost;
+      --left;
     }
-    --left;
-    const float2 tv = edge ? tab[k * S + l.j] : make_float2(0.0f, 0.0f);
+    const float2 tv = *row;
     const float xn = __shfl_down_sync(0xffffffffu, x, 1), yn = __shfl_down_sync(0xffffffffu, y, 1);
     float2 cur, dir;
     float L;
-    // lanes without an edge take a unit segment: a zero length would send the whole warp
-    // through the slow paths of the square root and the reciprocal
     if (NEAR) {
-      bool out = false;
-      cur.x = fmod_near((xn - x) + hx, Wf, out) - hx;
-      cur.y = fmod_near((yn - y) + hy, Hf, out) - hy;
-      cur = edge ? cur : make_float2(1.0f, 1.0f);
-      dir = unit_near(cur, L, out);
-      bad = bad || (out && edge && l.own);
+      const float dx = xn - x, dy = yn - y;
+      cur.x = fmod_near(dx + hx, Wf) - hx;
+      cur.y = fmod_near(dy + hy, Hf) - hy;
+      const float s = cur.x * cur.x + cur.y * cur.y;
+      dir = unit_near(cur, s, L);
+      far_x = max_track(far_x, dx);
+      far_y = max_track(far_y, dy);
+      s_min = min_track(s_min, s);
     } else {
       cur = min_image(xn, yn, x, y, Wf, Hf);
-      cur = edge ? cur : make_float2(1.0f, 1.0f);
       L = sqrtf(cur.x * cur.x + cur.y * cur.y);
       const float Lc = max_prop(L, 1e-8f);
       dir = make_float2(cur.x / Lc, cur.y / Lc);
@@ -271,10 +218,10 @@ __device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& 
     float fxp = __shfl_up_sync(0xffffffffu, fx, 1), fyp = __shfl_up_sync(0xffffffffu, fy, 1);
     fxp = prev ? fxp : 0.0f;
     fyp = prev ? fyp : 0.0f;
-    x = x + ((0.0f + fx) + (-fxp)) * ndg;
-    y = y + ((0.0f + fy) + (-fyp)) * ndg;
+    x = x + (fx - fxp) * ndg;
+    y = y + (fy - fyp) * ndg;
   }
-  return bad;
+  return NEAR && edge && l.own && !(far_x < kNear * Wf && far_y < kNear * Hf && s_min >= kNearLength2);
 }
 
 // All iterations of a PBD rod of rw warps.  The passes run without the slow paths of the modulo
@@ -288,7 +235,7 @@ __device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, i
   const bool act = tm.warp < rw, edge = l.j >= 0 && l.j < l.ne;
   const float Wf = (float)d.W, Hf = (float)d.H, ksh = d.k_shear, kst = d.k_stretch;
   float2* ex = tab + kThetaChunk * S;
-  const Team rod = {tm.warp, rw, tm.bar + 1};
+  const Team rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
   const int cycles = d.cycles;
   int buf = 0;
   for (int it0 = 0; it0 < cycles; it0 += kThetaChunk) {
@@ -331,6 +278,131 @@ __device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, i
   }
 }
 
+// a / b, correctly rounded, from r = RN(1 / b) and two corrections by the exact residual (see
+// unit_near); a zero or between 2^-80 and 2^80, b between 2^-30 and 2^30.
+__device__ __forceinline__ float div_near(float a, float b, float r) {
+  float q = a * r;
+  q = __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+}
+__device__ __forceinline__ float reciprocal(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return __fmaf_rn(__fmaf_rn(-b, r, 1.0f), r, r);
+}
+
+// Stable-Cosserat iterations of one rod (solver/stable_cosserat.py:13-119).  Phase 1: the bending
+// pass without over-relaxation, then theta += wrap(atan2(r) - theta) * 0.05 with r the segment's
+// min-image vector.  Phase 2: x += (w (y0 - x) + f_j - f_{j-1}) / ((w + H_j) + H_{j-1}), f =
+// (k_s/l)(r/l - d), H = k_s/l^2, y0 the inertial prediction (the positions the rod started from).
+// The angles depend on the positions here, so the two phases alternate; values travel two nodes
+// to the right per iteration, so the warps exchange after every second one.  The divisors do not
+// change, so NEAR divides by their reciprocals (div_near); it returns whether this lane left the
+// range where that and the one-period modulo are exact.
+template <bool NEAR, bool SEVERAL>
+__device__ __forceinline__ bool cosserat_iterations(const RDesc& d, const Team& rod, const RodLane& l, float& x,
+                                                    float& y, float& th, float l0, float ra, float kb, float edg,
+                                                    float2* ex, float* ext, int S) {
+  const int j = l.j;
+  const bool node = j >= 0 && j < l.nn, pair = j >= 0 && j < l.nb, pair_prev = j >= 1 && j - 1 < l.nb, prev = j >= 1;
+  const bool edge = j >= 0 && j < l.ne && (threadIdx.x & 31) < 31;
+  const float W = (float)d.W, H = (float)d.H, hx = W / 2.0f, hy = H / 2.0f;
+  const float w = d.cos_w, x0 = x, y0 = y;
+  const float le = edge ? l0 : 1.0f;
+  const float kl = edge ? d.k_stretch / le : 0.0f, he = edge ? d.k_stretch / (le * le) : 0.0f;
+  const float hep = __shfl_up_sync(0xffffffffu, he, 1);
+  float hh = w;
+  if (j < l.ne) hh = hh + he;
+  if (prev) hh = hh + hep;
+  const float rl = NEAR ? reciprocal(le) : 0.0f, rh = NEAR ? reciprocal(hh) : 0.0f;
+  float far_t = 0.0f, far_x = 0.0f, far_y = 0.0f, big = 0.0f, small = 1.0f;
+  int buf = 0, left = 2;
+  for (int it = 0; it < d.cycles; ++it) {
+    if (SEVERAL) {
+      if (left == 0) {
+        if (l.own) {
+          ex[buf * S + j] = make_float2(x, y);
+          ext[buf * S + j] = th;
+        }
+        rod.sync();
+        if (!l.own && node) {
+          const float2 p = ex[buf * S + j];
+          x = p.x;
+          y = p.y;
+          th = ext[buf * S + j];
+        }
+        buf ^= 1;
+        left = 2;
+      }
+      --left;
+    }
+    const float nx = __shfl_down_sync(0xffffffffu, th, 1);
+    const float xn = __shfl_down_sync(0xffffffffu, x, 1), yn = __shfl_down_sync(0xffffffffu, y, 1);
+    float c;
+    float2 r;
+    if (NEAR) {
+      const float dt = nx - th, dx = xn - x, dy = yn - y;
+      far_t = pair ? max_track(far_t, dt) : far_t;
+      far_x = max_track(far_x, dx);
+      far_y = max_track(far_y, dy);
+      c = (((fmod_near(dt + MC_PI_F, MC_2PI_F) - MC_PI_F) - ra) * kb) * 0.5f;
+      r = make_float2(fmod_near(dx + hx, W) - hx, fmod_near(dy + hy, H) - hy);
+    } else {
+      c = bend_corr(th, nx, ra, kb);
+      r = min_image(xn, yn, x, y, W, H);
+    }
+    // lanes without an edge take a unit segment, off the slow paths of atan2
+    if (!edge) r = make_float2(1.0f, 1.0f);
+    c = pair ? c : 0.0f;
+    float pv = __shfl_up_sync(0xffffffffu, c, 1);
+    pv = pair_prev ? pv : 0.0f;
+    th = th + (c - pv) * edg;
+    if (NEAR) {
+      const float a = atan2f(r.y, r.x) - th;
+      far_t = max_track(far_t, edge ? a : 0.0f);
+      th = th + (fmod_near(a + MC_PI_F, MC_2PI_F) - MC_PI_F) * 0.05f;
+    } else {
+      th = cos_pull(th, r.x, r.y);
+    }
+    float sn, cs;
+    sincosf(th, &sn, &cs);
+    const float qx = NEAR ? div_near(r.x, le, rl) : r.x / le, qy = NEAR ? div_near(r.y, le, rl) : r.y / le;
+    const float fx = edge ? kl * (qx - cs) : 0.0f, fy = edge ? kl * (qy - sn) : 0.0f;
+    float fxp = __shfl_up_sync(0xffffffffu, fx, 1), fyp = __shfl_up_sync(0xffffffffu, fy, 1);
+    fxp = prev ? fxp : 0.0f;
+    fyp = prev ? fyp : 0.0f;
+    const float ax = (w * (x0 - x) + fx) - fxp, ay = (w * (y0 - y) + fy) - fyp;
+    if (NEAR) {
+      big = max_track(max_track(big, ax), ay);
+      small = min_track(min_track(small, ax == 0.0f ? 1.0f : fabsf(ax)), ay == 0.0f ? 1.0f : fabsf(ay));
+      x = x + div_near(ax, hh, rh);
+      y = y + div_near(ay, hh, rh);
+    } else {
+      x = x + ax / hh;
+      y = y + ay / hh;
+    }
+  }
+  if (!NEAR || !l.own) return false;
+  const bool moves = !(big < 0x1p80f && small > 0x1p-80f && hh > 0x1p-30f && hh < 0x1p30f);
+  const bool turns = edge && !(far_t < kNear * MC_2PI_F && far_x < kNear * W && far_y < kNear * H && le > 0x1p-30f &&
+                               le < 0x1p30f);
+  return moves || turns;
+}
+
+template <bool SEVERAL>
+__device__ __forceinline__ void cosserat_rod(const RDesc& d, const Team& rod, const RodLane& l, float& x, float& y,
+                                             float& th, float l0, float ra, float kb, float edg, float2* tab, int S) {
+  float2* ex = tab + kThetaChunk * S;
+  float* ext = reinterpret_cast<float*>(tab);
+  const float xs = x, ys = y, ts = th;
+  if (rod.sync_or(cosserat_iterations<true, SEVERAL>(d, rod, l, x, y, th, l0, ra, kb, edg, ex, ext, S))) {
+    x = xs;
+    y = ys;
+    th = ts;
+    cosserat_iterations<false, SEVERAL>(d, rod, l, x, y, th, l0, ra, kb, edg, ex, ext, S);
+  }
+}
+
 // All cycles_per_step iterations at step t of the chain info = (first node, nodes, first edge, first
 // pair).  pos: the rollout's node positions (x, y), updated in place; tab: chain_smem(S) float2 of
 // shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.
@@ -366,9 +438,11 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
   const float edg = ((j < nb) + (j >= 1 && j - 1 < nb)) == 2 ? 0.5f : 1.0f;
   const float ndg = ((j < ne) + (j >= 1 && j - 1 < ne)) == 2 ? 0.5f : 1.0f;
   if (d.solver == 1) {
-    if (act)
-      cosserat_iterations(d, Team{tm.warp, rw, tm.bar + 1}, several, l.own, j, nn, ne, nb, x, y, th, l0, ra, kb, edg,
-                          tab + kThetaChunk * S, reinterpret_cast<float*>(tab), S);
+    const Team rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
+    if (act && several)
+      cosserat_rod<true>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
+    else if (act)
+      cosserat_rod<false>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
   }
   else if (several)
     pbd_iterations<true>(d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);

@@ -15,6 +15,8 @@
 
 #include "../../include/microcosmos_b200.h"
 #include "mc_internal.cuh"
+#include "node_step.cuh"
+#include "rod.cuh"
 
 using mc::RDesc;
 
@@ -42,6 +44,7 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 
 constexpr int kDefaultSortCap = 2048;  // contributions per tile sorted in shared memory by default
+constexpr int kNodeStepSmem = 220 * 1024;  // dynamic shared memory of a node-step CTA at most
 // largest plan (IB points over all rollouts) whose body force is computed by the last IB round
 constexpr long long kFuseFinalizeMaxPoints = 65536;
 
@@ -136,9 +139,14 @@ struct mc_plan {
   cudaError_t coop_err = cudaSuccess;
   std::vector<RDesc> desc;
   cudaStream_t cap_stream = nullptr;
-  // CUDA graphs, keyed by [steps-1][parity][recording variant][write_u][runs next pipeline]
-  cudaGraphExec_t graph[2][2][3][2][2] = {};
-  int64_t graph_kernels[2][2][3][2][2] = {};
+  // CUDA graphs by step variant (graph_key)
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t kernels = 0;
+  };
+  std::map<int, StepGraph> graphs;
+  bool compact_ok = false;   // small enough for the node-step kernel (compact_shape)
+  mc::NodeStepShape ns = {};
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t lbm_stream = nullptr;                  // the dense pass, beside the IB chain
@@ -681,7 +689,8 @@ mc::Launch L(mc_plan* p, Kind k, cudaStream_t s) {
 const char* const kProfNames[] = {"predict", "cic_bins",  "fft_rows",    "fft_cols", "chain",
                                    "node",    "ib_bins",   "ib_interp",   "ib_spread", "ib_finalize",
                                    "lbm",     "reaction",  "record_fields", "tick",    "steric",
-                                   "stencil", "ib_fused", "steric_conv", "collide_heads", "ib_cluster"};
+                                   "stencil", "ib_fused", "steric_conv", "collide_heads", "ib_cluster",
+                                   "node_step"};
 constexpr int kNumProf = sizeof(kProfNames) / sizeof(kProfNames[0]);
 
 cudaEvent_t take_event(mc_plan* p) {
@@ -785,7 +794,64 @@ void recount_steric(mc_plan* p) {
   for (int k : {K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12}) p->grid[k] = p->off[k][p->n];
 }
 
+// The steric filter of the deposit: row and column passes.
+int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool capture) {
+  int64_t k = 0;
+  if (p->grid[K_FR16]) {
+    timed(p, 2, s, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, s), p->fft_e); });
+    ++k;
+  }
+  if (p->grid[K_FR12]) {
+    timed(p, 2, s, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, s)); });
+    ++k;
+  }
+  if (p->grid[K_FFTR2]) {
+    timed(p, 2, s, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, s), p->fftr2_smem); });
+    ++k;
+  }
+  if (p->grid[K_FFTR]) {
+    timed(p, 2, s, capture, [&] { mc::launch_fft_rows(L(p, K_FFTR, s), p->fftr_smem); });
+    ++k;
+  }
+  if (p->grid[K_FC16]) {
+    timed(p, 3, s, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, s), p->fft_e, p->fft_tv); });
+    ++k;
+  }
+  if (p->grid[K_FC12]) {
+    timed(p, 3, s, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, s)); });
+    ++k;
+  }
+  if (p->grid[K_FFTC2]) {
+    timed(p, 3, s, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, s), p->fftc2_smem); });
+    ++k;
+  }
+  if (p->grid[K_FFTC]) {
+    timed(p, 3, s, capture, [&] { mc::launch_fft_cols(L(p, K_FFTC, s), p->fftc_smem); });
+    ++k;
+  }
+  if (p->grid[K_SCONV]) {
+    timed(p, 17, s, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, s), p->sconv_smem); });
+    ++k;
+  }
+  return k;
+}
+
+// Whether the plan's steps run the node-step kernel: it is small enough and no other layout of
+// the IB kernels has been asked for.
+bool is_compact(const mc_plan* p) { return p->compact_ok && !p->use_coop && p->ib_cluster == 0; }
+
+int64_t enqueue_node_step(mc_plan* p, int parity, int main, int next, cudaStream_t s, bool capture) {
+  timed(p, 20, s, capture, [&] {
+    mc::launch_node_step(at<RDesc>(p->ws, p->r_desc), p->n, at<int>(p->ws, p->r_tdev), p->ns, parity, main, next, s);
+  });
+  return 1;
+}
+
 int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
+  if (is_compact(p)) {
+    if (!p->any_steric) return 0;
+    return enqueue_node_step(p, 0, 0, 1, s, capture) + enqueue_filter(p, s, capture);
+  }
   int* tdev = at<int>(p->ws, p->r_tdev);
   int64_t k = 0;
   if (p->grid[K_NODES]) {
@@ -800,42 +866,7 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
                            p->bin_threads);
     });
     k += 1;
-    if (p->grid[K_FR16]) {
-      timed(p, 2, s, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, s), p->fft_e); });
-      ++k;
-    }
-    if (p->grid[K_FR12]) {
-      timed(p, 2, s, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, s)); });
-      ++k;
-    }
-    if (p->grid[K_FFTR2]) {
-      timed(p, 2, s, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, s), p->fftr2_smem); });
-      ++k;
-    }
-    if (p->grid[K_FFTR]) {
-      timed(p, 2, s, capture, [&] { mc::launch_fft_rows(L(p, K_FFTR, s), p->fftr_smem); });
-      ++k;
-    }
-    if (p->grid[K_FC16]) {
-      timed(p, 3, s, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, s), p->fft_e, p->fft_tv); });
-      ++k;
-    }
-    if (p->grid[K_FC12]) {
-      timed(p, 3, s, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, s)); });
-      ++k;
-    }
-    if (p->grid[K_FFTC2]) {
-      timed(p, 3, s, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, s), p->fftc2_smem); });
-      ++k;
-    }
-    if (p->grid[K_FFTC]) {
-      timed(p, 3, s, capture, [&] { mc::launch_fft_cols(L(p, K_FFTC, s), p->fftc_smem); });
-      ++k;
-    }
-    if (p->grid[K_SCONV]) {
-      timed(p, 17, s, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, s), p->sconv_smem); });
-      ++k;
-    }
+    k += enqueue_filter(p, s, capture);
   }
   if (p->grid[K_NODES]) {
     timed(p, 14, s, capture, [&] { mc::launch_steric(L(p, K_NODES, s)); });
@@ -919,29 +950,43 @@ int64_t enqueue_tail(mc_plan* p, int rec_fields, cudaStream_t s, bool capture) {
     ++k;
   }
   if (rec_fields) {
-    timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), tdev); });
+    timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), tdev, 0); });
     ++k;
   }
   timed(p, 13, s, capture, [&] { mc::launch_tick(tdev, s); });
   return k + 1;
 }
 
-// Everything of step t after its pipeline, plus pipeline(t+1) when has_next.
+// Everything of step t after its pipeline, plus pipeline(t+1) when has_next; with `first` the
+// step's own pipeline too.
 //   lbm stream: the dense pass lbm(t) (reads h[parity], writes h[parity^1]) from the start
-//               of the body, concurrently with the IB chain, which reads h[parity] only;
+//               of the body, concurrently with the pipeline and the IB chain, which reads
+//               h[parity] only;
 //   main:       ib(t) (bins, iterations, body force per touched cell), then, once lbm(t)
 //               is done, the touched cells' collision over its result;
 //   side:       after ib(t): tail(t) (node reaction) and pipeline(t+1).
-// The next body starts when all three have finished.
-int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool has_next, cudaStream_t s,
+// The next body starts when all three have finished.  In a compact plan one node-step launch
+// is pipeline(t) after the filter, ib(t), tail(t) and pipeline(t+1) up to the filter.
+int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool first, bool has_next, cudaStream_t s,
                      bool capture, mc_status* err) {
+  const bool compact = is_compact(p);
+  int64_t k = 0;
   if (rec_fields || p->profiling) {
     // sequential: field recording needs this order; profiling times kernels one at a time
-    int64_t k = enqueue_ib(p, parity, s, capture);
+    if (first) k += enqueue_pipeline(p, s, capture);
+    k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
     k += enqueue_lbm(p, parity, write_u, s, capture);
     k += enqueue_heads(p, parity, write_u, s, capture);
-    k += enqueue_tail(p, rec_fields, s, capture);
-    if (has_next) k += enqueue_pipeline(p, s, capture);
+    if (!compact) {
+      k += enqueue_tail(p, rec_fields, s, capture);
+      if (has_next) k += enqueue_pipeline(p, s, capture);
+      return k;
+    }
+    if (rec_fields) {
+      timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), at<int>(p->ws, p->r_tdev), 1); });
+      ++k;
+    }
+    if (has_next && p->any_steric) k += enqueue_filter(p, s, capture);
     return k;
   }
   auto fork = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to, const char* what) {
@@ -949,21 +994,26 @@ int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool h
     if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
     if (e != cudaSuccess && *err == MC_OK) *err = cuda_fail(e, what);
   };
-  int64_t k = 0;
   cudaStream_t s2 = p->side_stream, s3 = p->lbm_stream;
   if (p->any_fluid) {
     fork(p->ev_lfork, s, s3, "fork to the dense-pass stream");
     k += enqueue_lbm(p, parity, write_u, s3, capture);
   }
-  k += enqueue_ib(p, parity, s, capture);
-  fork(p->ev_fork, s, s2, "fork to the side stream");
-  k += enqueue_tail(p, 0, s2, capture);
-  if (has_next) k += enqueue_pipeline(p, s2, capture);
+  if (first) k += enqueue_pipeline(p, s, capture);
+  const bool side = !compact || (has_next && p->any_steric);
+  k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
+  if (side) fork(p->ev_fork, s, s2, "fork to the side stream");
+  if (compact) {
+    if (side) k += enqueue_filter(p, s2, capture);
+  } else {
+    k += enqueue_tail(p, 0, s2, capture);
+    if (has_next) k += enqueue_pipeline(p, s2, capture);
+  }
   if (p->any_fluid) {
     fork(p->ev_ljoin, s3, s, "join from the dense-pass stream");
     k += enqueue_heads(p, parity, write_u, s, capture);
   }
-  fork(p->ev_join, s2, s, "join from the side stream");
+  if (side) fork(p->ev_join, s2, s, "join from the side stream");
   return k;
 }
 
@@ -1001,49 +1051,49 @@ cudaError_t prioritise_graph(cudaGraph_t graph) {
 
 mc_status run_steps(mc_plan* p, int num, int use_graph, int last, cudaStream_t s, int64_t& launches) {
   const int recv = p->rec_fields ? (p->rec_fluid ? 2 : 1) : 0;
-  // the first step of this call needs its node pipeline unless the previous call left it
-  // pending (an advance with last != 0 finishes its step without starting the next one)
-  if (!p->pending_next && num > 0) launches += enqueue_pipeline(p, s, false);
   int remaining = num;
   while (remaining > 0) {
     const int parity = p->step & 1;
     const bool is_last = last && remaining == 1;
     const int write_u = (is_last || p->rec_fluid) ? 1 : 0;
     const bool has_next = !is_last;
+    // a step needs its own node pipeline unless the previous one left it pending (an advance with
+    // last != 0 finishes its step without starting the next one)
+    const bool first = !p->pending_next;
     mc_status err = MC_OK;
     if (use_graph && !p->profiling) {
       // two steps per graph where possible (parity 0 then 1, neither the final step)
       const int ns = (parity == 0 && remaining >= 3) ? 2 : 1;
       const int wu = ns == 2 ? p->rec_fluid : write_u;
-      const int nx = has_next ? 1 : 0;
-      cudaGraphExec_t& g = p->graph[ns - 1][parity][recv][wu][nx];
-      if (!g) {
+      const int key = ((((ns - 1) * 2 + parity) * 3 + recv) * 2 + wu) * 4 + (first ? 2 : 0) + (has_next ? 1 : 0);
+      mc_plan::StepGraph& g = p->graphs[key];
+      if (!g.exec) {
         cudaGraph_t graph;
         MC_CUDA(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
         int64_t kk = 0;
         for (int j = 0; j < ns && err == MC_OK; ++j)
-          kk += enqueue_body(p, (parity + j) & 1, wu, p->rec_fields, j + 1 < ns ? true : has_next, p->cap_stream,
-                             true, &err);
+          kk += enqueue_body(p, (parity + j) & 1, wu, p->rec_fields, first && j == 0, j + 1 < ns ? true : has_next,
+                             p->cap_stream, true, &err);
         cudaError_t e = cudaStreamEndCapture(p->cap_stream, &graph);
         if (err != MC_OK) return err;
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
         e = prioritise_graph(graph);
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) {
-          g = nullptr;
+          g.exec = nullptr;
           return cuda_fail(e, "cudaGraphInstantiate");
         }
-        p->graph_kernels[ns - 1][parity][recv][wu][nx] = kk;
+        g.kernels = kk;
       }
-      MC_CUDA(cudaGraphLaunch(g, s));
-      launches += p->graph_kernels[ns - 1][parity][recv][wu][nx];
+      MC_CUDA(cudaGraphLaunch(g.exec, s));
+      launches += g.kernels;
       p->step += ns;
       remaining -= ns;
       p->pending_next = has_next;
       continue;
     }
-    launches += enqueue_body(p, parity, write_u, p->rec_fields, has_next, s, false, &err);
+    launches += enqueue_body(p, parity, write_u, p->rec_fields, first, has_next, s, false, &err);
     if (err != MC_OK) return err;
     p->step += 1;
     remaining -= 1;
@@ -1053,15 +1103,71 @@ mc_status run_steps(mc_plan* p, int num, int use_graph, int last, cudaStream_t s
 }
 
 void destroy_graphs(mc_plan* p) {
-  for (auto& a : p->graph)
-    for (auto& b : a)
-      for (auto& c : b)
-        for (auto& e : c)
-          for (auto& g : e)
-            if (g) {
-              cudaGraphExecDestroy(g);
-              g = nullptr;
-            }
+  for (auto& g : p->graphs)
+    if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+  p->graphs.clear();
+}
+
+// Whether every rollout of the plan fits the node-step kernel (only chain rods, a kernel of at most
+// 4 points, everything it keeps in kNodeStepSmem bytes of shared memory), and its shape.  The line
+// lies at the shared memory of an SM (about 410 IB points with the 4-point kernel, 1,700 with the
+// 2-point one): up to there one CTA is faster than the separate launches (384 points: 60 against
+// about 90 us per step).
+bool compact_shape(const std::vector<HostRollout>& R, mc::NodeStepShape* out) {
+  int N = 0, NI = 0, C = 0, longest = 1, rods = 0, shortest = mc::chain_warps(256);
+  for (const HostRollout& h : R) {
+    if (h.dims.N < 1 || h.dims.N > 16384 || !h.generic_comp.empty() || h.cfg.ibm_kernel_size > 4) return false;
+    const int ni = h.dims.N * (h.cfg.synthetic_node_width > 0.0f ? 2 : 1);
+    if ((long long)ni * 16 > 65535) return false;
+    N = std::max(N, h.dims.N);
+    NI = std::max(NI, ni);
+    C = std::max(C, std::max(h.M, h.cfg.enable_steric ? 4 * h.dims.N : 0));
+    longest = std::max(longest, h.max_chain);
+    rods = std::max(rods, (int)h.chain_info.size());
+    for (const int4& c : h.chain_info) shortest = std::min(shortest, mc::chain_warps(c.y));
+  }
+  mc::NodeStepShape s = {};
+  // up to two contributions per thread, a full CTA on a large rollout
+  s.threads = C <= 256 ? 128 : C <= 512 ? 256 : C <= 1024 ? 512 : mc::kNodeStepMaxThreads;
+  s.hash = (3 * std::max(C, 4) / 2 + 3) / 4 * 4;  // half as many again: a probe always finds a free entry
+  int at = 0;
+  auto take = [&](long long bytes) {
+    const int o = at;
+    at = (int)(((long long)at + bytes + 15) / 16 * 16);
+    return o;
+  };
+  s.pos = take(8LL * N);
+  s.vel = take(8LL * N);
+  s.nvl = take(8LL * NI);
+  s.delta = take(8LL * NI);
+  s.w = take(4LL * C);
+  s.slot = take(2LL * C);
+  s.rw = take(4LL * C);
+  s.rn = take(2LL * C);
+  s.hcell = take(std::max(8LL * C, 4LL * s.hash));  // with hrun behind it: the hash's counts
+  s.hrun = s.hcell + 4 * C;
+  s.shared = at;
+  s.longest = longest;
+  const int tab = mc::chain_smem(longest) * (int)sizeof(float2);
+  const int group = std::max(8 * C, 8 * s.hash);  // the hash, later the touched cells' velocities
+  // Rods at a time: a team per rod if the warps allow it, of the warps that its nodes need and up
+  // to four for the sines and cosines of its iterations.  15 named barriers are left: a team
+  // needs one, and a second where some rod has fewer warps than the team.
+  const int need = mc::chain_warps(longest);
+  if (s.threads < 32 * need) s.threads = 32 * need;
+  const int warps = s.threads / 32;
+  s.rod_warps = std::max(need, std::min(4, warps / std::max(rods, 1)));
+  s.bars = s.rod_warps == shortest ? 1 : 2;
+  if (s.rod_warps > need && 15 / s.bars < std::min(rods, warps / s.rod_warps)) {
+    s.rod_warps = need;
+    s.bars = need == shortest ? 1 : 2;
+  }
+  s.teams = std::min(warps / s.rod_warps, s.rod_warps > 1 ? 15 / s.bars : 32);
+  s.teams = std::max(1, std::min(s.teams, std::max(group, kNodeStepSmem - at) / tab));
+  at += std::max(group, s.teams * tab);
+  s.bytes = (at + 15) / 16 * 16;
+  *out = s;
+  return s.bytes <= kNodeStepSmem;
 }
 
 }  // namespace
@@ -1264,7 +1370,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   p->R.resize(n);
   Layout lay;
   p->r_desc = lay.take(sizeof(RDesc) * n);
-  p->r_tdev = lay.take(sizeof(int));
+  p->r_tdev = lay.take(sizeof(int) * n);  // step counters (the node-step kernel keeps one per rollout)
   p->r_wl_ctl = lay.take(4 * sizeof(int));
   for (int k = 0; k < K_COUNT; ++k) p->r_off[k] = lay.take(sizeof(int) * (n + 1));
   int vec_all = -1;
@@ -1560,6 +1666,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   }
   int work = std::max(mcn, std::max(mce, mcb));
   p->node_bs = std::min(256, std::max(32, (work + 31) / 32 * 32));
+  p->compact_ok = compact_shape(p->R, &p->ns);
   p->desc.resize(n);
   *out = p;
   return MC_OK;
@@ -1746,6 +1853,7 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
       return fail(MC_ERR_UNSUPPORTED, "shared memory needed by the plan exceeds the device limit");
     MC_CUDA(mc::node_set_smem((size_t)optin));
     MC_CUDA(mc::tiles_set_smem((size_t)optin));
+    MC_CUDA(mc::node_step_set_smem((size_t)optin));
     if (p->lbm_stages > 0) {
       if (mc::lbm_staged_smem(p->lbm_stages) > (size_t)optin)
         return fail(MC_ERR_UNSUPPORTED, "the staged dense pass's shared memory exceeds the device limit");
@@ -1828,7 +1936,7 @@ mc_status mc_rollout_begin(mc_plan* p, const mc_state* states, const mc_actuatio
     const mc::Upload u{p->ws + p->r_desc.off, p->desc.data(), p->desc.size() * sizeof(RDesc)};
     MC_CUDA(mc::stage_uploads(&u, 1, s));
   }
-  MC_CUDA(cudaMemsetAsync(at<int>(p->ws, p->r_tdev), 0, sizeof(int), s));
+  MC_CUDA(cudaMemsetAsync(at<int>(p->ws, p->r_tdev), 0, sizeof(int) * p->n, s));
   p->rec_fields = rec_fields;
   p->rec_fluid = rec_fluid;
   p->step = 0;
