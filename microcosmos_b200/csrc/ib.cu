@@ -1,14 +1,14 @@
-// Immersed-boundary coupling (src/microcosmos/solver/fluid.py:202-386) and the
-// deterministic scatter-add machinery it shares with the steric cloud-in-cell deposit
-// (src/microcosmos/forces.py:98-115).
+// Immersed-boundary coupling (src/microcosmos/solver/fluid.py:202-386) and the deterministic
+// scatter-adds: of the stencils' contributions to their cells, and of the steric cloud-in-cell
+// deposit (src/microcosmos/forces.py:98-115).
 //
-// Scatter-adds are never done with float atomics.  Each contribution k (IB: k = n*K*K + s,
-// CIC: k = corner*N + n — the order in which the reference's scatters apply them) is
-// appended to the bin of its 16x16-cell tile with its cell's position in the tile packed
-// above it (an integer atomic picks the slot; a full bin spills to an overflow list).  One CTA per tile then counting-sorts the bin by cell,
-// orders each cell's run by k and sums it sequentially — the reference's in-order
-// scatter-add, bit-reproducibly.  The IB iterations work on the compact list of touched
-// cells ("heads") instead of full (H, W) grids.
+// Scatter-adds are never done with float atomics: integer atomics collect the contributions of a
+// cell in arrival order, then they are ordered by contribution index and summed one after another,
+// the reference's in-order scatter-add, bit-reproducibly.  IB contributions (k = point*K*K + entry)
+// are collected per cell (k_stencil4, k_stencil) and one thread per touched cell ("head") orders
+// them (k_ib_heads); the rounds work on the compact list of heads instead of full (H, W) grids.
+// CIC contributions (k = corner*N + node) are collected per 16x16-cell tile and one CTA per tile
+// counting-sorts them by cell (k_bin_tiles).
 #include "lbm_cell.cuh"
 
 namespace mc {
@@ -22,22 +22,16 @@ struct BinView {
   int* ctl;
   int cap;
   int count;
-  int gw;      // width of the grid the cells index (lattice for IB, domain grid for CIC)
+  int gw;      // width of the grid the cells index
   int ntx;     // bin tiles per row of that grid
   int ntiles;  // bin tiles of that grid
 };
 
-__device__ __forceinline__ BinView bin_view(const RDesc& d, int which) {
+__device__ __forceinline__ BinView bin_view(const RDesc& d) {
   BinView v;
-  if (which == 0) {
-    v.cell = d.ib_cell; v.w = d.ib_w; v.store = d.ib_store; v.tcount = d.ib_tcount; v.ovf = d.ib_ovf;
-    v.ctl = d.ib_ctl; v.cap = d.ib_cap; v.count = d.M;
-    v.gw = d.lW; v.ntx = d.lntile_x; v.ntiles = d.lntile_x * d.lntile_y;
-  } else {
-    v.cell = d.c_cell; v.w = d.c_w; v.store = d.c_store; v.tcount = d.c_tcount; v.ovf = d.c_ovf;
-    v.ctl = d.c_ctl; v.cap = d.c_cap; v.count = d.enable_steric ? 4 * d.N : 0;
-    v.gw = d.W; v.ntx = d.ntile_x; v.ntiles = d.ntile_x * d.ntile_y;
-  }
+  v.cell = d.c_cell; v.w = d.c_w; v.store = d.c_store; v.tcount = d.c_tcount; v.ovf = d.c_ovf;
+  v.ctl = d.c_ctl; v.cap = d.c_cap; v.count = d.enable_steric ? 4 * d.N : 0;
+  v.gw = d.W; v.ntx = d.ntile_x; v.ntiles = d.ntile_x * d.ntile_y;
   return v;
 }
 
@@ -78,50 +72,13 @@ __device__ __forceinline__ int lower_bound_u(const unsigned* a, int len, unsigne
   return lo;
 }
 
-// Per-cell reduction work.  IB: coverage -> 1/max(cov, 1), the macroscopic state pulled
-// from h[parity] (density, clamped velocity), u_corrected = velocity (fluid.py:268-290);
-// the caller has already linked the run's contributions to `slot`.
-__device__ __forceinline__ void ib_head(const RDesc& d, int parity, int cell, float cov, int slot, int len,
-                                        int run_pos) {
-  d.h_cell[slot] = cell;
-  d.h_start[slot] = run_pos;
-  d.h_len[slot] = len;
-  d.s_inv[slot] = 1.0f / max_prop(cov, 1.0f);
-  const int y = cell / d.lW, x = cell - y * d.lW;
-  const size_t HW = (size_t)d.lH * d.lW;
-  const int ex[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
-  const int ey[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
-  float f[9];
-  const float* hp = d.h[parity];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) {
-    const int ys = imod_floor(y - ey[q], d.lH), xs = imod_floor(x - ex[q], d.lW);
-    f[q] = hp[q * HW + (size_t)ys * d.lW + xs];
-  }
-  float rho, vx, vy;
-  macroscopic(f, d.vmax, d.vmax_q4, rho, vx, vy);
-  d.s_rho[slot] = rho;
-  d.s_vx[slot] = vx;
-  d.s_vy[slot] = vy;
-  d.s_ucx[slot] = vx;
-  d.s_ucy[slot] = vy;
-}
-
-// Work for one touched cell whose contributions are run[0..len) in increasing k, read
-// from global memory (spilled tiles only).  CIC: deposit = in-order sum (forces.py:98-115).
-__device__ __forceinline__ void head_work(const RDesc& d, const BinView& v, int which, int parity, const int* run,
-                                          int len, int run_pos) {
+// Deposit of one touched cell whose contributions are run[0..len) in increasing k, read from
+// global memory (spilled tiles only): the in-order sum (forces.py:98-115).
+__device__ __forceinline__ void deposit_cell(const RDesc& d, const BinView& v, const int* run, int len) {
   const int k0 = run[0];
-  const int cell = v.cell[k0];
   float acc = v.w[k0];
   for (int j = 1; j < len; ++j) acc = acc + v.w[run[j]];
-  if (which == 1) {
-    d.dep[cell] = acc;
-    return;
-  }
-  const int slot = atomicAdd(v.ctl + 2, 1);
-  for (int j = 0; j < len; ++j) d.ib_slot[run[j]] = slot;
-  ib_head(d, parity, cell, acc, slot, len, run_pos);
+  d.dep[v.cell[k0]] = acc;
 }
 
 // One CTA on one bin tile: sort the tile's contributions by (cell, k) and reduce every
@@ -130,7 +87,7 @@ __device__ __forceinline__ void head_work(const RDesc& d, const BinView& v, int 
 // bin capacity of every rollout of the launch (a power of two).
 __device__ __forceinline__ int pc(int c) { return c + (c >> 3); }
 
-__device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned* skeys, int capS) {
+__device__ void tile_work(const RDesc& d, int t, unsigned* skeys, int capS) {
   const int kCapS = capS;
   const int kChunk = 4 * capS;  // keys per shared-memory chunk sort on the spill path
   // per-cell counters at padded slots pc(c) = c + c / 8: the scan below gives each lane 8
@@ -139,8 +96,8 @@ __device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned
   __shared__ int cpos[kBinTile * kBinTile + kBinTile * kBinTile / 8];
   __shared__ int hpos[kBinTile * kBinTile + kBinTile * kBinTile / 8];  // rank of a touched cell among the tile's
   __shared__ int tlist[kBinTile * kBinTile];  // the touched cells, by rank
-  __shared__ int s_spill, s_heads, s_base, s_fill;
-  const BinView v = bin_view(d, which);
+  __shared__ int s_spill, s_heads, s_fill;
+  const BinView v = bin_view(d);
   if (v.count == 0) return;
   const int total = v.tcount[t];
   if (total == 0) return;
@@ -200,8 +157,7 @@ __device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned
       if (tid == 31) s_heads = inz;
     }
     __syncthreads();
-    // one slot range per tile for its touched cells (IB); the touched cells listed by rank
-    if (which == 0 && tid == 0) s_base = atomicAdd(v.ctl + 2, s_heads);
+    // the touched cells listed by rank
     for (int c = tid; c < kBinTile * kBinTile; c += blockDim.x)
       if (cnt[pc(c)] > 0) tlist[hpos[pc(c)]] = c;
     for (int i = tid; i < total; i += blockDim.x) {
@@ -233,24 +189,7 @@ __device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned
       }
       float acc = rw[0];
       for (int j = 1; j < len; ++j) acc = acc + rw[j];
-      const int cell = v.cell[rk[0]];
-      if (which == 1) {
-        d.dep[cell] = acc;
-      } else {
-        const int slot = s_base + hpos[pc(c)];
-        for (int j = 0; j < len; ++j) d.ib_slot[rk[j]] = slot;
-        ib_head(d, parity, cell, acc, slot, len, t * v.cap + cpos[pc(c)]);
-      }
-    }
-    __syncthreads();
-    if (which == 0) {
-      // runs for the spread: contributing node and weight, contiguous per touched cell
-      const int K2 = d.K * d.K;
-      float* binw = d.ib_store_w + (size_t)t * v.cap;
-      for (int i = tid; i < total; i += blockDim.x) {
-        bin[i] = kout[i] / K2;
-        binw[i] = wout[i];
-      }
+      d.dep[v.cell[rk[0]]] = acc;
     }
     if (tid == 0) v.tcount[t] = 0;
     return;
@@ -314,22 +253,12 @@ __device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned
   int* kv = reinterpret_cast<int*>(dst);
   for (int i = tid; i < m; i += blockDim.x) kv[i] = (int)(keys[i] & 0xffffffu);
   __syncthreads();
-  const int kv_pos = base + (int)(reinterpret_cast<unsigned*>(kv) - bufA);
   for (int i = tid; i < m; i += blockDim.x) {
     const unsigned lc = keys[i] >> 24;
     if (i > 0 && (keys[i - 1] >> 24) == lc) continue;
     int len = 1;
     while (i + len < m && (keys[i + len] >> 24) == lc) ++len;
-    head_work(d, v, which, parity, kv + i, len, kv_pos + i);
-  }
-  __syncthreads();
-  if (which == 0) {
-    const int K2 = d.K * d.K;
-    for (int i = tid; i < m; i += blockDim.x) {
-      const int k = kv[i];
-      d.ib_store_w[kv_pos + i] = v.w[k];
-      kv[i] = k / K2;
-    }
+    deposit_cell(d, v, kv + i, len);
   }
   if (tid == 0) v.tcount[t] = 0;
 }
@@ -340,7 +269,7 @@ __device__ void tile_work(const RDesc& d, int which, int parity, int t, unsigned
 // a time from a cursor (wl_count[2], reset with the list), so that no CTA is launched only
 // to find nothing to do and uneven tiles balance across the CTAs.
 __global__ void __launch_bounds__(256) k_bin_tiles(const RDesc* __restrict__ D, const int2* __restrict__ wl,
-                                                   int* __restrict__ wl_count, int which, int parity, int capS) {
+                                                   int* __restrict__ wl_count, int capS) {
   extern __shared__ unsigned dyn[];
   __shared__ int s_item;
   const int count = *wl_count;
@@ -350,19 +279,175 @@ __global__ void __launch_bounds__(256) k_bin_tiles(const RDesc* __restrict__ D, 
     const int i = s_item;
     if (i >= count) break;  // uniform across the CTA
     const int2 item = wl[i];
-    tile_work(D[item.x], which, parity, item.y, dyn, capS);
+    tile_work(D[item.x], item.y, dyn, capS);
     __syncthreads();  // the shared arrays and s_item are reused by the next item
   }
 }
 
-// Weighted sum of a head-indexed field over the K*K stencil of one node, in stencil order
+// ---------------------------------------------------------------- touched cells
+// Sorts R (key, value) pairs in registers by key.
+template <int R>
+__device__ __forceinline__ void sort_regs(int (&k)[R], float (&w)[R]) {
+#pragma unroll
+  for (int size = 2; size <= R; size <<= 1)
+#pragma unroll
+    for (int j = size >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int o = i ^ j;
+        if (o > i) {
+          const bool swap = ((i & size) == 0) ? k[i] > k[o] : k[i] < k[o];
+          const int ka = swap ? k[o] : k[i], kb = swap ? k[i] : k[o];
+          const float wa = swap ? w[o] : w[i], wb = swap ? w[i] : w[o];
+          k[i] = ka;
+          k[o] = kb;
+          w[i] = wa;
+          w[o] = wb;
+        }
+      }
+}
+
+// A head of at most R <= kRunRow contributions: its run in its row, its contributions linked to it; returns
+// the coverage (the weights' sum in order of k).
+template <int R>
+__device__ __forceinline__ float head_row(const RDesc& d, int h, int cell, int len, int K2) {
+  int k[R];
+  float w[R];
+  const int4* bucket = reinterpret_cast<const int4*>(d.ib_bucket + (size_t)cell * d.ib_cap);
+#pragma unroll
+  for (int q = 0; q < R; q += 4) {
+    int4 v = make_int4(0, 0, 0, 0);
+    if (q < len) v = bucket[q / 4];
+    k[q] = q < len ? v.x : 0x7fffffff;
+    k[q + 1] = q + 1 < len ? v.y : 0x7fffffff;
+    k[q + 2] = q + 2 < len ? v.z : 0x7fffffff;
+    k[q + 3] = q + 3 < len ? v.w : 0x7fffffff;
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q) w[q] = q < len ? d.ib_w[k[q]] : 0.0f;
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+    if (q < len) d.ib_slot[k[q]] = h;
+  sort_regs<R>(k, w);
+  float cov = w[0];
+#pragma unroll
+  for (int q = 1; q < R; ++q)
+    if (q < len) cov = cov + w[q];
+  int4* row = reinterpret_cast<int4*>(d.run + (size_t)h * kRunRow);
+#pragma unroll
+  for (int q = 0; q < R; q += 2)
+    if (q < len) {
+      const int a = K2 == 16 ? k[q] >> 4 : k[q] / K2, b = K2 == 16 ? k[q + 1] >> 4 : k[q + 1] / K2;
+      row[q / 2] = make_int4(a, __float_as_int(w[q]), b, __float_as_int(w[q + 1]));
+    }
+  return cov;
+}
+
+// A head with more contributions than a row holds, by its whole warp: gathered from the bucket and
+// the overflow list into the pool, ranked, and its run written behind them.
+__device__ __noinline__ float head_pool(const RDesc& d, int h, int cell, int len, int K2, int lane, int& start) {
+  int base = 0;
+  const int pad = (len + 1) & ~1;
+  if (lane == 0) base = atomicAdd(d.ib_ctl + 1, 2 * pad);
+  base = d.run_rows * kRunRow + __shfl_sync(0xffffffffu, base, 0);
+  int2* raw = d.run + base;
+  int2* run = raw + pad;
+  const int* bucket = d.ib_bucket + (size_t)cell * d.ib_cap;
+  const int held = min(len, d.ib_cap);
+  for (int i = lane; i < held; i += 32) raw[i].x = bucket[i];
+  if (lane == 0 && len > d.ib_cap) {
+    int e = d.ib_ovf_head[cell];
+    for (int i = d.ib_cap; i < len; ++i) {
+      raw[i].x = d.ib_ovf[e];
+      e = d.ib_ovf_next[e];
+    }
+    d.ib_ovf_head[cell] = -1;
+  }
+  __syncwarp();
+  for (int i = lane; i < len; i += 32) {
+    const int k = raw[i].x;
+    int rank = 0;
+    for (int q = 0; q < len; ++q) rank += raw[q].x < k ? 1 : 0;
+    run[rank] = make_int2(k / K2, __float_as_int(d.ib_w[k]));
+    d.ib_slot[k] = h;
+  }
+  __syncwarp();
+  float cov = __int_as_float(run[0].y);
+  for (int q = 1; q < len; ++q) cov = cov + __int_as_float(run[q].y);
+  start = base + pad;
+  return cov;
+}
+
+// One thread per touched cell: its contributions ordered by k, the coverage -> 1/max(cov, 1), the
+// macroscopic state pulled from h[parity] (density, clamped velocity), u_corrected = velocity
+// (fluid.py:268-290).  Bound by the latency of its three dependent loads (the cell, its bucket and
+// populations, the weights), with every head's loads in flight at once.
+// Before, one CTA per 16x16 tile counting-sorted the tile's contributions in shared memory, in
+// phases separated by barriers; a tile with more than 2,048 took a sort in global memory, whose
+// tail set the kernel's time on dense rollouts.  Measured (per launch in a step): 1024^2 with
+// 16,384 points 26 -> 11.3 us, a batch of 64 uneven rollouts with 74 k points 225 -> 54 us.  Rows
+// of 8 entries instead of 16 took 46 and 82 us: where rods cross, whole warps of cells then went
+// through the pool.
+__global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restrict__ D, const int* __restrict__ off,
+                                                           int n, int parity) {
+  const int r = find_rollout(off, n, blockIdx.x);
+  const RDesc& d = D[r];
+  const int h0 = (blockIdx.x - off[r]) * blockDim.x;
+  const int heads = d.ib_ctl[2];
+  if (h0 >= heads) return;
+  const int h = h0 + threadIdx.x, lane = threadIdx.x & 31;
+  const bool on = h < heads;
+  const int cell = on ? d.h_new[h] : 0;
+  const int len = on ? d.ib_cnt[cell] : 0;
+  const int lW = d.lW, lH = d.lH, K2 = d.K * d.K;
+  const int y = cell / lW, x = cell - y * lW;
+  const int xm = x == 0 ? lW - 1 : x - 1, xp = x == lW - 1 ? 0 : x + 1;
+  const int HW = lH * lW;
+  // populations are pulled from the cell opposite to their direction
+  const float* __restrict__ r0 = d.h[parity] + y * lW;
+  const float* __restrict__ rm = d.h[parity] + (y == 0 ? lH - 1 : y - 1) * lW;
+  const float* __restrict__ rp = d.h[parity] + (y == lH - 1 ? 0 : y + 1) * lW;
+  float f[9];
+  f[0] = r0[x];
+  f[1] = r0[HW + xm];
+  f[2] = rm[2 * HW + x];
+  f[3] = r0[3 * HW + xp];
+  f[4] = rp[4 * HW + x];
+  f[5] = rm[5 * HW + xm];
+  f[6] = rm[6 * HW + xp];
+  f[7] = rp[7 * HW + xp];
+  f[8] = rp[8 * HW + xm];
+  float cov = 0.0f;
+  int start = h * kRunRow;
+  if (len > 0 && len <= 8) cov = head_row<8>(d, h, cell, len, K2);
+  if (len > 8 && len <= kRunRow) cov = head_row<kRunRow>(d, h, cell, len, K2);
+  for (unsigned deep = __ballot_sync(0xffffffffu, len > kRunRow); deep; deep &= deep - 1) {
+    const int src = __ffs(deep) - 1;
+    int at;
+    const float c = head_pool(d, __shfl_sync(0xffffffffu, h, src), __shfl_sync(0xffffffffu, cell, src),
+                              __shfl_sync(0xffffffffu, len, src), K2, lane, at);
+    if (lane == src) {
+      cov = c;
+      start = at;
+    }
+  }
+  if (!on) return;
+  d.ib_cnt[cell] = 0;
+  float rho, vx, vy;
+  macroscopic(f, d.vmax, d.vmax_q4, rho, vx, vy);
+  d.h_cell[h] = cell;
+  d.h_run[h] = make_int2(start, len);
+  d.s_mac[h] = make_float4(rho, vx, vy, 1.0f / max_prop(cov, 1.0f));
+  d.s_uc[h] = make_float2(vx, vy);
+}
+
+// Weighted sum of a head-indexed field over the K*K stencil of one point, in stencil order
 // (the reference's sum over axis 1 of values * weights, fluid.py:90-97).
 template <int K2>
-__device__ __forceinline__ void stencil_sum(const RDesc& d, int node, const float* __restrict__ ax,
-                                            const float* __restrict__ ay, float& sx, float& sy) {
+__device__ __forceinline__ float2 stencil_sum(const RDesc& d, int point, const float2* __restrict__ field) {
   int slot[K2];
   float w[K2];
-  const int base = node * K2;
+  const int base = point * K2;
   if (K2 % 4 == 0) {
 #pragma unroll
     for (int s = 0; s < K2; s += 4) {
@@ -378,60 +463,52 @@ __device__ __forceinline__ void stencil_sum(const RDesc& d, int node, const floa
       w[s] = d.ib_w[base + s];
     }
   }
-  float vx[K2], vy[K2];
+  float2 v[K2];
 #pragma unroll
-  for (int s = 0; s < K2; ++s) {
-    vx[s] = ax[slot[s]];
-    vy[s] = ay[slot[s]];
-  }
+  for (int s = 0; s < K2; ++s) v[s] = field[slot[s]];
   float x = 0.0f, y = 0.0f;
 #pragma unroll
   for (int s = 0; s < K2; ++s) {
-    x = x + vx[s] * w[s];
-    y = y + vy[s] * w[s];
+    x = x + v[s].x * w[s];
+    y = y + v[s].y * w[s];
   }
-  sx = x;
-  sy = y;
+  return make_float2(x, y);
 }
 
-__device__ __forceinline__ void stencil_sum_any(const RDesc& d, int node, const float* __restrict__ ax,
-                                                const float* __restrict__ ay, float& sx, float& sy) {
+__device__ __forceinline__ float2 stencil_sum_any(const RDesc& d, int point, const float2* __restrict__ field) {
   switch (d.K) {
-    case 4: stencil_sum<16>(d, node, ax, ay, sx, sy); return;
-    case 2: stencil_sum<4>(d, node, ax, ay, sx, sy); return;
-    case 3: stencil_sum<9>(d, node, ax, ay, sx, sy); return;
+    case 4: return stencil_sum<16>(d, point, field);
+    case 2: return stencil_sum<4>(d, point, field);
+    case 3: return stencil_sum<9>(d, point, field);
     default: break;
   }
   const int K2 = d.K * d.K;
   float x = 0.0f, y = 0.0f;
   for (int s = 0; s < K2; ++s) {
-    const int k = node * K2 + s;
-    const int p = d.ib_slot[k];
+    const int k = point * K2 + s;
+    const float2 v = field[d.ib_slot[k]];
     const float w = d.ib_w[k];
-    x = x + ax[p] * w;
-    y = y + ay[p] * w;
+    x = x + v.x * w;
+    y = y + v.y * w;
   }
-  sx = x;
-  sy = y;
+  return make_float2(x, y);
 }
 
-// Body force of touched cell p from its corrected velocity after the last multi-direct
+// Body force of a touched cell from its corrected velocity after the last multi-direct
 // forcing round (fluid.py:327-339): post clamp of u_corrected, F = (u_c - u) rho, optional
 // force clamp.
-__device__ __forceinline__ void head_force(const RDesc& d, int p, float ucx, float ucy) {
-  const float c2 = clamp_factor(ucx, ucy, d.vmax);
-  ucx = ucx * c2;
-  ucy = ucy * c2;
-  const float rho = d.s_rho[p];
-  float Fx = (ucx - d.s_vx[p]) * rho;
-  float Fy = (ucy - d.s_vy[p]) * rho;
+__device__ __forceinline__ float2 head_force(const RDesc& d, float4 mac, float2 uc) {
+  const float c2 = clamp_factor_fast(uc.x, uc.y, d.vmax, d.vmax_q4);
+  uc.x = uc.x * c2;
+  uc.y = uc.y * c2;
+  float Fx = (uc.x - mac.y) * mac.x;
+  float Fy = (uc.y - mac.z) * mac.x;
   if (d.force_clamp) {
     const float c3 = clamp_factor(Fx, Fy, d.vmax);
     Fx = Fx * c3;
     Fy = Fy * c3;
   }
-  d.s_fx[p] = Fx;
-  d.s_fy[p] = Fy;
+  return make_float2(Fx, Fy);
 }
 
 // Multi-direct forcing, interpolation half (fluid.py:292-302): per IB point, u at the point
@@ -440,15 +517,44 @@ __global__ void __launch_bounds__(256) k_ib_interp(const RDesc* __restrict__ D, 
                                                    int it) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int node = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
-  if (node >= d.NI || it >= d.ib_iters) return;  // node = IB point
-  float ux, uy;
-  stencil_sum_any(d, node, d.s_ucx, d.s_ucy, ux, uy);
-  const float sx = (d.nvl[2 * node] - ux) * d.relax;
-  const float sy = (d.nvl[2 * node + 1] - uy) * d.relax;
-  const float cf = clamp_factor(sx, sy, d.vmax);
-  d.delta[2 * node] = sx * cf;
-  d.delta[2 * node + 1] = sy * cf;
+  const int p = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;  // IB point
+  if (p >= d.NI || it >= d.ib_iters) return;
+  const float2 v = d.nvl[p];
+  const float2 u = stencil_sum_any(d, p, d.s_uc);
+  const float sx = (v.x - u.x) * d.relax;
+  const float sy = (v.y - u.y) * d.relax;
+  const float cf = clamp_factor_fast(sx, sy, d.vmax, d.vmax_q4);
+  d.delta[p] = make_float2(sx * cf, sy * cf);
+}
+
+// In-order sum of correction * weight over a head's run (fluid.py:304-309).  Runs are short: 8
+// entries are fetched at a time (those that exist) so that all their loads are in flight together.
+__device__ __forceinline__ float2 run_sum(const int2* __restrict__ run, int len, const float2* __restrict__ delta) {
+  float dx = 0.0f, dy = 0.0f;
+  const int4* pairs = reinterpret_cast<const int4*>(run);  // runs start at even entries
+  for (int j = 0; j < len; j += 8) {
+    int4 e[4];
+    float2 v[8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = j + 2 * q < len ? pairs[j / 2 + q] : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      v[2 * q] = j + 2 * q < len ? delta[e[q].x] : make_float2(0.0f, 0.0f);
+      v[2 * q + 1] = j + 2 * q + 1 < len ? delta[e[q].z] : make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (j + 2 * q < len) {
+        dx = dx + v[2 * q].x * __int_as_float(e[q].y);
+        dy = dy + v[2 * q].y * __int_as_float(e[q].y);
+      }
+      if (j + 2 * q + 1 < len) {
+        dx = dx + v[2 * q + 1].x * __int_as_float(e[q].w);
+        dy = dy + v[2 * q + 1].y * __int_as_float(e[q].w);
+      }
+    }
+  }
+  return make_float2(dx, dy);
 }
 
 // Multi-direct forcing, spread half (fluid.py:304-310): per touched cell, the in-order sum
@@ -462,42 +568,16 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
   // the plan's last round also computes each touched cell's body force (k_ib_finalize's
   // work for the same cell) when every rollout of the plan runs the same number of rounds
   const bool fin = fuse_finalize && it == d.ib_iters - 1;
-  if (fin && p == 0) d.ib_ctl[5] = d.ib_ctl[2];
-  if (it >= d.ib_iters || p >= d.ib_ctl[2]) return;
-  const int len = d.h_len[p];
-  const int* rn = d.ib_store + d.h_start[p];      // contributing nodes, in k order
-  const float* rw = d.ib_store_w + d.h_start[p];  // their weights
-  float dx = 0.0f, dy = 0.0f;
-  // runs are short: fetch 8 entries at a time (the last group predicated) so that all
-  // their loads are in flight together; the sum keeps the run order
-  for (int j = 0; j < len; j += 8) {
-    int nd[8];
-    float w[8], ex[8], ey[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const bool ok = j + q < len;
-      nd[q] = ok ? rn[j + q] : 0;
-      w[q] = ok ? rw[j + q] : 0.0f;
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const bool ok = j + q < len;
-      ex[q] = ok ? d.delta[2 * nd[q]] : 0.0f;
-      ey[q] = ok ? d.delta[2 * nd[q] + 1] : 0.0f;
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (j + q < len) {
-        dx = dx + ex[q] * w[q];
-        dy = dy + ey[q] * w[q];
-      }
-    }
-  }
-  const float inv = d.s_inv[p];
-  const float ucx = d.s_ucx[p] + dx * inv, ucy = d.s_ucy[p] + dy * inv;
-  d.s_ucx[p] = ucx;
-  d.s_ucy[p] = ucy;
-  if (fin) head_force(d, p, ucx, ucy);
+  const int heads = d.ib_ctl[2];
+  if (fin && p == 0) d.ib_ctl[5] = heads;
+  if (it >= d.ib_iters || p >= heads) return;
+  const int2 run = d.h_run[p];
+  const float4 mac = d.s_mac[p];
+  float2 u = d.s_uc[p];
+  const float2 s = run_sum(d.run + run.x, run.y, d.delta);
+  u = make_float2(u.x + s.x * mac.w, u.y + s.y * mac.w);
+  d.s_uc[p] = u;
+  if (fin) d.s_f[p] = head_force(d, mac, u);
 }
 
 // ---------------------------------------------------------------- fused IB iterations
@@ -540,98 +620,58 @@ __device__ __forceinline__ void ib_iterations(const RDesc& d, int t0, int stride
   const int nheads = __ldcg(d.ib_ctl + 2);
   const int K2 = d.K * d.K;
   for (int it = 0; it < d.ib_iters; ++it) {
-    for (int node = t0; node < d.NI; node += stride) {  // IB points
+    for (int p = t0; p < d.NI; p += stride) {  // IB points
       float ux = 0.0f, uy = 0.0f;
-      const int base = node * K2;
-      if (K2 == 16) {
-        int slot[16];
-        float w[16];
+      const int base = p * K2;
+      for (int q0 = 0; q0 < K2; q0 += 8) {
+        float2 v[8];
+        float w[8];
 #pragma unroll
-        for (int q = 0; q < 16; q += 4) {
-          const int4 a = *reinterpret_cast<const int4*>(d.ib_slot + base + q);
-          const float4 b = *reinterpret_cast<const float4*>(d.ib_w + base + q);
-          slot[q] = a.x; slot[q + 1] = a.y; slot[q + 2] = a.z; slot[q + 3] = a.w;
-          w[q] = b.x; w[q + 1] = b.y; w[q + 2] = b.z; w[q + 3] = b.w;
-        }
-        float vx[16], vy[16];
+        for (int q = 0; q < 8; ++q)
+          if (q0 + q < K2) {
+            v[q] = __ldcg(d.s_uc + d.ib_slot[base + q0 + q]);
+            w[q] = d.ib_w[base + q0 + q];
+          }
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          vx[q] = __ldcg(d.s_ucx + slot[q]);
-          vy[q] = __ldcg(d.s_ucy + slot[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          ux = ux + vx[q] * w[q];
-          uy = uy + vy[q] * w[q];
-        }
-      } else {
-        for (int q = 0; q < K2; ++q) {
-          const int sl = d.ib_slot[base + q];
-          const float w = d.ib_w[base + q];
-          ux = ux + __ldcg(d.s_ucx + sl) * w;
-          uy = uy + __ldcg(d.s_ucy + sl) * w;
-        }
+        for (int q = 0; q < 8; ++q)
+          if (q0 + q < K2) {
+            ux = ux + v[q].x * w[q];
+            uy = uy + v[q].y * w[q];
+          }
       }
-      const float sx = (d.nvl[2 * node] - ux) * d.relax;
-      const float sy = (d.nvl[2 * node + 1] - uy) * d.relax;
+      const float2 nv = d.nvl[p];
+      const float sx = (nv.x - ux) * d.relax;
+      const float sy = (nv.y - uy) * d.relax;
       const float cf = clamp_factor(sx, sy, d.vmax);
-      d.delta[2 * node] = sx * cf;
-      d.delta[2 * node + 1] = sy * cf;
+      d.delta[p] = make_float2(sx * cf, sy * cf);
     }
     sync();
     for (int p = t0; p < nheads; p += stride) {
-      const int len = d.h_len[p];
-      const int* rn = d.ib_store + d.h_start[p];
-      const float* rw = d.ib_store_w + d.h_start[p];
+      const int2 run = d.h_run[p];
       float dx = 0.0f, dy = 0.0f;
-      int j = 0;
-      for (; j + 8 <= len; j += 8) {
-        int nd[8];
-        float w[8], ex[8], ey[8];
+      for (int j = 0; j < run.y; j += 8) {
+        int2 e[8];
+        float2 v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          nd[q] = rn[j + q];
-          w[q] = rw[j + q];
-        }
+        for (int q = 0; q < 8; ++q)
+          if (j + q < run.y) {
+            e[q] = d.run[run.x + j + q];
+            v[q] = __ldcg(d.delta + e[q].x);
+          }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          ex[q] = __ldcg(d.delta + 2 * nd[q]);
-          ey[q] = __ldcg(d.delta + 2 * nd[q] + 1);
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          dx = dx + ex[q] * w[q];
-          dy = dy + ey[q] * w[q];
-        }
+        for (int q = 0; q < 8; ++q)
+          if (j + q < run.y) {
+            dx = dx + v[q].x * __int_as_float(e[q].y);
+            dy = dy + v[q].y * __int_as_float(e[q].y);
+          }
       }
-      for (; j < len; ++j) {
-        const int node = rn[j];
-        const float w = rw[j];
-        dx = dx + __ldcg(d.delta + 2 * node) * w;
-        dy = dy + __ldcg(d.delta + 2 * node + 1) * w;
-      }
-      const float inv = d.s_inv[p];
-      d.s_ucx[p] = __ldcg(d.s_ucx + p) + dx * inv;
-      d.s_ucy[p] = __ldcg(d.s_ucy + p) + dy * inv;
+      const float inv = d.s_mac[p].w;
+      const float2 u = __ldcg(d.s_uc + p);
+      d.s_uc[p] = make_float2(u.x + dx * inv, u.y + dy * inv);
     }
     sync();
   }
-  for (int p = t0; p < nheads; p += stride) {
-    float ucx = __ldcg(d.s_ucx + p), ucy = __ldcg(d.s_ucy + p);
-    const float c2 = clamp_factor(ucx, ucy, d.vmax);
-    ucx = ucx * c2;
-    ucy = ucy * c2;
-    const float rho = d.s_rho[p];
-    float Fx = (ucx - d.s_vx[p]) * rho;
-    float Fy = (ucy - d.s_vy[p]) * rho;
-    if (d.force_clamp) {
-      const float c3 = clamp_factor(Fx, Fy, d.vmax);
-      Fx = Fx * c3;
-      Fy = Fy * c3;
-    }
-    d.s_fx[p] = Fx;
-    d.s_fy[p] = Fy;
-  }
+  for (int p = t0; p < nheads; p += stride) d.s_f[p] = head_force(d, d.s_mac[p], __ldcg(d.s_uc + p));
   if (t0 == 0) d.ib_ctl[5] = nheads;  // for k_collide_heads
 }
 
@@ -677,7 +717,7 @@ __global__ void __launch_bounds__(256) k_ib_finalize(const RDesc* __restrict__ D
   const int nheads = d.ib_ctl[2];
   if (p == 0) d.ib_ctl[5] = nheads;
   if (p >= nheads) return;
-  head_force(d, p, d.s_ucx[p], d.s_ucy[p]);
+  d.s_f[p] = head_force(d, d.s_mac[p], d.s_uc[p]);
 }
 
 // Node reaction (fluid.py:364-382), final wrap (simulate.py:97-98), non-finite check and
@@ -699,17 +739,14 @@ __global__ void __launch_bounds__(256) k_reaction(const RDesc* __restrict__ D, c
   if (node >= d.N) return;
   float vx = d.vel[2 * node], vy = d.vel[2 * node + 1];
   if (d.enable_fluid) {
-    float fx, fy;
-    stencil_sum_any(d, node, d.s_fx, d.s_fy, fx, fy);
+    float2 f = stencil_sum_any(d, node, d.s_f);
     if (d.NI > d.N) {
       // synthetic pair: the mean of the two points' forces (fluid.py:371-374)
-      float gx, gy;
-      stencil_sum_any(d, node + d.N, d.s_fx, d.s_fy, gx, gy);
-      fx = 0.5f * (fx + gx);
-      fy = 0.5f * (fy + gy);
+      const float2 g = stencil_sum_any(d, node + d.N, d.s_f);
+      f = make_float2(0.5f * (f.x + g.x), 0.5f * (f.y + g.y));
     }
-    vx = vx - (fx / d.node_mass) / d.sdt_x;
-    vy = vy - (fy / d.node_mass) / d.sdt_y;
+    vx = vx - (f.x / d.node_mass) / d.sdt_x;
+    vy = vy - (f.y / d.node_mass) / d.sdt_y;
     d.vel[2 * node] = vx;
     d.vel[2 * node + 1] = vy;
   }
@@ -809,9 +846,11 @@ __global__ void k_tick(int* tdev) { *tdev += 1; }
 cudaError_t tiles_blocks_per_sm(int threads, int capS, int* out) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k_bin_tiles, threads, (size_t)4 * capS * sizeof(unsigned));
 }
-void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int which, int parity, int capS,
-                      int threads) {
-  k_bin_tiles<<<L.grid, threads, (size_t)4 * capS * sizeof(unsigned), L.s>>>(L.d, wl, wl_count, which, parity, capS);
+void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int capS, int threads) {
+  k_bin_tiles<<<L.grid, threads, (size_t)4 * capS * sizeof(unsigned), L.s>>>(L.d, wl, wl_count, capS);
+}
+void launch_ib_heads(const Launch& L, int parity) {
+  k_ib_heads<<<L.grid, kHeadThreads, 0, L.s>>>(L.d, L.off, L.n, parity);
 }
 // `bytes` is the per-block opt-in limit; the kernel's static shared memory comes off it.
 cudaError_t tiles_set_smem(size_t bytes) {

@@ -371,15 +371,26 @@ __global__ void __launch_bounds__(kHeadThreads) k_collide_heads(const RDesc* __r
   const size_t HW = (size_t)H * W;
   const float* __restrict__ hin = d.h[parity];
   float* __restrict__ hout = d.h[parity ^ 1];
+  const int xm = x == 0 ? W - 1 : x - 1, xp = x == W - 1 ? 0 : x + 1;
+  // populations are pulled from the cell opposite to their direction
+  const float* __restrict__ r0 = hin + (size_t)y * W;
+  const float* __restrict__ rm = hin + (size_t)(y == 0 ? H - 1 : y - 1) * W;
+  const float* __restrict__ rp = hin + (size_t)(y == H - 1 ? 0 : y + 1) * W;
   float f[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const int ys = imod_floor(y - kEy[i], H), xs = imod_floor(x - kEx[i], W);
-    f[i] = hin[i * HW + (size_t)ys * W + xs];
-  }
+  f[0] = r0[x];
+  f[1] = r0[HW + xm];
+  f[2] = rm[2 * HW + x];
+  f[3] = r0[3 * HW + xp];
+  f[4] = rp[4 * HW + x];
+  f[5] = rm[5 * HW + xm];
+  f[6] = rm[6 * HW + xp];
+  f[7] = rp[7 * HW + xp];
+  f[8] = rp[8 * HW + xm];
   const float cp = 1.0f - 0.5f * d.wp, cm = 1.0f - 0.5f * d.wm;
   float o[9], usx, usy;
-  collide(f, d.s_rho[p], d.s_vx[p], d.s_vy[p], d.s_fx[p], d.s_fy[p], d.wp, d.wm, cp, cm, o, usx, usy);
+  const float4 mac = d.s_mac[p];
+  const float2 F = d.s_f[p];
+  collide(f, mac.x, mac.y, mac.z, F.x, F.y, d.wp, d.wm, cp, cm, o, usx, usy);
 #pragma unroll
   for (int i = 0; i < 9; ++i) hout[i * HW + cell] = o[i];
   if (write_u) {
@@ -439,8 +450,12 @@ __global__ void k_clear_ws(const RDesc* __restrict__ D, const int* __restrict__ 
   const size_t t0 = (size_t)lb * blockDim.x + threadIdx.x;
   if (d.dep)
     for (size_t i = t0; i < HW; i += stride) d.dep[i] = 0.0f;
-  const int nt = d.ntile_x * d.ntile_y, lnt = d.lntile_x * d.lntile_y;
-  for (size_t i = t0; i < (size_t)lnt; i += stride) d.ib_tcount[i] = 0;
+  if (d.M > 0)
+    for (size_t i = t0; i < (size_t)d.lH * d.lW; i += stride) {
+      d.ib_cnt[i] = 0;
+      d.ib_ovf_head[i] = -1;
+    }
+  const int nt = d.ntile_x * d.ntile_y;
   for (size_t i = t0; i < (size_t)nt; i += stride) d.c_tcount[i] = 0;
   if (t0 < 8) {
     d.ib_ctl[t0] = 0;

@@ -26,7 +26,7 @@ constexpr int kStageCells = 1024;  // staged dense pass: lattice cells per item 
 constexpr int kStagedThreads = 256;  // ... and threads per CTA (4 cells each)
 constexpr int kConvTile = 32;     // steric direct convolution: 32 x 32 outputs per CTA
 constexpr int kConvMaxR = 24;     // largest tap radius of the direct convolution       //                    8 rows
-constexpr int kIbCap = 1024;       // minimum IB bin capacity per 16x16 tile (grown with node density)
+constexpr int kRunRow = 16;        // entries of a touched cell's run row (k_ib_heads sorts as many in registers)
 constexpr int kCicCap = 512;       // minimum CIC bin capacity per tile
 constexpr int kMaxBinCap = 8192;   // largest bin capacity (the tile sort keeps 4 x cap words in shared memory)
 constexpr int kFftMaxN = 4096;     // largest FFT length (shared memory)
@@ -42,7 +42,6 @@ struct RDesc {
   int NI;                // IB points: N, or 2N with synthetic node pairs
   int M;                 // IB contributions = NI*K*K
   int ntile_x, ntile_y;  // binning tiles (kBinTile) of the domain grid (cloud-in-cell deposit)
-  int lntile_x, lntile_y;  // binning tiles of the lattice (IB contributions)
   float rs_inv_y, rs_ks_y, rs_inv_x, rs_ks_x;  // lattice -> domain resize of the recorded u*: 1/scale, kernel width
   int lbm_tx, lbm_ty;    // LBM tiles
   int lbm_tw;            // LBM tile width in cells (32 * cells per lane)
@@ -117,35 +116,34 @@ struct RDesc {
   float* prev;         // (N,2)
   float* pred;         // (N,2)
   float* predw;        // (N,2) prediction wrapped into the domain (steric sampling)
-  float* nvl;          // (NI,2) IB point velocity in lattice units
-  float* delta;        // (NI,2) IB per-iteration correction
-  // Deterministic scatter-add bins.  Contribution k goes to bin tile t at
-  // store[t * cap + atomic position]; a tile that fills up spills into the overflow list.
-  // store[ntiles * cap ...] is an arena for sorting tiles with more than cap entries.
-  // ctl[0] = overflow count, ctl[1] = arena use, ctl[2] = touched-cell (head) count,
-  // ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
-  // ctl[5] = the head count saved by the finalize step for k_collide_heads.
+  float2* nvl;         // (NI) IB point velocity in lattice units
+  float2* delta;       // (NI) its correction of the current round
+  // IB contributions k = point*K*K + entry.  Each is appended to its cell's bucket
+  // (ib_bucket[cell * ib_cap ...], an atomic on ib_cnt picks the place); beyond ib_cap it goes to
+  // the cell's overflow list (ib_ovf_head, ib_ovf_next, ib_ovf).  The first one of a cell makes it
+  // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of the run pool, ctl[2] =
+  // heads, ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
+  // ctl[5] = the head count saved for k_collide_heads.
   int ib_cap;
-  int* ib_cell;     // (M) cell of contribution k = n*K*K + s
   float* ib_w;      // (M) normalised stencil weight
-  int* ib_store;    // (ntiles * ib_cap + 2 * M); after the tile sort: contributing node per run entry
-  float* ib_store_w;  // same indexing: the run entry's weight
-  int* ib_tcount;   // (ntiles)
-  int* ib_ovf;      // (M)
-  int* ib_ctl;      // (4)
-  int* ib_slot;     // (M) contribution -> head slot of its cell
-  // per touched cell ("head"), slots in [0, ctl[2])
-  int* h_cell;
-  int* h_start;     // position of the cell's sorted run in ib_store
-  int* h_len;
-  float* s_rho;
-  float* s_vx;
-  float* s_vy;
-  float* s_inv;
-  float* s_ucx;
-  float* s_ucy;
-  float* s_fx;
-  float* s_fy;
+  int* ib_slot;     // (M) contribution -> head of its cell
+  int* ib_cnt;      // (lH lW) contributions of the cell, zero between steps
+  int* ib_bucket;   // (lH lW, ib_cap)
+  int* ib_ovf_head;  // (lH lW) first overflow entry of the cell, -1 between steps
+  int* ib_ovf_next;  // (M)
+  int* ib_ovf;      // (M) their contributions
+  int* ib_ctl;      // (8)
+  // runs: per head the (point, weight) pairs of its contributions in order of k, in its row
+  // [h * kRunRow ...] or, when longer, in the pool behind the rows
+  int2* run;        // (run_rows * kRunRow + 3 M)
+  int run_rows;
+  // per head, in [0, ctl[2])
+  int* h_new;       // cell, as the stencil kernel lists it (while k_collide_heads may still use h_cell)
+  int* h_cell;      // cell, from k_ib_heads on
+  int2* h_run;      // start and length of its run
+  float4* s_mac;    // density, clamped velocity, 1 / max(coverage, 1)
+  float2* s_uc;     // corrected velocity
+  float2* s_f;      // body force
   // CIC deposit contributions k = corner*N + n (4N)
   int c_cap;
   int* c_cell;
@@ -154,11 +152,10 @@ struct RDesc {
   int* c_tcount;
   int* c_ovf;       // (4N)
   int* c_ctl;       // (4)
-  // plan-wide lists of bin tiles that received contributions this step: (rollout, tile)
+  // plan-wide list of bin tiles that received CIC contributions this step: (rollout, tile)
   int ridx;            // this rollout's index in the plan
-  int2* wl_ib;
   int2* wl_cic;
-  int* wl_ctl;         // [0] IB list length, [1] CIC list length, [2] / [3] their cursors
+  int* wl_ctl;         // [1] its length, [3] its cursor
   // rod components: chains (warp kernel) and general graphs (CTA kernel)
   int nchain, ngeneric;
   const int4* chain_info;   // (nchain) first node, nodes, first edge, first pair
@@ -241,8 +238,7 @@ struct Launch {
 void launch_predict(const Launch& L);
 // wl_count: the list length; wl_count[2] is the cursor the CTAs take tiles from (reset to 0
 // with the list)
-void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int which, int parity, int capS,
-                      int threads = 256);
+void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int capS, int threads = 256);
 cudaError_t tiles_blocks_per_sm(int threads, int capS, int* out);
 cudaError_t tiles_set_smem(size_t bytes);
 void launch_fft_rows(const Launch& L, size_t smem);
@@ -251,7 +247,8 @@ void launch_node(const Launch& L, const int* tdev, size_t smem, int bs);
 void launch_chain(const Launch& L, const int* tdev, int longest);
 void launch_steric(const Launch& L);
 void launch_stencil(const Launch& L);
-void launch_stencil16(const Launch& L);
+void launch_stencil4(const Launch& L);
+void launch_ib_heads(const Launch& L, int parity);
 void launch_ib_interp(const Launch& L, int it);
 void launch_ib_spread(const Launch& L, int it, int fuse_finalize);
 void launch_ib_finalize(const Launch& L, int parity);

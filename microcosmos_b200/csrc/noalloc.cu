@@ -232,7 +232,6 @@ extern "C" mc_status mc_steric_potential_noalloc(const float* position, int32_t 
   d.flags = reinterpret_cast<unsigned*>(P(kOffFlags));
   d.ridx = 0;
   d.wl_cic = reinterpret_cast<int2*>(P(kOffWl));
-  d.wl_ib = reinterpret_cast<int2*>(P(kOffWl));  // unused (no IB here); k_predict resets its length
   d.wl_ctl = reinterpret_cast<int*>(P(kOffWlCtl));
 
   // CTA offset tables of the four kernels: deposit (nodes), bin tiles, FFT rows, FFT columns
@@ -254,7 +253,7 @@ extern "C" mc_status mc_steric_potential_noalloc(const float* position, int32_t 
   mc::launch_predict(l);
   l.off = off + 2;
   l.grid = cnt[1] < 1184 ? cnt[1] : 1184;
-  mc::launch_bin_tiles(l, reinterpret_cast<const int2*>(P(kOffWl)), reinterpret_cast<int*>(P(kOffWlCtl)) + 1, 1, 0,
+  mc::launch_bin_tiles(l, reinterpret_cast<const int2*>(P(kOffWl)), reinterpret_cast<int*>(P(kOffWlCtl)) + 1,
                        mc::kCicCap);
   l.off = off + 4;
   l.grid = cnt[2];

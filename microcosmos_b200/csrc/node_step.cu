@@ -243,11 +243,8 @@ __device__ __forceinline__ void forcing(const RDesc& d, const Smem& m, int NI, i
   const int tid = threadIdx.x, T = blockDim.x;
   const float vmax = d.vmax, q4 = d.vmax_q4, relax = d.relax;
   const int iters = d.ib_iters, clamp_force = d.force_clamp;
-  const float* __restrict__ s_rho = d.s_rho;
-  const float* __restrict__ s_vx = d.s_vx;
-  const float* __restrict__ s_vy = d.s_vy;
-  float* __restrict__ s_fx = d.s_fx;
-  float* __restrict__ s_fy = d.s_fy;
+  const float4* __restrict__ s_mac = d.s_mac;
+  float2* __restrict__ s_f = d.s_f;
   const float* const inv = m.inv();
   float2* const uc = m.uc();
   float2* const delta = m.delta();
@@ -297,18 +294,17 @@ __device__ __forceinline__ void forcing(const RDesc& d, const Smem& m, int NI, i
   }
   for (int h = tid; h < heads; h += T) {
     float2 u = uc[h];
-    const float rho = s_rho[h], vx = s_vx[h], vy = s_vy[h];
+    const float4 mac = s_mac[h];
     const float c2 = clamp_factor_fast(u.x, u.y, vmax, q4);
     u.x = u.x * c2;
     u.y = u.y * c2;
-    float Fx = (u.x - vx) * rho, Fy = (u.y - vy) * rho;
+    float Fx = (u.x - mac.y) * mac.x, Fy = (u.y - mac.z) * mac.x;
     if (clamp_force) {
       const float c3 = clamp_factor(Fx, Fy, vmax);
       Fx = Fx * c3;
       Fy = Fy * c3;
     }
-    s_fx[h] = Fx;
-    s_fy[h] = Fy;
+    s_f[h] = make_float2(Fx, Fy);
     uc[h] = make_float2(Fx, Fy);
   }
   __syncthreads();
@@ -331,9 +327,7 @@ __device__ __forceinline__ void couple(const RDesc& d, const Smem& m, int* warp_
   const size_t HW = (size_t)lH * lW;
   const float vmax = d.vmax, q4 = d.vmax_q4;
   int* __restrict__ h_cell = d.h_cell;
-  float* __restrict__ s_rho = d.s_rho;
-  float* __restrict__ s_vx = d.s_vx;
-  float* __restrict__ s_vy = d.s_vy;
+  float4* __restrict__ s_mac = d.s_mac;
   if (tid == 0) d.ib_ctl[5] = heads;  // for k_collide_heads
   for (int h = tid; h < heads; h += T) {
     const int cell = m.hcell()[h];
@@ -359,10 +353,9 @@ __device__ __forceinline__ void couple(const RDesc& d, const Smem& m, int* warp_
     float rho, vx, vy;
     macroscopic(f, vmax, q4, rho, vx, vy);
     h_cell[h] = cell;
-    s_rho[h] = rho;
-    s_vx[h] = vx;
-    s_vy[h] = vy;
-    m.inv()[h] = 1.0f / max_prop(cov, 1.0f);
+    const float inv = 1.0f / max_prop(cov, 1.0f);
+    s_mac[h] = make_float4(rho, vx, vy, inv);
+    m.inv()[h] = inv;
     m.uc()[h] = make_float2(vx, vy);
   }
   __syncthreads();

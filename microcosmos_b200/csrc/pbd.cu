@@ -21,14 +21,10 @@ __global__ void __launch_bounds__(256) k_predict(const RDesc* __restrict__ D, co
   const RDesc& d = D[r];
   const int node = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
   if (node == 0) {
-    // the previous step's IB work is complete: reset this step's IB bin controls
+    // the previous step's IB work is complete: reset this step's IB controls
     d.ib_ctl[0] = 0;
     d.ib_ctl[1] = 0;
     d.ib_ctl[2] = 0;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    d.wl_ctl[0] = 0;  // the plan's IB tile list and its cursor
-    d.wl_ctl[2] = 0;
   }
   if (node >= d.N) return;
   const float px = d.pos[2 * node], py = d.pos[2 * node + 1];
@@ -184,10 +180,23 @@ __device__ __forceinline__ float2 ib_point(const RDesc& d, int p, int node, floa
   return p < d.N ? make_float2(gx + ox, gy + oy) : make_float2(gx - ox, gy - oy);
 }
 
+// Contribution k appended to its cell; true when it is the cell's first of this step.
+__device__ __forceinline__ bool ib_append(const RDesc& d, int cell, int k) {
+  const int pos = atomicAdd(d.ib_cnt + cell, 1);
+  if (pos < d.ib_cap) {
+    d.ib_bucket[(size_t)cell * d.ib_cap + pos] = k;
+  } else {
+    const int e = atomicAdd(d.ib_ctl, 1);
+    d.ib_ovf[e] = k;
+    d.ib_ovf_next[e] = atomicExch(d.ib_ovf_head + cell, e);
+  }
+  return pos == 0;
+}
+
 // Velocity (simulate.py:83-84), the IB point in lattice units (fluid.py:236-239) and its
-// K x K stencil (fluid.py:40-79) appended to the IB bins, and the clearing of the node's
-// CIC deposit cells (the deposit grid stays zero between steps).  The stencil spans at
-// most 2 x 2 bin tiles, so its contributions take their bin slots with one atomic per tile.
+// K x K stencil (fluid.py:40-79), its contributions appended to their cells, the cells' first
+// ones making them touched cells; and the clearing of the node's CIC deposit cells (the deposit
+// grid stays zero between steps).  One thread per IB point, any K.
 __global__ void __launch_bounds__(256) k_stencil(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
@@ -208,8 +217,7 @@ __global__ void __launch_bounds__(256) k_stencil(const RDesc* __restrict__ D, co
   const int K = d.K, K2 = K * K;
   const float2 gp = ib_point(d, p, gi, x, y);
   const float gx = gp.x, gy = gp.y;
-  d.nvl[2 * p] = (vx * d.scale_x) * d.dt;
-  d.nvl[2 * p + 1] = (vy * d.scale_y) * d.dt;
+  d.nvl[p] = make_float2((vx * d.scale_x) * d.dt, (vy * d.scale_y) * d.dt);
   const int half = (K - 1) / 2;
   const float hw = (float)K / 2.0f;
   const float sx = floorf(gx) - (float)half, sy = floorf(gy) - (float)half;
@@ -233,139 +241,103 @@ __global__ void __launch_bounds__(256) k_stencil(const RDesc* __restrict__ D, co
     for (int b = 0; b < 8; ++b)
       if (a < K && b < K) sum = sum + wx[a] * wy[b];
   const float den = sum + MC_EPSIL;
-  // tile split of the stencil: columns (rows) whose tile differs from the first one's.
-  // A window of K <= 8 consecutive cells meets at most two tiles unless the grid's last
-  // tile is narrower than the window; then every contribution takes its own slot.
-  const int tx0 = cx[0] / kBinTile, ty0 = cy[0] / kBinTile;
-  int txo = -1, tyo = -1, nx1 = 0, ny1 = 0;
-  bool split_ok = true;
-#pragma unroll
-  for (int a = 1; a < 8; ++a) {
-    if (a < K) {
-      const int tx = cx[a] / kBinTile, ty = cy[a] / kBinTile;
-      if (tx != tx0) {
-        if (txo >= 0 && tx != txo) split_ok = false;
-        txo = tx;
-        ++nx1;
-      }
-      if (ty != ty0) {
-        if (tyo >= 0 && ty != tyo) split_ok = false;
-        tyo = ty;
-        ++ny1;
-      }
-    }
-  }
-  if (txo < 0) txo = tx0;
-  if (tyo < 0) tyo = ty0;
-  const int nx0 = K - nx1, ny0 = K - ny1;
-  int base[4];
-  const int tiles[4] = {ty0 * d.lntile_x + tx0, ty0 * d.lntile_x + txo, tyo * d.lntile_x + tx0, tyo * d.lntile_x + txo};
-  const int counts[4] = {nx0 * ny0, nx1 * ny0, nx0 * ny1, nx1 * ny1};
-  if (split_ok) {
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      base[g] = counts[g] ? atomicAdd(d.ib_tcount + tiles[g], counts[g]) : -1;
-      if (base[g] == 0) d.wl_ib[atomicAdd(d.wl_ctl, 1)] = make_int2(d.ridx, tiles[g]);
-    }
-  }
-  int rank[4] = {0, 0, 0, 0};
-  const int cap = d.ib_cap;
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
     if (a < K) {
-      const int xs = (cx[a] / kBinTile != tx0) ? 1 : 0;
 #pragma unroll
       for (int b = 0; b < 8; ++b) {
         if (b < K) {
-          const int ys = (cy[b] / kBinTile != ty0) ? 1 : 0;
-          const int g = xs + 2 * ys;
-          const int k = p * K2 + a * K + b;
-          d.ib_cell[k] = cy[b] * d.lW + cx[a];
+          const int k = p * K2 + a * K + b, cell = cy[b] * d.lW + cx[a];
           d.ib_w[k] = (wx[a] * wy[b]) / den;
-          int tile, pos;
-          if (split_ok) {
-            tile = tiles[g];
-            pos = base[g] + rank[g]++;
-          } else {
-            tile = (cy[b] / kBinTile) * d.lntile_x + cx[a] / kBinTile;
-            pos = atomicAdd(d.ib_tcount + tile, 1);
-            if (pos == 0) d.wl_ib[atomicAdd(d.wl_ctl, 1)] = make_int2(d.ridx, tile);
-          }
-          if (pos < cap) {
-            d.ib_store[(size_t)tile * cap + pos] = bin_entry(cy[b], cx[a], k);
-          } else {
-            d.ib_ovf[atomicAdd(d.ib_ctl, 1)] = k;
-          }
+          if (ib_append(d, cell, k)) d.h_new[atomicAdd(d.ib_ctl + 2, 1)] = cell;
         }
       }
     }
   }
 }
 
-// The same work with one 16-lane group per node (K <= 4): lane s = a*K + b owns stencil
-// entry s.  The weight normalisation sum is taken by the group's first lane in entry
-// order, so the result equals the one-thread-per-node kernel's; bin slots are taken with
-// one atomic per (warp, tile) group.
-__global__ void __launch_bounds__(256) k_stencil16(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+// The same work for K <= 4 with 4 lanes per IB point, lane a a column of the stencil: two cosines
+// and up to four contributions per lane.  The weights' sum is taken in entry order a * K + b by
+// every lane, so the result equals the one-thread-per-point kernel's.  The touched cells of a warp
+// (8 consecutive points) are numbered together, so that neighbours on a rod stay neighbours in the
+// list of touched cells.  Bound by the latency of the atomics.  Before, 16 lanes per point computed
+// all cosines 4 times over and took slots in 16x16 tiles: a batch of 64
+// uneven rollouts with 74 k points 39 -> 23 us per launch, 1024^2 with 16,384 points 8.8 -> 9.2 us
+// (latency on both sides; the kernel that follows gains more).
+__global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
   const int t = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
-  const int p = t >> 4, s = t & 15;  // IB point, stencil entry
-  const int lane = threadIdx.x & 31;
-  const unsigned gmask = 0xffffu << (lane & 16);
-  if (p >= d.NI) return;  // both halves of a warp exit together unless NI is odd
-  const int gi = p < d.N ? p : p - d.N;
+  const int NI = d.NI, N = d.N;
+  const int p = min(t >> 2, NI - 1), a = t & 3, lane = threadIdx.x & 31;
+  const bool on = (t >> 2) < NI;
+  const int gi = p < N ? p : p - N;
   const float x = d.pos[2 * gi], y = d.pos[2 * gi + 1];
   const float vx = (x - d.prev[2 * gi]) / d.dt, vy = (y - d.prev[2 * gi + 1]) / d.dt;
-  if (p < d.N) {
-    if (s == 0) {
+  if (on && p < N) {
+    if (a == 0) {
       d.vel[2 * gi] = vx;
       d.vel[2 * gi + 1] = vy;
     }
-    if (d.enable_steric && s < 4) d.dep[d.c_cell[s * d.N + gi]] = 0.0f;
+    if (d.enable_steric) d.dep[d.c_cell[a * N + gi]] = 0.0f;
   }
   if (!d.enable_fluid) return;
-  const int K = d.K, K2 = K * K;
-  const float2 gp = ib_point(d, p, gi, x, y);
-  const float gx = gp.x, gy = gp.y;
-  if (s == 0) {
-    d.nvl[2 * p] = (vx * d.scale_x) * d.dt;
-    d.nvl[2 * p + 1] = (vy * d.scale_y) * d.dt;
-  }
-  const int half = (K - 1) / 2;
-  const float hw = (float)K / 2.0f;
-  const float sx = floorf(gx) - (float)half, sy = floorf(gy) - (float)half;
-  const int a = s / K, b = s - (s / K) * K;
-  const bool act = s < K2;
-  const float rx = fabsf((sx + (float)a) - gx) / hw;
-  const float ry = fabsf((sy + (float)b) - gy) / hw;
+  const int K = d.K;
+  const float2 g = ib_point(d, p, gi, x, y);
+  if (on && a == 0) d.nvl[p] = make_float2((vx * d.scale_x) * d.dt, (vy * d.scale_y) * d.dt);
+  const float half = (float)((K - 1) / 2), hw = (float)K / 2.0f;
+  const float bx = (floorf(g.x) - half) + (float)a, by = (floorf(g.y) - half) + (float)a;
+  const float rx = fabsf(bx - g.x) / hw, ry = fabsf(by - g.y) / hw;
   const float wxa = rx <= 2.0f ? 0.25f * (1.0f + cosf((MC_PI_F * rx) / 2.0f)) : 0.0f;
-  const float wyb = ry <= 2.0f ? 0.25f * (1.0f + cosf((MC_PI_F * ry) / 2.0f)) : 0.0f;
-  const float w = wxa * wyb;
-  float sum = 0.0f;
-  for (int q = 0; q < K2; ++q) sum = sum + __shfl_sync(gmask, w, q, 16);
-  const float den = sum + MC_EPSIL;
-  if (!act) return;
-  const int cx = imod_floor((int)(sx + (float)a), d.lW);
-  const int cy = imod_floor((int)(sy + (float)b), d.lH);
-  const int k = p * K2 + s;
-  d.ib_cell[k] = cy * d.lW + cx;
-  d.ib_w[k] = w / den;
-  const int tile = (cy / kBinTile) * d.lntile_x + cx / kBinTile;
-  const unsigned active = __activemask();
-  const unsigned group = __match_any_sync(active, tile);
-  const int leader = __ffs(group) - 1;
-  int base = 0;
-  if (lane == leader) {
-    base = atomicAdd(d.ib_tcount + tile, __popc(group));
-    if (base == 0) d.wl_ib[atomicAdd(d.wl_ctl, 1)] = make_int2(d.ridx, tile);
+  const float wya = ry <= 2.0f ? 0.25f * (1.0f + cosf((MC_PI_F * ry) / 2.0f)) : 0.0f;
+  const int cx = imod_floor((int)bx, d.lW), cya = imod_floor((int)by, d.lH) * d.lW;
+  const unsigned full = 0xffffffffu;
+  float w[4];
+  int cell[4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    w[b] = wxa * __shfl_sync(full, wya, b, 4);
+    cell[b] = __shfl_sync(full, cya, b, 4) + cx;
   }
-  base = __shfl_sync(group, base, leader);
-  const int pos = base + __popc(group & ((1u << lane) - 1u));
-  if (pos < d.ib_cap) {
-    d.ib_store[(size_t)tile * d.ib_cap + pos] = bin_entry(cy, cx, k);
-  } else {
-    d.ib_ovf[atomicAdd(d.ib_ctl, 1)] = k;
+  float sum = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float we = __shfl_sync(full, w[b], e, 4);
+      if (e < K && b < K) sum = sum + we;
+    }
+  const float den = sum + MC_EPSIL;
+  const bool mine = on && a < K;
+  const int k0 = (p * K + a) * K;
+  int pos[4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) pos[b] = mine && b < K ? atomicAdd(d.ib_cnt + cell[b], 1) : -1;
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if (mine && b < K) d.ib_w[k0 + b] = w[b] / den;
+  int fresh = 0;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) fresh += pos[b] == 0 ? 1 : 0;
+  int before = fresh;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(full, before, o);
+    if (lane >= o) before += v;
+  }
+  int base = 0;
+  if (lane == 31 && before > 0) base = atomicAdd(d.ib_ctl + 2, before);
+  base = __shfl_sync(full, base, 31) + before - fresh;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    if (pos[b] == 0) d.h_new[base++] = cell[b];
+    if (pos[b] >= 0 && pos[b] < d.ib_cap) {
+      d.ib_bucket[(size_t)cell[b] * d.ib_cap + pos[b]] = k0 + b;
+    } else if (pos[b] >= 0) {
+      const int e = atomicAdd(d.ib_ctl, 1);
+      d.ib_ovf[e] = k0 + b;
+      d.ib_ovf_next[e] = atomicExch(d.ib_ovf_head + cell[b], e);
+    }
   }
 }
 
@@ -527,8 +499,7 @@ __global__ void k_node(const RDesc* __restrict__ D, const int* __restrict__ off,
 void launch_predict(const Launch& L) { k_predict<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
 void launch_steric(const Launch& L) { k_steric<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
 void launch_stencil(const Launch& L) { k_stencil<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
-// 8 IB points (16 lanes each) per 128-thread CTA (measured 0.5% faster steps than 16 per 256)
-void launch_stencil16(const Launch& L) { k_stencil16<<<L.grid, 128, 0, L.s>>>(L.d, L.off, L.n); }
+void launch_stencil4(const Launch& L) { k_stencil4<<<L.grid, 128, 0, L.s>>>(L.d, L.off, L.n); }
 void launch_node(const Launch& L, const int* tdev, size_t smem, int bs) {
   k_node<<<L.grid, bs, smem, L.s>>>(L.d, L.off, L.n, tdev);
 }

@@ -48,7 +48,7 @@ constexpr int kNodeStepSmem = 220 * 1024;  // dynamic shared memory of a node-st
 // largest plan (IB points over all rollouts) whose body force is computed by the last IB round
 constexpr long long kFuseFinalizeMaxPoints = 65536;
 
-enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES16, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_COUNT };
+enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES4, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_COUNT };
 
 // CTAs of the steric filter kernels for one rollout: the radix-16 register kernels for
 // power-of-two sides >= 16, the mixed-radix Stockham kernels for the other FFT sides, or
@@ -90,14 +90,14 @@ struct HostRollout {
   Region r_cgW, r_cgH;
   int M = 0, ntx = 0, nty = 0, lbm_tx = 0, lbm_ty = 0, vec = 4, lbm_th = 4;
   int lH = 0, lW = 0;      // the fluid lattice (= dims.H, dims.W unless dims.fluid_H/W are set)
-  int lntx = 0, lnty = 0;  // bin tiles of the lattice (IB); ntx, nty: of the domain grid (CIC)
-  int ib_cap = 0, c_cap = 0;  // bin capacities (powers of two)
+  int ib_cap = 0, c_cap = 0;  // capacities of a cell's bucket (IB) and of a tile's bin (CIC), powers of two
   int logW = -1, logH = -1;   // log2 of power-of-two grid sides (-1: mixed radix path)
   int T_r = 0, P_r = 0, T_c = 0, P_c = 0;
   // workspace regions (offsets relative to the workspace base)
   Region r_h0, r_h1, r_dep, r_tmp, r_prev, r_pred, r_predw, r_nvl, r_delta;
-  Region r_ibcell, r_ibw, r_ibstore, r_ibstorew, r_ibtc, r_ibovf, r_ibctl, r_ibslot, r_hcell, r_hstart, r_hlen, r_srho, r_svx,
-      r_svy, r_sinv, r_sucx, r_sucy, r_sfx, r_sfy;
+  Region r_ibw, r_ibslot, r_ibcnt, r_ibbucket, r_ibovh, r_ibovn, r_ibovf, r_ibctl, r_run, r_hnew, r_hcell, r_hrun, r_smac, r_suc,
+      r_sf;
+  int run_rows = 0;
   Region r_ccell, r_cw, r_cstore, r_ctc, r_covf, r_cctl, r_chain, r_generic;
   Region r_pairs, r_bpairs, r_compn, r_compe, r_compb, r_epo, r_epi, r_neo, r_nei, r_edeg, r_ndeg;
   Region r_twW, r_twH, r_ptW, r_ptH, r_gW, r_gH, r_flags;
@@ -109,16 +109,18 @@ struct mc_plan {
   int n = 0;
   std::vector<HostRollout> R;
   size_t ws_bytes = 0;
-  Region r_desc, r_tdev, r_wl_ib, r_wl_cic, r_wl_ctl;
-  int tile_grid = 1;     // CTAs walking the tile lists (set at bind: as many as the GPU holds)
-  int tile_grid_c = 1;   // the same for the cloud-in-cell tiles (their shared sort capacity differs)
+  Region r_desc, r_tdev, r_wl_cic, r_wl_ctl;
+  int tile_grid_c = 1;   // CTAs walking the list of cloud-in-cell tiles (set at bind: as many as the GPU holds)
   long long n_tiles = 0;  // bin tiles of all rollouts
   int bin_threads = 128;  // threads per CTA of the tile kernel
   int lbm_vec = 2, lbm_rows = 4;  // tile of the direct dense-pass kernel: cells per lane, rows per CTA
   int lbm_stages = 0;       // > 0: the staged dense-pass kernel, with that many bands in flight per CTA
   int lbm_staged_ctas = 0;  // its persistent grid (set at bind: as many CTAs as the GPU holds)
-  int ib_capS = 0, c_capS = 0;  // largest bin capacity of the plan
-  int ib_smem = 0, c_smem = 0;  // contributions a tile may hold to be sorted in shared memory
+  int c_capS = 0;    // largest bin capacity of the plan
+  int dense_cap = 0;  // contributions per 16x16 tile that the densest rollout's stencils call for: the upper end
+                      // of the sort capacity (mc_plan_bin_sort_capacity)
+  int sort_cap = 0;  // mc_plan_set_bin_sort_capacity
+  int c_smem = 0;    // contributions a tile may hold to be sorted in shared memory
   Region r_off[K_COUNT];
   std::vector<int> off[K_COUNT];
   int grid[K_COUNT] = {};
@@ -464,8 +466,6 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.ntile_y = h.nty;
   d.lH = h.lH;
   d.lW = h.lW;
-  d.lntile_x = h.lntx;
-  d.lntile_y = h.lnty;
   d.lbm_tx = h.lbm_tx;
   d.lbm_ty = h.lbm_ty;
   d.lbm_tw = 32 * h.vec;
@@ -600,28 +600,25 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.prev = at<float>(b, h.r_prev);
   d.pred = at<float>(b, h.r_pred);
   d.predw = at<float>(b, h.r_predw);
-  d.nvl = at<float>(b, h.r_nvl);
-  d.delta = at<float>(b, h.r_delta);
+  d.nvl = at<float2>(b, h.r_nvl);
+  d.delta = at<float2>(b, h.r_delta);
   d.ib_cap = h.ib_cap;
-  d.ib_cell = at<int>(b, h.r_ibcell);
+  d.run_rows = h.run_rows;
   d.ib_w = at<float>(b, h.r_ibw);
-  d.ib_store = at<int>(b, h.r_ibstore);
-  d.ib_store_w = at<float>(b, h.r_ibstorew);
-  d.ib_tcount = at<int>(b, h.r_ibtc);
+  d.ib_slot = at<int>(b, h.r_ibslot);
+  d.ib_cnt = at<int>(b, h.r_ibcnt);
+  d.ib_bucket = at<int>(b, h.r_ibbucket);
+  d.ib_ovf_head = at<int>(b, h.r_ibovh);
+  d.ib_ovf_next = at<int>(b, h.r_ibovn);
   d.ib_ovf = at<int>(b, h.r_ibovf);
   d.ib_ctl = at<int>(b, h.r_ibctl);
-  d.ib_slot = at<int>(b, h.r_ibslot);
+  d.run = at<int2>(b, h.r_run);
+  d.h_new = at<int>(b, h.r_hnew);
   d.h_cell = at<int>(b, h.r_hcell);
-  d.h_start = at<int>(b, h.r_hstart);
-  d.h_len = at<int>(b, h.r_hlen);
-  d.s_rho = at<float>(b, h.r_srho);
-  d.s_vx = at<float>(b, h.r_svx);
-  d.s_vy = at<float>(b, h.r_svy);
-  d.s_inv = at<float>(b, h.r_sinv);
-  d.s_ucx = at<float>(b, h.r_sucx);
-  d.s_ucy = at<float>(b, h.r_sucy);
-  d.s_fx = at<float>(b, h.r_sfx);
-  d.s_fy = at<float>(b, h.r_sfy);
+  d.h_run = at<int2>(b, h.r_hrun);
+  d.s_mac = at<float4>(b, h.r_smac);
+  d.s_uc = at<float2>(b, h.r_suc);
+  d.s_f = at<float2>(b, h.r_sf);
   d.c_cap = h.c_cap;
   d.c_cell = at<int>(b, h.r_ccell);
   d.c_w = at<float>(b, h.r_cw);
@@ -630,7 +627,6 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.c_ovf = at<int>(b, h.r_covf);
   d.c_ctl = at<int>(b, h.r_cctl);
   d.ridx = i;
-  d.wl_ib = at<int2>(b, p->r_wl_ib);
   d.wl_cic = at<int2>(b, p->r_wl_cic);
   d.wl_ctl = at<int>(b, p->r_wl_ctl);
   d.nchain = (int)h.chain_info.size();
@@ -862,7 +858,7 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
     timed(p, 1, s, capture, [&] {
       mc::Launch l = L(p, K_TILES, s);
       l.grid = p->tile_grid_c;
-      mc::launch_bin_tiles(l, at<int2>(p->ws, p->r_wl_cic), at<int>(p->ws, p->r_wl_ctl) + 1, 1, 0, p->c_smem,
+      mc::launch_bin_tiles(l, at<int2>(p->ws, p->r_wl_cic), at<int>(p->ws, p->r_wl_ctl) + 1, p->c_smem,
                            p->bin_threads);
     });
     k += 1;
@@ -882,7 +878,7 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
   }
   if (p->grid[K_NODES]) {
     if (p->max_k <= 4)
-      timed(p, 15, s, capture, [&] { mc::launch_stencil16(L(p, K_NODES16, s)); });
+      timed(p, 15, s, capture, [&] { mc::launch_stencil4(L(p, K_NODES4, s)); });
     else
       timed(p, 15, s, capture, [&] { mc::launch_stencil(L(p, K_NODES, s)); });
     ++k;
@@ -893,13 +889,10 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
 int64_t enqueue_ib(mc_plan* p, int parity, cudaStream_t s, bool capture) {
   if (!p->any_fluid) return 0;
   int64_t k = 0;
-  timed(p, 6, s, capture, [&] {
-    mc::Launch l = L(p, K_TILES, s);
-    l.grid = p->tile_grid;
-    mc::launch_bin_tiles(l, at<int2>(p->ws, p->r_wl_ib), at<int>(p->ws, p->r_wl_ctl), 0, parity, p->ib_smem,
-                         p->bin_threads);
-  });
-  ++k;
+  if (p->grid[K_IB]) {
+    timed(p, 6, s, capture, [&] { mc::launch_ib_heads(L(p, K_IB, s), parity); });
+    ++k;
+  }
   if (p->ib_cluster > 0 && p->grid[K_NODES]) {
     timed(p, 19, s, capture, [&] {
       // a lone rollout needs all the threads a cluster can hold; a batch many small clusters
@@ -1488,10 +1481,8 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     if (vec_all != h.vec) vec_all = 1;
     h.ntx = div_up(D.W, mc::kBinTile);
     h.nty = div_up(D.H, mc::kBinTile);
-    h.lntx = div_up(h.lW, mc::kBinTile);
-    h.lnty = div_up(h.lH, mc::kBinTile);
     const size_t HW = (size_t)D.H * D.W, LHW = (size_t)h.lH * h.lW;
-    const size_t N = D.N, E = D.E, B = D.B, nt = (size_t)h.ntx * h.nty, lnt = (size_t)h.lntx * h.lnty;
+    const size_t N = D.N, E = D.E, B = D.B, nt = (size_t)h.ntx * h.nty;
     h.r_h0 = lay.take(9 * LHW * 4);
     h.r_h1 = lay.take(9 * LHW * 4);
     h.r_dep = lay.take(HW * 4);
@@ -1503,8 +1494,6 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     h.r_nvl = lay.take(2 * NIz * 4);
     h.r_delta = lay.take(2 * NIz * 4);
     const size_t Mz = (size_t)M;
-    h.r_ibcell = lay.take(Mz * 4);
-    h.r_ibw = lay.take(Mz * 4);
     // bin capacity: at least 3x the mean contributions per tile, a power of two
     auto cap_for = [&](long long contributions, int minimum, size_t tiles) {
       long long want = std::max<long long>(minimum, (3 * contributions + (long long)tiles - 1) / (long long)tiles);
@@ -1512,25 +1501,29 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
       while (c < want && c < mc::kMaxBinCap) c <<= 1;
       return c;
     };
-    h.ib_cap = cap_for((long long)Mz, mc::kIbCap, lnt);
+    p->dense_cap = std::max(p->dense_cap, cap_for((long long)Mz, 1024, (size_t)div_up(h.lW, mc::kBinTile) *
+                                                                           div_up(h.lH, mc::kBinTile)));
     h.c_cap = cap_for(4LL * (long long)N, mc::kCicCap, nt);
-    h.r_ibstore = lay.take((lnt * h.ib_cap + 2 * Mz) * 4);
-    h.r_ibstorew = lay.take((lnt * h.ib_cap + 2 * Mz) * 4);
-    h.r_ibtc = lay.take(lnt * 4);
+    // contributions of a cell that stay in its bucket: where two rods of unit spacing cross a cell
+    // collects about 8 with the 4-point kernel, more where rods crowd (mean over all cells above 2)
+    h.ib_cap = (double)M < 2.0 * (double)LHW ? 16 : 32;
+    h.run_rows = (int)std::min(Mz, LHW);
+    const size_t cells = M > 0 ? LHW : 0;
+    h.r_ibw = lay.take(Mz * 4);
+    h.r_ibslot = lay.take(Mz * 4);
+    h.r_ibcnt = lay.take(cells * 4);
+    h.r_ibbucket = lay.take(cells * h.ib_cap * 4);
+    h.r_ibovh = lay.take(cells * 4);
+    h.r_ibovn = lay.take(Mz * 4);
     h.r_ibovf = lay.take(Mz * 4);
     h.r_ibctl = lay.take(8 * 4);
-    h.r_ibslot = lay.take(Mz * 4);
+    h.r_run = lay.take(((size_t)h.run_rows * mc::kRunRow + 3 * Mz) * 8);
+    h.r_hnew = lay.take(Mz * 4);
     h.r_hcell = lay.take(Mz * 4);
-    h.r_hstart = lay.take(Mz * 4);
-    h.r_hlen = lay.take(Mz * 4);
-    h.r_srho = lay.take(Mz * 4);
-    h.r_svx = lay.take(Mz * 4);
-    h.r_svy = lay.take(Mz * 4);
-    h.r_sinv = lay.take(Mz * 4);
-    h.r_sucx = lay.take(Mz * 4);
-    h.r_sucy = lay.take(Mz * 4);
-    h.r_sfx = lay.take(Mz * 4);
-    h.r_sfy = lay.take(Mz * 4);
+    h.r_hrun = lay.take(Mz * 8);
+    h.r_smac = lay.take(Mz * 16);
+    h.r_suc = lay.take(Mz * 8);
+    h.r_sf = lay.take(Mz * 8);
     h.r_ccell = lay.take(4 * N * 4);
     h.r_cw = lay.take(4 * N * 4);
     h.r_cstore = lay.take((nt * h.c_cap + 8 * N) * 4);
@@ -1588,25 +1581,14 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   p->lbm_stages = 0;
   lbm_tiles(p);
   {
-    long long tiles = 0, ltiles = 0;
+    long long tiles = 0;
     for (auto& h : p->R) {
       tiles += (long long)h.ntx * h.nty;
-      ltiles += (long long)h.lntx * h.lnty;
-    }
-    p->r_wl_ib = lay.take((size_t)ltiles * sizeof(int2));
-    p->r_wl_cic = lay.take((size_t)tiles * sizeof(int2));
-    tiles = std::max(tiles, ltiles);
-    p->n_tiles = tiles;
-    for (auto& h : p->R) {
-      p->ib_capS = std::max(p->ib_capS, h.ib_cap);
       p->c_capS = std::max(p->c_capS, h.c_cap);
     }
-    // up to 2048 contributions per tile are sorted in shared memory (32 KB per CTA, and only
-    // when some rollout's bins are that deep: sparse plans keep their 1024-entry bins): the
-    // dense rollouts of a batch then rarely take the global-arena sort, while the residency
-    // of the launch's CTAs is not cut further (measured: 2.05 vs 2.10 ms per step of the
-    // 256-rollout batch against 1024, 2.23 ms at 4096)
-    p->ib_smem = std::min(p->ib_capS, kDefaultSortCap);
+    p->r_wl_cic = lay.take((size_t)tiles * sizeof(int2));
+    p->n_tiles = tiles;
+    p->sort_cap = std::min(p->dense_cap, kDefaultSortCap);
     p->c_smem = std::min(p->c_capS, kDefaultSortCap);
   }
   p->ws_bytes = lay.cur;
@@ -1622,7 +1604,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     // node-only kernels return for indices >= N
     const long long npts = (long long)h.dims.N * (c.synthetic_node_width > 0.0f ? 2 : 1);
     cnt[K_NODES] = div_up(npts, mc::kNodeThreads);
-    cnt[K_NODES16] = div_up(16LL * npts, 128);
+    cnt[K_NODES4] = div_up(4LL * npts, 128);
     // fused IB kernel: one thread per touched-cell candidate / 4 (scaled down at bind if
     // the plan's CTAs would not all be resident)
     cnt[K_IBCOOP] = c.enable_fluid ? std::max(1, div_up(h.M, 1024)) : 0;
@@ -1691,12 +1673,12 @@ mc_status mc_plan_set_bin_sort_capacity(mc_plan* p, int32_t entries) {
   if (entries != 0 && (entries < 256 || entries > 8192 || (entries & (entries - 1))))
     return fail(MC_ERR_INVALID, "entries must be 0 (default 2048) or a power of two in 256..8192");
   const int e = entries ? entries : kDefaultSortCap;
-  p->ib_smem = std::min(p->ib_capS, e);
+  p->sort_cap = std::min(p->dense_cap, e);
   p->c_smem = std::min(p->c_capS, e);
   return MC_OK;
 }
 
-int32_t mc_plan_bin_sort_capacity(const mc_plan* p) { return p ? p->ib_smem : 0; }
+int32_t mc_plan_bin_sort_capacity(const mc_plan* p) { return p ? p->sort_cap : 0; }
 
 mc_status mc_plan_set_fft_values_per_thread(mc_plan* p, int32_t values) {
   g_err.clear();
@@ -1867,12 +1849,10 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
   MC_CUDA(cudaMemsetAsync(p->ws + p->r_wl_ctl.off, 0, 4 * sizeof(int), s));
   {
     // the tile kernels take listed tiles from a cursor: launch as many CTAs as fit at once
-    int dev = 0, sms = 0, nib = 0, nc = 0;
+    int dev = 0, sms = 0, nc = 0;
     MC_CUDA(cudaGetDevice(&dev));
     MC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MC_CUDA(mc::tiles_blocks_per_sm(p->bin_threads, std::max(p->ib_smem, 1), &nib));
     MC_CUDA(mc::tiles_blocks_per_sm(p->bin_threads, std::max(p->c_smem, 1), &nc));
-    p->tile_grid = std::max(1, sms * nib);
     p->tile_grid_c = std::max(1, sms * nc);
     if (p->lbm_stages > 0) {
       int nl = 0;
