@@ -399,45 +399,64 @@ __global__ void __launch_bounds__(kHeadThreads) k_collide_heads(const RDesc* __r
   }
 }
 
-// h_i(y, x) = f_grid_i((y + cy) % H, (x + cx) % W): the inverse of the push streaming, so
-// that the first pulled step reads exactly fields.f_grid.
-__global__ void k_unstream(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
-  const int r = find_rollout(off, n, blockIdx.x);
-  const RDesc& d = D[r];
-  const int lb = blockIdx.x - off[r];
-  const size_t HW = (size_t)d.lH * d.lW;
+// out_i(y, x) = max(in_i((y + sign cy) % H, (x + sign cx) % W), EPSIL) for the 9 populations, by the
+// warps of a rollout's CTAs: a warp takes 128 cells of a row at a time, 4 per lane, whose 9 source
+// rows are found once; the 36 loads of a lane are in flight together.  Bound by HBM (72 B per cell).
+// Before, every cell divided its index and took 18 modulos: 25 M cells in 256 lattices 760 us in and
+// 618 us out, 317 and 310 us now (0.88 of the measured HBM rate); 1024^2 34 and 22 -> 11.7 us.
+template <int SIGN>
+__device__ __forceinline__ void shift_populations(const float* __restrict__ in, float* __restrict__ out, int H, int W,
+                                                  int warp, int warps, int lane) {
   const int ex[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
   const int ey[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
-  for (size_t idx = (size_t)lb * blockDim.x + threadIdx.x; idx < HW; idx += (size_t)(off[r + 1] - off[r]) * blockDim.x) {
-    int y = (int)(idx / d.lW), x = (int)(idx % d.lW);
+  const int HW = H * W, parts = (W + 127) / 128;
+  for (int u = warp; u < H * parts; u += warps) {
+    const int y = u / parts, x0 = (u - y * parts) * 128 + lane;
+    const int row = y * W, rowm = (y == 0 ? H - 1 : y - 1) * W, rowp = (y == H - 1 ? 0 : y + 1) * W;
+    float v[4][9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      int ys = imod_floor(y + ey[i], d.lH), xs = imod_floor(x + ex[i], d.lW);
-      d.h[0][i * HW + idx] = max_prop(d.f_grid[i * HW + (size_t)ys * d.lW + xs], MC_EPSIL);
+    for (int c = 0; c < 4; ++c) {
+      const int x = x0 + 32 * c;
+      if (x < W) {
+        const int xm = x == 0 ? W - 1 : x - 1, xp = x == W - 1 ? 0 : x + 1;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          const int dy = SIGN * ey[i], dx = SIGN * ex[i];
+          v[c][i] = in[i * HW + (dy == 0 ? row : dy > 0 ? rowp : rowm) + (dx == 0 ? x : dx > 0 ? xp : xm)];
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int x = x0 + 32 * c;
+      if (x < W) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) out[i * HW + row + x] = max_prop(v[c][i], MC_EPSIL);
+      }
     }
   }
 }
 
-// fields.f_grid_i(y, x) = max(h_i((y - cy) % H, (x - cx) % W), EPSIL): the push streaming
-// of the reference (fluid.py:352-357) applied to the final post-collision state.
-__global__ void k_stream_out(const RDesc* __restrict__ D, const int* __restrict__ off, int n, int parity,
-                             float* __restrict__ dst) {
+// h_i(y, x) = f_grid_i((y + cy) % H, (x + cx) % W): the inverse of the push streaming, so that the
+// first pulled step reads exactly fields.f_grid.
+__global__ void __launch_bounds__(256) k_unstream(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int lb = blockIdx.x - off[r];
-  const size_t HW = (size_t)d.lH * d.lW;
-  const int ex[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
-  const int ey[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
-  const float* h = d.h[parity];
-  float* out = dst ? dst : d.f_grid;  // dst: a snapshot buffer of a one-rollout plan
-  for (size_t idx = (size_t)lb * blockDim.x + threadIdx.x; idx < HW; idx += (size_t)(off[r + 1] - off[r]) * blockDim.x) {
-    int y = (int)(idx / d.lW), x = (int)(idx % d.lW);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      int ys = imod_floor(y - ey[i], d.lH), xs = imod_floor(x - ex[i], d.lW);
-      out[i * HW + idx] = max_prop(h[i * HW + (size_t)ys * d.lW + xs], MC_EPSIL);
-    }
-  }
+  if (!d.f_grid) return;
+  shift_populations<1>(d.f_grid, d.h[0], d.lH, d.lW, (blockIdx.x - off[r]) * 8 + (threadIdx.x >> 5),
+                       (off[r + 1] - off[r]) * 8, threadIdx.x & 31);
+}
+
+// fields.f_grid_i(y, x) = max(h_i((y - cy) % H, (x - cx) % W), EPSIL): the push streaming
+// of the reference (fluid.py:352-357) applied to the final post-collision state.
+__global__ void __launch_bounds__(256) k_stream_out(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
+                                                    int parity, float* __restrict__ dst) {
+  const int r = find_rollout(off, n, blockIdx.x);
+  const RDesc& d = D[r];
+  if (!dst && !d.f_grid) return;
+  // dst: a snapshot buffer of a one-rollout plan
+  shift_populations<-1>(d.h[parity], dst ? dst : d.f_grid, d.lH, d.lW, (blockIdx.x - off[r]) * 8 + (threadIdx.x >> 5),
+                        (off[r + 1] - off[r]) * 8, threadIdx.x & 31);
 }
 
 // Workspace initialisation: deposit grid = 0, counters = 0.

@@ -48,7 +48,7 @@ constexpr int kNodeStepSmem = 220 * 1024;  // dynamic shared memory of a node-st
 // largest plan (IB points over all rollouts) whose body force is computed by the last IB round
 constexpr long long kFuseFinalizeMaxPoints = 65536;
 
-enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES4, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_COUNT };
+enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES4, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_SHIFT, K_COUNT };
 
 // CTAs of the steric filter kernels for one rollout: the radix-16 register kernels for
 // power-of-two sides >= 16, the mixed-radix Stockham kernels for the other FFT sides, or
@@ -1298,7 +1298,7 @@ cudaError_t stage_uploads(const Upload* items, int count, cudaStream_t s) {
 mc_status rollout_snapshot_f(mc_plan* p, float* dst, cudaStream_t s) {
   if (!p || !p->active || p->n != 1 || !dst) return fail(MC_ERR_INVALID, "snapshot outside a one-rollout rollout");
   if (p->pending_next) return fail(MC_ERR_INVALID, "snapshot while the next step's pipeline is in flight");
-  if (p->any_fluid) launch_stream_out(L(p, K_CELLS, s), p->step & 1, dst);
+  if (p->any_fluid) launch_stream_out(L(p, K_SHIFT, s), p->step & 1, dst);
   MC_CUDA(cudaGetLastError());
   return MC_OK;
 }
@@ -1614,6 +1614,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     cnt[K_TILES] = h.ntx * h.nty;
     cnt[K_LBM] = c.enable_fluid ? h.lbm_tx * h.lbm_ty : 0;
     cnt[K_CELLS] = std::min(div_up(HW, 256), 1024);
+    cnt[K_SHIFT] = std::min(div_up((long long)h.lH * div_up(h.lW, 128), 8), 2048);  // 8 warps, 128 cells each
     // every length goes through the multi-transform kernels (the one-transform-per-CTA
     // kernels serve the allocation-free entry point)
     cnt[K_FFTR] = 0;
@@ -1923,7 +1924,7 @@ mc_status mc_rollout_begin(mc_plan* p, const mc_state* states, const mc_actuatio
   p->active = true;
   p->last_launches = 0;
   if (p->any_fluid) {
-    mc::launch_unstream(L(p, K_CELLS, s));
+    mc::launch_unstream(L(p, K_SHIFT, s));
     p->last_launches += 1;
   }
   p->pending_next = false;  // the first advance launches step 0's pipeline
@@ -1958,7 +1959,7 @@ mc_status mc_rollout_end(mc_plan* p, void* stream) {
     return fail(MC_ERR_INVALID, "the last mc_rollout_advance() before mc_rollout_end() must pass last != 0");
   }
   if (p->any_fluid) {
-    mc::launch_stream_out(L(p, K_CELLS, (cudaStream_t)stream), p->step & 1);
+    mc::launch_stream_out(L(p, K_SHIFT, (cudaStream_t)stream), p->step & 1);
     p->last_launches += 1;
   }
   p->active = false;
