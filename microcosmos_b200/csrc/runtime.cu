@@ -133,6 +133,9 @@ struct mc_plan {
   int max_k = 0;  // largest IB kernel size of the plan
   int fft_e = 4;  // values per thread of the register-radix FFT kernels
   bool fuse_finalize = false;  // body force computed by the last IB spread round
+  bool filter_split = true;  // every rollout's two sides belong to one family of filter kernels
+  cudaStream_t filter_stream = nullptr;
+  cudaEvent_t ev_ffork = nullptr, ev_fjoin = nullptr;
   int fft_tv = 4096;  // values per CTA of the register-radix column pass (4096 or 2048)
   bool use_coop = false, coop_cap_checked = false;
   bool fused_ib = false;  // mc_plan_set_fused_ib (separate launches measured faster)
@@ -261,26 +264,36 @@ void fft_tables_compute(int N, double sigma, std::vector<float2>& tw, std::vecto
   }
 }
 
-// The twiddles of the register-radix Stockham passes (steric.cu, pass_reg) for a
-// power-of-two length N and E values per thread, laid out per pass: the pass with Ns
-// (the product of the earlier radices) and radix R keeps, for each k < Ns, the R - 1
-// factors tw[(m k) << (log N - log Ns - log R)], m = 1..R-1, at (Ns - 1) + k (R - 1) + m - 1
-// (the passes' tables fill [0, N - 1) exactly).  The same values as the root table, so
-// the transform's results are unchanged; a thread reads its factors from one base address.
+// The twiddles of the register-radix Stockham passes (steric.cu, pass_load) of a length N with E
+// values per thread (N a power of two), or of a length 3 * 2^a, laid out per pass: the pass with Ns
+// (the product of the earlier radices) and radix R keeps, for each m = 1..R-1, its factors
+// tw[m k N / (Ns R)] of k < Ns at (Ns - 1) + (m - 1) Ns + k (the passes' tables fill [0, N - 1)
+// exactly).  The same values as the root table; neighbouring threads, which hold neighbouring k,
+// read neighbouring factors.
 void pass_twiddles(const std::vector<float2>& tw, int E, std::vector<float2>& pt) {
   const int N = (int)tw.size();
   pt.assign(N, make_float2(0.f, 0.f));
-  if (N < 2 || (N & (N - 1))) return;
-  int logN = 0;
-  while ((1 << logN) < N) ++logN;
-  const int LE = E == 4 ? 2 : E == 8 ? 3 : 4;
-  int logNs = 0;
-  while (logNs < logN) {
-    const int LR = logNs + LE <= logN ? LE : logN - logNs;
-    const int R = 1 << LR, Ns = 1 << logNs, tsh = logN - logNs - LR;
-    for (int k = 0; k < Ns; ++k)
-      for (int m = 1; m < R; ++m) pt[(Ns - 1) + k * (R - 1) + (m - 1)] = tw[(m * k) << tsh];
-    logNs += LR;
+  if (N < 2) return;
+  std::vector<int> radices;
+  int Ns = 1;
+  if (three_pow2(N)) {
+    const int P = N / 3;
+    while (Ns * 4 <= P) {
+      radices.push_back(4);
+      Ns *= 4;
+    }
+    if (Ns < P) radices.push_back(2);
+    radices.push_back(3);
+  } else if ((N & (N - 1)) == 0) {
+    for (; Ns * E <= N; Ns *= E) radices.push_back(E);
+    if (Ns < N) radices.push_back(N / Ns);
+  }
+  Ns = 1;
+  for (int R : radices) {
+    const int step = N / (Ns * R);
+    for (int m = 1; m < R; ++m)
+      for (int k = 0; k < Ns; ++k) pt[(Ns - 1) + (m - 1) * Ns + k] = tw[m * k * step];
+    Ns *= R;
   }
 }
 
@@ -777,8 +790,10 @@ void recount_steric(mc_plan* p);
 void recount_steric(mc_plan* p) {
   p->fft_tv = default_fft_cols_tv(p->R, p->fft_e);
   for (int k : {K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12}) p->off[k][0] = 0;
+  p->filter_split = true;
   for (int i = 0; i < p->n; ++i) {
     const StericCtas c = steric_ctas(p->R[i], p->fft_e, p->fft_tv);
+    if ((c.fr16 > 0) != (c.fc16 > 0)) p->filter_split = false;
     p->off[K_FFTR2][i + 1] = p->off[K_FFTR2][i] + c.fftr2;
     p->off[K_FFTC2][i + 1] = p->off[K_FFTC2][i] + c.fftc2;
     p->off[K_SCONV][i + 1] = p->off[K_SCONV][i] + c.sconv;
@@ -790,45 +805,64 @@ void recount_steric(mc_plan* p) {
   for (int k : {K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12}) p->grid[k] = p->off[k][p->n];
 }
 
-// The steric filter of the deposit: row and column passes.
-int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool capture) {
+// The steric filter of the deposit: row and column passes, by family of side lengths (powers of two;
+// 3 * 2^a; others; the direct form).  When every rollout's sides are of one family, the families
+// share nothing and run beside each other: each alone leaves SMs idle (64 uneven rollouts: rows and
+// columns of two families 73 us in turn, 59 us beside each other).
+int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool capture, mc_status* err) {
   int64_t k = 0;
-  if (p->grid[K_FR16]) {
-    timed(p, 2, s, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, s), p->fft_e); });
-    ++k;
+  auto regular = [&](cudaStream_t q) {
+    if (p->grid[K_FR16]) {
+      timed(p, 2, q, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, q), p->fft_e); });
+      ++k;
+    }
+    if (p->grid[K_FC16] && p->filter_split) {
+      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q), p->fft_e, p->fft_tv); });
+      ++k;
+    }
+  };
+  auto others = [&](cudaStream_t q) {
+    if (p->grid[K_FR12]) {
+      timed(p, 2, q, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, q)); });
+      ++k;
+    }
+    if (p->grid[K_FFTR2]) {
+      timed(p, 2, q, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, q), p->fftr2_smem); });
+      ++k;
+    }
+    if (p->grid[K_FC16] && !p->filter_split) {
+      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q), p->fft_e, p->fft_tv); });
+      ++k;
+    }
+    if (p->grid[K_FC12]) {
+      timed(p, 3, q, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, q)); });
+      ++k;
+    }
+    if (p->grid[K_FFTC2]) {
+      timed(p, 3, q, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, q), p->fftc2_smem); });
+      ++k;
+    }
+    if (p->grid[K_SCONV]) {
+      timed(p, 17, q, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, q), p->sconv_smem); });
+      ++k;
+    }
+  };
+  const bool two = p->filter_split && p->grid[K_FR16] &&
+                   (p->grid[K_FR12] || p->grid[K_FFTR2] || p->grid[K_SCONV]) && !p->profiling;
+  if (!two) {
+    regular(s);
+    others(s);
+    return k;
   }
-  if (p->grid[K_FR12]) {
-    timed(p, 2, s, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, s)); });
-    ++k;
-  }
-  if (p->grid[K_FFTR2]) {
-    timed(p, 2, s, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, s), p->fftr2_smem); });
-    ++k;
-  }
-  if (p->grid[K_FFTR]) {
-    timed(p, 2, s, capture, [&] { mc::launch_fft_rows(L(p, K_FFTR, s), p->fftr_smem); });
-    ++k;
-  }
-  if (p->grid[K_FC16]) {
-    timed(p, 3, s, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, s), p->fft_e, p->fft_tv); });
-    ++k;
-  }
-  if (p->grid[K_FC12]) {
-    timed(p, 3, s, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, s)); });
-    ++k;
-  }
-  if (p->grid[K_FFTC2]) {
-    timed(p, 3, s, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, s), p->fftc2_smem); });
-    ++k;
-  }
-  if (p->grid[K_FFTC]) {
-    timed(p, 3, s, capture, [&] { mc::launch_fft_cols(L(p, K_FFTC, s), p->fftc_smem); });
-    ++k;
-  }
-  if (p->grid[K_SCONV]) {
-    timed(p, 17, s, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, s), p->sconv_smem); });
-    ++k;
-  }
+  auto fork = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
+    cudaError_t e = cudaEventRecord(ev, from);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
+    if (e != cudaSuccess && *err == MC_OK) *err = cuda_fail(e, "fork to the filter stream");
+  };
+  fork(p->ev_ffork, s, p->filter_stream);
+  others(p->filter_stream);
+  regular(s);
+  fork(p->ev_fjoin, p->filter_stream, s);
   return k;
 }
 
@@ -843,10 +877,10 @@ int64_t enqueue_node_step(mc_plan* p, int parity, int main, int next, cudaStream
   return 1;
 }
 
-int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
+int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture, mc_status* err) {
   if (is_compact(p)) {
     if (!p->any_steric) return 0;
-    return enqueue_node_step(p, 0, 0, 1, s, capture) + enqueue_filter(p, s, capture);
+    return enqueue_node_step(p, 0, 0, 1, s, capture) + enqueue_filter(p, s, capture, err);
   }
   int* tdev = at<int>(p->ws, p->r_tdev);
   int64_t k = 0;
@@ -862,7 +896,7 @@ int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture) {
                            p->bin_threads);
     });
     k += 1;
-    k += enqueue_filter(p, s, capture);
+    k += enqueue_filter(p, s, capture, err);
   }
   if (p->grid[K_NODES]) {
     timed(p, 14, s, capture, [&] { mc::launch_steric(L(p, K_NODES, s)); });
@@ -966,20 +1000,20 @@ int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool f
   int64_t k = 0;
   if (rec_fields || p->profiling) {
     // sequential: field recording needs this order; profiling times kernels one at a time
-    if (first) k += enqueue_pipeline(p, s, capture);
+    if (first) k += enqueue_pipeline(p, s, capture, err);
     k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
     k += enqueue_lbm(p, parity, write_u, s, capture);
     k += enqueue_heads(p, parity, write_u, s, capture);
     if (!compact) {
       k += enqueue_tail(p, rec_fields, s, capture);
-      if (has_next) k += enqueue_pipeline(p, s, capture);
+      if (has_next) k += enqueue_pipeline(p, s, capture, err);
       return k;
     }
     if (rec_fields) {
       timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), at<int>(p->ws, p->r_tdev), 1); });
       ++k;
     }
-    if (has_next && p->any_steric) k += enqueue_filter(p, s, capture);
+    if (has_next && p->any_steric) k += enqueue_filter(p, s, capture, err);
     return k;
   }
   auto fork = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to, const char* what) {
@@ -992,15 +1026,15 @@ int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool f
     fork(p->ev_lfork, s, s3, "fork to the dense-pass stream");
     k += enqueue_lbm(p, parity, write_u, s3, capture);
   }
-  if (first) k += enqueue_pipeline(p, s, capture);
+  if (first) k += enqueue_pipeline(p, s, capture, err);
   const bool side = !compact || (has_next && p->any_steric);
   k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
   if (side) fork(p->ev_fork, s, s2, "fork to the side stream");
   if (compact) {
-    if (side) k += enqueue_filter(p, s2, capture);
+    if (side) k += enqueue_filter(p, s2, capture, err);
   } else {
     k += enqueue_tail(p, 0, s2, capture);
-    if (has_next) k += enqueue_pipeline(p, s2, capture);
+    if (has_next) k += enqueue_pipeline(p, s2, capture, err);
   }
   if (p->any_fluid) {
     fork(p->ev_ljoin, s3, s, "join from the dense-pass stream");
@@ -1773,6 +1807,9 @@ void mc_plan_destroy(mc_plan* p) {
   if (p->side_stream) cudaStreamDestroy(p->side_stream);
   if (p->ev_fork) cudaEventDestroy(p->ev_fork);
   if (p->ev_join) cudaEventDestroy(p->ev_join);
+  if (p->filter_stream) cudaStreamDestroy(p->filter_stream);
+  if (p->ev_ffork) cudaEventDestroy(p->ev_ffork);
+  if (p->ev_fjoin) cudaEventDestroy(p->ev_fjoin);
   if (p->lbm_stream) cudaStreamDestroy(p->lbm_stream);
   if (p->ev_lfork) cudaEventDestroy(p->ev_lfork);
   if (p->ev_ljoin) cudaEventDestroy(p->ev_ljoin);
@@ -1878,6 +1915,9 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
     p->coop_possible = coop && p->grid[K_IBCOOP] > 0 && p->grid[K_IBCOOP] <= per_sm * sms;
     p->use_coop = p->fused_ib && p->coop_possible;
   }
+  if (!p->filter_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->filter_stream, cudaStreamNonBlocking));
+  if (!p->ev_ffork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_ffork, cudaEventDisableTiming));
+  if (!p->ev_fjoin) MC_CUDA(cudaEventCreateWithFlags(&p->ev_fjoin, cudaEventDisableTiming));
   if (!p->ev_fork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
   if (!p->ev_join) MC_CUDA(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
   if (!p->ev_lfork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_lfork, cudaEventDisableTiming));

@@ -494,16 +494,22 @@ void launch_steric_conv(const Launch& L, size_t smem) {
 
 
 // ---------------------------------------------------------------- register-radix path
-// Power-of-two lengths: G = N / E threads per transform, each holding E = 4, 8 or 16
+// Power-of-two lengths: L = N / E threads per transform, each holding E = 4, 8 or 16
 // complex values in registers.  A Stockham pass of radix R (E, or a smaller power of two
-// for the last pass) loads R-strided operands from shared memory, twiddles them, runs an
-// R-point DFT in registers and stores the autosorted result back in place: a length-1024
-// transform takes three shared-memory passes with E = 16 (16, 16, 4), five with E = 4.
-// Fewer values per thread give more threads for small problems; more give fewer
-// instructions per value for large batches.  Shared-memory addresses are padded by one
-// element every 16 (a -> a + a / 16) so the strided stores of the first pass spread over
-// the banks.  Twiddles are the float64-derived roots, read from a table laid out per pass
-// (the host's pass_twiddles) so that a butterfly's R - 1 factors sit at one base address.
+// for the last pass) takes R-strided operands, twiddles them, runs an R-point DFT in
+// registers and stores the autosorted result: a length-1024 transform takes three passes with
+// E = 16 (16, 16, 4), five with E = 4.  Fewer values per thread give more threads for small
+// problems; more give fewer instructions per value for large batches.
+// What bounds it is the latency of the exchanges between passes, so there are as few as the passes
+// allow: the first pass reads global memory, the spectrum is applied where the forward transform
+// ends, the last pass writes global memory, and a transform held by one warp needs no CTA barrier.
+// Shared-memory addresses are padded by one element every 16 (a -> a + a / 16) so the strided stores
+// of the first pass spread over the banks.  Twiddles are the float64-derived roots, in a table laid
+// out per pass (the host's pass_twiddles) whose neighbours are read by neighbouring threads; the
+// R - 1 factors of a butterfly side by side instead put every lane's read on a line of its own.
+// Measured (rows + columns per step; before: staging passes at both ends and around the spectrum):
+// 128^2 13.0 -> 7.5 us, 1024^2 26.3 -> 23.4 us, 2048^2 79 -> 66 us, 64 uneven rollouts 114 -> 73 us,
+// 256 uneven rollouts 453 -> 291 us.
 
 __device__ __forceinline__ int pad16(int a) { return a + (a >> 4); }
 
@@ -599,259 +605,301 @@ __device__ __forceinline__ constexpr int dft_slot(int k) {
   return k;
 }
 
-// One in-place Stockham pass of radix R over a padded buffer of N = 2^logN values,
-// G = N / E threads (local index lt) holding E values each, Ns = 2^logNs.
-// `pt`: this length's per-pass twiddle table (pass_twiddles on the host): the R - 1 factors of
-// butterfly k of the pass with Ns = 2^logNs start at pt[(Ns - 1) + k (R - 1)].
-template <int E, int R>
-__device__ __forceinline__ void pass_reg(float2* buf, int logN, int logNs, int lt, const float2* __restrict__ pt) {
-  constexpr int LR = R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 4;
-  constexpr int LE = E == 4 ? 2 : E == 8 ? 3 : 4;
-  constexpr int C = E / R;  // butterflies per thread
-  const int G = 1 << (logN - LE);
-  const int S = 1 << (logN - LR);  // butterflies in the pass
-  const int Ns = 1 << logNs;
-  float2 v[E];
+// A Stockham pass of radix R over transforms of N = L * E values, L threads each with E values
+// (E / R butterflies), Ns the product of the earlier radices.  Output index of butterfly j:
+// (j - k) R + k + m Ns with k = j mod Ns.
+//   In::load(i):     value i of the transform, from global memory (the first pass) or shared memory;
+//   Out::store(i,v): value i, to shared memory, scaled by the spectrum and conjugated (the last
+//                    pass of the forward transform), or to global memory (of the inverse one).
+// The pass's twiddles (pt, per-pass table of the host's pass_twiddles): factor m of butterfly k at
+// pt[(Ns - 1) + (m - 1) Ns + k], so that neighbouring threads read neighbouring factors.
+template <int E, int R, bool TWIDDLE, typename In>
+__device__ __forceinline__ void pass_load(float2 (&v)[E], const In& in, int L, int S, int Ns, int lt,
+                                          const float2* __restrict__ pt) {
+  constexpr int C = E / R;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
-    const int j = lt + c * G;
+    const int j = lt + c * L;
     const int k = j & (Ns - 1);
-    const float2* __restrict__ tk = pt + (Ns - 1) + k * (R - 1) - 1;  // tk[m], m = 1..R-1
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      float2 a = buf[pad16(j + m * S)];
-      if (m > 0 && k > 0) a = cmul(a, __ldg(tk + m));
+      float2 a = in.load(j + m * S);
+      if (TWIDDLE && m > 0 && k > 0) a = cmul(a, __ldg(pt + (Ns - 1) + (m - 1) * Ns + k));
       v[c * R + m] = a;
     }
     dft_reg<R>(v + c * R);
   }
-  (void)S;
-  __syncthreads();
+}
+template <int E, int R, typename Out>
+__device__ __forceinline__ void pass_store(const float2 (&v)[E], const Out& out, int L, int Ns, int lt) {
+  constexpr int C = E / R;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
-    const int j = lt + c * G;
+    const int j = lt + c * L;
     const int k = j & (Ns - 1);
-    const int dst = ((j - k) << LR) + k;
+    const int dst = (j - k) * R + k;
 #pragma unroll
-    for (int m = 0; m < R; ++m) buf[pad16(dst + m * Ns)] = v[c * R + dft_slot<R>(m)];
-  }
-  __syncthreads();
-}
-
-// Forward transform in place (natural order in and out), N = 2^logN >= E.
-template <int E>
-__device__ __forceinline__ void fft_reg(float2* buf, int logN, int lt, const float2* __restrict__ pt) {
-  constexpr int LE = E == 4 ? 2 : E == 8 ? 3 : 4;
-  int logNs = 0;
-  while (logNs + LE <= logN) {
-    pass_reg<E, E>(buf, logN, logNs, lt, pt);
-    logNs += LE;
-  }
-  const int rem = logN - logNs;
-  if (rem == 1) pass_reg<E, 2>(buf, logN, logNs, lt, pt);
-  if constexpr (E >= 8) {
-    if (rem == 2) pass_reg<E, 4>(buf, logN, logNs, lt, pt);
-  }
-  if constexpr (E >= 16) {
-    if (rem == 3) pass_reg<E, 8>(buf, logN, logNs, lt, pt);
+    for (int m = 0; m < R; ++m) out.store(dst + m * Ns, v[c * R + dft_slot<R>(m)]);
   }
 }
 
-// x -> IFFT(G * FFT(x)) with 1/N folded into g: conj(FFT(conj(G * FFT(x)))).
-template <int E>
-__device__ __forceinline__ void filter_reg(float2* buf, int logN, int lt, const float2* __restrict__ pt,
-                                           const float* __restrict__ g) {
-  const int N = 1 << logN, G = N / E;
-  fft_reg<E>(buf, logN, lt, pt);
-  for (int i = lt; i < N; i += G) {
+struct SharedValues {  // a transform's buffer, padded by one value every 16
+  float2* buf;
+  __device__ __forceinline__ float2 load(int i) const { return buf[pad16(i)]; }
+  __device__ __forceinline__ void store(int i, float2 v) const { buf[pad16(i)] = v; }
+};
+struct Filtered {  // conj(G X) with 1/N folded into G
+  float2* buf;
+  const float* __restrict__ g;
+  __device__ __forceinline__ void store(int i, float2 v) const {
     const float gk = __ldg(g + i);
-    const float2 v = buf[pad16(i)];
     buf[pad16(i)] = make_float2(v.x * gk, -(v.y * gk));
   }
-  __syncthreads();
-  fft_reg<E>(buf, logN, lt, pt);
+};
+// Two real rows y0, y0 + 1 (columns x0, x0 + 1) as one complex sequence; the second may not exist.
+struct RowPair {
+  const float* __restrict__ r0;
+  const float* __restrict__ r1;
+  float* o0;
+  float* o1;
+  bool on0, on1;
+  __device__ __forceinline__ float2 load(int x) const { return make_float2(on0 ? r0[x] : 0.0f, on1 ? r1[x] : 0.0f); }
+  __device__ __forceinline__ void store(int x, float2 v) const {
+    if (on0) o0[x] = v.x;
+    if (on1) o1[x] = -v.y;
+  }
+};
+struct ColumnPair {
+  const float* __restrict__ in;
+  float* out;
+  int W;
+  bool on0, on1;
+  bool even;  // rows of even length: a pair of columns is one 8-byte load (the workspace is aligned)
+  __device__ __forceinline__ float2 load(int y) const {
+    const float* p = in + y * W;
+    if (even) return on0 ? *reinterpret_cast<const float2*>(p) : make_float2(0.0f, 0.0f);
+    return make_float2(on0 ? p[0] : 0.0f, on1 ? p[1] : 0.0f);
+  }
+  __device__ __forceinline__ void store(int y, float2 v) const {
+    float* p = out + y * W;
+    if (on0) p[0] = v.x;
+    if (on1) p[1] = -v.y;
+  }
+};
+
+// Barrier among the threads of a transform: those of a warp when it is held by one, else the CTA.
+__device__ __forceinline__ void fft_sync(bool in_warp) {
+  if (in_warp)
+    __syncwarp();
+  else
+    __syncthreads();
 }
 
-// Row pass: 256 / G row pairs per CTA (one packed transform each), G = W / E.
+// A middle pass, in place.
+template <int E, int R>
+__device__ __forceinline__ void pass_middle(float2* buf, int L, int S, int Ns, int lt, const float2* __restrict__ pt,
+                                            bool in_warp) {
+  float2 v[E];
+  const SharedValues sv{buf};
+  pass_load<E, R, true>(v, sv, L, S, Ns, lt, pt);
+  fft_sync(in_warp);
+  pass_store<E, R>(v, sv, L, Ns, lt);
+  fft_sync(in_warp);
+}
+
+// x -> IFFT(G FFT(x)) of one packed transform as conj(FFT(conj(G FFT(x)))): values come from and go
+// to global memory in the first and last pass, the spectrum is applied where the forward transform
+// ends, so a transform of p passes takes 2 p - 1 exchanges through shared memory.
+// `ends`: this thread's place (t0, l0) in the global accesses (transform, index), which the column
+// pass arranges so that a row's neighbouring columns lie on neighbouring threads; (buf, lt): its
+// place in the passes between, where a transform's threads are neighbours.  RL: radix of the last
+// pass.  radix(p): the radix of pass p < passes - 1 is R.
+template <int E, int R, int RL, typename Pair>
+__device__ __forceinline__ void filter_passes(const Pair& pair, float2* buf_end, int l_end, float2* buf, int lt, int L,
+                                              int full, int Ns_last, bool in_warp, bool same,
+                                              const float2* __restrict__ pt, const float* __restrict__ g) {
+  // `full` passes of radix R, then one of radix RL with Ns_last (RL = 1: none)
+  const int N = L * E;
+  const int S = N / R;
+  // the barrier between a pass on the ends' mapping and one on the inner mapping
+  const bool edge_warp = in_warp && same;
+  float2 v[E];
+  if (RL == 1 && full == 1) {
+    pass_load<E, R, false>(v, pair, L, S, 1, l_end, pt);
+    pass_store<E, R>(v, Filtered{buf_end, g}, L, 1, l_end);
+    fft_sync(edge_warp);
+    pass_load<E, R, false>(v, SharedValues{buf_end}, L, S, 1, l_end, pt);
+    pass_store<E, R>(v, pair, L, 1, l_end);
+    return;
+  }
+  pass_load<E, R, false>(v, pair, L, S, 1, l_end, pt);
+  pass_store<E, R>(v, SharedValues{buf_end}, L, 1, l_end);
+  fft_sync(edge_warp);
+  int Ns = R;
+  const int mid = RL == 1 ? full - 1 : full;
+  for (int p = 1; p < mid; ++p, Ns *= R) pass_middle<E, R>(buf, L, S, Ns, lt, pt, in_warp);
+  if constexpr (RL == 1) {
+    pass_load<E, R, true>(v, SharedValues{buf}, L, S, Ns, lt, pt);
+    fft_sync(in_warp);
+    pass_store<E, R>(v, Filtered{buf, g}, L, Ns, lt);
+  } else {
+    pass_load<E, RL, true>(v, SharedValues{buf}, L, N / RL, Ns_last, lt, pt);
+    fft_sync(in_warp);
+    pass_store<E, RL>(v, Filtered{buf, g}, L, Ns_last, lt);
+  }
+  fft_sync(in_warp);
+  {
+    pass_load<E, R, false>(v, SharedValues{buf}, L, S, 1, lt, pt);
+    fft_sync(in_warp);
+    pass_store<E, R>(v, SharedValues{buf}, L, 1, lt);
+  }
+  Ns = R;
+  for (int p = 1; p < mid; ++p, Ns *= R) {
+    fft_sync(in_warp);
+    pass_load<E, R, true>(v, SharedValues{buf}, L, S, Ns, lt, pt);
+    fft_sync(in_warp);
+    pass_store<E, R>(v, SharedValues{buf}, L, Ns, lt);
+  }
+  fft_sync(edge_warp);
+  if constexpr (RL == 1) {
+    pass_load<E, R, true>(v, SharedValues{buf_end}, L, S, Ns, l_end, pt);
+    pass_store<E, R>(v, pair, L, Ns, l_end);
+  } else {
+    pass_load<E, RL, true>(v, SharedValues{buf_end}, L, N / RL, Ns_last, l_end, pt);
+    pass_store<E, RL>(v, pair, L, Ns_last, l_end);
+  }
+}
+
+// Power-of-two lengths N = 2^logN >= E: passes of radix E, then the remaining factor.
+template <int E, typename Pair>
+__device__ __forceinline__ void filter_reg(const Pair& pair, float2* buf_end, int l_end, float2* buf, int lt, int logN,
+                                           bool in_warp, bool same, const float2* __restrict__ pt,
+                                           const float* __restrict__ g) {
+  constexpr int LE = E == 4 ? 2 : E == 8 ? 3 : 4;
+  const int full = logN / LE, rem = logN - full * LE, L = 1 << (logN - LE), Ns_last = 1 << (full * LE);
+  if (rem == 0) filter_passes<E, E, 1>(pair, buf_end, l_end, buf, lt, L, full, Ns_last, in_warp, same, pt, g);
+  if (rem == 1) filter_passes<E, E, 2>(pair, buf_end, l_end, buf, lt, L, full, Ns_last, in_warp, same, pt, g);
+  if constexpr (E >= 8) {
+    if (rem == 2) filter_passes<E, E, 4>(pair, buf_end, l_end, buf, lt, L, full, Ns_last, in_warp, same, pt, g);
+  }
+  if constexpr (E >= 16) {
+    if (rem == 3) filter_passes<E, E, 8>(pair, buf_end, l_end, buf, lt, L, full, Ns_last, in_warp, same, pt, g);
+  }
+}
+
+__device__ __forceinline__ RowPair row_pair(const RDesc& d, int q) {
+  const int W = d.W, H = d.H, y0 = 2 * q;
+  RowPair p;
+  p.on0 = y0 < H;
+  p.on1 = y0 + 1 < H;
+  const size_t a = (size_t)(p.on0 ? y0 : 0) * W, b = (size_t)(p.on1 ? y0 + 1 : 0) * W;
+  p.r0 = d.dep + a;
+  p.r1 = d.dep + b;
+  p.o0 = d.tmp + a;
+  p.o1 = d.tmp + b;
+  return p;
+}
+__device__ __forceinline__ ColumnPair column_pair(const RDesc& d, int x) {
+  ColumnPair p;
+  p.W = d.W;
+  p.on0 = x < d.W;
+  p.on1 = x + 1 < d.W;
+  p.even = d.W % 2 == 0;
+  p.in = d.tmp + (p.on0 ? x : 0);
+  p.out = d.steric + (p.on0 ? x : 0);
+  return p;
+}
+
+// Row pass: 256 / L row pairs per CTA (one packed transform each), L = W / E threads each.
 template <int E>
-__global__ void __launch_bounds__(256) k_fftreg_rows(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+__global__ void __launch_bounds__(256, E == 16 ? 2 : 3) k_fftreg_rows(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   extern __shared__ float2 smr[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int W = d.W, H = d.H, logN = d.fft_logW;
-  const int G = W / E, P = 256 / G;
-  const int tr = threadIdx.x / G, lt = threadIdx.x - tr * G;
-  const int q = (blockIdx.x - off[r]) * P + tr;
-  const int y0 = 2 * q, y1 = 2 * q + 1;
+  const int W = d.W, L = W / E, P = 256 / L;
+  const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
   float2* buf = smr + (size_t)tr * (W + (W >> 4));
-  const bool act0 = y0 < H, act1 = y1 < H;
-  const float* r0 = d.dep + (size_t)(act0 ? y0 : 0) * W;
-  const float* r1 = d.dep + (size_t)(act1 ? y1 : 0) * W;
-  for (int x = lt; x < W; x += G) buf[pad16(x)] = make_float2(act0 ? r0[x] : 0.0f, act1 ? r1[x] : 0.0f);
-  __syncthreads();
-  filter_reg<E>(buf, logN, lt, d.ptW, d.gW);
-  if (act0) {
-    float* o = d.tmp + (size_t)y0 * W;
-    for (int x = lt; x < W; x += G) o[x] = buf[pad16(x)].x;
-  }
-  if (act1) {
-    float* o = d.tmp + (size_t)y1 * W;
-    for (int x = lt; x < W; x += G) o[x] = -buf[pad16(x)].y;
-  }
+  filter_reg<E>(row_pair(d, (blockIdx.x - off[r]) * P + tr), buf, lt, buf, lt, d.fft_logW, L <= 32, true, d.ptW, d.gW);
 }
 
-// Column pass: TV / H column pairs per CTA of TV / E threads (G = H / E per pair), TV = 4096
+// Column pass: TV / H column pairs per CTA of TV / E threads (L = H / E per pair), TV = 4096
 // values per CTA, or 2048 when a plan has too few columns to give every SM two CTAs (a single
-// 1024^2 lattice: 256 CTAs instead of 128); staged from the row-pass output: at H = 1024 a
-// CTA reads 32-byte (TV = 4096) or 16-byte row segments.  Every column pair is transformed
-// by the same code whatever TV is, so both give the same bits.
+// 1024^2 lattice: 256 CTAs instead of 128).  Every column pair is transformed by the same code
+// whatever TV is, so both give the same bits.
 template <int E, int TV>
-__global__ void __launch_bounds__(TV / E) k_fftreg_cols(const RDesc* __restrict__ D, const int* __restrict__ off,
+__global__ void __launch_bounds__(TV / E, E == 16 ? TV == 4096 ? 3 : 5 : 1) k_fftreg_cols(const RDesc* __restrict__ D, const int* __restrict__ off,
                                                         int n) {
   extern __shared__ float2 smr[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int W = d.W, H = d.H, logN = d.fft_logH;
-  const int G = H / E, P = blockDim.x / G;
-  // one extra slot per column pair staggers the pairs over the shared-memory banks when the
-  // tile is staged row by row
+  const int H = d.H, L = H / E, P = blockDim.x / L;
+  // one extra slot per column pair staggers the pairs over the shared-memory banks
   const int S = H + (H >> 4) + 1;
   const int xbase = (blockIdx.x - off[r]) * 2 * P;
-  for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
-    const int y = idx / P, t = idx - y * P;
-    const int xr = xbase + 2 * t, xi = xr + 1;
-    const float* row = d.tmp + (size_t)y * W;
-    smr[(size_t)t * S + pad16(y)] = make_float2(xr < W ? row[xr] : 0.0f, xi < W ? row[xi] : 0.0f);
-  }
-  __syncthreads();
-  const int tr = threadIdx.x / G, lt = threadIdx.x - tr * G;
-  filter_reg<E>(smr + (size_t)tr * S, logN, lt, d.ptH, d.gH);
-  for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
-    const int y = idx / P, t = idx - y * P;
-    const int xr = xbase + 2 * t, xi = xr + 1;
-    const float2 v = smr[(size_t)t * S + pad16(y)];
-    float* row = d.steric + (size_t)y * W;
-    if (xr < W) row[xr] = v.x;
-    if (xi < W) row[xi] = -v.y;
-  }
+  const int l_end = threadIdx.x / P, t_end = threadIdx.x - l_end * P;
+  const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
+  filter_reg<E>(column_pair(d, xbase + 2 * t_end), smr + (size_t)t_end * S, l_end, smr + (size_t)tr * S, lt,
+                d.fft_logH, L <= 32, P == 1, d.ptH, d.gH);
 }
 
 // ---------------------------------------------------------------- sides N = 3 * 2^a
-// Twelve values per thread (G = N / 12 threads per transform): the power-of-two factor
+// Twelve values per thread (L = N / 12 threads per transform): the power-of-two factor
 // in radix-4 passes (three butterflies per thread; one radix-2 pass if a is odd), then a
 // final radix-3 pass (four butterflies per thread) with Ns = N / 3, so every k = j mod Ns
-// is still a mask.  Twiddle index steps N / (Ns R) are integers but not powers of two.
-template <int R>
-__device__ __forceinline__ void pass12(float2* buf, int N, int Ns, int lt, const float2* __restrict__ tw) {
-  constexpr int C = 12 / R;
-  const int G = N / 12;
-  const int S = N / R;
-  const int step = N / (Ns * R);
-  float2 v[12];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int j = lt + c * G;
-    const int k = j & (Ns - 1);
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      float2 a = buf[pad16(j + m * S)];
-      if (m > 0 && k > 0) a = cmul(a, __ldg(tw + m * k * step));
-      v[c * R + m] = a;
-    }
-    dft_reg<R>(v + c * R);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int j = lt + c * G;
-    const int k = j & (Ns - 1);
-    const int dst = (j - k) * R + k;
-#pragma unroll
-    for (int m = 0; m < R; ++m) buf[pad16(dst + m * Ns)] = v[c * R + dft_slot<R>(m)];
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ void fft12(float2* buf, int N, int lt, const float2* __restrict__ tw) {
-  const int P = N / 3;  // power of two >= 4
-  int Ns = 1;
-  while (Ns * 4 <= P) {
-    pass12<4>(buf, N, Ns, lt, tw);
-    Ns *= 4;
-  }
-  if (Ns < P) {
-    pass12<2>(buf, N, Ns, lt, tw);
-    Ns *= 2;
-  }
-  pass12<3>(buf, N, Ns, lt, tw);
-}
-
-__device__ __forceinline__ void filter12(float2* buf, int N, int lt, const float2* __restrict__ tw,
+// is still a mask.
+template <typename Pair>
+__device__ __forceinline__ void filter12(const Pair& pair, float2* buf_end, int l_end, float2* buf, int lt, int N,
+                                         bool in_warp, bool same, const float2* __restrict__ pt,
                                          const float* __restrict__ g) {
-  const int G = N / 12;
-  fft12(buf, N, lt, tw);
-  for (int i = lt; i < N; i += G) {
-    const float gk = __ldg(g + i);
-    const float2 v = buf[pad16(i)];
-    buf[pad16(i)] = make_float2(v.x * gk, -(v.y * gk));
-  }
-  __syncthreads();
-  fft12(buf, N, lt, tw);
+  const int L = N / 12, P = N / 3;  // P: a power of two >= 4
+  const bool edge_warp = in_warp && same;
+  const bool odd = (__ffs(P) - 1) & 1;
+  const int four = odd ? P / 2 : P;  // radix-4 passes have Ns = 1, 4, ... < four
+  float2 v[12];
+  const SharedValues sv{buf};
+  pass_load<12, 4, false>(v, pair, L, N / 4, 1, l_end, pt);
+  pass_store<12, 4>(v, SharedValues{buf_end}, L, 1, l_end);
+  fft_sync(edge_warp);
+  for (int Ns = 4; Ns < four; Ns *= 4) pass_middle<12, 4>(buf, L, N / 4, Ns, lt, pt, in_warp);
+  if (odd) pass_middle<12, 2>(buf, L, N / 2, P / 2, lt, pt, in_warp);
+  pass_load<12, 3, true>(v, sv, L, N / 3, P, lt, pt);
+  fft_sync(in_warp);
+  pass_store<12, 3>(v, Filtered{buf, g}, L, P, lt);
+  fft_sync(in_warp);
+  pass_load<12, 4, false>(v, sv, L, N / 4, 1, lt, pt);
+  fft_sync(in_warp);
+  pass_store<12, 4>(v, sv, L, 1, lt);
+  fft_sync(in_warp);
+  for (int Ns = 4; Ns < four; Ns *= 4) pass_middle<12, 4>(buf, L, N / 4, Ns, lt, pt, in_warp);
+  if (odd) pass_middle<12, 2>(buf, L, N / 2, P / 2, lt, pt, in_warp);
+  if (!edge_warp) __syncthreads();
+  pass_load<12, 3, true>(v, SharedValues{buf_end}, L, N / 3, P, l_end, pt);
+  pass_store<12, 3>(v, pair, L, P, l_end);
 }
 
-// Row pass for W = 3 * 2^a: 256 / G row pairs per CTA, G = W / 12.
-__global__ void __launch_bounds__(256) k_fft12_rows(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+// Row pass for W = 3 * 2^a: 256 / L row pairs per CTA, L = W / 12.
+__global__ void __launch_bounds__(256, 2) k_fft12_rows(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   extern __shared__ float2 sm12[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int W = d.W, H = d.H;
-  const int G = W / 12, P = 256 / G;
-  const int tr = threadIdx.x / G, lt = threadIdx.x - tr * G;
-  const int q = (blockIdx.x - off[r]) * P + tr;
-  const int y0 = 2 * q, y1 = 2 * q + 1;
+  const int W = d.W, L = W / 12, P = 256 / L;
+  const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
   float2* buf = sm12 + (size_t)tr * (W + (W >> 4));
-  const bool act0 = y0 < H, act1 = y1 < H;
-  const float* r0 = d.dep + (size_t)(act0 ? y0 : 0) * W;
-  const float* r1 = d.dep + (size_t)(act1 ? y1 : 0) * W;
-  for (int x = lt; x < W; x += G) buf[pad16(x)] = make_float2(act0 ? r0[x] : 0.0f, act1 ? r1[x] : 0.0f);
-  __syncthreads();
-  filter12(buf, W, lt, d.twW, d.gW);
-  if (act0) {
-    float* o = d.tmp + (size_t)y0 * W;
-    for (int x = lt; x < W; x += G) o[x] = buf[pad16(x)].x;
-  }
-  if (act1) {
-    float* o = d.tmp + (size_t)y1 * W;
-    for (int x = lt; x < W; x += G) o[x] = -buf[pad16(x)].y;
-  }
+  filter12(row_pair(d, (blockIdx.x - off[r]) * P + tr), buf, lt, buf, lt, W, L <= 32 && 32 % L == 0, true, d.ptW, d.gW);
 }
 
-// Column pass for H = 3 * 2^a: 384 / G column pairs per CTA of 384 threads, G = H / 12.
+// Column pass for H = 3 * 2^a: 384 / L column pairs per CTA of 384 threads, L = H / 12.
 __global__ void __launch_bounds__(384) k_fft12_cols(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   extern __shared__ float2 sm12[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int W = d.W, H = d.H;
-  const int G = H / 12, P = blockDim.x / G;
+  const int H = d.H, L = H / 12, P = blockDim.x / L;
   const int S = H + (H >> 4) + 1;  // staggered over the banks, as in k_fftreg_cols
   const int xbase = (blockIdx.x - off[r]) * 2 * P;
-  for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
-    const int y = idx / P, t = idx - y * P;
-    const int xr = xbase + 2 * t, xi = xr + 1;
-    const float* row = d.tmp + (size_t)y * W;
-    sm12[(size_t)t * S + pad16(y)] = make_float2(xr < W ? row[xr] : 0.0f, xi < W ? row[xi] : 0.0f);
-  }
-  __syncthreads();
-  const int tr = threadIdx.x / G, lt = threadIdx.x - tr * G;
-  filter12(sm12 + (size_t)tr * S, H, lt, d.twH, d.gH);
-  for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
-    const int y = idx / P, t = idx - y * P;
-    const int xr = xbase + 2 * t, xi = xr + 1;
-    const float2 v = sm12[(size_t)t * S + pad16(y)];
-    float* row = d.steric + (size_t)y * W;
-    if (xr < W) row[xr] = v.x;
-    if (xi < W) row[xi] = -v.y;
-  }
+  const int l_end = threadIdx.x / P, t_end = threadIdx.x - l_end * P;
+  const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
+  filter12(column_pair(d, xbase + 2 * t_end), sm12 + (size_t)t_end * S, l_end, sm12 + (size_t)tr * S, lt, H,
+           L <= 32 && 32 % L == 0, P == 1, d.ptH, d.gH);
 }
 
 // 256 * 12 / N (rows) or 384 * 12 / N (columns) transforms of N + N / 16 values
