@@ -33,8 +33,14 @@ mc_status rollout_snapshot_f(mc_plan* p, float* dst, cudaStream_t s);
 namespace {
 
 constexpr int kMaxKK = 64;       // stencil entries per node (kernel size <= 8)
-constexpr int kScanChunk = 4096;  // cells per scan block (1024 threads x 4)
-constexpr int kPbdThreads = 128;  // threads per rod component in the PBD kernels
+// IB points per CTA of the forcing rounds: bound by the load latency of a point's 16 gathers, so a
+// few hundred points go over a dozen SMs and not over two (384 points: interpolation 5.6 -> 3.7 us,
+// node side of the reverse 6.3 -> 3.3 us against 256 threads)
+constexpr int kPointThreads = 32;
+constexpr int kCellBucket = 16;  // entries of a cell ordered in registers
+constexpr long long kMaxCells = 4096LL * 4096;  // largest grid of the gradient path
+constexpr int kPbdThreads = 256;  // threads per rod component in the PBD kernels
+constexpr int kPbdRod = 128;      // edges, nodes and pairs of a component kept one per thread
 
 // Per-step inputs of one reverse step, read on the device so that the same CUDA graph
 // replays every step of a segment (sa[*jp], jp counts down).
@@ -95,21 +101,26 @@ struct AD {
   float* ib_w;    // NI x KK
   float2* sraw;   // iters x NI
   float2* s_tmp;  // NI
-  float* uc;      // 2 x lHW
+  float2* uc;     // lHW
   float* inv;     // lHW
-  // CSR over cells
-  int* cnt;    // max(HW, lHW) (all zero between builds)
-  int* start;  // max(HW, lHW) + 1
-  int* bsum;   // scan block sums
-  int* ent;    // entries
-  int* touched;   // cells with at least one entry (any order), M entries at most
-  int* ntouched;  // their count
-  int max_entries;
+  // entries (stencil entries of the IB points, or steric samples) by cell: a cell's entries are
+  // collected in its bucket (beyond kCellBucket in its overflow list) as they arrive, then ordered
+  // into its run of ent; used for the lattice, then for the domain grid
+  int* cnt;       // max(HW, lHW): entries of the cell, zero between uses
+  int* bucket;    // max(HW, lHW) x kCellBucket
+  int* ovf_head;  // max(HW, lHW): first overflow entry of the cell, -1 between uses
+  int* ovf_next;
+  int* ovf;
+  int* start;     // max(HW, lHW): run of a cell with entries
+  int* ent;       // runs: kCellBucket per touched cell, longer ones in the pool behind
+  int pool;       // where the pool begins
+  int* touched;   // cells with at least one entry (any order)
+  int* ntouched;  // [0] their count, [1] overflow entries, [2] use of the pool
   // adjoint
   float* lf0p;   // 9 x lHW
   float* lv;     // 2 x lHW
   float* lrho;   // lHW
-  float* luc;    // 2 x lHW
+  float2* luc;   // lHW
   float2* lnv;   // NI
   float2* lprev;  // N
   float2* lpos;   // N   (state cotangent)
@@ -132,7 +143,6 @@ struct AD {
   float* d_len;
   float* d_kb;
   // steric
-  int* st_cell;    // 16 N
   float* st_val;   // 16 N
   float2* lpred1;  // N
   float2* lpred0p;  // N
@@ -188,40 +198,53 @@ __global__ void k_rest(AD d) {
   d.rest_acc[b] = 0.0f;
 }
 
-__global__ void k_pred(AD d) {
+// 4 lanes per node, as the forward node-step kernel: one finite-difference sample and a quarter of
+// the neighbours each, their terms added in neighbour order.  384 nodes: 8.6 -> 4.1 us against one
+// thread per node.
+__global__ void __launch_bounds__(128) k_pred(AD d) {
   const StepArgs a = d.sa[*d.jp];
   const float2* __restrict__ pos = reinterpret_cast<const float2*>(a.pos);
   const float2* __restrict__ vel = reinterpret_cast<const float2*>(a.vel);
   const float* __restrict__ theta = a.th;
   const float* __restrict__ V = a.V;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < d.E) d.tt[i] = theta[i];
-  if (i >= d.N) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < d.E) d.tt[t] = theta[t];
+  const int i = min(t >> 2, d.N - 1), qs = t & 3;
+  const bool on = (t >> 2) < d.N;
+  const unsigned full = 0xffffffffu;
   const float2 p = pos[i], v = vel[i];
   float2 q = make_float2(p.x + (v.x * d.damp) * d.dt, p.y + (v.y * d.damp) * d.dt);
-  d.pred0[i] = q;
+  if (on && qs == 0) d.pred0[i] = q;
   if (d.steric) {
     const float Wf = (float)d.W, Hf = (float)d.H;
     const float x = mc::fmod_floor(q.x, Wf), y = mc::fmod_floor(q.y, Hf);
-    const float e = 0.5f, den = 1.0f;
-    const float gx = (sample_wrap(V, d.H, d.W, y, x + e) - sample_wrap(V, d.H, d.W, y, x - e)) / den;
-    const float gy = (sample_wrap(V, d.H, d.W, y + e, x) - sample_wrap(V, d.H, d.W, y - e, x)) / den;
-    float fx = -gx, fy = -gy;
+    const float e = (qs & 1) ? -0.5f : 0.5f, den = 1.0f;
+    const float s = sample_wrap(V, d.H, d.W, qs < 2 ? y : y + e, qs < 2 ? x + e : x);
+    const float xp = __shfl_sync(full, s, 0, 4), xm = __shfl_sync(full, s, 1, 4);
+    const float yp = __shfl_sync(full, s, 2, 4), ym = __shfl_sync(full, s, 3, 4);
+    float fx = -((xp - xm) / den), fy = -((yp - ym) / den);
     if (d.nskip > 0) {
       const float inv2s2 = 2.0f * d.sigma * d.sigma;
       const float norm = (float)(2.0 * M_PI) * d.sigma * d.sigma;
       float ax = 0.0f, ay = 0.0f;
       // the neighbours' wrapped predictions, recomputed from their positions and velocities
-      for (int o = -d.nskip; o <= d.nskip; ++o) {
-        const int j = i + o;
-        if (j < 0 || j >= d.N) continue;
-        const float2 pj0 = pos[j], vj = vel[j];
-        const float qx = pj0.x + (vj.x * d.damp) * d.dt, qy = pj0.y + (vj.y * d.damp) * d.dt;
-        const float2 r = mc::min_image(x, y, mc::fmod_floor(qx, Wf), mc::fmod_floor(qy, Hf), Wf, Hf);
-        const float d2 = r.x * r.x + r.y * r.y;
-        const float K = expf(-d2 / inv2s2) / norm;
-        ax = ax + K * r.x;
-        ay = ay + K * r.y;
+      for (int o0 = -d.nskip; o0 <= d.nskip; o0 += 4) {
+        const int o = o0 + qs, j = i + o;
+        float tx = 0.0f, ty = 0.0f;
+        if (o <= d.nskip && o != 0 && j >= 0 && j < d.N) {  // a node's own term is zero
+          const float2 pj0 = pos[j], vj = vel[j];
+          const float qx = pj0.x + (vj.x * d.damp) * d.dt, qy = pj0.y + (vj.y * d.damp) * d.dt;
+          const float2 r = mc::min_image(x, y, mc::fmod_floor(qx, Wf), mc::fmod_floor(qy, Hf), Wf, Hf);
+          const float d2 = r.x * r.x + r.y * r.y;
+          const float K = expf(-d2 / inv2s2) / norm;
+          tx = K * r.x;
+          ty = K * r.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          ax = ax + __shfl_sync(full, tx, k, 4);
+          ay = ay + __shfl_sync(full, ty, k, 4);
+        }
       }
       const float pre = d.scatter / (d.sigma * d.sigma);
       fx = fx - pre * ax;
@@ -230,7 +253,7 @@ __global__ void k_pred(AD d) {
     q.x = q.x + (fx * d.st_strength) * d.dt;
     q.y = q.y + (fy * d.st_strength) * d.dt;
   }
-  d.pp[i] = q;
+  if (on && qs == 0) d.pp[i] = q;
 }
 
 // ------------------------------------------------------------------ tape: PBD iterates (one CTA)
@@ -270,8 +293,8 @@ __device__ __forceinline__ float2 edge_force(const AD& d, const float2* p, float
 // first; the sines, cosines and (in the reverse pass) everything else that depends on the tape
 // alone is computed for all iterations at once, by all threads; the recurrences that remain are a
 // few operations per iteration.  Same operands and summation order as the general loops below, so
-// the same bits.  Measured (256^2, 8 x 48 nodes, per launch): tape 33.7 -> 22.7 us, reverse 33.9 ->
-// 29.2 us; before, each phase of an iteration went through the tape in global memory.
+// the same bits.  Measured (256^2, 8 x 48 nodes, per launch): tape 33.7 -> 21.6 us, reverse 33.9 ->
+// 26.9 us; before, each phase of an iteration went through the tape in global memory.
 constexpr int kPbdGather = 4;
 constexpr int kTapeChunk = 20;  // iterations whose angles and rest vectors the tape kernel keeps at a time
 constexpr int kRevChunk = 10;   // iterations whose tables the reverse kernel keeps at a time
@@ -352,14 +375,14 @@ __device__ __forceinline__ bool pbd_load_node(const AD& d, int in, int nb, PbdNo
 
 // The tape of a component that fits; false (nothing done) when it does not.
 __device__ __forceinline__ bool pbd_fwd_fast(const AD& d, int ea, int eb, int na, int nb) {
-  __shared__ float ths[kTapeChunk + 1][kPbdThreads];  // row k: the angles before pass k of the chunk
-  __shared__ float2 vec[kTapeChunk][kPbdThreads];     // rest vectors after pass k
-  __shared__ float2 ps[kPbdThreads], fs[kPbdThreads];
-  __shared__ float l0s[kPbdThreads];
+  __shared__ float ths[kTapeChunk + 1][kPbdRod];  // row k: the angles before pass k of the chunk
+  __shared__ float2 vec[kTapeChunk][kPbdRod];     // rest vectors after pass k
+  __shared__ float2 ps[kPbdRod], fs[kPbdRod];
+  __shared__ float l0s[kPbdRod];
   const int tid = threadIdx.x, ne = eb - ea;
   PbdEdgeReg re;
   PbdNodeReg rn;
-  bool ok = ne <= (int)blockDim.x && nb - na <= (int)blockDim.x;
+  bool ok = ne <= kPbdRod && nb - na <= kPbdRod;
   if (ok) ok = pbd_load_edge(d, ea + tid, eb, re) && pbd_load_node(d, na + tid, nb, rn);
   // places in the component instead of global indices
   int2 ends = make_int2(0, 0);
@@ -450,7 +473,7 @@ __device__ __forceinline__ bool pbd_fwd_fast(const AD& d, int ea, int eb, int na
 }
 
 // one CTA per rod component: the components never interact in the PBD passes
-__global__ void __launch_bounds__(kPbdThreads) k_pbd_fwd(AD d) {
+__global__ void __launch_bounds__(kPbdThreads, 2) k_pbd_fwd(AD d) {
   const int c = blockIdx.x;
   const int ea = d.c_estart[c], eb = d.c_estart[c + 1], na = d.c_nstart[c], nb = d.c_nstart[c + 1];
   if (pbd_fwd_fast(d, ea, eb, na, nb)) return;
@@ -492,14 +515,107 @@ __global__ void __launch_bounds__(kPbdThreads) k_pbd_fwd(AD d) {
   }
 }
 
+// ------------------------------------------------------------------ entries by cell
+__device__ __forceinline__ void cell_append(const AD& d, int cell, int e) {
+  const int pos = atomicAdd(d.cnt + cell, 1);
+  if (pos == 0) d.touched[atomicAdd(d.ntouched, 1)] = cell;
+  if (pos < kCellBucket) {
+    d.bucket[(size_t)cell * kCellBucket + pos] = e;
+  } else {
+    const int o = atomicAdd(d.ntouched + 1, 1);
+    d.ovf[o] = e;
+    d.ovf_next[o] = atomicExch(d.ovf_head + cell, o);
+  }
+}
+
+// Sorts R keys in registers.
+template <int R>
+__device__ __forceinline__ void sort_keys(int (&k)[R]) {
+#pragma unroll
+  for (int size = 2; size <= R; size <<= 1)
+#pragma unroll
+    for (int j = size >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int o = i ^ j;
+        if (o > i) {
+          const int lo = min(k[i], k[o]), hi = max(k[i], k[o]);
+          k[i] = (i & size) == 0 ? lo : hi;
+          k[o] = (i & size) == 0 ? hi : lo;
+        }
+      }
+}
+
+template <int R>
+__device__ __forceinline__ void order_row(const AD& d, int i, int cell, int len) {
+  int k[R];
+  const int4* bucket = reinterpret_cast<const int4*>(d.bucket + (size_t)cell * kCellBucket);
+  int4* row = reinterpret_cast<int4*>(d.ent + (size_t)i * kCellBucket);
+#pragma unroll
+  for (int q = 0; q < R; q += 4) {
+    int4 v = make_int4(0, 0, 0, 0);
+    if (q < len) v = bucket[q / 4];
+    k[q] = q < len ? v.x : 0x7fffffff;
+    k[q + 1] = q + 1 < len ? v.y : 0x7fffffff;
+    k[q + 2] = q + 2 < len ? v.z : 0x7fffffff;
+    k[q + 3] = q + 3 < len ? v.w : 0x7fffffff;
+  }
+  sort_keys<R>(k);
+#pragma unroll
+  for (int q = 0; q < R; q += 4)
+    if (q < len) row[q / 4] = make_int4(k[q], k[q + 1], k[q + 2], k[q + 3]);
+}
+
+// The entries of each touched cell in increasing index (the order np.add.at applies them): one
+// thread per cell sorts up to 16 in registers, its warp ranks longer ones.  Replaces a count, three
+// scans over all cells, a fill, a compaction and an insertion sort in global memory (24 to 31 us at
+// 256^2) by this launch of 3.6 us.
+__global__ void __launch_bounds__(128) k_cell_order(AD d) {
+  const int n = *d.ntouched;
+  const int i0 = blockIdx.x * blockDim.x;
+  if (i0 >= n) return;
+  const int i = i0 + threadIdx.x, lane = threadIdx.x & 31;
+  const bool on = i < n;
+  const int cell = on ? d.touched[i] : 0;
+  const int len = on ? d.cnt[cell] : 0;
+  if (len > 0 && len <= 8) order_row<8>(d, i, cell, len);
+  if (len > 8 && len <= kCellBucket) order_row<kCellBucket>(d, i, cell, len);
+  if (len > 0 && len <= kCellBucket) d.start[cell] = i * kCellBucket;
+  for (unsigned deep = __ballot_sync(0xffffffffu, len > kCellBucket); deep; deep &= deep - 1) {
+    const int src = __ffs(deep) - 1;
+    const int c = __shfl_sync(0xffffffffu, cell, src), m = __shfl_sync(0xffffffffu, len, src);
+    int base = 0;
+    if (lane == 0) base = atomicAdd(d.ntouched + 2, 2 * m);
+    int* raw = d.ent + d.pool + __shfl_sync(0xffffffffu, base, 0);
+    int* run = raw + m;
+    const int* bucket = d.bucket + (size_t)c * kCellBucket;
+    if (lane < kCellBucket) raw[lane] = bucket[lane];
+    if (lane == 0) {
+      int e = d.ovf_head[c];
+      for (int q = kCellBucket; q < m; ++q) {
+        raw[q] = d.ovf[e];
+        e = d.ovf_next[e];
+      }
+      d.ovf_head[c] = -1;
+      d.start[c] = (int)(run - d.ent);
+    }
+    __syncwarp();
+    for (int q = lane; q < m; q += 32) {
+      const int k = raw[q];
+      int rank = 0;
+      for (int o = 0; o < m; ++o) rank += raw[o] < k ? 1 : 0;
+      run[rank] = k;
+    }
+    __syncwarp();
+  }
+}
+
 // ------------------------------------------------------------------ tape: IB stencils
 // The stencil of IB point n at the step's final PBD positions; with synthetic pairs the
 // point is offset by +-syn_w * syn_ms along the normal of its node's chain tangent (the sum
 // of its edges' min-image vectors, src roles first, as the forward computes it).  The
 // positions are stop_gradient-ed: constants of the derivative.
-__global__ void k_ib_weights(AD d) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= d.NI) return;
+__device__ __forceinline__ float2 tape_point(const AD& d, int n) {
   const int gi = n < d.N ? n : n - d.N;
   const float2* pc = d.pp + (size_t)d.C * d.N;
   const float2 p = pc[gi];
@@ -523,6 +639,15 @@ __global__ void k_ib_weights(AD d) {
       y = y - oy;
     }
   }
+  return make_float2(x, y);
+}
+
+// any kernel size, one thread per IB point
+__global__ void k_ib_weights(AD d) {
+  int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= d.NI) return;
+  const float2 g = tape_point(d, n);
+  const float x = g.x, y = g.y;
   const int K = d.K;
   const float half = (float)((K - 1) / 2);
   const float hw = (float)K / 2.0f;
@@ -538,121 +663,52 @@ __global__ void k_ib_weights(AD d) {
       const int q = a * K + b;
       w[q] = px * py;
       s = s + w[q];
-      d.ib_idx[(size_t)n * d.KK + q] = cell_of((int)ny, (int)nx, d.lH, d.lW);
+      const int cell = cell_of((int)ny, (int)nx, d.lH, d.lW);
+      d.ib_idx[(size_t)n * d.KK + q] = cell;
+      cell_append(d, cell, n * d.KK + q);
     }
   }
   for (int q = 0; q < d.KK; ++q) d.ib_w[(size_t)n * d.KK + q] = w[q] / (s + MC_EPSIL);
 }
 
-// ------------------------------------------------------------------ CSR over cells
-__global__ void k_csr_count(const int* __restrict__ cells, int M, int* cnt) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < M) atomicAdd(cnt + cells[e], 1);
-}
-
-__device__ __forceinline__ int block_exclusive_scan(int v, int* smem, int& total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int x = v;
+// K <= 4: 4 lanes per IB point, lane a a column of the stencil (as k_stencil4 of the forward).
+// 384 points: 9.4 -> 5.8 us against one thread per point.
+__global__ void __launch_bounds__(128) k_ib_weights4(AD d) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = min(t >> 2, d.NI - 1), a = t & 3, K = d.K;
+  const bool mine = (t >> 2) < d.NI && a < K;
+  const float2 g = tape_point(d, n);
+  const float half = (float)((K - 1) / 2), hw = (float)K / 2.0f;
+  const float nx = (floorf(g.x) - half) + (float)a, ny = (floorf(g.y) - half) + (float)a;
+  const float rx = fabsf(nx - g.x) / hw, ry = fabsf(ny - g.y) / hw;
+  const float px = rx <= 2.0f ? 0.25f * (1.0f + cosf(((float)M_PI * rx) / 2.0f)) : 0.0f;
+  const float py = ry <= 2.0f ? 0.25f * (1.0f + cosf(((float)M_PI * ry) / 2.0f)) : 0.0f;
+  const int cx = mc::imod_floor((int)nx, d.lW), cy = mc::imod_floor((int)ny, d.lH) * d.lW;
+  const unsigned full = 0xffffffffu;
+  float w[4];
+  int cell[4];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  for (int b = 0; b < 4; ++b) {
+    w[b] = px * __shfl_sync(full, py, b, 4);
+    cell[b] = __shfl_sync(full, cy, b, 4) + cx;
   }
-  if (lane == 31) smem[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    int w = lane < (int)(blockDim.x >> 5) ? smem[lane] : 0;
+  float s = 0.0f;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float we = __shfl_sync(full, w[b], e, 4);
+      if (e < K && b < K) s = s + we;
     }
-    smem[lane] = w;
-  }
-  __syncthreads();
-  const int before = (wid > 0 ? smem[wid - 1] : 0) + x - v;
-  total = smem[(blockDim.x >> 5) - 1];
-  __syncthreads();
-  return before;
-}
-
-__global__ void __launch_bounds__(1024) k_scan1(const int* __restrict__ cnt, int n, int* start, int* bsum) {
-  __shared__ int smem[32];
-  const int base = blockIdx.x * kScanChunk + threadIdx.x * 4;
-  int v[4];
-  int s = 0;
+  if (!mine) return;
+  const int q0 = (n * K + a) * K;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    v[j] = base + j < n ? cnt[base + j] : 0;
-    s += v[j];
-  }
-  int total;
-  int run = block_exclusive_scan(s, smem, total);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (base + j < n) start[base + j] = run;
-    run += v[j];
-  }
-  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(1024) k_scan2(int* bsum, int nb) {
-  __shared__ int smem[32];
-  const int base = threadIdx.x * 4;
-  int v[4];
-  int s = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    v[j] = base + j < nb ? bsum[base + j] : 0;
-    s += v[j];
-  }
-  int total;
-  int run = block_exclusive_scan(s, smem, total);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (base + j < nb) bsum[base + j] = run;
-    run += v[j];
-  }
-}
-
-__global__ void k_scan3(int* start, const int* __restrict__ bsum, int n, int M) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) start[i] += bsum[i / kScanChunk];
-  if (i == 0) start[n] = M;
-}
-
-__global__ void k_csr_fill(const int* __restrict__ cells, int M, const int* __restrict__ start, int* cnt, int* ent) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= M) return;
-  const int c = cells[e];
-  const int slot = start[c] + atomicSub(cnt + c, 1) - 1;  // leaves cnt at zero
-  ent[slot] = e;
-}
-
-// entries of each cell in increasing flat index (the order np.add.at applies them)
-// the cells that received entries, compacted (their order does not matter: every
-// per-cell kernel below writes only its own cell)
-__global__ void k_csr_touched(const int* __restrict__ start, int n, int* touched, int* ntouched) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n || start[c + 1] == start[c]) return;
-  touched[atomicAdd(ntouched, 1)] = c;
-}
-
-__global__ void k_csr_sort(const int* __restrict__ start, const int* __restrict__ touched,
-                           const int* __restrict__ ntouched, int* ent) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *ntouched) return;
-  const int c = touched[i];
-  const int a = start[c], b = start[c + 1];
-  for (int i = a + 1; i < b; ++i) {
-    const int v = ent[i];
-    int j = i - 1;
-    while (j >= a && ent[j] > v) {
-      ent[j + 1] = ent[j];
-      --j;
+  for (int b = 0; b < 4; ++b)
+    if (b < K) {
+      d.ib_idx[q0 + b] = cell[b];
+      d.ib_w[q0 + b] = w[b] / (s + MC_EPSIL);
+      cell_append(d, cell[b], q0 + b);
     }
-    ent[j + 1] = v;
-  }
 }
 
 // ------------------------------------------------------------------ tape: macroscopic + IB iterations
@@ -672,50 +728,151 @@ __global__ void k_macro(AD d) {
   const float ux = (((((fv[1] - fv[3]) + fv[5]) - fv[6]) - fv[7]) + fv[8]) / rho;
   const float uy = (((((fv[2] - fv[4]) + fv[5]) + fv[6]) - fv[7]) - fv[8]) / rho;
   const float c1 = mc::clamp_factor(ux, uy, d.vmax);
-  d.uc[c] = ux * c1;
-  d.uc[d.lHW + c] = uy * c1;
+  d.uc[c] = make_float2(ux * c1, uy * c1);
   float cov = 0.0f;
-  for (int q = d.start[c]; q < d.start[c + 1]; ++q) cov = cov + d.ib_w[d.ent[q]];
+  const int len = d.cnt[c];
+  if (len > 0)
+    for (int q = d.start[c], end = q + len; q < end; ++q) cov = cov + d.ib_w[d.ent[q]];
   d.inv[c] = 1.0f / mc::max_prop(cov, 1.0f);
 }
 
-__global__ void k_ib_interp(AD d, int it) {
-  const float2* __restrict__ prev = reinterpret_cast<const float2*>(d.sa[*d.jp].pos);
-  int n = blockIdx.x * blockDim.x + threadIdx.x;  // IB point
-  if (n >= d.NI) return;
-  const int gi = n < d.N ? n : n - d.N;
+// Sum of field(cell) * weight over a point's stencil in stencil order (scale: the field is first
+// multiplied by it); all loads of a point in flight together.
+template <int KK>
+__device__ __forceinline__ float2 tape_gather(const AD& d, int n, const float2* __restrict__ field, const float* __restrict__ scale) {
+  const int base = n * (KK ? KK : d.KK);
   float ix = 0.0f, iy = 0.0f;
-  for (int q = 0; q < d.KK; ++q) {
-    const int c = d.ib_idx[(size_t)n * d.KK + q];
-    const float w = d.ib_w[(size_t)n * d.KK + q];
-    ix = ix + d.uc[c] * w;
-    iy = iy + d.uc[d.lHW + c] * w;
+  if constexpr (KK == 0) {
+    for (int q = 0; q < d.KK; ++q) {
+      const int c = d.ib_idx[base + q];
+      const float w = d.ib_w[base + q];
+      float2 v = field[c];
+      if (scale) v = make_float2(scale[c] * v.x, scale[c] * v.y);
+      ix = ix + v.x * w;
+      iy = iy + v.y * w;
+    }
+  } else {
+    int c[KK];
+    float w[KK];
+    if constexpr (KK % 4 == 0) {
+#pragma unroll
+      for (int q = 0; q < KK; q += 4) {
+        const int4 i4 = *reinterpret_cast<const int4*>(d.ib_idx + base + q);
+        const float4 w4 = *reinterpret_cast<const float4*>(d.ib_w + base + q);
+        c[q] = i4.x; c[q + 1] = i4.y; c[q + 2] = i4.z; c[q + 3] = i4.w;
+        w[q] = w4.x; w[q + 1] = w4.y; w[q + 2] = w4.z; w[q + 3] = w4.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < KK; ++q) {
+        c[q] = d.ib_idx[base + q];
+        w[q] = d.ib_w[base + q];
+      }
+    }
+    float2 v[KK];
+#pragma unroll
+    for (int q = 0; q < KK; ++q) {
+      v[q] = field[c[q]];
+      if (scale) {
+        const float sc = scale[c[q]];
+        v[q] = make_float2(sc * v[q].x, sc * v[q].y);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < KK; ++q) {
+      ix = ix + v[q].x * w[q];
+      iy = iy + v[q].y * w[q];
+    }
   }
+  return make_float2(ix, iy);
+}
+__device__ __forceinline__ float2 tape_gather_any(const AD& d, int n, const float2* __restrict__ field, const float* __restrict__ scale) {
+  if (d.KK == 16) return tape_gather<16>(d, n, field, scale);
+  if (d.KK == 9) return tape_gather<9>(d, n, field, scale);
+  if (d.KK == 4) return tape_gather<4>(d, n, field, scale);
+  return tape_gather<0>(d, n, field, scale);
+}
+
+// Sum of point value * weight over a cell's run, in order; 4 entries in flight.
+__device__ __forceinline__ float2 tape_run(const AD& d, int c, const float2* __restrict__ value) {
+  const int a = d.start[c], len = d.cnt[c];
+  float ax = 0.0f, ay = 0.0f;
+  for (int j = 0; j < len; j += 4) {
+    float2 v[4];
+    float w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j + q < len) {
+        const int e = d.ent[a + j + q];
+        w[q] = d.ib_w[e];
+        v[q] = value[d.KK == 16 ? e >> 4 : e / d.KK];
+      }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j + q < len) {
+        ax = ax + v[q].x * w[q];
+        ay = ay + v[q].y * w[q];
+      }
+  }
+  return make_float2(ax, ay);
+}
+
+__device__ __forceinline__ void tape_interp(const AD& d, int n, int it, const float2* prev) {
+  const int gi = n < d.N ? n : n - d.N;
+  const float2 u = tape_gather_any(d, n, d.uc, nullptr);
   const float2 pc = d.pp[(size_t)d.C * d.N + gi], p0 = prev[gi];
   const float v1x = (pc.x - p0.x) / d.dt, v1y = (pc.y - p0.y) / d.dt;
   const float nvx = (v1x * d.scx) * d.dt, nvy = (v1y * d.scy) * d.dt;
-  const float sx = (nvx - ix) * d.relax, sy = (nvy - iy) * d.relax;
+  const float sx = (nvx - u.x) * d.relax, sy = (nvy - u.y) * d.relax;
   d.sraw[(size_t)it * d.NI + n] = make_float2(sx, sy);
   const float cf = mc::clamp_factor(sx, sy, d.vmax);
   d.s_tmp[n] = make_float2(sx * cf, sy * cf);
 }
+__device__ __forceinline__ void tape_spread(const AD& d, int i) {
+  const int c = d.touched[i];
+  const float2 a = tape_run(d, c, d.s_tmp);
+  const float iv = d.inv[c];
+  const float2 u = d.uc[c];
+  d.uc[c] = make_float2(u.x + a.x * iv, u.y + a.y * iv);
+}
+__device__ __forceinline__ void rev_node(const AD& d, int n, int it) {
+  const float2 s = tape_gather_any(d, n, d.luc, d.inv);
+  const float2 r = d.sraw[(size_t)it * d.NI + n];
+  const float2 lr = clamp_vjp(r.x, r.y, d.vmax, s.x, s.y);
+  float2 a = it == d.iters - 1 ? make_float2(0.0f, 0.0f) : d.lnv[n];
+  a.x += d.relax * lr.x;
+  a.y += d.relax * lr.y;
+  d.lnv[n] = a;
+  d.s_tmp[n] = make_float2(-d.relax * lr.x, -d.relax * lr.y);
+}
+__device__ __forceinline__ void rev_cell(const AD& d, int i) {
+  const int c = d.touched[i];
+  const float2 a = tape_run(d, c, d.s_tmp);
+  const float2 u = d.luc[c];
+  d.luc[c] = make_float2(u.x + a.x, u.y + a.y);
+}
+__device__ __forceinline__ const float2* step_positions(const AD& d) {
+  return reinterpret_cast<const float2*>(d.sa[*d.jp].pos);
+}
 
+// The multi-direct forcing rounds and their reverse, one launch per phase.  (All phases in one
+// launch of a cluster of 8 CTAs with its hardware barrier between them took as long, 48 us against
+// 51 for five rounds of 384 points, and longer from 4,096 points: a phase is its dependent loads.)
+__global__ void k_ib_interp(AD d, int it) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;  // IB point
+  if (n < d.NI) tape_interp(d, n, it, step_positions(d));
+}
 __global__ void k_ib_spread(AD d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *d.ntouched) return;
-  const int c = d.touched[i];
-  const int a = d.start[c], b = d.start[c + 1];
-  float ax = 0.0f, ay = 0.0f;
-  for (int q = a; q < b; ++q) {
-    const int e = d.ent[q];
-    const float w = d.ib_w[e];
-    const float2 s = d.s_tmp[e / d.KK];
-    ax = ax + s.x * w;
-    ay = ay + s.y * w;
-  }
-  const float iv = d.inv[c];
-  d.uc[c] = d.uc[c] + ax * iv;
-  d.uc[d.lHW + c] = d.uc[d.lHW + c] + ay * iv;
+  if (i < *d.ntouched) tape_spread(d, i);
+}
+__global__ void k_ib_rev_node(AD d, int it) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < d.NI) rev_node(d, n, it);
+}
+__global__ void k_ib_rev_cell(AD d) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < *d.ntouched) rev_cell(d, i);
 }
 
 // ------------------------------------------------------------------ adjoint: stream + collide + F
@@ -744,7 +901,8 @@ __global__ void k_lbm_adj1(AD d) {
   const float uy = ((((f0[2] - f0[4]) + f0[5]) + f0[6]) - f0[7]) - f0[8];
   const float c1 = mc::clamp_factor(ux / rho, uy / rho, d.vmax);
   const float vx = (ux / rho) * c1, vy = (uy / rho) * c1;
-  const float u5x = d.uc[c], u5y = d.uc[d.lHW + c];
+  const float2 u5 = d.uc[c];
+  const float u5x = u5.x, u5y = u5.y;
   const float c2 = mc::clamp_factor(u5x, u5y, d.vmax);
   const float ucx = u5x * c2, ucy = u5y * c2;
   const float Frx = (ucx - vx) * rho, Fry = (ucy - vy) * rho;
@@ -809,7 +967,8 @@ __global__ void k_lbm_adj1(AD d) {
   // pairs, nf of a node = 0.5 (nf of its + point + nf of its - point))
   const bool syn = d.NI > d.N;
   float rx = 0.0f, ry = 0.0f;
-  for (int q = d.start[c]; q < d.start[c + 1]; ++q) {
+  const int len = d.cnt[c], first = len > 0 ? d.start[c] : 0;
+  for (int q = first; q < first + len; ++q) {
     const int e = d.ent[q];
     const float w = d.ib_w[e];
     const int pt = e / d.KK;
@@ -835,50 +994,12 @@ __global__ void k_lbm_adj1(AD d) {
   lvy -= lFy * rho;
   lrho += lFx * (ucx - vx) + lFy * (ucy - vy);  // through F_raw = (ucc - v) rho
   const float2 l5 = clamp_vjp(u5x, u5y, d.vmax, lccx, lccy);
-  d.luc[c] = l5.x;
-  d.luc[d.lHW + c] = l5.y;
+  d.luc[c] = l5;
   d.lv[c] = lvx;
   d.lv[d.lHW + c] = lvy;
   d.lrho[c] = lrho;
 #pragma unroll
   for (int i = 0; i < 9; ++i) d.lf0p[(size_t)i * d.lHW + c] = lf0[i];
-}
-
-__global__ void k_ib_rev_node(AD d, int it) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;  // IB point
-  if (n >= d.NI) return;
-  float sx = 0.0f, sy = 0.0f;
-  for (int q = 0; q < d.KK; ++q) {
-    const int c = d.ib_idx[(size_t)n * d.KK + q];
-    const float w = d.ib_w[(size_t)n * d.KK + q];
-    const float iv = d.inv[c];
-    sx = sx + (iv * d.luc[c]) * w;
-    sy = sy + (iv * d.luc[d.lHW + c]) * w;
-  }
-  const float2 r = d.sraw[(size_t)it * d.NI + n];
-  const float2 lr = clamp_vjp(r.x, r.y, d.vmax, sx, sy);
-  float2 a = d.lnv[n];
-  a.x += d.relax * lr.x;
-  a.y += d.relax * lr.y;
-  d.lnv[n] = a;
-  d.s_tmp[n] = make_float2(-d.relax * lr.x, -d.relax * lr.y);
-}
-
-__global__ void k_ib_rev_cell(AD d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *d.ntouched) return;
-  const int c = d.touched[i];
-  const int a = d.start[c], b = d.start[c + 1];
-  float ax = 0.0f, ay = 0.0f;
-  for (int q = a; q < b; ++q) {
-    const int e = d.ent[q];
-    const float w = d.ib_w[e];
-    const float2 s = d.s_tmp[e / d.KK];
-    ax = ax + s.x * w;
-    ay = ay + s.y * w;
-  }
-  d.luc[c] = d.luc[c] + ax;
-  d.luc[d.lHW + c] = d.luc[d.lHW + c] + ay;
 }
 
 __global__ void k_lbm_adj2(AD d) {
@@ -896,7 +1017,9 @@ __global__ void k_lbm_adj2(AD d) {
   const float rho = mc::max_prop(rr, 0.1f);
   const float ux = (((((f0[1] - f0[3]) + f0[5]) - f0[6]) - f0[7]) + f0[8]) / rho;
   const float uy = (((((f0[2] - f0[4]) + f0[5]) + f0[6]) - f0[7]) - f0[8]) / rho;
-  const float lvx = d.lv[c] + d.luc[c], lvy = d.lv[d.lHW + c] + d.luc[d.lHW + c];
+  const float2 lu5 = d.luc[c];
+  const float lvx = d.lv[c] + lu5.x, lvy = d.lv[d.lHW + c] + lu5.y;
+  d.cnt[c] = 0;  // the lattice's entries have been used
   const float2 lu = clamp_vjp(ux, uy, d.vmax, lvx, lvy);
   const float lrho = d.lrho[c] - (lu.x * ux + lu.y * uy) / rho;
   const float lraw = lrho * dmaxf(rr, 0.1f);
@@ -910,6 +1033,7 @@ __global__ void k_lbm_adj2(AD d) {
 // ------------------------------------------------------------------ adjoint: node velocity / position
 __global__ void k_node_adj(AD d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 3) d.ntouched[i] = 0;
   if (i < d.E) d.lt[0][i] = d.lth[i];
   if (i >= d.N) return;
   float2 lv1 = d.lvel[i];
@@ -943,7 +1067,7 @@ __device__ __forceinline__ bool pbd_rev_fast(const AD& d, int ea, int eb, int na
   float ns = 1.0f, nt = 1.0f, L0 = 0.0f, ed_x = 1.0f, ed_y = 1.0f, kbb = 0.0f, rst = 0.0f;
   int bq[kPbdGather];
   bool negq[kPbdGather];
-  bool ok = eb - ea <= (int)blockDim.x && nb - na <= (int)blockDim.x && bb - ba <= (int)blockDim.x;
+  bool ok = eb - ea <= kPbdRod && nb - na <= kPbdRod && bb - ba <= kPbdRod;
   if (ok) ok = pbd_load_node(d, na + tid, nb, rn);
   if (ok && ea + tid < eb) {
     e = d.c_edges[ea + tid];
@@ -991,13 +1115,13 @@ __device__ __forceinline__ bool pbd_rev_fast(const AD& d, int ea, int eb, int na
     if (bpl.x < 0 || bpl.y < 0) ok = false;
   }
   if (!__syncthreads_and(ok)) return false;
-  __shared__ float2 lp[kPbdThreads], lcur[kPbdThreads];
-  __shared__ float lthn[kPbdThreads], gb[kPbdThreads], l0s[kPbdThreads];
-  __shared__ int2 ends[kPbdThreads];
+  __shared__ float2 lp[kPbdRod], lcur[kPbdRod];
+  __shared__ float lthn[kPbdRod], gb[kPbdRod], l0s[kPbdRod];
+  __shared__ int2 ends[kPbdRod];
   // per (iteration, edge): segment, (L - L0) / m and its derivative, m, the new angle's cosine and
   // sine; per (iteration, pair): deviation from the rest angle
-  __shared__ float2 seg[kRevChunk][kPbdThreads], stretch[kRevChunk][kPbdThreads], turn[kRevChunk][kPbdThreads];
-  __shared__ float length[kRevChunk][kPbdThreads], bend[kRevChunk][kPbdThreads];
+  __shared__ float2 seg[kRevChunk][kPbdRod], stretch[kRevChunk][kPbdRod], turn[kRevChunk][kPbdRod];
+  __shared__ float length[kRevChunk][kPbdRod], bend[kRevChunk][kPbdRod];
   const int ne = eb - ea;
   if (rn.n >= 0) lp[tid] = d.lp[0][rn.n];
   if (e >= 0) {
@@ -1407,56 +1531,74 @@ __device__ __forceinline__ void sample_adj(const AD& d, const float* V, float yy
   const int y0 = mc::imod_floor(iy, d.H), y1 = mc::imod_floor(iy + 1, d.H);
   const int x0 = mc::imod_floor(ix, d.W), x1 = mc::imod_floor(ix + 1, d.W);
   const float v00 = V[y0 * d.W + x0], v01 = V[y0 * d.W + x1], v10 = V[y1 * d.W + x0], v11 = V[y1 * d.W + x1];
-  lpx += coef * ((1.0f - ty) * (v01 - v00) + ty * (v11 - v10));
-  lpy += coef * ((1.0f - tx) * (v10 - v00) + tx * (v11 - v01));
-  const size_t base = (size_t)n * 16 + qs * 4;
-  d.st_cell[base + 0] = y0 * d.W + x0;
+  lpx = coef * ((1.0f - ty) * (v01 - v00) + ty * (v11 - v10));
+  lpy = coef * ((1.0f - tx) * (v10 - v00) + tx * (v11 - v01));
+  const int base = n * 16 + qs * 4;
   d.st_val[base + 0] = coef * ((1.0f - ty) * (1.0f - tx));
-  d.st_cell[base + 1] = y0 * d.W + x1;
   d.st_val[base + 1] = coef * ((1.0f - ty) * tx);
-  d.st_cell[base + 2] = y1 * d.W + x0;
   d.st_val[base + 2] = coef * (ty * (1.0f - tx));
-  d.st_cell[base + 3] = y1 * d.W + x1;
   d.st_val[base + 3] = coef * (ty * tx);
+  cell_append(d, y0 * d.W + x0, base);
+  cell_append(d, y0 * d.W + x1, base + 1);
+  cell_append(d, y1 * d.W + x0, base + 2);
+  cell_append(d, y1 * d.W + x1, base + 3);
 }
 
-__global__ void k_steric_adj_node(AD d) {
+// 4 lanes per node: lane q one of the four bilinear samples and a quarter of the neighbours; the
+// terms are added in the order samples, then neighbours.  384 nodes: 12.6 -> 7.6 us against one
+// thread per node.
+__global__ void __launch_bounds__(128) k_steric_adj_node(AD d) {
   const float* __restrict__ V = d.sa[*d.jp].V;
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= d.N) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = min(t >> 2, d.N - 1), qs = t & 3;
+  const bool on = (t >> 2) < d.N;
+  const unsigned full = 0xffffffffu;
   const float Wf = (float)d.W, Hf = (float)d.H;
   const float2 lp1 = d.lpred1[n];
   const float lfx = (lp1.x * d.st_strength) * d.dt, lfy = (lp1.y * d.st_strength) * d.dt;
   const float2 q = d.pred0[n];
   const float x = mc::fmod_floor(q.x, Wf), y = mc::fmod_floor(q.y, Hf);
   const float e = 0.5f;
+  float tx = 0.0f, ty = 0.0f;
+  if (on)
+    sample_adj(d, V, qs < 2 ? y : (qs == 2 ? y + e : y - e), qs > 1 ? x : (qs == 0 ? x + e : x - e),
+               qs == 0 ? -lfx : qs == 1 ? lfx : qs == 2 ? -lfy : lfy, n, qs, tx, ty);
   float lpx = 0.0f, lpy = 0.0f;
-  sample_adj(d, V, y, x + e, -lfx, n, 0, lpx, lpy);
-  sample_adj(d, V, y, x - e, lfx, n, 1, lpx, lpy);
-  sample_adj(d, V, y + e, x, -lfy, n, 2, lpx, lpy);
-  sample_adj(d, V, y - e, x, lfy, n, 3, lpx, lpy);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    lpx += __shfl_sync(full, tx, i, 4);
+    lpy += __shfl_sync(full, ty, i, 4);
+  }
   if (d.nskip > 0) {
     const float s2 = d.sigma * d.sigma;
     const float inv2s2 = 2.0f * d.sigma * d.sigma;
     const float norm = (float)(2.0 * M_PI) * d.sigma * d.sigma;
     const float pre = d.scatter / (d.sigma * d.sigma);
-    for (int o = -d.nskip; o <= d.nskip; ++o) {
-      const int j = n + o;
-      if (o == 0 || j < 0 || j >= d.N) continue;
-      const float2 qj = d.pred0[j];
-      const float2 r = mc::min_image(x, y, mc::fmod_floor(qj.x, Wf), mc::fmod_floor(qj.y, Hf), Wf, Hf);
-      const float d2 = r.x * r.x + r.y * r.y;
-      const float K = expf(-d2 / inv2s2) / norm;
-      const float2 lpj = d.lpred1[j];
-      const float ljx = (lpj.x * d.st_strength) * d.dt, ljy = (lpj.y * d.st_strength) * d.dt;
-      // J(r) (g_n - g_j) with g = -pre * lf and J = K (I - r r^T / sigma^2)
-      const float gx = -pre * (lfx - ljx), gy = -pre * (lfy - ljy);
-      const float rg = (r.x * gx + r.y * gy) / s2;
-      lpx += K * (gx - r.x * rg);
-      lpy += K * (gy - r.y * rg);
+    for (int o0 = -d.nskip; o0 <= d.nskip; o0 += 4) {
+      const int o = o0 + qs, j = n + o;
+      const bool there = o != 0 && o <= d.nskip && j >= 0 && j < d.N;
+      tx = ty = 0.0f;
+      if (there) {
+        const float2 qj = d.pred0[j];
+        const float2 r = mc::min_image(x, y, mc::fmod_floor(qj.x, Wf), mc::fmod_floor(qj.y, Hf), Wf, Hf);
+        const float d2 = r.x * r.x + r.y * r.y;
+        const float K = expf(-d2 / inv2s2) / norm;
+        const float2 lpj = d.lpred1[j];
+        const float ljx = (lpj.x * d.st_strength) * d.dt, ljy = (lpj.y * d.st_strength) * d.dt;
+        // J(r) (g_n - g_j) with g = -pre * lf and J = K (I - r r^T / sigma^2)
+        const float gx = -pre * (lfx - ljx), gy = -pre * (lfy - ljy);
+        const float rg = (r.x * gx + r.y * gy) / s2;
+        tx = K * (gx - r.x * rg);
+        ty = K * (gy - r.y * rg);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        lpx += __shfl_sync(full, tx, i, 4);
+        lpy += __shfl_sync(full, ty, i, 4);
+      }
     }
   }
-  d.lpred0p[n] = make_float2(lp1.x + lpx, lp1.y + lpy);
+  if (on && qs == 0) d.lpred0p[n] = make_float2(lp1.x + lpx, lp1.y + lpy);
 }
 
 // out must be zero outside the touched cells
@@ -1465,8 +1607,9 @@ __global__ void k_gather_field(AD d, const float* __restrict__ val, float* out) 
   if (i >= *d.ntouched) return;
   const int c = d.touched[i];
   float a = 0.0f;
-  for (int q = d.start[c]; q < d.start[c + 1]; ++q) a = a + val[d.ent[q]];
+  for (int q = d.start[c], end = q + d.cnt[c]; q < end; ++q) a = a + val[d.ent[q]];
   out[c] = a;
+  d.cnt[c] = 0;  // used
 }
 
 __global__ void k_steric_adj_cic(AD d) {
@@ -1493,6 +1636,7 @@ __global__ void k_steric_adj_cic(AD d) {
 }
 
 __global__ void k_step_next(AD d) {
+  if (threadIdx.x < 3 && blockIdx.x == 0) d.ntouched[threadIdx.x] = 0;
   if (threadIdx.x == 0 && blockIdx.x == 0) *d.jp -= 1;
 }
 
@@ -1525,9 +1669,11 @@ struct mc_grad_plan {
       r_fdesc;
   bool filter_ready = false;
   R r_wpos, r_wvel, r_wth, r_wra, r_wst, r_wfu, r_wf, r_ck, r_seg, r_segV;
-  R r_rest, r_pred0, r_pp, r_tt, r_ibidx, r_ibw, r_sraw, r_stmp, r_uc, r_inv, r_cnt, r_start, r_bsum, r_ent, r_touch;
+  R r_rest, r_pred0, r_pp, r_tt, r_ibidx, r_ibw, r_sraw, r_stmp, r_uc, r_inv, r_cnt, r_start, r_bucket, r_ovh, r_ovn, r_ovf,
+      r_ent, r_touch;
+  long long pool = 0;  // where the pool of runs begins in r_ent
   R r_lf0p, r_lv, r_lrho, r_luc, r_lnv, r_lprev, r_lpos, r_lvel, r_lth, r_lp0, r_lp1, r_lt0, r_lt1, r_lcur, r_lthn,
-      r_gb, r_racc, r_dc, r_da, r_dp, r_do, r_dr, r_dl, r_dk, r_stc, r_stv, r_lpred1, r_lpred0p, r_lV, r_ctmp, r_ldep, r_lf0,
+      r_gb, r_racc, r_dc, r_da, r_dp, r_do, r_dr, r_dl, r_dk, r_stv, r_lpred1, r_lpred0p, r_lV, r_ctmp, r_ldep, r_lf0,
       r_lf1;
   size_t state_ck_bytes = 0;  // one checkpoint: pos, vel, theta, f
   AD ad{};
@@ -1560,20 +1706,6 @@ size_t al(size_t x) { return (x + 255) / 256 * 256; }
 template <typename T>
 T* at(unsigned char* ws, const mc_grad_plan::R& r) {
   return reinterpret_cast<T*>(ws + r.off);
-}
-
-// CSR of M entries over ncells cells (the lattice for the IB stencils, the domain grid for
-// the steric samples)
-void csr_build(const AD& d, const int* cells, int M, int ncells, cudaStream_t s) {
-  const int nb = nblk(ncells, kScanChunk);
-  if (M > 0) k_csr_count<<<nblk(M, 256), 256, 0, s>>>(cells, M, d.cnt);
-  k_scan1<<<nb, 1024, 0, s>>>(d.cnt, ncells, d.start, d.bsum);
-  k_scan2<<<1, 1024, 0, s>>>(d.bsum, nb);
-  k_scan3<<<nblk(ncells, 256), 256, 0, s>>>(d.start, d.bsum, ncells, M);
-  if (M > 0) k_csr_fill<<<nblk(M, 256), 256, 0, s>>>(cells, M, d.start, d.cnt, d.ent);
-  cudaMemsetAsync(d.ntouched, 0, sizeof(int), s);
-  k_csr_touched<<<nblk(ncells, 256), 256, 0, s>>>(d.start, ncells, d.touched, d.ntouched);
-  k_csr_sort<<<nblk(std::max(M, 1), 256), 256, 0, s>>>(d.start, d.touched, d.ntouched, d.ent);
 }
 
 mc_status copy_state_to(mc_grad_plan* p, float* pos, float* vel, float* th, float* f, const float* spos, const float* svel,
@@ -1667,24 +1799,28 @@ void reverse_step(mc_grad_plan* p, cudaStream_t s) {
   const int TB = 256;
   const int nNE = std::max(d.N, d.E);
   k_rest<<<nblk(std::max(d.B, 1), TB), TB, 0, s>>>(d);
-  k_pred<<<nblk(nNE, TB), TB, 0, s>>>(d);
+  k_pred<<<nblk(std::max(4LL * d.N, (long long)d.E), 128), 128, 0, s>>>(d);
   if (d.solver == MC_SOLVER_COSSERAT)
     k_cos_fwd<<<d.ncomp, kPbdThreads, 0, s>>>(d);
   else
     k_pbd_fwd<<<d.ncomp, kPbdThreads, 0, s>>>(d);
   if (d.fluid) {
-    k_ib_weights<<<nblk(d.NI, TB), TB, 0, s>>>(d);
-    csr_build(d, d.ib_idx, d.NI * d.KK, d.lHW, s);
+    if (d.K <= 4)
+      k_ib_weights4<<<nblk(4LL * d.NI, 128), 128, 0, s>>>(d);
+    else
+      k_ib_weights<<<nblk(d.NI, TB), TB, 0, s>>>(d);
+    const int most = std::min((long long)d.NI * d.KK, (long long)d.lHW);  // touched cells at most
+    k_cell_order<<<nblk(most, 128), 128, 0, s>>>(d);
     k_macro<<<nblk(d.lHW, TB), TB, 0, s>>>(d);
     for (int it = 0; it < d.iters; ++it) {
-      k_ib_interp<<<nblk(d.NI, TB), TB, 0, s>>>(d, it);
-      k_ib_spread<<<nblk(d.NI * d.KK, TB), TB, 0, s>>>(d);
+      k_ib_interp<<<nblk(d.NI, kPointThreads), kPointThreads, 0, s>>>(d, it);
+      k_ib_spread<<<nblk(most, 128), 128, 0, s>>>(d);
     }
     k_lbm_adj1<<<nblk(d.lHW, TB), TB, 0, s>>>(d);
-    cudaMemsetAsync(d.lnv, 0, (size_t)d.NI * 8, s);
+    if (d.iters == 0) cudaMemsetAsync(d.lnv, 0, (size_t)d.NI * 8, s);
     for (int it = d.iters - 1; it >= 0; --it) {
-      k_ib_rev_node<<<nblk(d.NI, TB), TB, 0, s>>>(d, it);
-      k_ib_rev_cell<<<nblk(d.NI * d.KK, TB), TB, 0, s>>>(d);
+      k_ib_rev_node<<<nblk(d.NI, kPointThreads), kPointThreads, 0, s>>>(d, it);
+      k_ib_rev_cell<<<nblk(most, 128), 128, 0, s>>>(d);
     }
     k_lbm_adj2<<<nblk(d.lHW, TB), TB, 0, s>>>(d);
   }
@@ -1694,10 +1830,11 @@ void reverse_step(mc_grad_plan* p, cudaStream_t s) {
   else
     k_pbd_rev<<<d.ncomp, kPbdThreads, 0, s>>>(d);
   if (d.steric) {
-    k_steric_adj_node<<<nblk(d.N, TB), TB, 0, s>>>(d);
-    csr_build(d, d.st_cell, d.N * 16, d.HW, s);
+    const int most = std::min(16LL * d.N, (long long)d.HW);
+    k_steric_adj_node<<<nblk(4LL * d.N, 128), 128, 0, s>>>(d);
+    k_cell_order<<<nblk(most, 128), 128, 0, s>>>(d);
     cudaMemsetAsync(d.lV, 0, (size_t)d.HW * 4, s);
-    k_gather_field<<<nblk(d.N * 16, TB), TB, 0, s>>>(d, d.st_val, d.lV);
+    k_gather_field<<<nblk(most, TB), TB, 0, s>>>(d, d.st_val, d.lV);
     // the spectral filter is real and even, so it is its own adjoint: the forward plan's
     // filter kernels map the sample cotangent lV to the deposit cotangent ldep
     mc::filter_launch(p->fwd, p->ws + p->r_fdesc.off, s);
@@ -1722,13 +1859,13 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
   if (D.N < 1 || D.E < 0 || D.B < 0 || D.H < 4 || D.W < 4) return gfail(MC_ERR_INVALID, "bad dims");
   if ((D.E && !pairs) || (D.B && !bending_pairs)) return gfail(MC_ERR_INVALID, "null topology");
   if (num_steps < 0) return gfail(MC_ERR_INVALID, "negative num_steps");
-  if ((long long)D.H * D.W > (long long)kScanChunk * 4096) return gfail(MC_ERR_UNSUPPORTED, "grid too large for the gradient path");
+  if ((long long)D.H * D.W > kMaxCells) return gfail(MC_ERR_UNSUPPORTED, "grid too large for the gradient path");
   if (cfg->ibm_kernel_size < 1 || cfg->ibm_kernel_size * cfg->ibm_kernel_size > kMaxKK)
     return gfail(MC_ERR_UNSUPPORTED, "ibm_kernel_size outside 1..8");
   if (cfg->synthetic_node_width < 0.0f) return gfail(MC_ERR_INVALID, "synthetic_node_width must be >= 0");
   if ((D.fluid_H > 0) != (D.fluid_W > 0) || D.fluid_H < 0 || D.fluid_W < 0)
     return gfail(MC_ERR_INVALID, "fluid_H and fluid_W must both be 0 (the domain grid) or both > 0");
-  if ((long long)std::max(D.fluid_H, 0) * std::max(D.fluid_W, 0) > (long long)kScanChunk * 4096)
+  if ((long long)std::max(D.fluid_H, 0) * std::max(D.fluid_W, 0) > kMaxCells)
     return gfail(MC_ERR_UNSUPPORTED, "fluid lattice too large for the gradient path");
   if (cfg->solver_type != MC_SOLVER_PBD && cfg->solver_type != MC_SOLVER_COSSERAT)
     return gfail(MC_ERR_INVALID, "solver_type must be MC_SOLVER_PBD or MC_SOLVER_COSSERAT");
@@ -1875,11 +2012,17 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
   take(p->r_stmp, NI * 8);
   take(p->r_uc, 2 * LHW * 4);
   take(p->r_inv, LHW * 4);
+  const size_t entries = std::max<size_t>(NI * KK, 16 * N);
+  const size_t rows = std::min(entries, CHW);
+  p->pool = (long long)(rows * kCellBucket);
   take(p->r_cnt, CHW * 4);
-  take(p->r_start, (CHW + 1) * 4);
-  take(p->r_bsum, 4096 * 4);
-  take(p->r_ent, std::max<size_t>(NI * KK, 16 * N) * 4);
-  take(p->r_touch, std::max<size_t>(NI * KK, 16 * N) * 4 + 256);
+  take(p->r_bucket, CHW * kCellBucket * 4);
+  take(p->r_ovh, CHW * 4);
+  take(p->r_ovn, entries * 4);
+  take(p->r_ovf, entries * 4);
+  take(p->r_start, CHW * 4);
+  take(p->r_ent, (rows * kCellBucket + 2 * entries) * 4);
+  take(p->r_touch, rows * 4 + 256);
   take(p->r_lf0p, 9 * LHW * 4);
   take(p->r_lv, 2 * LHW * 4);
   take(p->r_lrho, LHW * 4);
@@ -1907,7 +2050,6 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
   take(p->r_dr, B * 4);
   take(p->r_dl, E * 4);
   take(p->r_dk, B * 4);
-  take(p->r_stc, 16 * N * 4);
   take(p->r_stv, 16 * N * 4);
   take(p->r_lpred1, N * 8);
   take(p->r_lpred0p, N * 8);
@@ -1978,6 +2120,8 @@ mc_status mc_grad_plan_bind(mc_grad_plan* p, void* workspace, size_t bytes, void
   p->filter_ready = false;
   if (!p->cap_stream) GC(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
   GC(cudaMemsetAsync(p->ws + p->r_cnt.off, 0, p->r_cnt.bytes, s));
+  GC(cudaMemsetAsync(p->ws + p->r_ovh.off, 0xff, p->r_ovh.bytes, s));
+  GC(cudaMemsetAsync(p->ws + p->r_touch.off, 0, 256, s));
   const mc_config& c = p->cfg;
   const mc_dims& D = p->dims;
   AD& d = p->ad;
@@ -2056,18 +2200,22 @@ mc_status mc_grad_plan_bind(mc_grad_plan* p, void* workspace, size_t bytes, void
   d.ib_w = at<float>(w, p->r_ibw);
   d.sraw = at<float2>(w, p->r_sraw);
   d.s_tmp = at<float2>(w, p->r_stmp);
-  d.uc = at<float>(w, p->r_uc);
+  d.uc = at<float2>(w, p->r_uc);
   d.inv = at<float>(w, p->r_inv);
   d.cnt = at<int>(w, p->r_cnt);
   d.start = at<int>(w, p->r_start);
-  d.bsum = at<int>(w, p->r_bsum);
+  d.bucket = at<int>(w, p->r_bucket);
+  d.ovf_head = at<int>(w, p->r_ovh);
+  d.ovf_next = at<int>(w, p->r_ovn);
+  d.ovf = at<int>(w, p->r_ovf);
+  d.pool = (int)p->pool;
   d.ent = at<int>(w, p->r_ent);
   d.ntouched = at<int>(w, p->r_touch);
   d.touched = d.ntouched + 64;
   d.lf0p = at<float>(w, p->r_lf0p);
   d.lv = at<float>(w, p->r_lv);
   d.lrho = at<float>(w, p->r_lrho);
-  d.luc = at<float>(w, p->r_luc);
+  d.luc = at<float2>(w, p->r_luc);
   d.lnv = at<float2>(w, p->r_lnv);
   d.lprev = at<float2>(w, p->r_lprev);
   d.lpos = at<float2>(w, p->r_lpos);
@@ -2091,7 +2239,6 @@ mc_status mc_grad_plan_bind(mc_grad_plan* p, void* workspace, size_t bytes, void
   d.d_rest = at<float>(w, p->r_dr);
   d.d_len = at<float>(w, p->r_dl);
   d.d_kb = at<float>(w, p->r_dk);
-  d.st_cell = at<int>(w, p->r_stc);
   d.st_val = at<float>(w, p->r_stv);
   d.lpred1 = at<float2>(w, p->r_lpred1);
   d.lpred0p = at<float2>(w, p->r_lpred0p);
