@@ -268,10 +268,11 @@ __device__ void tile_work(const RDesc& d, int t, unsigned* skeys, int capS) {
 // listed).  A grid of as many CTAs as the GPU holds at once takes the listed tiles one at
 // a time from a cursor (wl_count[2], reset with the list), so that no CTA is launched only
 // to find nothing to do and uneven tiles balance across the CTAs.
-__global__ void __launch_bounds__(256) k_bin_tiles(const RDesc* __restrict__ D, const int2* __restrict__ wl,
-                                                   int* __restrict__ wl_count, int capS) {
+__global__ void __launch_bounds__(256) k_bin_tiles(const RDesc* __restrict__ D, const int2* wl, int* wl_count,
+                                                   int capS) {
   extern __shared__ unsigned dyn[];
   __shared__ int s_item;
+  after_previous();
   const int count = *wl_count;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(wl_count + 2, 1);
@@ -392,6 +393,7 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
                                                            int n, int parity) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int h0 = (blockIdx.x - off[r]) * blockDim.x;
   const int heads = d.ib_ctl[2];
   if (h0 >= heads) return;
@@ -442,40 +444,51 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
 }
 
 // Weighted sum of a head-indexed field over the K*K stencil of one point, in stencil order
-// (the reference's sum over axis 1 of values * weights, fluid.py:90-97).
+// (the reference's sum over axis 1 of values * weights, fluid.py:90-97).  The slots and weights
+// are read past the L1: a chained kernel reads them before it waits (after_previous).
 template <int K2>
-__device__ __forceinline__ float2 stencil_sum(const RDesc& d, int point, const float2* __restrict__ field) {
+struct Taps {
   int slot[K2];
   float w[K2];
-  const int base = point * K2;
-  if (K2 % 4 == 0) {
+  __device__ __forceinline__ void load(const RDesc& d, int point) {
+    const int base = point * K2;
+    if (K2 % 4 == 0) {
 #pragma unroll
-    for (int s = 0; s < K2; s += 4) {
-      const int4 q = *reinterpret_cast<const int4*>(d.ib_slot + base + s);
-      const float4 v = *reinterpret_cast<const float4*>(d.ib_w + base + s);
-      slot[s] = q.x; slot[s + 1] = q.y; slot[s + 2] = q.z; slot[s + 3] = q.w;
-      w[s] = v.x; w[s + 1] = v.y; w[s + 2] = v.z; w[s + 3] = v.w;
+      for (int s = 0; s < K2; s += 4) {
+        const int4 q = __ldcg(reinterpret_cast<const int4*>(d.ib_slot + base + s));
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(d.ib_w + base + s));
+        slot[s] = q.x; slot[s + 1] = q.y; slot[s + 2] = q.z; slot[s + 3] = q.w;
+        w[s] = v.x; w[s + 1] = v.y; w[s + 2] = v.z; w[s + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < K2; ++s) {
+        slot[s] = __ldcg(d.ib_slot + base + s);
+        w[s] = __ldcg(d.ib_w + base + s);
+      }
     }
-  } else {
+  }
+  __device__ __forceinline__ float2 sum(const float2* field) const {
+    float2 v[K2];
+#pragma unroll
+    for (int s = 0; s < K2; ++s) v[s] = field[slot[s]];
+    float x = 0.0f, y = 0.0f;
 #pragma unroll
     for (int s = 0; s < K2; ++s) {
-      slot[s] = d.ib_slot[base + s];
-      w[s] = d.ib_w[base + s];
+      x = x + v[s].x * w[s];
+      y = y + v[s].y * w[s];
     }
+    return make_float2(x, y);
   }
-  float2 v[K2];
-#pragma unroll
-  for (int s = 0; s < K2; ++s) v[s] = field[slot[s]];
-  float x = 0.0f, y = 0.0f;
-#pragma unroll
-  for (int s = 0; s < K2; ++s) {
-    x = x + v[s].x * w[s];
-    y = y + v[s].y * w[s];
-  }
-  return make_float2(x, y);
+};
+template <int K2>
+__device__ __forceinline__ float2 stencil_sum(const RDesc& d, int point, const float2* field) {
+  Taps<K2> taps;
+  taps.load(d, point);
+  return taps.sum(field);
 }
 
-__device__ __forceinline__ float2 stencil_sum_any(const RDesc& d, int point, const float2* __restrict__ field) {
+__device__ __forceinline__ float2 stencil_sum_any(const RDesc& d, int point, const float2* field) {
   switch (d.K) {
     case 4: return stencil_sum<16>(d, point, field);
     case 2: return stencil_sum<4>(d, point, field);
@@ -511,6 +524,29 @@ __device__ __forceinline__ float2 head_force(const RDesc& d, float4 mac, float2 
   return make_float2(Fx, Fy);
 }
 
+// The correction of one point from u at the point (fluid.py:297-302).
+__device__ __forceinline__ void ib_correct(const RDesc& d, int p, float2 v, float2 u) {
+  const float sx = (v.x - u.x) * d.relax;
+  const float sy = (v.y - u.y) * d.relax;
+  const float cf = clamp_factor_fast(sx, sy, d.vmax, d.vmax_q4);
+  d.delta[p] = make_float2(sx * cf, sy * cf);
+}
+
+// What a round reads that the kernel before it does not write (the point's velocity, slots and
+// weights, after the first round) is read before the wait for that kernel.
+template <int K2>
+__device__ __forceinline__ void interp_point(const RDesc& d, int p, bool on, int it) {
+  if (it == 0) after_previous();  // k_ib_heads writes the slots
+  Taps<K2> taps;
+  float2 v;
+  if (on) {
+    v = __ldcg(d.nvl + p);
+    taps.load(d, p);
+  }
+  if (it > 0) after_previous();
+  if (on) ib_correct(d, p, v, taps.sum(d.s_uc));
+}
+
 // Multi-direct forcing, interpolation half (fluid.py:292-302): per IB point, u at the point
 // = sum_s w_s u_corrected(cell_s); correction = (U_point - u) * relaxation, clamped.
 __global__ void __launch_bounds__(256) k_ib_interp(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
@@ -518,25 +554,28 @@ __global__ void __launch_bounds__(256) k_ib_interp(const RDesc* __restrict__ D, 
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
   const int p = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;  // IB point
-  if (p >= d.NI || it >= d.ib_iters) return;
-  const float2 v = d.nvl[p];
-  const float2 u = stencil_sum_any(d, p, d.s_uc);
-  const float sx = (v.x - u.x) * d.relax;
-  const float sy = (v.y - u.y) * d.relax;
-  const float cf = clamp_factor_fast(sx, sy, d.vmax, d.vmax_q4);
-  d.delta[p] = make_float2(sx * cf, sy * cf);
+  const bool on = p < d.NI && it < d.ib_iters;
+  switch (d.K) {
+    case 4: return interp_point<16>(d, p, on, it);
+    case 2: return interp_point<4>(d, p, on, it);
+    case 3: return interp_point<9>(d, p, on, it);
+    default: break;
+  }
+  after_previous();
+  if (on) ib_correct(d, p, d.nvl[p], stencil_sum_any(d, p, d.s_uc));
 }
 
 // In-order sum of correction * weight over a head's run (fluid.py:304-309).  Runs are short: 8
 // entries are fetched at a time (those that exist) so that all their loads are in flight together.
-__device__ __forceinline__ float2 run_sum(const int2* __restrict__ run, int len, const float2* __restrict__ delta) {
-  float dx = 0.0f, dy = 0.0f;
-  const int4* pairs = reinterpret_cast<const int4*>(run);  // runs start at even entries
-  for (int j = 0; j < len; j += 8) {
-    int4 e[4];
-    float2 v[8];
+struct RunChunk {
+  int4 e[4];
+  __device__ __forceinline__ void load(const int2* run, int len, int j) {
+    const int4* pairs = reinterpret_cast<const int4*>(run);  // runs start at even entries
 #pragma unroll
-    for (int q = 0; q < 4; ++q) e[q] = j + 2 * q < len ? pairs[j / 2 + q] : make_int4(0, 0, 0, 0);
+    for (int q = 0; q < 4; ++q) e[q] = j + 2 * q < len ? __ldcg(pairs + j / 2 + q) : make_int4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ void add(int len, int j, const float2* delta, float2& sum) const {
+    float2 v[8];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       v[2 * q] = j + 2 * q < len ? delta[e[q].x] : make_float2(0.0f, 0.0f);
@@ -545,17 +584,16 @@ __device__ __forceinline__ float2 run_sum(const int2* __restrict__ run, int len,
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (j + 2 * q < len) {
-        dx = dx + v[2 * q].x * __int_as_float(e[q].y);
-        dy = dy + v[2 * q].y * __int_as_float(e[q].y);
+        sum.x = sum.x + v[2 * q].x * __int_as_float(e[q].y);
+        sum.y = sum.y + v[2 * q].y * __int_as_float(e[q].y);
       }
       if (j + 2 * q + 1 < len) {
-        dx = dx + v[2 * q + 1].x * __int_as_float(e[q].w);
-        dy = dy + v[2 * q + 1].y * __int_as_float(e[q].w);
+        sum.x = sum.x + v[2 * q + 1].x * __int_as_float(e[q].w);
+        sum.y = sum.y + v[2 * q + 1].y * __int_as_float(e[q].w);
       }
     }
   }
-  return make_float2(dx, dy);
-}
+};
 
 // Multi-direct forcing, spread half (fluid.py:304-310): per touched cell, the in-order sum
 // of correction * weight over its contributions, times 1/max(coverage, 1), added to
@@ -568,13 +606,28 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
   // the plan's last round also computes each touched cell's body force (k_ib_finalize's
   // work for the same cell) when every rollout of the plan runs the same number of rounds
   const bool fin = fuse_finalize && it == d.ib_iters - 1;
-  const int heads = d.ib_ctl[2];
+  // k_ib_interp, the kernel before, writes delta only: all else is read before the wait for it
+  const int heads = __ldcg(d.ib_ctl + 2);
+  const bool on = it < d.ib_iters && p < heads;
+  int2 run = make_int2(0, 0);
+  float4 mac;
+  float2 u;
+  if (on) {
+    run = __ldcg(d.h_run + p);
+    mac = __ldcg(d.s_mac + p);
+    u = __ldcg(d.s_uc + p);
+  }
+  RunChunk c;
+  c.load(d.run + run.x, run.y, 0);
+  after_previous();
   if (fin && p == 0) d.ib_ctl[5] = heads;
-  if (it >= d.ib_iters || p >= heads) return;
-  const int2 run = d.h_run[p];
-  const float4 mac = d.s_mac[p];
-  float2 u = d.s_uc[p];
-  const float2 s = run_sum(d.run + run.x, run.y, d.delta);
+  if (!on) return;
+  float2 s = make_float2(0.0f, 0.0f);
+  c.add(run.y, 0, d.delta, s);
+  for (int j = 8; j < run.y; j += 8) {
+    c.load(d.run + run.x, run.y, j);
+    c.add(run.y, j, d.delta, s);
+  }
   u = make_float2(u.x + s.x * mac.w, u.y + s.y * mac.w);
   d.s_uc[p] = u;
   if (fin) d.s_f[p] = head_force(d, mac, u);
@@ -713,6 +766,7 @@ __global__ void __launch_bounds__(256) k_ib_finalize(const RDesc* __restrict__ D
                                                      int parity) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int p = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
   const int nheads = d.ib_ctl[2];
   if (p == 0) d.ib_ctl[5] = nheads;
@@ -723,9 +777,10 @@ __global__ void __launch_bounds__(256) k_ib_finalize(const RDesc* __restrict__ D
 // Node reaction (fluid.py:364-382), final wrap (simulate.py:97-98), non-finite check and
 // per-step node recording (simulate.py:21-32).
 __global__ void __launch_bounds__(256) k_reaction(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
-                                                  const int* __restrict__ tdev) {
+                                                  const int* tdev) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int node = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
   if (node == 0) {
     // this step's deposit has been reduced: reset the CIC bin controls
@@ -841,16 +896,19 @@ __global__ void k_record_fields(const RDesc* __restrict__ D, const int* __restri
   }
 }
 
-__global__ void k_tick(int* tdev) { *tdev += 1; }
+__global__ void k_tick(int* tdev) {
+  after_previous();
+  *tdev += 1;
+}
 
 cudaError_t tiles_blocks_per_sm(int threads, int capS, int* out) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k_bin_tiles, threads, (size_t)4 * capS * sizeof(unsigned));
 }
 void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int capS, int threads) {
-  k_bin_tiles<<<L.grid, threads, (size_t)4 * capS * sizeof(unsigned), L.s>>>(L.d, wl, wl_count, capS);
+  launch(L, k_bin_tiles, threads, (size_t)4 * capS * sizeof(unsigned), L.d, wl, wl_count, capS);
 }
 void launch_ib_heads(const Launch& L, int parity) {
-  k_ib_heads<<<L.grid, kHeadThreads, 0, L.s>>>(L.d, L.off, L.n, parity);
+  launch(L, k_ib_heads, kHeadThreads, 0, L.d, L.off, L.n, parity);
 }
 // `bytes` is the per-block opt-in limit; the kernel's static shared memory comes off it.
 cudaError_t tiles_set_smem(size_t bytes) {
@@ -860,9 +918,9 @@ cudaError_t tiles_set_smem(size_t bytes) {
   return cudaFuncSetAttribute(k_bin_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(bytes - a.sharedSizeBytes));
 }
-void launch_ib_interp(const Launch& L, int it) { k_ib_interp<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n, it); }
+void launch_ib_interp(const Launch& L, int it) { launch(L, k_ib_interp, kNodeThreads, 0, L.d, L.off, L.n, it); }
 void launch_ib_spread(const Launch& L, int it, int fuse_finalize) {
-  k_ib_spread<<<L.grid, kHeadThreads, 0, L.s>>>(L.d, L.off, L.n, it, fuse_finalize);
+  launch(L, k_ib_spread, kHeadThreads, 0, L.d, L.off, L.n, it, fuse_finalize);
 }
 cudaError_t launch_ib_coop(const Launch& L, int parity) {
   cudaLaunchConfig_t cfg = {};
@@ -905,14 +963,18 @@ cudaError_t ib_coop_blocks_per_sm(int* out) {
 }
 
 void launch_ib_finalize(const Launch& L, int parity) {
-  k_ib_finalize<<<L.grid, kHeadThreads, 0, L.s>>>(L.d, L.off, L.n, parity);
+  launch(L, k_ib_finalize, kHeadThreads, 0, L.d, L.off, L.n, parity);
 }
 void launch_reaction(const Launch& L, const int* tdev) {
-  k_reaction<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n, tdev);
+  launch(L, k_reaction, kNodeThreads, 0, L.d, L.off, L.n, tdev);
 }
 void launch_record_fields(const Launch& L, const int* tdev, int advanced) {
   k_record_fields<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n, tdev, advanced);
 }
-void launch_tick(int* tdev, cudaStream_t s) { k_tick<<<1, 1, 0, s>>>(tdev); }
+void launch_tick(const Launch& L, int* tdev) {
+  Launch one = L;
+  one.grid = 1;
+  launch(one, k_tick, 1, 0, tdev);
+}
 
 }  // namespace mc

@@ -177,6 +177,16 @@ __device__ __forceinline__ int find_rollout(const int* __restrict__ off, int n, 
   return lo;
 }
 
+// Head of every kernel that may be launched chained: waits until the kernels before it have finished
+// and their writes are visible, then lets the next kernel's CTAs come in.  All threads pass here
+// before they read or write anything that another kernel touches, and before any return; so when a
+// kernel starts, the one before its predecessor has finished, and a finished kernel means that all
+// before it have.  Without a chained launch both instructions do nothing.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Floored float modulo, the semantics of jnp.mod / numpy.mod for floats (y > 0 here):
 // r = fmodf(x, y); r += y if r is nonzero with the sign opposite to y.
 // For |x| < 2y, fmodf(x, y) is x or x -/+ y, and both subtractions are exact (Sterbenz),
@@ -233,9 +243,28 @@ struct Launch {
   int n;
   int grid;
   cudaStream_t s;
+  bool chained = false;  // directly behind a kernel of the same stream, which may still be draining
 };
 
-void launch_predict(const Launch& L);
+// Launches `kernel` on L.s.  A chained launch is a programmatic dependent one: the CTAs come onto
+// the SMs while the kernel before drains and wait in after_previous(), so that the launch itself
+// and the look-up of the descriptor do not lie between the two kernels.
+template <class... P, class... A>
+inline void launch(const Launch& L, void (*kernel)(P...), int threads, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)L.grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = L.s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = L.chained ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+void launch_predict(const Launch& L, int* tdev);
 // wl_count: the list length; wl_count[2] is the cursor the CTAs take tiles from (reset to 0
 // with the list)
 void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int capS, int threads = 256);
@@ -273,7 +302,7 @@ void launch_record_fields(const Launch& L, const int* tdev, int advanced);
 void launch_unstream(const Launch& L);
 void launch_stream_out(const Launch& L, int parity, float* dst = nullptr);
 void launch_clear_ws(const Launch& L);
-void launch_tick(int* tdev, cudaStream_t s);
+void launch_tick(const Launch& L, int* tdev);
 cudaError_t fft_set_smem(size_t rows, size_t cols);
 void launch_fft_rows_p2(const Launch& L, size_t smem);
 void launch_fft_cols_p2(const Launch& L, size_t smem);

@@ -250,7 +250,7 @@ extern "C" mc_status mc_steric_potential_noalloc(const float* position, int32_t 
   const mc::RDesc* dd = reinterpret_cast<const mc::RDesc*>(P(kOffDesc));
   const int* off = reinterpret_cast<const int*>(P(kOffOff));
   mc::Launch l{dd, off, 1, cnt[0], s};
-  mc::launch_predict(l);
+  mc::launch_predict(l, nullptr);
   l.off = off + 2;
   l.grid = cnt[1] < 1184 ? cnt[1] : 1184;
   mc::launch_bin_tiles(l, reinterpret_cast<const int2*>(P(kOffWl)), reinterpret_cast<int*>(P(kOffWlCtl)) + 1,

@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kNodeStepMaxThreads, 1)
       const int tw = shape.rod_warps, team = warp / tw;
       if (team < shape.teams)
         for (int c = team; c < d.nchain; c += shape.teams)
-          chain_rod(d, d.chain_info[c], t, Team{warp - team * tw, tw, 1 + shape.bars * team}, m.pos(),
+          chain_rod<false>(d, d.chain_info[c], t, Team{warp - team * tw, tw, 1 + shape.bars * team}, m.pos(),
                     m.tab() + (size_t)team * chain_smem(shape.longest), shape.longest);
     }
     __syncthreads();
@@ -580,6 +580,7 @@ __global__ void __launch_bounds__(kNodeStepMaxThreads, 1)
     if (tid == 0) tdev[r] = t + 1;
     __syncthreads();
   }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the filter's CTAs may come and wait
 
   if (next && d.enable_steric) {
     int* const cell = m.cell();

@@ -16,10 +16,13 @@ __device__ __forceinline__ int bin_tile(const RDesc& d, int cy, int cx) {
   return (cy / kBinTile) * d.ntile_x + cx / kBinTile;
 }
 
-__global__ void __launch_bounds__(256) k_predict(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+__global__ void __launch_bounds__(256) k_predict(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
+                                                 int* tdev) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int node = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
+  if (tdev && blockIdx.x == 0 && threadIdx.x == 0) *tdev += 1;  // the step before ends here
   if (node == 0) {
     // the previous step's IB work is complete: reset this step's IB controls
     d.ib_ctl[0] = 0;
@@ -87,63 +90,6 @@ __global__ void __launch_bounds__(256) k_predict(const RDesc* __restrict__ D, co
   }
 }
 
-// map_coordinates(V, [yy, xx], order=1, mode="wrap") (forces.py:30-34)
-__device__ __forceinline__ float sample_wrap(const float* __restrict__ V, int H, int W, float yy, float xx) {
-  const float ly = floorf(yy), lx = floorf(xx);
-  const float ty = yy - ly, tx = xx - lx;
-  const float wy0 = 1.0f - ty, wx0 = 1.0f - tx;
-  const int iy = (int)ly, ix = (int)lx;
-  const int iy0 = imod_floor(iy, H), iy1 = imod_floor(iy + 1, H);
-  const int ix0 = imod_floor(ix, W), ix1 = imod_floor(ix + 1, W);
-  float acc = (wy0 * wx0) * V[(size_t)iy0 * W + ix0];
-  acc = acc + (wy0 * tx) * V[(size_t)iy0 * W + ix1];
-  acc = acc + (ty * wx0) * V[(size_t)iy1 * W + ix0];
-  acc = acc + (ty * tx) * V[(size_t)iy1 * W + ix1];
-  return acc;
-}
-
-// compute_field_steric_force_corrected for node gi (forces.py:41-81): -grad V by central
-// differences of bilinear samples, minus the analytic Gaussian of global neighbours
-// gi-n..gi+n (the 0 <= j < N mask only, as in the reference).
-__device__ float2 steric_force(const RDesc& d, int gi) {
-  const float W = (float)d.W, H = (float)d.H;
-  const float px = d.predw[2 * gi], py = d.predw[2 * gi + 1];
-  const float* V = d.steric;
-  const float gx = (sample_wrap(V, d.H, d.W, py, px + 0.5f) - sample_wrap(V, d.H, d.W, py, px - 0.5f)) / 1.0f;
-  const float gy = (sample_wrap(V, d.H, d.W, py + 0.5f, px) - sample_wrap(V, d.H, d.W, py - 0.5f, px)) / 1.0f;
-  float fx = -gx, fy = -gy;
-  const int nsk = d.st_skip;
-  if (nsk > 0) {
-    float ax = 0.0f, ay = 0.0f;
-    for (int o = -nsk; o <= nsk; ++o) {
-      const int j = gi + o;
-      const float valid = (j >= 0 && j < d.N) ? 1.0f : 0.0f;
-      const int js = j < 0 ? 0 : (j >= d.N ? d.N - 1 : j);
-      const float qx = d.predw[2 * js], qy = d.predw[2 * js + 1];
-      const float2 rr = min_image(px, py, qx, qy, W, H);
-      const float d2 = rr.x * rr.x + rr.y * rr.y;
-      const float K = expf(-d2 / d.st_2s2) / d.st_norm;
-      const float kv = K * valid;
-      ax = ax + kv * rr.x;
-      ay = ay + kv * rr.y;
-    }
-    fx = fx - d.st_coef * ax;
-    fy = fy - d.st_coef * ay;
-  }
-  return make_float2(fx, fy);
-}
-
-// Predicted position of node gi after the steric displacement (simulate.py:55-63).
-__device__ __forceinline__ float2 node_start(const RDesc& d, int gi) {
-  float qx = d.pred[2 * gi], qy = d.pred[2 * gi + 1];
-  if (d.enable_steric) {
-    const float2 f = steric_force(d, gi);
-    qx = qx + (f.x * d.st_strength) * d.dt;
-    qy = qy + (f.y * d.st_strength) * d.dt;
-  }
-  return make_float2(qx, qy);
-}
-
 // One edge force (pbd.py:60-81).
 __device__ __forceinline__ float2 edge_force(const RDesc& d, float th, float L0, float xs, float ys, float xt,
                                              float yt) {
@@ -200,6 +146,7 @@ __device__ __forceinline__ bool ib_append(const RDesc& d, int cell, int k) {
 __global__ void __launch_bounds__(256) k_stencil(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int p = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;  // IB point
   if (p >= d.NI) return;
   const int gi = p < d.N ? p : p - d.N;
@@ -272,14 +219,19 @@ __global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, c
   const int p = min(t >> 2, NI - 1), a = t & 3, lane = threadIdx.x & 31;
   const bool on = (t >> 2) < NI;
   const int gi = p < N ? p : p - N;
+  // the rods' kernel before writes positions and angles only
+  const float2 pv = __ldcg(reinterpret_cast<const float2*>(d.prev) + gi);
+  int dep = -1;
+  if (on && p < N && d.enable_steric) dep = __ldcg(d.c_cell + a * N + gi);
+  after_previous();
   const float x = d.pos[2 * gi], y = d.pos[2 * gi + 1];
-  const float vx = (x - d.prev[2 * gi]) / d.dt, vy = (y - d.prev[2 * gi + 1]) / d.dt;
+  const float vx = (x - pv.x) / d.dt, vy = (y - pv.y) / d.dt;
   if (on && p < N) {
     if (a == 0) {
       d.vel[2 * gi] = vx;
       d.vel[2 * gi + 1] = vy;
     }
-    if (d.enable_steric) d.dep[d.c_cell[a * N + gi]] = 0.0f;
+    if (dep >= 0) d.dep[dep] = 0.0f;
   }
   if (!d.enable_fluid) return;
   const int K = d.K;
@@ -341,36 +293,100 @@ __global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, c
   }
 }
 
-// The prediction displaced by the steric force (simulate.py:55-65), written to the node
-// positions the rod kernels start from.
-__global__ void __launch_bounds__(256) k_steric(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+// The prediction displaced by the steric force (simulate.py:55-65), written to the node positions
+// the rod kernels start from.  The force (compute_field_steric_force_corrected, forces.py:41-81):
+// -grad V by central differences of bilinear samples (map_coordinates order=1, mode="wrap",
+// forces.py:30-34), minus the analytic Gaussian of global neighbours gi-n..gi+n (the 0 <= j < N
+// mask only, as in the reference).
+//
+// 4 lanes per node: lane q takes one of the four samples and every fourth neighbour, whose terms
+// are added in neighbour order.  Bound by latency; the neighbours do not need the field, so their
+// part is done while the filter before drains.
+__global__ void __launch_bounds__(128) k_steric(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const int gi = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
-  if (gi >= d.N) return;
-  const float2 s = node_start(d, gi);
-  d.pos[2 * gi] = s.x;
-  d.pos[2 * gi + 1] = s.y;
+  const int t = (blockIdx.x - off[r]) * blockDim.x + threadIdx.x;
+  const int gi = min(t >> 2, d.N - 1), q = t & 3;
+  if (!d.enable_steric) {
+    after_previous();
+    if ((t >> 2) < d.N && q < 2) d.pos[2 * gi + q] = d.pred[2 * gi + q];
+    return;
+  }
+  const unsigned full = 0xffffffffu;
+  const float2* predw = reinterpret_cast<const float2*>(d.predw);
+  const float W = (float)d.W, H = (float)d.H;
+  const float2 p = __ldcg(predw + gi);
+  float2 x = __ldcg(reinterpret_cast<const float2*>(d.pred) + gi);
+  const int nsk = d.st_skip;
+  float ax = 0.0f, ay = 0.0f;
+  for (int o0 = -nsk; o0 <= nsk; o0 += 4) {
+    float tx = 0.0f, ty = 0.0f;
+    if (o0 + q <= nsk) {
+      const int j = gi + o0 + q;
+      const float valid = (j >= 0 && j < d.N) ? 1.0f : 0.0f;
+      const float2 pj = __ldcg(predw + (j < 0 ? 0 : (j >= d.N ? d.N - 1 : j)));
+      const float2 rr = min_image(p.x, p.y, pj.x, pj.y, W, H);
+      const float d2 = rr.x * rr.x + rr.y * rr.y;
+      const float K = expf(-d2 / d.st_2s2) / d.st_norm;
+      const float kv = K * valid;
+      tx = kv * rr.x;
+      ty = kv * rr.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      ax = ax + __shfl_sync(full, tx, k, 4);
+      ay = ay + __shfl_sync(full, ty, k, 4);
+    }
+  }
+  // sample q: +x, -x, +y, -y by half a cell
+  const float e = (q & 1) ? -0.5f : 0.5f;
+  const float xx = q < 2 ? p.x + e : p.x, yy = q < 2 ? p.y : p.y + e;
+  const float ly = floorf(yy), lx = floorf(xx);
+  const float sy = yy - ly, sx = xx - lx;
+  const float wy0 = 1.0f - sy, wx0 = 1.0f - sx;
+  const int iy = (int)ly, ix = (int)lx;
+  const int ix0 = imod_floor(ix, d.W), ix1 = imod_floor(ix + 1, d.W);
+  const float* V0 = d.steric + (size_t)imod_floor(iy, d.H) * d.W;
+  const float* V1 = d.steric + (size_t)imod_floor(iy + 1, d.H) * d.W;
+  after_previous();
+  float v = (wy0 * wx0) * V0[ix0];
+  v = v + (wy0 * sx) * V0[ix1];
+  v = v + (sy * wx0) * V1[ix0];
+  v = v + (sy * sx) * V1[ix1];
+  const float vxp = __shfl_sync(full, v, 0, 4), vxm = __shfl_sync(full, v, 1, 4);
+  const float vyp = __shfl_sync(full, v, 2, 4), vym = __shfl_sync(full, v, 3, 4);
+  float fx = -((vxp - vxm) / 1.0f), fy = -((vyp - vym) / 1.0f);
+  if (nsk > 0) {
+    fx = fx - d.st_coef * ax;
+    fy = fy - d.st_coef * ay;
+  }
+  x.x = x.x + (fx * d.st_strength) * d.dt;
+  x.y = x.y + (fy * d.st_strength) * d.dt;
+  if ((t >> 2) < d.N && q == 0) {  // the caller's buffer: no alignment beyond a float's
+    d.pos[2 * gi] = x.x;
+    d.pos[2 * gi + 1] = x.y;
+  }
 }
 
 // ---------------------------------------------------------------- chains: CTA per rod
 // One CTA (one team) per chain rod; S: the longest chain of the plan.  At least four warps, so
 // that the sines and cosines of a short rod's iterations do not fall to a single warp.
 __global__ void __launch_bounds__(384) k_chain(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
-                                               const int* __restrict__ tdev, int S) {
+                                               const int* tdev, int S) {
   extern __shared__ float2 chain_tab[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
   const Team tm = {(int)threadIdx.x >> 5, (int)blockDim.x >> 5, 1};
-  chain_rod(d, d.chain_info[blockIdx.x - off[r]], *tdev, tm, d.pos, chain_tab, S);
+  chain_rod<true>(d, d.chain_info[blockIdx.x - off[r]], __ldcg(tdev), tm, d.pos, chain_tab, S);
 }
 
 // ---------------------------------------------------------------- general rods: CTA per rod
 __global__ void k_node(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
-                       const int* __restrict__ tdev) {
+                       const int* tdev) {
   extern __shared__ float sm[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int comp = d.generic_comp[blockIdx.x - off[r]];
   const int n0 = d.comp_n[comp], nn = d.comp_n[comp + 1] - n0;
   const int e0 = d.comp_e[comp], ne = d.comp_e[comp + 1] - e0;
@@ -496,16 +512,16 @@ __global__ void k_node(const RDesc* __restrict__ D, const int* __restrict__ off,
   }
 }
 
-void launch_predict(const Launch& L) { k_predict<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
-void launch_steric(const Launch& L) { k_steric<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
-void launch_stencil(const Launch& L) { k_stencil<<<L.grid, kNodeThreads, 0, L.s>>>(L.d, L.off, L.n); }
-void launch_stencil4(const Launch& L) { k_stencil4<<<L.grid, 128, 0, L.s>>>(L.d, L.off, L.n); }
+void launch_predict(const Launch& L, int* tdev) { launch(L, k_predict, kNodeThreads, 0, L.d, L.off, L.n, tdev); }
+void launch_steric(const Launch& L) { launch(L, k_steric, 128, 0, L.d, L.off, L.n); }
+void launch_stencil(const Launch& L) { launch(L, k_stencil, kNodeThreads, 0, L.d, L.off, L.n); }
+void launch_stencil4(const Launch& L) { launch(L, k_stencil4, 128, 0, L.d, L.off, L.n); }
 void launch_node(const Launch& L, const int* tdev, size_t smem, int bs) {
-  k_node<<<L.grid, bs, smem, L.s>>>(L.d, L.off, L.n, tdev);
+  launch(L, k_node, bs, smem, L.d, L.off, L.n, tdev);
 }
 void launch_chain(const Launch& L, const int* tdev, int longest) {
   const int warps = chain_warps(longest) < 4 ? 4 : chain_warps(longest);
-  k_chain<<<L.grid, 32 * warps, (size_t)chain_smem(longest) * sizeof(float2), L.s>>>(L.d, L.off, L.n, tdev, longest);
+  launch(L, k_chain, 32 * warps, (size_t)chain_smem(longest) * sizeof(float2), L.d, L.off, L.n, tdev, longest);
 }
 cudaError_t node_set_smem(size_t bytes) {
   return cudaFuncSetAttribute(k_node, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

@@ -106,7 +106,7 @@ __device__ __forceinline__ float2 unit_near(float2 v, float s, float& L) {
 // Rest angle of pair gb at step t (the caller-side curvature actuation, if any); `store` keeps
 // it in the state.
 __device__ __forceinline__ float rest_angle(const RDesc& d, int gb, int t, bool store = true) {
-  if (!d.act_amp) return d.rest_ang[gb];
+  if (!d.act_amp) return __ldcg(d.rest_ang + gb);
   const float arg = d.act_omega[gb] * (float)(d.act_t0 + t) + d.act_phase[gb];
   const float a = d.act_c[gb] + d.act_amp[gb] * sinf(arg);
   if (store) d.rest_ang[gb] = a;
@@ -226,9 +226,10 @@ __device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& 
 
 // All iterations of a PBD rod of rw warps.  The passes run without the slow paths of the modulo
 // and the divisions first (their branches would lie on the dependent chain); if any lane needed
-// one, the chunk is done again from its start with them.
-template <bool SEVERAL>
-__device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, int rw, const RodLane& l, int e0,
+// one, the chunk is done again from its start with them.  start() gives the positions; the first
+// chunk's angles and rest vectors do not need them.
+template <bool SEVERAL, class F>
+__device__ __forceinline__ void pbd_iterations(const F& start, const RDesc& d, const Team& tm, int rw, const RodLane& l, int e0,
                                                float& x, float& y, float& th, float l0, float ra, float kb, float edg,
                                                float ndg, float2* tab, int S) {
   const int lane = threadIdx.x & 31;
@@ -238,6 +239,7 @@ __device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, i
   const Team rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
   const int cycles = d.cycles;
   int buf = 0;
+  if (cycles <= 0) start();
   for (int it0 = 0; it0 < cycles; it0 += kThetaChunk) {
     const int q = min(kThetaChunk, cycles - it0);
     const float th0 = th;
@@ -263,6 +265,7 @@ __device__ __forceinline__ void pbd_iterations(const RDesc& d, const Team& tm, i
       }
     }
     tm.sync();
+    if (it0 == 0) start();
     const float x0 = x, y0 = y;
     const int buf0 = buf;
     bad = false;
@@ -406,6 +409,7 @@ __device__ __forceinline__ void cosserat_rod(const RDesc& d, const Team& rod, co
 // All cycles_per_step iterations at step t of the chain info = (first node, nodes, first edge, first
 // pair).  pos: the rollout's node positions (x, y), updated in place; tab: chain_smem(S) float2 of
 // shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.
+template <bool CHAINED>
 __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, const Team& tm, float* pos, float2* tab,
                                           int S) {
   const int lane = threadIdx.x & 31;
@@ -420,13 +424,21 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
   l.own = act && l.j < nn && (!several || (lane >= kSegGhost && lane < kSegGhost + kSegOwn));
   const int j = l.j, ne = l.ne, nb = l.nb;
   float x = 0.0f, y = 0.0f, th = 0.0f, l0 = 0.0f, ra = 0.0f, kb = 0.0f;
-  if (act && j >= 0) {
-    if (j < nn) {
+  // CHAINED: the kernel before writes the positions; what a PBD rod does without them comes first
+  auto start = [&] {
+    if (CHAINED) after_previous();
+    if (act && j >= 0 && j < nn) {
       x = pos[2 * (n0 + j)];
       y = pos[2 * (n0 + j) + 1];
     }
+  };
+  auto late = [&] {
+    if (CHAINED) start();
+  };
+  if (!CHAINED || d.solver == 1) start();
+  if (act && j >= 0) {
     if (j < ne) {
-      th = d.theta[e0 + j];
+      th = __ldcg(d.theta + e0 + j);
       l0 = d.rest_len[e0 + j];
     }
     if (j < nb) {
@@ -445,9 +457,9 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
       cosserat_rod<false>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
   }
   else if (several)
-    pbd_iterations<true>(d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
+    pbd_iterations<true>(late, d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
   else
-    pbd_iterations<false>(d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
+    pbd_iterations<false>(late, d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
   if (l.own) {
     if (j < ne) d.theta[e0 + j] = th;
     pos[2 * (n0 + j)] = x;

@@ -152,10 +152,9 @@ struct mc_plan {
   std::map<int, StepGraph> graphs;
   bool compact_ok = false;   // small enough for the node-step kernel (compact_shape)
   mc::NodeStepShape ns = {};
-  cudaStream_t side_stream = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t lbm_stream = nullptr;                  // the dense pass, beside the IB chain
-  cudaEvent_t ev_lfork = nullptr, ev_ljoin = nullptr;
+  cudaEvent_t ev_lfork = nullptr, ev_ljoin = nullptr, ev_ifork = nullptr;
+  bool chain = false;  // chained launches in the steps being enqueued (chain_launches)
   bool pending_next = false;  // the next step's pipeline has already been launched
   int64_t last_launches = 0;
   // rollout in progress (mc_rollout_begin .. mc_rollout_end)
@@ -685,13 +684,14 @@ void lbm_tiles(mc_plan* p) {
   }
 }
 
-mc::Launch L(mc_plan* p, Kind k, cudaStream_t s) {
+mc::Launch L(mc_plan* p, Kind k, cudaStream_t s, bool chained = false) {
   mc::Launch l;
   l.d = at<RDesc>(p->ws, p->r_desc);
   l.off = at<int>(p->ws, p->r_off[k]);
   l.n = p->n;
   l.grid = p->grid[k];
   l.s = s;
+  l.chained = chained;
   return l;
 }
 
@@ -809,49 +809,60 @@ void recount_steric(mc_plan* p) {
 // 3 * 2^a; others; the direct form).  When every rollout's sides are of one family, the families
 // share nothing and run beside each other: each alone leaves SMs idle (64 uneven rollouts: rows and
 // columns of two families 73 us in turn, 59 us beside each other).
-int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool capture, mc_status* err) {
+bool filter_forks(const mc_plan* p) {
+  return p->filter_split && p->grid[K_FR16] && (p->grid[K_FR12] || p->grid[K_FFTR2] || p->grid[K_SCONV]) &&
+         !p->profiling;
+}
+
+int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool chained, bool capture, mc_status* err) {
   int64_t k = 0;
-  auto regular = [&](cudaStream_t q) {
+  auto regular = [&](cudaStream_t q, bool c) {
     if (p->grid[K_FR16]) {
-      timed(p, 2, q, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, q), p->fft_e); });
+      timed(p, 2, q, capture, [&] { mc::launch_fftreg_rows(L(p, K_FR16, q, c), p->fft_e); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_FC16] && p->filter_split) {
-      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q), p->fft_e, p->fft_tv); });
+      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q, c), p->fft_e, p->fft_tv); });
+      c = p->chain;
       ++k;
     }
   };
-  auto others = [&](cudaStream_t q) {
+  auto others = [&](cudaStream_t q, bool c) {
     if (p->grid[K_FR12]) {
-      timed(p, 2, q, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, q)); });
+      timed(p, 2, q, capture, [&] { mc::launch_fft12_rows(L(p, K_FR12, q, c)); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_FFTR2]) {
-      timed(p, 2, q, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, q), p->fftr2_smem); });
+      timed(p, 2, q, capture, [&] { mc::launch_fft_rows_p2(L(p, K_FFTR2, q, c), p->fftr2_smem); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_FC16] && !p->filter_split) {
-      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q), p->fft_e, p->fft_tv); });
+      timed(p, 3, q, capture, [&] { mc::launch_fftreg_cols(L(p, K_FC16, q, c), p->fft_e, p->fft_tv); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_FC12]) {
-      timed(p, 3, q, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, q)); });
+      timed(p, 3, q, capture, [&] { mc::launch_fft12_cols(L(p, K_FC12, q, c)); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_FFTC2]) {
-      timed(p, 3, q, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, q), p->fftc2_smem); });
+      timed(p, 3, q, capture, [&] { mc::launch_fft_cols_p2(L(p, K_FFTC2, q, c), p->fftc2_smem); });
+      c = p->chain;
       ++k;
     }
     if (p->grid[K_SCONV]) {
-      timed(p, 17, q, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, q), p->sconv_smem); });
+      timed(p, 17, q, capture, [&] { mc::launch_steric_conv(L(p, K_SCONV, q, c), p->sconv_smem); });
+      c = p->chain;
       ++k;
     }
   };
-  const bool two = p->filter_split && p->grid[K_FR16] &&
-                   (p->grid[K_FR12] || p->grid[K_FFTR2] || p->grid[K_SCONV]) && !p->profiling;
-  if (!two) {
-    regular(s);
-    others(s);
+  if (!filter_forks(p)) {
+    regular(s, chained);
+    others(s, chained || (k > 0 && p->chain));
     return k;
   }
   auto fork = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
@@ -860,8 +871,8 @@ int64_t enqueue_filter(mc_plan* p, cudaStream_t s, bool capture, mc_status* err)
     if (e != cudaSuccess && *err == MC_OK) *err = cuda_fail(e, "fork to the filter stream");
   };
   fork(p->ev_ffork, s, p->filter_stream);
-  others(p->filter_stream);
-  regular(s);
+  others(p->filter_stream, false);
+  regular(s, chained);
   fork(p->ev_fjoin, p->filter_stream, s);
   return k;
 }
@@ -877,54 +888,57 @@ int64_t enqueue_node_step(mc_plan* p, int parity, int main, int next, cudaStream
   return 1;
 }
 
-int64_t enqueue_pipeline(mc_plan* p, cudaStream_t s, bool capture, mc_status* err) {
+int64_t enqueue_pipeline(mc_plan* p, bool tick, cudaStream_t s, bool chained, bool capture, mc_status* err) {
   if (is_compact(p)) {
     if (!p->any_steric) return 0;
-    return enqueue_node_step(p, 0, 0, 1, s, capture) + enqueue_filter(p, s, capture, err);
+    return enqueue_node_step(p, 0, 0, 1, s, capture) + enqueue_filter(p, s, false, capture, err);
   }
   int* tdev = at<int>(p->ws, p->r_tdev);
+  const bool on = p->chain;
   int64_t k = 0;
   if (p->grid[K_NODES]) {
-    timed(p, 0, s, capture, [&] { mc::launch_predict(L(p, K_NODES, s)); });
+    timed(p, 0, s, capture, [&] { mc::launch_predict(L(p, K_NODES, s, chained), tick ? tdev : nullptr); });
     ++k;
   }
   if (p->any_steric) {
     timed(p, 1, s, capture, [&] {
-      mc::Launch l = L(p, K_TILES, s);
+      mc::Launch l = L(p, K_TILES, s, p->grid[K_NODES] ? on : chained);
       l.grid = p->tile_grid_c;
       mc::launch_bin_tiles(l, at<int2>(p->ws, p->r_wl_cic), at<int>(p->ws, p->r_wl_ctl) + 1, p->c_smem,
                            p->bin_threads);
     });
     k += 1;
-    k += enqueue_filter(p, s, capture, err);
+    k += enqueue_filter(p, s, on, capture, err);
   }
+  const bool behind = on && !(p->any_steric && filter_forks(p));  // not behind a join
   if (p->grid[K_NODES]) {
-    timed(p, 14, s, capture, [&] { mc::launch_steric(L(p, K_NODES, s)); });
+    timed(p, 14, s, capture, [&] { mc::launch_steric(L(p, K_NODES4, s, behind)); });
     ++k;
   }
   if (p->grid[K_CHAIN]) {
-    timed(p, 4, s, capture, [&] { mc::launch_chain(L(p, K_CHAIN, s), tdev, p->max_chain); });
+    timed(p, 4, s, capture, [&] { mc::launch_chain(L(p, K_CHAIN, s, on), tdev, p->max_chain); });
     ++k;
   }
   if (p->grid[K_COMP]) {
-    timed(p, 5, s, capture, [&] { mc::launch_node(L(p, K_COMP, s), tdev, p->node_smem, p->node_bs); });
+    timed(p, 5, s, capture, [&] { mc::launch_node(L(p, K_COMP, s, on), tdev, p->node_smem, p->node_bs); });
     ++k;
   }
   if (p->grid[K_NODES]) {
     if (p->max_k <= 4)
-      timed(p, 15, s, capture, [&] { mc::launch_stencil4(L(p, K_NODES4, s)); });
+      timed(p, 15, s, capture, [&] { mc::launch_stencil4(L(p, K_NODES4, s, on)); });
     else
-      timed(p, 15, s, capture, [&] { mc::launch_stencil(L(p, K_NODES, s)); });
+      timed(p, 15, s, capture, [&] { mc::launch_stencil(L(p, K_NODES, s, on)); });
     ++k;
   }
   return k;
 }
 
-int64_t enqueue_ib(mc_plan* p, int parity, cudaStream_t s, bool capture) {
+int64_t enqueue_ib(mc_plan* p, int parity, cudaStream_t s, bool chained, bool capture) {
   if (!p->any_fluid) return 0;
+  const bool on = p->chain;
   int64_t k = 0;
   if (p->grid[K_IB]) {
-    timed(p, 6, s, capture, [&] { mc::launch_ib_heads(L(p, K_IB, s), parity); });
+    timed(p, 6, s, capture, [&] { mc::launch_ib_heads(L(p, K_IB, s, chained), parity); });
     ++k;
   }
   if (p->ib_cluster > 0 && p->grid[K_NODES]) {
@@ -943,12 +957,12 @@ int64_t enqueue_ib(mc_plan* p, int parity, cudaStream_t s, bool capture) {
   // when every rollout runs max_iters rounds, the last spread also computes the body force
   const int fuse = p->fuse_finalize ? 1 : 0;
   for (int it = 0; it < p->max_iters; ++it) {
-    timed(p, 7, s, capture, [&] { mc::launch_ib_interp(L(p, K_NODES, s), it); });
-    timed(p, 8, s, capture, [&] { mc::launch_ib_spread(L(p, K_IB, s), it, fuse); });
+    timed(p, 7, s, capture, [&] { mc::launch_ib_interp(L(p, K_NODES, s, on), it); });
+    timed(p, 8, s, capture, [&] { mc::launch_ib_spread(L(p, K_IB, s, on), it, fuse); });
     k += 2;
   }
   if (fuse) return k;
-  timed(p, 9, s, capture, [&] { mc::launch_ib_finalize(L(p, K_IB, s), parity); });
+  timed(p, 9, s, capture, [&] { mc::launch_ib_finalize(L(p, K_IB, s, on), parity); });
   return k + 1;
 }
 
@@ -969,51 +983,62 @@ int64_t enqueue_heads(mc_plan* p, int parity, int write_u, cudaStream_t s, bool 
   return 1;
 }
 
-int64_t enqueue_tail(mc_plan* p, int rec_fields, cudaStream_t s, bool capture) {
+// The step counter is advanced by the next step's k_predict when one follows at once, else here.
+int64_t enqueue_tail(mc_plan* p, int rec_fields, bool has_next, cudaStream_t s, bool chained, bool capture) {
   int* tdev = at<int>(p->ws, p->r_tdev);
   int64_t k = 0;
   if (p->grid[K_NODES]) {
-    timed(p, 11, s, capture, [&] { mc::launch_reaction(L(p, K_NODES, s), tdev); });
+    timed(p, 11, s, capture, [&] { mc::launch_reaction(L(p, K_NODES, s, chained), tdev); });
     ++k;
   }
   if (rec_fields) {
     timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), tdev, 0); });
     ++k;
   }
-  timed(p, 13, s, capture, [&] { mc::launch_tick(tdev, s); });
+  if (has_next && p->grid[K_NODES]) return k;
+  timed(p, 13, s, capture, [&] { mc::launch_tick(L(p, K_NODES, s, k > 0 && p->chain && !rec_fields), tdev); });
   return k + 1;
 }
+
+// Whether a step's kernels are launched chained.  Not while kernels are timed one at a time, and not
+// where the node grid is more than half of what the GPU holds at once (148 SMs x 16 CTAs of 128
+// threads): the CTAs that wait then take the slots the dense pass beside them would run in.  Per
+// pass without and with: 1024^2 (128 CTAs) 2390 and 2210 us, 64 uneven rollouts (610) 4204 and 4000,
+// 256 of them (2300) 7650 and 7820.
+bool chain_launches(const mc_plan* p) { return !p->profiling && p->grid[K_NODES] <= 8 * 148; }
 
 // Everything of step t after its pipeline, plus pipeline(t+1) when has_next; with `first` the
 // step's own pipeline too.
 //   lbm stream: the dense pass lbm(t) (reads h[parity], writes h[parity^1]) from the start
 //               of the body, concurrently with the pipeline and the IB chain, which reads
-//               h[parity] only;
-//   main:       ib(t) (bins, iterations, body force per touched cell), then, once lbm(t)
-//               is done, the touched cells' collision over its result;
-//   side:       after ib(t): tail(t) (node reaction) and pipeline(t+1).
-// The next body starts when all three have finished.  In a compact plan one node-step launch
+//               h[parity] only; then, once ib(t) is done, the touched cells' collision over
+//               its result;
+//   main:       ib(t) (touched cells, iterations, body force per touched cell), tail(t) (node
+//               reaction) and pipeline(t+1), each kernel chained to the one before.
+// The next body starts when both have finished.  In a compact plan one node-step launch
 // is pipeline(t) after the filter, ib(t), tail(t) and pipeline(t+1) up to the filter.
 int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool first, bool has_next, cudaStream_t s,
                      bool capture, mc_status* err) {
   const bool compact = is_compact(p);
   int64_t k = 0;
+  p->chain = chain_launches(p);
   if (rec_fields || p->profiling) {
     // sequential: field recording needs this order; profiling times kernels one at a time
-    if (first) k += enqueue_pipeline(p, s, capture, err);
-    k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
+    if (first) k += enqueue_pipeline(p, false, s, false, capture, err);
+    k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture)
+                 : enqueue_ib(p, parity, s, false, capture);
     k += enqueue_lbm(p, parity, write_u, s, capture);
     k += enqueue_heads(p, parity, write_u, s, capture);
     if (!compact) {
-      k += enqueue_tail(p, rec_fields, s, capture);
-      if (has_next) k += enqueue_pipeline(p, s, capture, err);
+      k += enqueue_tail(p, rec_fields, has_next, s, false, capture);
+      if (has_next) k += enqueue_pipeline(p, true, s, false, capture, err);
       return k;
     }
     if (rec_fields) {
       timed(p, 12, s, capture, [&] { mc::launch_record_fields(L(p, K_CELLS, s), at<int>(p->ws, p->r_tdev), 1); });
       ++k;
     }
-    if (has_next && p->any_steric) k += enqueue_filter(p, s, capture, err);
+    if (has_next && p->any_steric) k += enqueue_filter(p, s, false, capture, err);
     return k;
   }
   auto fork = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to, const char* what) {
@@ -1021,26 +1046,28 @@ int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool f
     if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
     if (e != cudaSuccess && *err == MC_OK) *err = cuda_fail(e, what);
   };
-  cudaStream_t s2 = p->side_stream, s3 = p->lbm_stream;
+  cudaStream_t s2 = p->lbm_stream;
   if (p->any_fluid) {
-    fork(p->ev_lfork, s, s3, "fork to the dense-pass stream");
-    k += enqueue_lbm(p, parity, write_u, s3, capture);
+    fork(p->ev_lfork, s, s2, "fork to the dense-pass stream");
+    k += enqueue_lbm(p, parity, write_u, s2, capture);
   }
-  if (first) k += enqueue_pipeline(p, s, capture, err);
-  const bool side = !compact || (has_next && p->any_steric);
-  k += compact ? enqueue_node_step(p, parity, 1, has_next, s, capture) : enqueue_ib(p, parity, s, capture);
-  if (side) fork(p->ev_fork, s, s2, "fork to the side stream");
+  if (first) k += enqueue_pipeline(p, false, s, false, capture, err);
+  const int64_t ib = compact ? enqueue_node_step(p, parity, 1, has_next, s, capture)
+                             : enqueue_ib(p, parity, s, first && p->grid[K_NODES] && p->chain, capture);
+  k += ib;
+  if (p->any_fluid) {
+    fork(p->ev_ifork, s, s2, "fork to the touched cells' collision");
+    k += enqueue_heads(p, parity, write_u, s2, capture);
+  }
   if (compact) {
-    if (side) k += enqueue_filter(p, s2, capture, err);
+    if (has_next && p->any_steric) k += enqueue_filter(p, s, p->chain, capture, err);
   } else {
-    k += enqueue_tail(p, 0, s2, capture);
-    if (has_next) k += enqueue_pipeline(p, s2, capture, err);
+    const bool rounds = ib > 0 && !p->use_coop && p->ib_cluster == 0;  // those launches are not chained
+    const int64_t tail = enqueue_tail(p, 0, has_next, s, rounds && p->chain, capture);
+    k += tail;
+    if (has_next) k += enqueue_pipeline(p, true, s, tail > 0 && p->chain, capture, err);
   }
-  if (p->any_fluid) {
-    fork(p->ev_ljoin, s3, s, "join from the dense-pass stream");
-    k += enqueue_heads(p, parity, write_u, s, capture);
-  }
-  if (side) fork(p->ev_join, s2, s, "join from the side stream");
+  if (p->any_fluid) fork(p->ev_ljoin, s2, s, "join from the dense-pass stream");
   return k;
 }
 
@@ -1804,9 +1831,7 @@ void mc_plan_destroy(mc_plan* p) {
   }
   for (auto e : p->ev_pool) cudaEventDestroy(e);
   if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
-  if (p->side_stream) cudaStreamDestroy(p->side_stream);
-  if (p->ev_fork) cudaEventDestroy(p->ev_fork);
-  if (p->ev_join) cudaEventDestroy(p->ev_join);
+  if (p->ev_ifork) cudaEventDestroy(p->ev_ifork);
   if (p->filter_stream) cudaStreamDestroy(p->filter_stream);
   if (p->ev_ffork) cudaEventDestroy(p->ev_ffork);
   if (p->ev_fjoin) cudaEventDestroy(p->ev_fjoin);
@@ -1903,7 +1928,6 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
   MC_CUDA(cudaGetLastError());
   destroy_graphs(p);
   if (!p->cap_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
-  if (!p->side_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->side_stream, cudaStreamNonBlocking));
   if (!p->lbm_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->lbm_stream, cudaStreamNonBlocking));
   {
     // the fused IB kernel needs every CTA resident at once (cooperative launch)
@@ -1918,8 +1942,7 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
   if (!p->filter_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->filter_stream, cudaStreamNonBlocking));
   if (!p->ev_ffork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_ffork, cudaEventDisableTiming));
   if (!p->ev_fjoin) MC_CUDA(cudaEventCreateWithFlags(&p->ev_fjoin, cudaEventDisableTiming));
-  if (!p->ev_fork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
-  if (!p->ev_join) MC_CUDA(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
+  if (!p->ev_ifork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_ifork, cudaEventDisableTiming));
   if (!p->ev_lfork) MC_CUDA(cudaEventCreateWithFlags(&p->ev_lfork, cudaEventDisableTiming));
   if (!p->ev_ljoin) MC_CUDA(cudaEventCreateWithFlags(&p->ev_ljoin, cudaEventDisableTiming));
   p->bound = true;

@@ -357,6 +357,7 @@ __global__ void __launch_bounds__(256) k_fft_rows_p2(const RDesc* __restrict__ D
   extern __shared__ float2 sm[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int W = d.W, H = d.H, T = d.fft_T_r, P = d.fft_tpc_r, logW = d.fft_logW;
   const int tr = threadIdx.x / T, lt = threadIdx.x - tr * T;  // P * T == blockDim.x
   const int q = (blockIdx.x - off[r]) * P + tr;
@@ -386,6 +387,7 @@ __global__ void __launch_bounds__(512) k_fft_cols_p2(const RDesc* __restrict__ D
   extern __shared__ float2 sm[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int W = d.W, H = d.H, T = d.fft_T_c, P = d.fft_tpc_c, logH = d.fft_logH;
   const int S = H + 1;
   const int xbase = (blockIdx.x - off[r]) * 2 * P;
@@ -414,10 +416,10 @@ __global__ void __launch_bounds__(512) k_fft_cols_p2(const RDesc* __restrict__ D
 }
 
 void launch_fft_rows_p2(const Launch& L, size_t smem) {
-  k_fft_rows_p2<<<L.grid, 256, smem, L.s>>>(L.d, L.off, L.n);
+  launch(L, k_fft_rows_p2, 256, smem, L.d, L.off, L.n);
 }
 void launch_fft_cols_p2(const Launch& L, size_t smem) {
-  k_fft_cols_p2<<<L.grid, 512, smem, L.s>>>(L.d, L.off, L.n);
+  launch(L, k_fft_cols_p2, 512, smem, L.d, L.off, L.n);
 }
 cudaError_t fft_p2_set_smem(size_t bytes) {
   cudaError_t e = cudaFuncSetAttribute(k_fft_rows_p2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -453,6 +455,7 @@ cudaError_t fft_set_smem(size_t rows, size_t cols) {
 __global__ void __launch_bounds__(256) k_steric_conv(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int lb = blockIdx.x - off[r];
   const int tx = lb % d.conv_ntx, ty = lb / d.conv_ntx;
   const int H = d.H, W = d.W, Rx = d.conv_RW, Ry = d.conv_RH;
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(256) k_steric_conv(const RDesc* __restrict__ D
 }
 
 void launch_steric_conv(const Launch& L, size_t smem) {
-  k_steric_conv<<<L.grid, 256, smem, L.s>>>(L.d, L.off, L.n);
+  launch(L, k_steric_conv, 256, smem, L.d, L.off, L.n);
 }
 
 
@@ -816,6 +819,7 @@ __global__ void __launch_bounds__(256, E == 16 ? 2 : 3) k_fftreg_rows(const RDes
   extern __shared__ float2 smr[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int W = d.W, L = W / E, P = 256 / L;
   const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
   float2* buf = smr + (size_t)tr * (W + (W >> 4));
@@ -832,6 +836,7 @@ __global__ void __launch_bounds__(TV / E, E == 16 ? TV == 4096 ? 3 : 5 : 1) k_ff
   extern __shared__ float2 smr[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int H = d.H, L = H / E, P = blockDim.x / L;
   // one extra slot per column pair staggers the pairs over the shared-memory banks
   const int S = H + (H >> 4) + 1;
@@ -882,6 +887,7 @@ __global__ void __launch_bounds__(256, 2) k_fft12_rows(const RDesc* __restrict__
   extern __shared__ float2 sm12[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int W = d.W, L = W / 12, P = 256 / L;
   const int tr = threadIdx.x / L, lt = threadIdx.x - tr * L;
   float2* buf = sm12 + (size_t)tr * (W + (W >> 4));
@@ -893,6 +899,7 @@ __global__ void __launch_bounds__(384) k_fft12_cols(const RDesc* __restrict__ D,
   extern __shared__ float2 sm12[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
+  after_previous();
   const int H = d.H, L = H / 12, P = blockDim.x / L;
   const int S = H + (H >> 4) + 1;  // staggered over the banks, as in k_fftreg_cols
   const int xbase = (blockIdx.x - off[r]) * 2 * P;
@@ -905,8 +912,8 @@ __global__ void __launch_bounds__(384) k_fft12_cols(const RDesc* __restrict__ D,
 // 256 * 12 / N (rows) or 384 * 12 / N (columns) transforms of N + N / 16 values
 constexpr size_t kFft12RowsSmem = (size_t)256 * 12 * 17 / 16 * sizeof(float2) + 256;
 constexpr size_t kFft12ColsSmem = ((size_t)384 * 12 * 17 / 16 + 384) * sizeof(float2) + 256;
-void launch_fft12_rows(const Launch& L) { k_fft12_rows<<<L.grid, 256, kFft12RowsSmem, L.s>>>(L.d, L.off, L.n); }
-void launch_fft12_cols(const Launch& L) { k_fft12_cols<<<L.grid, 384, kFft12ColsSmem, L.s>>>(L.d, L.off, L.n); }
+void launch_fft12_rows(const Launch& L) { launch(L, k_fft12_rows, 256, kFft12RowsSmem, L.d, L.off, L.n); }
+void launch_fft12_cols(const Launch& L) { launch(L, k_fft12_cols, 384, kFft12ColsSmem, L.d, L.off, L.n); }
 
 // shared memory of a CTA: (row pass, 256 threads) 256 E / N transforms or (column pass,
 // TV / E threads) TV / N transforms, of N + N / 16 values each (+1 per column pair)
@@ -914,21 +921,21 @@ size_t fftreg_smem(int e) { return (size_t)256 * e * 17 / 16 * sizeof(float2); }
 size_t fftreg_cols_smem(int tv) { return ((size_t)tv * 17 / 16 + 256) * sizeof(float2); }
 
 void launch_fftreg_rows(const Launch& L, int e) {
-  if (e == 16) k_fftreg_rows<16><<<L.grid, 256, fftreg_smem(16), L.s>>>(L.d, L.off, L.n);
-  else if (e == 8) k_fftreg_rows<8><<<L.grid, 256, fftreg_smem(8), L.s>>>(L.d, L.off, L.n);
-  else k_fftreg_rows<4><<<L.grid, 256, fftreg_smem(4), L.s>>>(L.d, L.off, L.n);
+  if (e == 16) launch(L, k_fftreg_rows<16>, 256, fftreg_smem(16), L.d, L.off, L.n);
+  else if (e == 8) launch(L, k_fftreg_rows<8>, 256, fftreg_smem(8), L.d, L.off, L.n);
+  else launch(L, k_fftreg_rows<4>, 256, fftreg_smem(4), L.d, L.off, L.n);
 }
 void launch_fftreg_cols(const Launch& L, int e, int tv) {
   const size_t sm = fftreg_cols_smem(tv);
   if (tv == 2048) {
-    if (e == 16) k_fftreg_cols<16, 2048><<<L.grid, 128, sm, L.s>>>(L.d, L.off, L.n);
-    else if (e == 8) k_fftreg_cols<8, 2048><<<L.grid, 256, sm, L.s>>>(L.d, L.off, L.n);
-    else k_fftreg_cols<4, 2048><<<L.grid, 512, sm, L.s>>>(L.d, L.off, L.n);
+    if (e == 16) launch(L, k_fftreg_cols<16, 2048>, 128, sm, L.d, L.off, L.n);
+    else if (e == 8) launch(L, k_fftreg_cols<8, 2048>, 256, sm, L.d, L.off, L.n);
+    else launch(L, k_fftreg_cols<4, 2048>, 512, sm, L.d, L.off, L.n);
     return;
   }
-  if (e == 16) k_fftreg_cols<16, 4096><<<L.grid, 256, sm, L.s>>>(L.d, L.off, L.n);
-  else if (e == 8) k_fftreg_cols<8, 4096><<<L.grid, 512, sm, L.s>>>(L.d, L.off, L.n);
-  else k_fftreg_cols<4, 4096><<<L.grid, 1024, sm, L.s>>>(L.d, L.off, L.n);
+  if (e == 16) launch(L, k_fftreg_cols<16, 4096>, 256, sm, L.d, L.off, L.n);
+  else if (e == 8) launch(L, k_fftreg_cols<8, 4096>, 512, sm, L.d, L.off, L.n);
+  else launch(L, k_fftreg_cols<4, 4096>, 1024, sm, L.d, L.off, L.n);
 }
 
 
