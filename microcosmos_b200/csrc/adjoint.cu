@@ -39,6 +39,7 @@ constexpr int kMaxKK = 64;       // stencil entries per node (kernel size <= 8)
 constexpr int kPointThreads = 32;
 constexpr int kCellBucket = 16;  // entries of a cell ordered in registers
 constexpr long long kMaxCells = 4096LL * 4096;  // largest grid of the gradient path
+constexpr size_t kOverlapBytes = size_t(1) << 30;  // of a segment's inputs, up to which they are kept twice
 constexpr int kPbdThreads = 256;  // threads per rod component in the PBD kernels
 constexpr int kPbdRod = 128;      // edges, nodes and pairs of a component kept one per thread
 
@@ -1682,6 +1683,10 @@ struct mc_grad_plan {
   R r_ly, r_lfn, r_lhn;
   std::vector<StepArgs> sargs;
   cudaStream_t cap_stream = nullptr;
+  // The recomputation of a segment beside the reverse steps of the one after it (replay_segment)
+  bool overlap = false;
+  cudaStream_t replay_stream = nullptr;
+  cudaEvent_t ev_replayed[2] = {nullptr, nullptr}, ev_reversed[2] = {nullptr, nullptr}, ev_begin = nullptr;
   cudaGraphExec_t rev_graph = nullptr;  // one reverse step, replayed per step
   int rev_graph_act = -1;               // has_act the graph was captured with
 };
@@ -1770,6 +1775,42 @@ mc_status begin_fwd(mc_grad_plan* p, int t0, cudaStream_t s) {
   }
   const mc_actuation* const acts[1] = {ap};
   return mc_rollout_begin(p->fwd, &w, acts, nullptr, s);
+}
+
+// Where the inputs of step j of segment k are kept: neighbouring segments apart when they overlap.
+int segment_slot(const mc_grad_plan* p, int k, int j) { return (p->overlap && (k & 1) ? p->S : 0) + j; }
+
+// The step inputs of segment k from its checkpoint: one rollout over the segment, the populations
+// of every step's input snapshot from the open rollout (no per-step entry/exit conversion).
+mc_status replay_segment(mc_grad_plan* p, int k, cudaStream_t s) {
+  const mc_dims& D = p->dims;
+  const size_t HW = (size_t)D.H * D.W, LHW = (size_t)p->ad.lHW;
+  unsigned char* w = p->ws;
+  const int t0 = k * p->S, len = std::min(p->S, p->T - t0);
+  Slot ck = slot(p, p->r_ck, k);
+  mc_status st = copy_state_to(p, at<float>(w, p->r_wpos), at<float>(w, p->r_wvel), at<float>(w, p->r_wth),
+                               at<float>(w, p->r_wf), ck.pos, ck.vel, ck.th, ck.f, s);
+  if (st != MC_OK) return st;
+  st = begin_fwd(p, t0, s);
+  if (st != MC_OK) return st;
+  for (int j = 0; j < len; ++j) {
+    const int at_j = segment_slot(p, k, j);
+    Slot sj = slot(p, p->r_seg, at_j);
+    GC(cudaMemcpyAsync(sj.pos, at<float>(w, p->r_wpos), (size_t)D.N * 8, cudaMemcpyDeviceToDevice, s));
+    GC(cudaMemcpyAsync(sj.vel, at<float>(w, p->r_wvel), (size_t)D.N * 8, cudaMemcpyDeviceToDevice, s));
+    if (D.E) GC(cudaMemcpyAsync(sj.th, at<float>(w, p->r_wth), (size_t)D.E * 4, cudaMemcpyDeviceToDevice, s));
+    if (p->ad.fluid) {
+      st = mc::rollout_snapshot_f(p->fwd, sj.f, s);
+      if (st != MC_OK) return st;
+    } else {
+      GC(cudaMemcpyAsync(sj.f, at<float>(w, p->r_wf), 9 * LHW * 4, cudaMemcpyDeviceToDevice, s));
+    }
+    st = mc_rollout_advance(p->fwd, 1, 1, 1, s);
+    if (st != MC_OK) return st;
+    GC(cudaMemcpyAsync(w + p->r_segV.off + (size_t)at_j * al(HW * 4), w + p->r_wst.off, HW * 4,
+                       cudaMemcpyDeviceToDevice, s));
+  }
+  return mc_rollout_end(p->fwd, s);
 }
 
 mc_status run_fwd(mc_grad_plan* p, int steps, int t0, cudaStream_t s) {
@@ -2000,8 +2041,12 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
   take(p->r_wf, 9 * LHW * 4);
   p->state_ck_bytes = al(N * 8) * 2 + al(E * 4) + al(9 * LHW * 4);
   take(p->r_ck, std::max(p->nseg, 1) * p->state_ck_bytes);
-  take(p->r_seg, (size_t)S * p->state_ck_bytes);
-  take(p->r_segV, (size_t)S * al(HW * 4));
+  // a second copy of the segment's inputs, unless it is of a size that a user would notice
+  const size_t seg_bytes = (size_t)S * (p->state_ck_bytes + al(HW * 4));
+  p->overlap = p->nseg > 1 && seg_bytes <= kOverlapBytes;
+  const size_t copies = p->overlap ? 2 : 1;
+  take(p->r_seg, copies * S * p->state_ck_bytes);
+  take(p->r_segV, copies * S * al(HW * 4));
   take(p->r_rest, B * 4);
   take(p->r_pred0, N * 8);
   take(p->r_pp, (size_t)(C + 1) * N * 8);
@@ -2076,6 +2121,9 @@ void mc_grad_plan_destroy(mc_grad_plan* p) {
   if (!p) return;
   if (p->rev_graph) cudaGraphExecDestroy(p->rev_graph);
   if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
+  if (p->replay_stream) cudaStreamDestroy(p->replay_stream);
+  for (cudaEvent_t e : {p->ev_replayed[0], p->ev_replayed[1], p->ev_reversed[0], p->ev_reversed[1], p->ev_begin})
+    if (e) cudaEventDestroy(e);
   if (p->fwd) mc_plan_destroy(p->fwd);
   delete p;
 }
@@ -2119,6 +2167,11 @@ mc_status mc_grad_plan_bind(mc_grad_plan* p, void* workspace, size_t bytes, void
   }
   p->filter_ready = false;
   if (!p->cap_stream) GC(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
+  if (p->overlap) {
+    if (!p->replay_stream) GC(cudaStreamCreateWithFlags(&p->replay_stream, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&p->ev_replayed[0], &p->ev_replayed[1], &p->ev_reversed[0], &p->ev_reversed[1], &p->ev_begin})
+      if (!*e) GC(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
   GC(cudaMemsetAsync(p->ws + p->r_cnt.off, 0, p->r_cnt.bytes, s));
   GC(cudaMemsetAsync(p->ws + p->r_ovh.off, 0xff, p->r_ovh.bytes, s));
   GC(cudaMemsetAsync(p->ws + p->r_touch.off, 0, 256, s));
@@ -2351,46 +2404,52 @@ mc_status mc_grad_backward(mc_grad_plan* p, const mc_state_cot* final_cot, mc_st
     p->filter_ready = true;
   }
   int lfcur = 0;
+  // Replay of segment k - 1 beside the reverse of segment k: a replayed step keeps one SM busy for
+  // most of its time and a reverse step a few, and they share nothing but the two copies of the
+  // segment's inputs.
+  cudaStream_t rs = p->overlap ? p->replay_stream : s;
+  auto after = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
+    cudaError_t e = cudaEventRecord(ev, from);
+    return e == cudaSuccess ? cudaStreamWaitEvent(to, ev, 0) : e;
+  };
+  if (p->overlap) GC(after(p->ev_begin, s, rs));
+  // whatever happens, the caller's stream waits for the replay's
+  struct Join {
+    mc_grad_plan* p;
+    cudaStream_t from, to;
+    ~Join() {
+      if (from != to && cudaEventRecord(p->ev_begin, from) == cudaSuccess) cudaStreamWaitEvent(to, p->ev_begin, 0);
+    }
+  } join{p, rs, s};
+  mc_status st = p->nseg > 0 ? replay_segment(p, p->nseg - 1, rs) : MC_OK;
+  if (st != MC_OK) return st;
   for (int k = p->nseg - 1; k >= 0; --k) {
     const int t0 = k * p->S;
     const int len = std::min(p->S, p->T - t0);
-    Slot ck = slot(p, p->r_ck, k);
-    mc_status st = copy_state_to(p, at<float>(w, p->r_wpos), at<float>(w, p->r_wvel), at<float>(w, p->r_wth),
-                                 at<float>(w, p->r_wf), ck.pos, ck.vel, ck.th, ck.f, s);
-    if (st != MC_OK) return st;
-    // the segment's step inputs: one rollout over the segment, the populations of every
-    // step's input snapshot from the open rollout (no per-step entry/exit conversion)
-    st = begin_fwd(p, t0, s);
-    if (st != MC_OK) return st;
-    for (int j = 0; j < len; ++j) {
-      Slot sj = slot(p, p->r_seg, j);
-      GC(cudaMemcpyAsync(sj.pos, at<float>(w, p->r_wpos), (size_t)D.N * 8, cudaMemcpyDeviceToDevice, s));
-      GC(cudaMemcpyAsync(sj.vel, at<float>(w, p->r_wvel), (size_t)D.N * 8, cudaMemcpyDeviceToDevice, s));
-      if (D.E) GC(cudaMemcpyAsync(sj.th, at<float>(w, p->r_wth), (size_t)D.E * 4, cudaMemcpyDeviceToDevice, s));
-      if (d.fluid) {
-        st = mc::rollout_snapshot_f(p->fwd, sj.f, s);
+    if (p->overlap) {
+      GC(after(p->ev_replayed[k & 1], rs, s));
+      if (k > 0) {
+        // segment k - 1 goes where segment k + 1 was
+        if (k + 1 < p->nseg) GC(cudaStreamWaitEvent(rs, p->ev_reversed[(k + 1) & 1], 0));
+        st = replay_segment(p, k - 1, rs);
         if (st != MC_OK) return st;
-      } else {
-        GC(cudaMemcpyAsync(sj.f, at<float>(w, p->r_wf), 9 * LHW * 4, cudaMemcpyDeviceToDevice, s));
       }
-      st = mc_rollout_advance(p->fwd, 1, 1, 1, s);
+    } else if (k < p->nseg - 1) {
+      st = replay_segment(p, k, s);
       if (st != MC_OK) return st;
-      GC(cudaMemcpyAsync(w + p->r_segV.off + (size_t)j * al(HW * 4), w + p->r_wst.off, HW * 4,
-                         cudaMemcpyDeviceToDevice, s));
     }
-    st = mc_rollout_end(p->fwd, s);
-    if (st != MC_OK) return st;
     // per-step inputs of the segment (the cotangent of f alternates between two buffers)
     p->sargs.assign(len, StepArgs{});
     for (int j = len - 1; j >= 0; --j) {
-      Slot sj = slot(p, p->r_seg, j);
+      const int at_j = segment_slot(p, k, j);
+      Slot sj = slot(p, p->r_seg, at_j);
       StepArgs& a = p->sargs[j];
       a.t = t0 + j;
       a.pos = sj.pos;
       a.vel = sj.vel;
       a.th = sj.th;
       a.f = sj.f;
-      a.V = reinterpret_cast<const float*>(w + p->r_segV.off + (size_t)j * al(HW * 4));
+      a.V = reinterpret_cast<const float*>(w + p->r_segV.off + (size_t)at_j * al(HW * 4));
       a.lf_in = at<float>(w, lfcur ? p->r_lf1 : p->r_lf0);
       a.lf_out = at<float>(w, lfcur ? p->r_lf0 : p->r_lf1);
       if (d.fluid) lfcur ^= 1;
@@ -2423,8 +2482,8 @@ mc_status mc_grad_backward(mc_grad_plan* p, const mc_state_cot* final_cot, mc_st
     }
     for (int j = len - 1; j >= 0; --j) GC(cudaGraphLaunch(p->rev_graph, s));
     GC(cudaGetLastError());
+    if (p->overlap) GC(cudaEventRecord(p->ev_reversed[k & 1], s));
   }
-  (void)d;
   auto out = [&](float* dst, const mc_grad_plan::R& r, size_t n) -> cudaError_t {
     if (!dst || n == 0) return cudaSuccess;
     return cudaMemcpyAsync(dst, w + r.off, n, cudaMemcpyDeviceToDevice, s);

@@ -44,3 +44,14 @@ def test_rod_lengths(nodes):
 def test_iteration_counts(cycles):
     check(case(32, 32, 2, 10, seed=cycles),
           O.Config(enable_fluid=False, enable_steric=False, cycles_per_step=cycles))
+
+
+@pytest.mark.parametrize("every", [1, 2, 3, 6])
+def test_segments_recomputed_beside_the_reverse(every):
+    """The recomputed inputs of neighbouring segments are kept apart: the same bits as one segment."""
+    sc, steps = case(40, 32, 3, 12, seed=every), 7
+    cot = cotangent(sc, 2)
+    want = gpu_grads(sc, O.Config(), steps, cot, ckpt=steps)[1]
+    got = gpu_grads(sc, O.Config(), steps, cot, ckpt=every)[1]
+    for k in want:
+        assert got[k].tobytes() == want[k].tobytes(), k
