@@ -330,7 +330,7 @@ namespace mc {
 // it: the filter is its own adjoint).  filter_prepare writes a descriptor and CTA offset
 // tables (filter_desc_bytes() bytes at `dev`) naming in -> tmp -> out; it needs the plan's
 // descriptor of a rollout call (mc_rollout_begin has run once).  filter_launch enqueues
-// the same row and column kernels as a step.
+// the same row and column kernels as a step, chained to the kernel before on `s`.
 size_t filter_desc_bytes();
 cudaError_t filter_prepare(mc_plan* p, void* dev, const float* in, float* tmp, float* out, cudaStream_t s);
 void filter_launch(mc_plan* p, const void* dev, cudaStream_t s);

@@ -1397,6 +1397,7 @@ void filter_launch(mc_plan* p, const void* dev, cudaStream_t s) {
     l.n = 1;
     l.grid = cnt[k];
     l.s = s;
+    l.chained = true;
     return l;
   };
   if (cnt[0]) launch_fftreg_rows(launch(0), p->fft_e);
