@@ -41,6 +41,8 @@ constexpr int kPointThreads = 32;
 constexpr int kCellBucket = 16;  // entries of a cell ordered in registers
 constexpr long long kMaxCells = 4096LL * 4096;  // largest grid of the gradient path
 constexpr size_t kOverlapBytes = size_t(1) << 30;  // of a segment's inputs, up to which they are kept twice
+constexpr int kDirectSteps = 64;    // steps up to which forward steps are launched without graphs (step_graphs)
+constexpr int kDirectReverse = 16;  // the same for reverse steps
 constexpr int kPbdThreads = 256;  // threads per rod component in the PBD kernels
 constexpr int kPbdRod = 128;      // edges, nodes and pairs of a component kept one per thread
 
@@ -1850,6 +1852,25 @@ mc_state working_state(mc_grad_plan* p) {
   return w;
 }
 
+// Values grouped by key, in the order given: each(put) calls put(key, value) for all of them, the
+// same ones each time.
+template <class F>
+void group_by(int groups, std::vector<int>& start, std::vector<int>& list, F&& each) {
+  start.assign(groups + 1, 0);
+  each([&](int key, int) { ++start[key + 1]; });
+  for (int g = 0; g < groups; ++g) start[g + 1] += start[g];
+  list.resize(start[groups]);
+  std::vector<int> next(start.begin(), start.end() - 1);
+  each([&](int key, int value) { list[next[key]++] = value; });
+}
+
+// Short rollouts launch their kernels directly: a plan of one gradient would spend more on making
+// its graphs (some 0.25 ms each to capture and instantiate, 0.14 to destroy, with the GPU idle
+// before the first and after the last) than on launching each kernel (2 us).  48 steps at 256^2
+// 13.9 -> 12.9 ms, 12 steps at 640^2 8.6 -> 7.4.  A reverse step has three times the kernels of a
+// forward one, so that its graphs pay from fewer steps on.
+int step_graphs(const mc_grad_plan* p) { return p->T > kDirectSteps; }
+
 // Open a rollout of the forward plan on the working state, actuated from step t0 (the
 // static rest angles restored first when there is no actuation).
 mc_status begin_fwd(mc_grad_plan* p, int t0, cudaStream_t s) {
@@ -1899,7 +1920,7 @@ mc_status replay_segment(mc_grad_plan* p, int k, cudaStream_t s) {
     } else {
       GC(cudaMemcpyAsync(sj.f, at<float>(w, p->r_wf), 9 * LHW * 4, cudaMemcpyDeviceToDevice, s));
     }
-    st = mc_rollout_advance(p->fwd, 1, 1, 1, s);
+    st = mc_rollout_advance(p->fwd, 1, step_graphs(p), 1, s);
     if (st != MC_OK) return st;
     GC(cudaMemcpyAsync(w + p->r_segV.off + (size_t)at_j * al(HW * 4), w + p->r_wst.off, HW * 4,
                        cudaMemcpyDeviceToDevice, s));
@@ -1924,7 +1945,7 @@ mc_status run_fwd(mc_grad_plan* p, int steps, int t0, cudaStream_t s) {
                        cudaMemcpyDeviceToDevice, s));
   }
   const mc_actuation* const acts[1] = {ap};
-  return mc_rollout(p->fwd, &w, steps, acts, nullptr, 1, s);
+  return mc_rollout(p->fwd, &w, steps, acts, nullptr, step_graphs(p), s);
 }
 
 // Enqueues kernels, each chained to the one before on its stream.
@@ -1992,11 +2013,11 @@ void reverse_step(mc_grad_plan* p, const AD& d, cudaStream_t s) {
   go(k_steric_adj_cic, nblk(d.N, TB), TB, d);
 }
 
-// The graphs a segment's reverse is made of.  With two tapes (steps of odd and even number), the
+// What a segment's reverse is made of, graphs or direct launches.  With two tapes (steps of odd and even number), the
 // tape of step j - 1 runs beside the reverse of step j: neither fills more than a few SMs.
 enum RevGraph { kTapeEven, kTapeOdd, kBothEven, kBothOdd, kReverseEven, kWhole };
 
-void capture_reverse(mc_grad_plan* p, int which, cudaStream_t s) {
+void enqueue_reverse(mc_grad_plan* p, int which, cudaStream_t s) {
   const int par = which & 1;
   AD d = p->ad;
   if (which == kWhole) {
@@ -2029,7 +2050,7 @@ mc_status rev_graph(mc_grad_plan* p, int which, cudaGraphExec_t* out) {
   if (!x) {
     cudaGraph_t g;
     GC(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
-    capture_reverse(p, which, p->cap_stream);
+    enqueue_reverse(p, which, p->cap_stream);
     cudaError_t e = cudaStreamEndCapture(p->cap_stream, &g);
     if (e != cudaSuccess) return gfail(MC_ERR_CUDA, std::string("capture of the reverse step: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(&x, g, 0);
@@ -2100,26 +2121,18 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
         return gfail(MC_ERR_INVALID, "bending_pairs index out of range");
       }
   // gather lists in scatter order: sources first (in edge order), then targets
-  p->n_start.assign(D.N + 1, 0);
-  std::vector<std::vector<int>> nl(D.N);
-  for (int e = 0; e < D.E; ++e) nl[p->pairs[2 * e]].push_back(e * 2);
-  for (int e = 0; e < D.E; ++e) nl[p->pairs[2 * e + 1]].push_back(e * 2 + 1);
+  auto ends = [](const std::vector<int>& ab, int count) {
+    return [&ab, count](auto&& put) {
+      for (int q = 0; q < 2; ++q)
+        for (int i = 0; i < count; ++i) put(ab[2 * i + q], i * 2 + q);
+    };
+  };
+  group_by(D.N, p->n_start, p->n_list, ends(p->pairs, D.E));
   p->ndeg.resize(D.N);
-  for (int n = 0; n < D.N; ++n) {
-    p->n_start[n + 1] = p->n_start[n] + (int)nl[n].size();
-    p->n_list.insert(p->n_list.end(), nl[n].begin(), nl[n].end());
-    p->ndeg[n] = std::max((float)nl[n].size(), 1.0f);
-  }
-  p->e_start.assign(D.E + 1, 0);
-  std::vector<std::vector<int>> el(D.E);
-  for (int b = 0; b < D.B; ++b) el[p->bpairs[2 * b]].push_back(b * 2);
-  for (int b = 0; b < D.B; ++b) el[p->bpairs[2 * b + 1]].push_back(b * 2 + 1);
+  for (int n = 0; n < D.N; ++n) p->ndeg[n] = std::max((float)(p->n_start[n + 1] - p->n_start[n]), 1.0f);
+  group_by(D.E, p->e_start, p->e_list, ends(p->bpairs, D.B));
   p->edeg.resize(D.E);
-  for (int e = 0; e < D.E; ++e) {
-    p->e_start[e + 1] = p->e_start[e] + (int)el[e].size();
-    p->e_list.insert(p->e_list.end(), el[e].begin(), el[e].end());
-    p->edeg[e] = std::max((float)el[e].size(), 1.0f);
-  }
+  for (int e = 0; e < D.E; ++e) p->edeg[e] = std::max((float)(p->e_start[e + 1] - p->e_start[e]), 1.0f);
   {
     // rod components: union-find over the edges; members listed in ascending order
     std::vector<int> par(D.N);
@@ -2142,21 +2155,15 @@ mc_status mc_grad_plan_create(const mc_dims* dims, const mc_config* cfg, float d
       if (cid[r] < 0) cid[r] = nc++;
       cid[n] = cid[r];
     }
-    std::vector<std::vector<int>> cn(nc), ce(nc), cb(nc);
-    for (int n = 0; n < D.N; ++n) cn[cid[n]].push_back(n);
-    for (int e = 0; e < D.E; ++e) ce[cid[p->pairs[2 * e]]].push_back(e);
-    for (int b = 0; b < D.B; ++b) cb[cid[p->pairs[2 * p->bpairs[2 * b]]]].push_back(b);
-    p->c_nstart.assign(1, 0);
-    p->c_estart.assign(1, 0);
-    p->c_bstart.assign(1, 0);
-    for (int c = 0; c < nc; ++c) {
-      p->c_nodes.insert(p->c_nodes.end(), cn[c].begin(), cn[c].end());
-      p->c_edges.insert(p->c_edges.end(), ce[c].begin(), ce[c].end());
-      p->c_bps.insert(p->c_bps.end(), cb[c].begin(), cb[c].end());
-      p->c_nstart.push_back((int)p->c_nodes.size());
-      p->c_estart.push_back((int)p->c_edges.size());
-      p->c_bstart.push_back((int)p->c_bps.size());
-    }
+    group_by(nc, p->c_nstart, p->c_nodes, [&](auto&& put) {
+      for (int n = 0; n < D.N; ++n) put(cid[n], n);
+    });
+    group_by(nc, p->c_estart, p->c_edges, [&](auto&& put) {
+      for (int e = 0; e < D.E; ++e) put(cid[p->pairs[2 * e]], e);
+    });
+    group_by(nc, p->c_bstart, p->c_bps, [&](auto&& put) {
+      for (int b = 0; b < D.B; ++b) put(cid[p->pairs[2 * p->bpairs[2 * b]]], b);
+    });
   }
   // forward plan (same kernels as mc_rollout)
   const int32_t* pp[1] = {pairs};
@@ -2640,6 +2647,10 @@ mc_status mc_grad_backward(mc_grad_plan* p, const mc_state_cot* final_cot, mc_st
     if (p->rev_graph_act != d.has_act) drop_rev_graphs(p);
     p->rev_graph_act = d.has_act;
     auto run = [&](int which) -> mc_status {
+      if (p->T <= kDirectReverse) {
+        enqueue_reverse(p, which, s);
+        return MC_OK;
+      }
       cudaGraphExec_t g;
       mc_status gs = rev_graph(p, which, &g);
       if (gs == MC_OK) GC(cudaGraphLaunch(g, s));

@@ -1381,9 +1381,7 @@ cudaError_t filter_prepare(mc_plan* p, void* dev, const float* in, float* tmp, f
     std::memcpy(host.data() + align_up(sizeof(RDesc), 256) + 256 * k, off, sizeof(off));
   }
   const Upload u{dev, host.data(), host.size()};
-  cudaError_t e = stage_uploads(&u, 1, s);
-  if (e != cudaSuccess) return e;
-  return cudaStreamSynchronize(s);  // `host` is a temporary
+  return stage_uploads(&u, 1, s);
 }
 
 void filter_launch(mc_plan* p, const void* dev, cudaStream_t s) {
