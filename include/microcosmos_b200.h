@@ -391,6 +391,21 @@ mc_status mc_env_act(const void* table, int32_t n, void* stream);
  * base.py:140-149); the energy source, step counter and done flag are left alone. */
 mc_status mc_env_observe(const void* table, int32_t n, int32_t advance, void* stream);
 
+/* The same for a batch of environments of equal sizes whose actions and results are rows of
+ * the caller's arrays: the actions are read from d_rest (n x E) and d_angle (n x B) instead of
+ * the buffers named in the table (null: from those), the results are written to the arrays of
+ * `outputs` as well (a null member, or null outputs: not). */
+typedef struct mc_env_outputs {
+  float* observation;   /* n x 5N */
+  float* reward;        /* n */
+  uint8_t* done;        /* n: 0 or 1 */
+  int32_t* steps;       /* n: the step counters */
+  float* energy_center; /* n x 2 */
+} mc_env_outputs;
+mc_status mc_env_act_batch(const void* table, int32_t n, const float* d_rest, const float* d_angle, void* stream);
+mc_status mc_env_observe_batch(const void* table, int32_t n, int32_t advance, const mc_env_outputs* outputs,
+                               void* stream);
+
 /* ------------------------------------------------------------------ frames
  * The reference's render() of a recorded rollout (src/microcosmos/rendering.py:20-80)
  * into a caller-owned device buffer, no display or graphics API involved.  Inputs (device):

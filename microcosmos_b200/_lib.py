@@ -102,6 +102,10 @@ class McEnv(ctypes.Structure):
                 ("segment_fitness", ctypes.c_void_p)]
 
 
+class McEnvOutputs(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("observation", "reward", "done", "steps", "energy_center")]
+
+
 # name -> (restype, argtypes); every symbol declared in include/microcosmos_b200.h
 SIGNATURES = {
     "mc_plan_create": (ctypes.c_int, [ctypes.c_int32, ctypes.POINTER(McDims), ctypes.POINTER(McConfig),
@@ -162,6 +166,10 @@ SIGNATURES = {
     "mc_env_table_upload": (ctypes.c_int, [ctypes.POINTER(McEnv), ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]),
     "mc_env_act": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]),
     "mc_env_observe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]),
+    "mc_env_act_batch": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p,
+                                        ctypes.c_void_p]),
+    "mc_env_observe_batch": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32,
+                                            ctypes.POINTER(McEnvOutputs), ctypes.c_void_p]),
     "mc_render_scratch_bytes": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
     "mc_render_frames": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,

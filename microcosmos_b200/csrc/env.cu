@@ -17,13 +17,15 @@ namespace mc {
 
 constexpr int kEnvThreads = 256;
 
-__global__ void __launch_bounds__(kEnvThreads) k_env_act(const mc_env* __restrict__ envs) {
+// d_rest, d_angle: the batch's actions, rows of E and B per environment, or null for the table's own
+__global__ void __launch_bounds__(kEnvThreads) k_env_act(const mc_env* __restrict__ envs, const float* d_rest,
+                                                         const float* d_angle) {
   const mc_env& e = envs[blockIdx.x];
-  for (int i = threadIdx.x; i < e.E; i += blockDim.x)
-    e.rest_lengths[i] = e.d_rest_length ? e.base_rest_lengths[i] + e.d_rest_length[i] : e.base_rest_lengths[i] + 0.0f;
+  const float* dr = d_rest ? d_rest + (size_t)blockIdx.x * e.E : e.d_rest_length;
+  const float* da = d_angle ? d_angle + (size_t)blockIdx.x * e.B : e.d_bending_angle;
+  for (int i = threadIdx.x; i < e.E; i += blockDim.x) e.rest_lengths[i] = e.base_rest_lengths[i] + (dr ? dr[i] : 0.0f);
   for (int i = threadIdx.x; i < e.B; i += blockDim.x)
-    e.bending_rest_angles[i] =
-        e.d_bending_angle ? e.base_bending_rest_angles[i] + e.d_bending_angle[i] : e.base_bending_rest_angles[i] + 0.0f;
+    e.bending_rest_angles[i] = e.base_bending_rest_angles[i] + (da ? da[i] : 0.0f);
 }
 
 // Sum of one value per thread over the CTA in a fixed order; every thread gets the result.
@@ -39,7 +41,11 @@ __device__ float block_sum(float v, float* scratch) {
   return t;
 }
 
-__global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __restrict__ envs, int advance) {
+// `to`: where the results are written a second time for the caller, or nulls.  A batch's results
+// were copied out by five more launches, 2 us each for a few KB (64 environments at 256^2: 124 us a
+// step with them and the copies of the actions, 102 without).
+__global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __restrict__ envs, int advance,
+                                                             mc_env_outputs to) {
   __shared__ float scratch[kEnvThreads / 32];
   __shared__ float s_center[2];
   const mc_env& e = envs[blockIdx.x];
@@ -47,6 +53,8 @@ __global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __res
   if (threadIdx.x == 0 && !advance) {
     s_center[0] = e.energy_center[0];
     s_center[1] = e.energy_center[1];
+    if (to.steps) to.steps[blockIdx.x] = *e.time;
+    if (to.done) to.done[blockIdx.x] = *e.done != 0;
   }
   if (threadIdx.x == 0 && advance) {
     // (center + normal * std) % (w, h), floored (base.py:187-190)
@@ -62,6 +70,8 @@ __global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __res
     const int t = *e.time + 1;
     *e.time = t;
     *e.done = t >= e.max_steps ? 1 : 0;
+    if (to.steps) to.steps[blockIdx.x] = t;
+    if (to.done) to.done[blockIdx.x] = t >= e.max_steps;
   }
   // centre of mass (base.py:114-115)
   float sx = 0.0f, sy = 0.0f;
@@ -87,6 +97,9 @@ __global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __res
     obs[4 * N + i] = e.energy_amplitude * expf(-d2 / e.energy_two_size_sq);
   }
   __syncthreads();
+  if (to.observation)
+    for (int i = threadIdx.x; i < 5 * N; i += blockDim.x) to.observation[(size_t)blockIdx.x * 5 * N + i] = obs[i];
+  if (to.energy_center && threadIdx.x < 2) to.energy_center[2 * blockIdx.x + threadIdx.x] = s_center[threadIdx.x];
   // per node range: sum of its energies; reward = sum over the ranges (multi_agent.py:201-212)
   const int nseg = e.num_segments > 0 ? e.num_segments : 1;
   float reward = 0.0f;
@@ -99,7 +112,10 @@ __global__ void __launch_bounds__(kEnvThreads) k_env_observe(const mc_env* __res
     if (threadIdx.x == 0 && e.segment_fitness) e.segment_fitness[g] = s;
     reward = reward + s;
   }
-  if (threadIdx.x == 0) *e.reward = reward;
+  if (threadIdx.x == 0) {
+    *e.reward = reward;
+    if (to.reward) to.reward[blockIdx.x] = reward;
+  }
 }
 
 }  // namespace mc
@@ -138,15 +154,26 @@ mc_status mc_env_table_upload(const mc_env* envs, int32_t n, void* table, void* 
 }
 
 mc_status mc_env_act(const void* table, int32_t n, void* stream) {
+  return mc_env_act_batch(table, n, nullptr, nullptr, stream);
+}
+
+mc_status mc_env_act_batch(const void* table, int32_t n, const float* d_rest, const float* d_angle, void* stream) {
   if (n <= 0 || !table) return env_fail(MC_ERR_INVALID, "mc_env_act: empty table");
-  mc::k_env_act<<<n, mc::kEnvThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const mc_env*>(table));
+  mc::k_env_act<<<n, mc::kEnvThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const mc_env*>(table), d_rest,
+                                                                              d_angle);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? MC_OK : env_fail(MC_ERR_CUDA, cudaGetErrorString(err));
 }
 
 mc_status mc_env_observe(const void* table, int32_t n, int32_t advance, void* stream) {
+  return mc_env_observe_batch(table, n, advance, nullptr, stream);
+}
+
+mc_status mc_env_observe_batch(const void* table, int32_t n, int32_t advance, const mc_env_outputs* outputs,
+                               void* stream) {
   if (n <= 0 || !table) return env_fail(MC_ERR_INVALID, "mc_env_observe: empty table");
-  mc::k_env_observe<<<n, mc::kEnvThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const mc_env*>(table), advance ? 1 : 0);
+  mc::k_env_observe<<<n, mc::kEnvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const mc_env*>(table), advance ? 1 : 0, outputs ? *outputs : mc_env_outputs{});
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? MC_OK : env_fail(MC_ERR_CUDA, cudaGetErrorString(err));
 }

@@ -41,6 +41,12 @@ class BatchedState:
         return self._owner._centers
 
 
+def _readable(a, buf):
+    """Whether the kernels can read tensor ``a`` in the place of ``buf``."""
+    return (type(a) is torch.Tensor and a.dtype == buf.dtype and a.device == buf.device and a.layout == torch.strided
+            and a.is_contiguous() and a.numel() == buf.numel() and not a.is_neg())
+
+
 class BatchedEnv:
     def __init__(self, env: Environment, batch_size: int, device="cuda"):
         if batch_size < 1:
@@ -93,31 +99,37 @@ class BatchedEnv:
         if state is not self._state:
             raise ValueError("step() takes the state returned by this batch's reset()/step()")
         B = self.batch_size
-        if actions is not None:
-            for name, buf in (("d_rest_length", self._d_rest), ("d_bending_angle", self._d_ang)):
-                a = actions.get(name)
-                if a is None:
-                    buf.zero_()
-                else:
-                    buf.copy_(torch.as_tensor(a, dtype=_F32).reshape(buf.shape))
-        else:
-            self._d_rest.zero_()
-            self._d_ang.zero_()
+        acts = []
+        for name, buf in (("d_rest_length", self._d_rest), ("d_bending_angle", self._d_ang)):
+            a = None if actions is None else actions.get(name)
+            if _readable(a, buf):
+                acts.append(ctypes.c_void_p(a.data_ptr()))  # read in place
+                continue
+            if a is None:
+                buf.zero_()
+            else:
+                buf.copy_(torch.as_tensor(a, dtype=_F32).reshape(buf.shape))
+            acts.append(None)
         if self._noise is not None:
             g = np.random.default_rng(None if keys is None else [int(np.asarray(k).ravel()[-1]) for k in keys])
             self._noise.copy_(torch.as_tensor(g.standard_normal((B, 2)).astype(np.float32)))
         lib = _lib.load()
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
         ptr = ctypes.c_void_p(self._table["ptr"])
-        _lib.check(lib.mc_env_act(ptr, B, stream))
+        _lib.check(lib.mc_env_act_batch(ptr, B, acts[0], acts[1], stream))
         if not self._open:
             self._plan.begin([s.device for s in state.states])
             self._open = True
         self._plan.advance(1, last=True)
-        self._observe(advance=True)
+        # the results straight into tensors of the caller's
         out = self._table["out"]
-        info = {"steps": state.time.clone(), "energy_center": state.energy_center.clone()}
-        return out["obs"].clone(), state, out["reward"].clone(), out["done"].bool(), info
+        obs, reward = torch.empty_like(out["obs"]), torch.empty_like(out["reward"])
+        done = torch.empty_like(out["done"], dtype=torch.bool)
+        info = {"steps": torch.empty_like(state.time), "energy_center": torch.empty_like(state.energy_center)}
+        to = _lib.McEnvOutputs(obs.data_ptr(), reward.data_ptr(), done.data_ptr(), info["steps"].data_ptr(),
+                               info["energy_center"].data_ptr())
+        _lib.check(lib.mc_env_observe_batch(ptr, B, 1, ctypes.byref(to), stream))
+        return obs, state, reward, done, info
 
     def fitness_per_creature(self, state: BatchedState):
         self._observe(advance=False)
