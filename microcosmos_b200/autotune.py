@@ -6,7 +6,7 @@ Three kernels have a free shape:
     up to 4 warps per CTA, each looping over rows_per_cta / 4 rows);
   * the power-of-two FFT kernels of the steric filter: each thread holds 4, 8 or 16
     values in registers (more values: fewer instructions per value; fewer: more threads);
-  * the tile kernel that sorts the IB and cloud-in-cell contributions: 128 or 256 threads
+  * the tile kernel that sorts the cloud-in-cell contributions: 128 or 256 threads
     per CTA, and 512 or 1024 contributions per tile sorted in shared memory;
   * the IB iterations: separate launches per phase, or (when asked for) one thread-block
     cluster of CTAs per rollout with hardware cluster barriers between the phases.

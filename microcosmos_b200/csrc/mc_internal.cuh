@@ -25,7 +25,7 @@ constexpr int kLbmTileX = 128;     // dense LBM CTA tile: 32 lanes x 4 cells
 constexpr int kStageCells = 1024;  // staged dense pass: lattice cells per item (a band of whole rows)
 constexpr int kStagedThreads = 256;  // ... and threads per CTA (4 cells each)
 constexpr int kConvTile = 32;     // steric direct convolution: 32 x 32 outputs per CTA
-constexpr int kConvMaxR = 24;     // largest tap radius of the direct convolution       //                    8 rows
+constexpr int kConvMaxR = 24;     // largest tap radius of the direct convolution
 constexpr int kRunRow = 16;        // entries of a touched cell's run row (k_ib_heads sorts as many in registers)
 constexpr int kCicCap = 512;       // minimum CIC bin capacity per tile
 constexpr int kMaxBinCap = 8192;   // largest bin capacity (the tile sort keeps 4 x cap words in shared memory)

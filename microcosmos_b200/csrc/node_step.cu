@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kNodeStepMaxThreads, 1)
   __shared__ __align__(16) unsigned char desc_bytes[sizeof(RDesc)];
   __shared__ int warp_sum[kNodeStepMaxThreads / 32];
   const int r = blockIdx.x;
-  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5;
   // the descriptor, once: its fields are used in every phase
   {
     static_assert(sizeof(RDesc) % 4 == 0, "copied by words");
@@ -602,7 +602,6 @@ __global__ void __launch_bounds__(kNodeStepMaxThreads, 1)
       d.dep[m.hcell()[h]] = acc;
     }
   }
-  (void)lane;
 }
 
 void launch_node_step(const RDesc* d, int n, int* tdev, const NodeStepShape& shape, int parity, int main, int next,

@@ -223,7 +223,7 @@ class Plan:
         ``steric_method``: 0 = per rollout (direct convolution where it applies, else
         FFT), 1 = FFT, 2 = direct convolution.  ``fft_values``: values per thread of the
         power-of-two FFT kernels (4, 8, 16; 0 = the library's choice).  ``bin_threads``:
-        threads per CTA of the contribution-sorting tile kernel (64, 128, 256; 0 = 128).
+        threads per CTA of the tile kernel of the steric deposit (64, 128, 256; 0 = 128).
         ``bin_sort_capacity``: contributions per tile sorted in shared memory (0 = 2048).
         ``ib_cluster``: CTAs per rollout cluster for the IB iterations (0 = separate launches).
         ``lbm_stages``: 2..6 runs the staged dense pass (row bands copied into shared
