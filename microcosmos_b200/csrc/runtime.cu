@@ -1015,10 +1015,11 @@ bool chain_launches(const mc_plan* p) { return !p->profiling && p->grid[K_NODES]
 //               its result;
 //   main:       ib(t) (touched cells, iterations, body force per touched cell), tail(t) (node
 //               reaction) and pipeline(t+1), each kernel chained to the one before.
-// The next body starts when both have finished.  In a compact plan one node-step launch
+// The next body starts when both have finished (`follows`: it is the next in the same graph, and its
+// dense pass may start on its own, see there).  In a compact plan one node-step launch
 // is pipeline(t) after the filter, ib(t), tail(t) and pipeline(t+1) up to the filter.
-int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool first, bool has_next, cudaStream_t s,
-                     bool capture, mc_status* err) {
+int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool first, bool follows, bool has_next,
+                     cudaStream_t s, bool capture, mc_status* err) {
   const bool compact = is_compact(p);
   int64_t k = 0;
   p->chain = chain_launches(p);
@@ -1048,7 +1049,11 @@ int64_t enqueue_body(mc_plan* p, int parity, int write_u, int rec_fields, bool f
   };
   cudaStream_t s2 = p->lbm_stream;
   if (p->any_fluid) {
-    fork(p->ev_lfork, s, s2, "fork to the dense-pass stream");
+    // Behind the touched cells' collision of the step before it in the same graph, the dense pass
+    // does not wait for that step's pipeline(t+1) but runs beside it.  Per pass 2522 -> 2490 us at
+    // 2048^2, 2158 -> 2131 at 1024^2, 3991 -> 3949 for 64 uneven rollouts; 256 of them, which fill
+    // the GPU, took 7680 -> 7930, and a 180 x 300 lattice with the node step 3878 -> 3905.
+    if (!follows || compact || !p->chain) fork(p->ev_lfork, s, s2, "fork to the dense-pass stream");
     k += enqueue_lbm(p, parity, write_u, s2, capture);
   }
   if (first) k += enqueue_pipeline(p, false, s, false, capture, err);
@@ -1126,7 +1131,7 @@ mc_status run_steps(mc_plan* p, int num, int use_graph, int last, cudaStream_t s
         MC_CUDA(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
         int64_t kk = 0;
         for (int j = 0; j < ns && err == MC_OK; ++j)
-          kk += enqueue_body(p, (parity + j) & 1, wu, p->rec_fields, first && j == 0, j + 1 < ns ? true : has_next,
+          kk += enqueue_body(p, (parity + j) & 1, wu, p->rec_fields, first && j == 0, j > 0, j + 1 < ns ? true : has_next,
                              p->cap_stream, true, &err);
         cudaError_t e = cudaStreamEndCapture(p->cap_stream, &graph);
         if (err != MC_OK) return err;
@@ -1147,7 +1152,7 @@ mc_status run_steps(mc_plan* p, int num, int use_graph, int last, cudaStream_t s
       p->pending_next = has_next;
       continue;
     }
-    launches += enqueue_body(p, parity, write_u, p->rec_fields, first, has_next, s, false, &err);
+    launches += enqueue_body(p, parity, write_u, p->rec_fields, first, false, has_next, s, false, &err);
     if (err != MC_OK) return err;
     p->step += 1;
     remaining -= 1;
