@@ -33,7 +33,8 @@ __host__ __device__ constexpr int chain_smem(int S) { return (kThetaChunk + 2) *
 // own (chain_warps) help with the sines and cosines.
 struct Team {
   int warp, warps;  // this warp's index in the team, and the team's warps
-  int bar;          // the team's named barrier; bar + 1 is that of its first warps, when the rod has fewer
+  int bar;          // the team's named barrier; bar + 1 is that of its first warps, when the rod has fewer:
+                    // its count changes from rod to rod, so the whole team meets at `bar` in between
   __device__ __forceinline__ void sync() const {
     if (warps == 1)
       __syncwarp();
@@ -455,6 +456,10 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
       cosserat_rod<true>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
     else if (act)
       cosserat_rod<false>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
+    // All warps of the team, those the rod does not use too: its exchange buffers and its barrier
+    // (bar + 1, with this rod's warps) are free for the team's next rod.  A PBD rod ends with such
+    // a barrier in pbd_iterations.  (A team of the chain kernel has one rod.)
+    if (!CHAINED) tm.sync();
   }
   else if (several)
     pbd_iterations<true>(late, d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
