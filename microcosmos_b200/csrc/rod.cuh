@@ -80,11 +80,12 @@ __device__ __forceinline__ float fmod_near(float x, float y) {
 // "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
 // 34, 1990): for the square root, g ~ sqrt(s) and h ~ 1 / (2 sqrt(s)) are refined together and
 // the exact residual s - g g corrects g; for a quotient, with r = RN(1 / L), two corrections by
-// the exact residual v - L q.  The root equals sqrtf for every significand (all floats of [1, 4)
-// times even powers of two in 2^+-38 compared) and r equals 1 / L for all 2^23 significands.
-// Valid for s >= 2^-50 (a segment's components are min-image differences, so multiples of 2^-23,
-// and below 2^35); there the reference's floor of the length (1e-8) does not act either.  A zero
-// component may lose its sign, which no later sum can show.
+// the exact residual v - L q.  The root equals sqrtf for every float from 2^-50 to 2^38 and r equals
+// 1 / L for every significand (tests/rod_arithmetic.cu compares them, and quotients and whole rods
+// with the general path).  The bounds: s >= 2^-50, where the reference's floor of the length (1e-8)
+// does not act either; components are min-image differences, so multiples of 2^-23, and at most
+// half a domain's side, so that s stays far below 2^38.  A zero component may lose its sign, which
+// no later sum can show.
 constexpr float kNearLength2 = 0x1p-50f;
 __device__ __forceinline__ float2 unit_near(float2 v, float s, float& L) {
   float y, r;
