@@ -853,7 +853,10 @@ __device__ __forceinline__ const float2* step_positions(const AD& d) {
 // The multi-direct forcing rounds and their reverse, one launch per phase.  (All phases in one
 // launch of a cluster of 8 CTAs with its hardware barrier between them took as long, 48 us against
 // 51 for five rounds of 384 points, and longer from 4,096 points: a phase is its dependent loads.)
-// Each phase reads its indices and weights before it waits for the phase before.
+// Each phase reads before the wait what its predecessor does not write.  k_ib_interp comes behind
+// k_macro (uc, inv) or k_ib_spread (uc); k_ib_spread behind k_ib_interp (sraw, s_tmp); k_ib_rev_node
+// behind k_lbm_adj1 (luc, lv, lrho, lf0p) or k_ib_rev_cell (luc); k_ib_rev_cell behind k_ib_rev_node
+// (lnv, s_tmp).
 template <int KK>
 __device__ __forceinline__ void tape_interp(const AD& d, int n, int it) {
   PointTaps<KK, false> taps;

@@ -589,8 +589,9 @@ __device__ __forceinline__ void ib_correct(const RDesc& d, int p, float2 v, floa
   d.delta[p] = make_float2(sx * cf, sy * cf);
 }
 
-// What a round reads that the kernel before it does not write (the point's velocity, slots and
-// weights, after the first round) is read before the wait for that kernel.
+// What a round reads that its predecessor does not write is read before the wait: after the first
+// round the predecessor is k_ib_spread, which writes s_uc and s_f, and the point's velocity, slots
+// and weights are older.
 template <int K2>
 __device__ __forceinline__ void interp_point(const RDesc& d, int p, bool on, int it) {
   if (it == 0) after_previous();  // k_ib_heads writes the slots
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
   // the plan's last round also computes each touched cell's body force (k_ib_finalize's
   // work for the same cell) when every rollout of the plan runs the same number of rounds
   const bool fin = fuse_finalize && it == d.ib_iters - 1;
-  // k_ib_interp, the kernel before, writes delta only: all else is read before the wait for it
+  // the predecessor, k_ib_interp, writes delta only: all else is read before the wait for it
   const int heads = __ldcg(d.ib_ctl + 2);
   const bool on = it < d.ib_iters && p < heads;
   int2 run = make_int2(0, 0);

@@ -177,11 +177,16 @@ __device__ __forceinline__ int find_rollout(const int* __restrict__ off, int n, 
   return lo;
 }
 
-// Head of every kernel that may be launched chained: waits until the kernels before it have finished
-// and their writes are visible, then lets the next kernel's CTAs come in.  All threads pass here
-// before they read or write anything that another kernel touches, and before any return; so when a
-// kernel starts, the one before its predecessor has finished, and a finished kernel means that all
-// before it have.  Without a chained launch both instructions do nothing.
+// In every kernel that may be launched chained: waits until the kernels before it have finished and
+// their writes are visible, then lets the next kernel's CTAs come in.  All threads pass here, before
+// any return, and nothing lets the next kernel in earlier (k_node_step does, but is never launched
+// chained itself); so when a kernel starts, all but its predecessor have finished.  Before the wait a
+// kernel may therefore
+//   read what its predecessor does not write (past the L1, __ldcg, unless it is constant in a call),
+//   write what its predecessor neither reads nor writes;
+// all else comes after it.  Beside each access before the wait stands the predecessor that it counts
+// on: another kernel put between the two has to be held against it.  Without a chained launch both
+// instructions do nothing.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, c
   const int p = min(t >> 2, NI - 1), a = t & 3, lane = threadIdx.x & 31;
   const bool on = (t >> 2) < NI;
   const int gi = p < N ? p : p - N;
-  // the rods' kernel before writes positions and angles only
+  // the predecessor (k_chain or k_node, without rods k_steric) writes positions and angles only
   const float2 pv = __ldcg(reinterpret_cast<const float2*>(d.prev) + gi);
   int dep = -1;
   if (on && p < N && d.enable_steric) dep = __ldcg(d.c_cell + a * N + gi);
@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, c
 //
 // 4 lanes per node: lane q takes one of the four samples and every fourth neighbour, whose terms
 // are added in neighbour order.  Bound by latency; the neighbours do not need the field, so their
-// part is done while the filter before drains.
+// part is done while the predecessor drains (the filter's last pass, which writes the field alone; pred
+// and predw are k_predict's, three kernels before).
 __global__ void __launch_bounds__(128) k_steric(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];

@@ -426,7 +426,9 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
   l.own = act && l.j < nn && (!several || (lane >= kSegGhost && lane < kSegGhost + kSegOwn));
   const int j = l.j, ne = l.ne, nb = l.nb;
   float x = 0.0f, y = 0.0f, th = 0.0f, l0 = 0.0f, ra = 0.0f, kb = 0.0f;
-  // CHAINED: the kernel before writes the positions; what a PBD rod does without them comes first
+  // CHAINED: the predecessor, k_steric, writes the positions and touches nothing else of a rod; what a
+  // PBD rod does without them comes first (the step counter, the angles and their passes, the rest
+  // angles read and, under actuation, written)
   auto start = [&] {
     if (CHAINED) after_previous();
     if (act && j >= 0 && j < nn) {
