@@ -418,16 +418,16 @@ __device__ __forceinline__ float head_pool(const RDesc& d, int h, int cell, int 
   return cov;
 }
 
-// The CTA's heads with more contributions than a row holds, a warp each, shared among its warps: the
+// The CTA's heads with more contributions than a row holds (deep), a warp each, shared among its warps: the
 // cells around one spot are neighbours in the list.  Returns the coverage (its bits) and the start of
 // the calling thread's run.
-__device__ __noinline__ int2 deep_heads(const RDesc& d, int h0, int cell, int len, int K2) {
+__device__ __noinline__ int2 deep_heads(const RDesc& d, int h0, int cell, int len, bool deep, int K2) {
   __shared__ int s_deep, s_head[kHeadThreads];
   __shared__ int2 s_cell[kHeadThreads], s_run[kHeadThreads];
   if (threadIdx.x == 0) s_deep = 0;
   s_cell[threadIdx.x] = make_int2(cell, len);
   __syncthreads();
-  if (len > kRunRow) s_head[atomicAdd(&s_deep, 1)] = threadIdx.x;
+  if (deep) s_head[atomicAdd(&s_deep, 1)] = threadIdx.x;
   __syncthreads();
   for (int i = threadIdx.x >> 5; i < s_deep; i += kHeadThreads / 32) {
     const int t = s_head[i], lane = threadIdx.x & 31;
@@ -482,10 +482,11 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
   float cov = 0.0f;
   int start = h * kRunRow;
   if (len > 0 && len <= 8) cov = head_row<8>(d, h, cell, len, K2);
-  if (len > 8 && len <= kRunRow) cov = head_row<kRunRow>(d, h, cell, len, K2);
-  if (__syncthreads_or(len > kRunRow)) {
-    const int2 long_run = deep_heads(d, h0, cell, len, K2);
-    if (len > kRunRow) {
+  const int row = min(kRunRow, d.ib_cap);  // contributions that a run row and a bucket both hold
+  if (len > 8 && len <= row) cov = head_row<kRunRow>(d, h, cell, len, K2);
+  if (__syncthreads_or(len > row)) {
+    const int2 long_run = deep_heads(d, h0, cell, len, len > row, K2);
+    if (len > row) {
       cov = __int_as_float(long_run.x);
       start = long_run.y;
     }

@@ -1541,6 +1541,12 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
       h.T_c = threads_for(D.H, 512);
       h.P_c = 512 / h.T_c;
     }
+  }
+  p->compact_ok = compact_shape(p->R, &p->ns);
+  for (int i = 0; i < n; ++i) {
+    HostRollout& h = p->R[i];
+    const mc_dims& D = h.dims;
+    const mc_config& c = h.cfg;
     h.vec = (h.lW % 4 == 0) ? 4 : (h.lW % 2 == 0) ? 2 : 1;
     if (vec_all == -1) vec_all = h.vec;
     if (vec_all != h.vec) vec_all = 1;
@@ -1558,7 +1564,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     const size_t NIz = N * (c.synthetic_node_width > 0.0f ? 2 : 1);
     h.r_nvl = lay.take(2 * NIz * 4);
     h.r_delta = lay.take(2 * NIz * 4);
-    const size_t Mz = (size_t)M;
+    const size_t Mz = (size_t)h.M;
     // bin capacity: at least 3x the mean contributions per tile, a power of two
     auto cap_for = [&](long long contributions, int minimum, size_t tiles) {
       long long want = std::max<long long>(minimum, (3 * contributions + (long long)tiles - 1) / (long long)tiles);
@@ -1570,10 +1576,14 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
                                                                            div_up(h.lH, mc::kBinTile)));
     h.c_cap = cap_for(4LL * (long long)N, mc::kCicCap, nt);
     // contributions of a cell that stay in its bucket: where two rods of unit spacing cross a cell
-    // collects about 8 with the 4-point kernel, more where rods crowd (mean over all cells above 2)
-    h.ib_cap = (double)M < 2.0 * (double)LHW ? 16 : 32;
+    // collects about 8 with the 4-point kernel, more where rods crowd (mean over all cells above 2).
+    // The buckets are the largest part of the workspace behind the populations (64 of 217 B per cell
+    // at 1024^2 with 16,384 points); plans of the node-step kernel, which uses none and needs them
+    // only when another layout of the IB kernels is asked for, keep half as many (256 lattices of
+    // 128^2 with 16 points each 677 -> 543 MB).
+    h.ib_cap = p->compact_ok ? 8 : (double)Mz < 2.0 * (double)LHW ? 16 : 32;
     h.run_rows = (int)std::min(Mz, LHW);
-    const size_t cells = M > 0 ? LHW : 0;
+    const size_t cells = h.M > 0 ? LHW : 0;
     h.r_ibw = lay.take(Mz * 4);
     h.r_ibslot = lay.take(Mz * 4);
     h.r_ibcnt = lay.take(cells * 4);
@@ -1714,7 +1724,6 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   }
   int work = std::max(mcn, std::max(mce, mcb));
   p->node_bs = std::min(256, std::max(32, (work + 31) / 32 * 32));
-  p->compact_ok = compact_shape(p->R, &p->ns);
   p->desc.resize(n);
   *out = p;
   return MC_OK;
