@@ -41,7 +41,8 @@ constexpr int kPointThreads = 32;
 constexpr int kCellBucket = 16;  // entries of a cell ordered in registers
 constexpr long long kMaxCells = 4096LL * 4096;  // largest grid of the gradient path
 constexpr size_t kOverlapBytes = size_t(1) << 30;  // of a segment's inputs, up to which they are kept twice
-constexpr int kDirectSteps = 64;    // steps up to which forward steps are launched without graphs (step_graphs)
+constexpr int kDirectSteps = 64;    // steps up to which a plan's first gradient launches forward steps without
+                                    // graphs (step_graphs)
 constexpr int kDirectReverse = 16;  // the same for reverse steps
 constexpr int kPbdThreads = 256;  // threads per rod component in the PBD kernels
 constexpr int kPbdRod = 128;      // edges, nodes and pairs of a component kept one per thread
@@ -1747,6 +1748,7 @@ struct mc_grad_plan {
   size_t fwd_bytes = 0, total = 0;
   unsigned char* ws = nullptr;
   bool bound = false, have_forward = false, has_act = false;
+  long long forwards = 0, backwards = 0;  // calls so far, the present one included (step_graphs)
   // region offsets
   struct R {
     size_t off = 0, bytes = 0;
@@ -1867,12 +1869,18 @@ void group_by(int groups, std::vector<int>& start, std::vector<int>& list, F&& e
   each([&](int key, int value) { list[next[key]++] = value; });
 }
 
-// Short rollouts launch their kernels directly: a plan of one gradient would spend more on making
-// its graphs (some 0.25 ms each to capture and instantiate, 0.14 to destroy, with the GPU idle
-// before the first and after the last) than on launching each kernel (2 us).  48 steps at 256^2
-// 13.9 -> 12.9 ms, 12 steps at 640^2 8.6 -> 7.4.  A reverse step has three times the kernels of a
-// forward one, so that its graphs pay from fewer steps on.
-int step_graphs(const mc_grad_plan* p) { return p->T > kDirectSteps; }
+// The first gradient of a short rollout launches its kernels directly: a plan of one gradient would
+// spend more on making its graphs (some 0.25 ms each to capture and instantiate, 0.14 to destroy, with
+// the GPU idle before the first and after the last) than on launching each kernel (2 us).  48 steps at
+// 256^2 13.9 -> 12.9 ms, 12 steps at 640^2 8.6 -> 7.4.  A reverse step has three times the kernels of
+// a forward one, so that its graphs pay from fewer steps on.  First pass of a plan in us, launched
+// directly and by graphs: forward of 48 and 64 steps at 256^2 4,397 and 4,717, 5,792 and 6,173, at
+// 640^2 5,321 and 5,500, 6,947 and 7,014 (of 96 at 256^2, always by graphs, 8,923); reverse of 16 steps
+// of a 64^2 lattice 2,872 and 2,920, at 256^2 2,806 and 2,946, of 48 there 7,210 and 7,146.
+// A plan that is kept makes its graphs at the second gradient, since each further one is then faster:
+// forward of 48 steps at 640^2 5,279 -> 4,998, reverse of 16 steps of a 64^2 lattice 2,837 -> 2,346.
+int step_graphs(const mc_grad_plan* p) { return p->T > kDirectSteps || p->forwards > 1; }
+bool reverse_graphs(const mc_grad_plan* p) { return p->T > kDirectReverse || p->backwards > 1; }
 
 // Open a rollout of the forward plan on the working state, actuated from step t0 (the
 // static rest angles restored first when there is no actuation).
@@ -2534,6 +2542,7 @@ mc_status mc_grad_forward(mc_grad_plan* p, const mc_state* state, const mc_actua
     GC(cp(p->r_ap, act->phase, (size_t)D.B * 4));
   }
   p->ad.has_act = p->has_act ? 1 : 0;
+  ++p->forwards;
   for (int k = 0; k < p->nseg; ++k) {
     Slot ck = slot(p, p->r_ck, k);
     mc_status st = copy_state_to(p, ck.pos, ck.vel, ck.th, ck.f, at<float>(w, p->r_wpos), at<float>(w, p->r_wvel),
@@ -2588,6 +2597,7 @@ mc_status mc_grad_backward(mc_grad_plan* p, const mc_state_cot* final_cot, mc_st
     GC(mc::filter_prepare(p->fwd, w + p->r_fdesc.off, d.lV, d.ctmp, d.ldep, s));
     p->filter_ready = true;
   }
+  ++p->backwards;
   int lfcur = 0;
   // Replay of segment k - 1 beside the reverse of segment k: a replayed step keeps one SM busy for
   // most of its time and a reverse step a few, and they share nothing but the two copies of the
@@ -2650,7 +2660,7 @@ mc_status mc_grad_backward(mc_grad_plan* p, const mc_state_cot* final_cot, mc_st
     if (p->rev_graph_act != d.has_act) drop_rev_graphs(p);
     p->rev_graph_act = d.has_act;
     auto run = [&](int which) -> mc_status {
-      if (p->T <= kDirectReverse) {
+      if (!reverse_graphs(p)) {
         enqueue_reverse(p, which, s);
         return MC_OK;
       }
