@@ -191,9 +191,12 @@ mc_status mc_plan_set_bin_threads(mc_plan* plan, int32_t threads);
 int32_t mc_plan_bin_threads(const mc_plan* plan);
 
 /* Cloud-in-cell contributions a touched tile may hold to be sorted in shared memory (a power of two in
- * 256..8192, capped by the plan's bin capacity; 0 = 2048).  Denser tiles sort in a global
- * arena.  Smaller capacities keep more CTAs resident.  Results do not depend on it.  Only
- * before mc_plan_bind().  No counterpart in the reference. */
+ * 256..8192; 0 = 2048).  Denser tiles sort in a global arena.  Smaller capacities keep more CTAs
+ * resident.  Results do not depend on it.  Only before mc_plan_bind().
+ * mc_plan_bin_sort_capacity returns the setting, capped by the IB contributions per tile that the
+ * plan's densest rollout calls for (at least 1024).  The kernel itself sorts no more than the
+ * plan's largest cloud-in-cell bin holds (three times the mean per tile, at least 512), so on a
+ * sparse plan settings above that are the same launch.  No counterpart in the reference. */
 mc_status mc_plan_set_bin_sort_capacity(mc_plan* plan, int32_t entries);
 int32_t mc_plan_bin_sort_capacity(const mc_plan* plan);
 

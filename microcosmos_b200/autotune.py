@@ -7,7 +7,7 @@ Three kernels have a free shape:
   * the power-of-two FFT kernels of the steric filter: each thread holds 4, 8 or 16
     values in registers (more values: fewer instructions per value; fewer: more threads);
   * the tile kernel that sorts the cloud-in-cell contributions: 128 or 256 threads
-    per CTA, and 512 or 1024 contributions per tile sorted in shared memory;
+    per CTA, and 512, 1024 or 2048 contributions per tile sorted in shared memory;
   * the IB iterations: separate launches per phase, or (when asked for) one thread-block
     cluster of CTAs per rollout with hardware cluster barriers between the phases.
 Which shape is fastest depends on the rollout sizes of a plan (grid widths, how many CTAs
@@ -30,6 +30,7 @@ from .engine import DeviceState, Plan
 CELLS_PER_LANE = (1, 2, 4)
 ROWS_PER_CTA = (4, 8, 16, 32)
 FFT_VALUES = (4, 8, 16)
+# settings above what a plan's largest bin holds (512 in sparse plans) are the same launch
 BIN_SHAPES = ((128, 2048), (256, 2048), (128, 1024), (256, 1024), (128, 512))  # (threads per CTA, shared sort capacity)
 # CTAs per rollout cluster of the IB iterations tried besides the separate launches: none by
 # default (measured slower everywhere: 1.886 vs 1.852 ms per 256-rollout batch step with 8

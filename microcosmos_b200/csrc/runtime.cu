@@ -117,10 +117,10 @@ struct mc_plan {
   int lbm_stages = 0;       // > 0: the staged dense-pass kernel, with that many bands in flight per CTA
   int lbm_staged_ctas = 0;  // its persistent grid (set at bind: as many CTAs as the GPU holds)
   int c_capS = 0;    // largest bin capacity of the plan
-  int dense_cap = 0;  // contributions per 16x16 tile that the densest rollout's stencils call for: the upper end
-                      // of the sort capacity (mc_plan_bin_sort_capacity)
-  int sort_cap = 0;  // mc_plan_set_bin_sort_capacity
-  int c_smem = 0;    // contributions a tile may hold to be sorted in shared memory
+  int dense_cap = 0;  // IB contributions per 16x16 tile that the densest rollout calls for: the upper end of
+                      // sort_cap
+  int sort_cap = 0;  // the setting of mc_plan_set_bin_sort_capacity, as mc_plan_bin_sort_capacity reports it
+  int c_smem = 0;    // what runs: contributions a tile may hold to be sorted in shared memory, at most c_capS
   Region r_off[K_COUNT];
   std::vector<int> off[K_COUNT];
   int grid[K_COUNT] = {};
@@ -1001,10 +1001,12 @@ int64_t enqueue_tail(mc_plan* p, int rec_fields, bool has_next, cudaStream_t s, 
 }
 
 // Whether a step's kernels are launched chained.  Not while kernels are timed one at a time, and not
-// where the node grid is more than half of what the GPU holds at once (148 SMs x 16 CTAs of 128
-// threads): the CTAs that wait then take the slots the dense pass beside them would run in.  Per
-// pass without and with: 1024^2 (128 CTAs) 2390 and 2210 us, 64 uneven rollouts (610) 4204 and 4000,
-// 256 of them (2300) 7650 and 7820.
+// where the node grid is more than half of what a B200 holds at once (148 SMs x 16 CTAs of 128
+// threads): the CTAs that wait then take the slots the dense pass beside them would run in.  us per
+// step without and with, by node CTAs: one lattice of 1024^2 (128) 126 and 114; uneven rollouts 931:
+// 751 and 726, 1,295: 1,004 and 1,037, 1,578: 1,199 and 1,242, 2,091: 1,557 and 1,657, 2,344: 1,947 and
+// 2,068.  Equal rollouts, whose CTAs all end together, gain beyond the line too, but less and less
+// (1,024: 472 and 449, 1,536: 672 and 650, 2,048: 897 and 878); uneven ones are what is batched.
 bool chain_launches(const mc_plan* p) { return !p->profiling && p->grid[K_NODES] <= 8 * 148; }
 
 // Everything of step t after its pipeline, plus pipeline(t+1) when has_next; with `first` the
@@ -1169,9 +1171,18 @@ void destroy_graphs(mc_plan* p) {
 
 // Whether every rollout of the plan fits the node-step kernel (only chain rods, a kernel of at most
 // 4 points, everything it keeps in kNodeStepSmem bytes of shared memory), and its shape.  The line
-// lies at the shared memory of an SM (about 410 IB points with the 4-point kernel, 1,700 with the
-// 2-point one): up to there one CTA is faster than the separate launches (384 points: 60 against
-// about 90 us per step).
+// lies at the shared memory of an SM: about 410 IB points with the 4-point kernel, 700 with the 3-point
+// and 1,400 with the 2-point one.  One CTA's time grows with the points; the separate launches of a few
+// rollouts cost about 55 us a step whatever their size, those of many rollouts grow with all points.
+// Measured, us per step in the node-step kernel and in separate launches (128^2 or 64^2 lattices):
+//   one rollout, 4-point: 32 points 36 and 54; 128: 46 and 55; 192: 55 and 54; 256: 64 and 55;
+//     384: 82 and 57;  3-point: 128: 39 and 54; 256: 51 and 54; 384: 60 and 56; 640: 91 and 57;
+//     2-point: 128: 43 and 52; 384: 53 and 54; 640: 71 and 54; 1,280: 123 and 55;
+//   384 points, 4-point: 8 rollouts 80 and 65; 32: 85 and 88; 64: 86 and 124; 148: 107 and 233;
+//     1,024: 809 and 1,641.  16 points: 256 rollouts 121 and 157; 1,024: 218 and 248.
+// So for fewer than some 30 rollouts the line lies too high (it was set when the separate launches
+// were not chained and took 90 us at 384 points); below about 190, 320 and 400 points, and for
+// more rollouts at every size, the kernel is the faster form.
 bool compact_shape(const std::vector<HostRollout>& R, mc::NodeStepShape* out) {
   int N = 0, NI = 0, C = 0, longest = 1, rods = 0, shortest = mc::chain_warps(256);
   for (const HostRollout& h : R) {
