@@ -370,14 +370,20 @@ __global__ void __launch_bounds__(128) k_steric(const RDesc* __restrict__ D, con
 }
 
 // ---------------------------------------------------------------- chains: CTA per rod
-// One CTA (one team) per chain rod; S: the longest chain of the plan.  At least four warps, so
-// that the sines and cosines of a short rod's iterations do not fall to a single warp.
+// One CTA (one team) per chain rod; S: the longest chain of the plan.  At least four warps where all
+// CTAs run at once (kChainFill: 6 of 4 warps of 80 registers on each of 148 SMs), so that the sines
+// and cosines of a short rod's iterations do not fall to a single warp; beyond, issue slots are what
+// is short, and a rod takes the warps that its nodes need.  Per launch with 4 warps and with the rod's
+// own, rods of 32 nodes: 512 12.8 and 14.8 us, 888 14.8 and 14.7, 1,500 22.7 and 16.7, 8,000 78 and 39
+// (one warp per rod with all phases in one loop: 17, 19, 18.6 and 43); of 64: 888 19.0 and 18.9, 4,000
+// 62 and 56 (27 and 42: two nodes per lane need no ghosts, which count once the SMs are full).
+constexpr int kChainFill = 6 * 148;
 __global__ void __launch_bounds__(384) k_chain(const RDesc* __restrict__ D, const int* __restrict__ off, int n,
                                                const int* tdev, int S) {
   extern __shared__ float2 chain_tab[];
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
-  const Team tm = {(int)threadIdx.x >> 5, (int)blockDim.x >> 5, 1};
+  const TeamOf<1> tm = {(int)threadIdx.x >> 5, (int)blockDim.x >> 5, 1};
   chain_rod<true>(d, d.chain_info[blockIdx.x - off[r]], __ldcg(tdev), tm, d.pos, chain_tab, S);
 }
 
@@ -521,7 +527,7 @@ void launch_node(const Launch& L, const int* tdev, size_t smem, int bs) {
   launch(L, k_node, bs, smem, L.d, L.off, L.n, tdev);
 }
 void launch_chain(const Launch& L, const int* tdev, int longest) {
-  const int warps = chain_warps(longest) < 4 ? 4 : chain_warps(longest);
+  const int need = chain_warps(longest), warps = need < 4 && L.grid <= kChainFill ? 4 : need;
   launch(L, k_chain, 32 * warps, (size_t)chain_smem(longest) * sizeof(float2), L.d, L.off, L.n, tdev, longest);
 }
 cudaError_t node_set_smem(size_t bytes) {

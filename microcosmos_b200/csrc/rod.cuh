@@ -31,29 +31,53 @@ __host__ __device__ constexpr int chain_smem(int S) { return (kThetaChunk + 2) *
 
 // The threads working on one rod.  All of them call chain_rod together; warps beyond the rod's
 // own (chain_warps) help with the sines and cosines.
-struct Team {
+// BAR: the number of the team's first barrier where it is known at compile time, else 0.  A barrier
+// whose number is in a register makes the compiler reserve all 16 of a CTA, so that no more than 4
+// such CTAs fit on an SM (8,000 rods of 32 nodes in the chain kernel: 107 us per launch that way).
+template <int BAR>
+struct TeamOf {
   int warp, warps;  // this warp's index in the team, and the team's warps
   int bar;          // the team's named barrier; bar + 1 is that of its first warps, when the rod has fewer:
                     // its count changes from rod to rod, so the whole team meets at `bar` in between
   __device__ __forceinline__ void sync() const {
     if (warps == 1)
       __syncwarp();
-    else
+    else if (BAR == 0)
       asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(warps * 32) : "memory");
+    else if (bar == BAR)
+      asm volatile("bar.sync %0, %1;" ::"n"(BAR), "r"(warps * 32) : "memory");
+    else
+      asm volatile("bar.sync %0, %1;" ::"n"(BAR + 1), "r"(warps * 32) : "memory");
   }
   // sync, and whether `p` holds for any thread of the team
   __device__ __forceinline__ bool sync_or(bool p) const {
     if (warps == 1) return __any_sync(0xffffffffu, p) != 0;
     int r;
-    asm volatile(
-        "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
-        "selp.s32 %0, 1, 0, b;\n\t}"
-        : "=r"(r)
-        : "r"((int)p), "r"(bar), "r"(warps * 32)
-        : "memory");
+    if (BAR == 0)
+      asm volatile(
+          "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
+          "selp.s32 %0, 1, 0, b;\n\t}"
+          : "=r"(r)
+          : "r"((int)p), "r"(bar), "r"(warps * 32)
+          : "memory");
+    else if (bar == BAR)
+      asm volatile(
+          "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
+          "selp.s32 %0, 1, 0, b;\n\t}"
+          : "=r"(r)
+          : "r"((int)p), "n"(BAR), "r"(warps * 32)
+          : "memory");
+    else
+      asm volatile(
+          "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
+          "selp.s32 %0, 1, 0, b;\n\t}"
+          : "=r"(r)
+          : "r"((int)p), "n"(BAR + 1), "r"(warps * 32)
+          : "memory");
     return r != 0;
   }
 };
+using Team = TeamOf<0>;
 
 // max that propagates NaN, for the range checks of the fast passes
 __device__ __forceinline__ float max_track(float m, float v) {
@@ -130,8 +154,8 @@ struct RodLane {
 
 // q angle passes (pbd.py:23-49); row k of tab keeps the angles after pass k.  NEAR: without the
 // slow path of the floored modulo; returns whether this lane would have needed it.
-template <bool NEAR, bool SEVERAL>
-__device__ __forceinline__ bool theta_passes(const Team& rod, const RodLane& l, int q, float& th, float ra, float kb,
+template <bool NEAR, bool SEVERAL, class T>
+__device__ __forceinline__ bool theta_passes(const T& rod, const RodLane& l, int q, float& th, float ra, float kb,
                                              float edg, float2* tab, int S) {
   const bool pair = l.j >= 0 && l.j < l.nb, prev = l.j >= 1 && l.j - 1 < l.nb, edge = l.j >= 0 && l.j < l.ne;
   const bool keep = l.own && edge;
@@ -168,8 +192,8 @@ __device__ __forceinline__ bool theta_passes(const Team& rod, const RodLane& l, 
 
 // q position passes (pbd.py:51-89) with the rest vectors in tab; first: no pass came before them.
 // NEAR: without the slow paths of the modulo, the square root and the divisions.
-template <bool NEAR, bool SEVERAL>
-__device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& l, int q, bool first, float& x,
+template <bool NEAR, bool SEVERAL, class T>
+__device__ __forceinline__ bool position_passes(const T& rod, const RodLane& l, int q, bool first, float& x,
                                                 float& y, float l0, float ndg, float Wf, float Hf, float ksh,
                                                 float kst, const float2* tab, float2* ex, int& buf, int S) {
   // (lane 31 of a warp sees no next node: with several warps its edge is a neighbour's)
@@ -230,15 +254,15 @@ __device__ __forceinline__ bool position_passes(const Team& rod, const RodLane& 
 // and the divisions first (their branches would lie on the dependent chain); if any lane needed
 // one, the chunk is done again from its start with them.  start() gives the positions; the first
 // chunk's angles and rest vectors do not need them.
-template <bool SEVERAL, class F>
-__device__ __forceinline__ void pbd_iterations(const F& start, const RDesc& d, const Team& tm, int rw, const RodLane& l, int e0,
+template <bool SEVERAL, class F, class T>
+__device__ __forceinline__ void pbd_iterations(const F& start, const RDesc& d, const T& tm, int rw, const RodLane& l, int e0,
                                                float& x, float& y, float& th, float l0, float ra, float kb, float edg,
                                                float ndg, float2* tab, int S) {
   const int lane = threadIdx.x & 31;
   const bool act = tm.warp < rw, edge = l.j >= 0 && l.j < l.ne;
   const float Wf = (float)d.W, Hf = (float)d.H, ksh = d.k_shear, kst = d.k_stretch;
   float2* ex = tab + kThetaChunk * S;
-  const Team rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
+  const T rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
   const int cycles = d.cycles;
   int buf = 0;
   if (cycles <= 0) start();
@@ -304,8 +328,8 @@ __device__ __forceinline__ float reciprocal(float b) {
 // to the right per iteration, so the warps exchange after every second one.  The divisors do not
 // change, so NEAR divides by their reciprocals (div_near); it returns whether this lane left the
 // range where that and the one-period modulo are exact.
-template <bool NEAR, bool SEVERAL>
-__device__ __forceinline__ bool cosserat_iterations(const RDesc& d, const Team& rod, const RodLane& l, float& x,
+template <bool NEAR, bool SEVERAL, class T>
+__device__ __forceinline__ bool cosserat_iterations(const RDesc& d, const T& rod, const RodLane& l, float& x,
                                                     float& y, float& th, float l0, float ra, float kb, float edg,
                                                     float2* ex, float* ext, int S) {
   const int j = l.j;
@@ -394,8 +418,8 @@ __device__ __forceinline__ bool cosserat_iterations(const RDesc& d, const Team& 
   return moves || turns;
 }
 
-template <bool SEVERAL>
-__device__ __forceinline__ void cosserat_rod(const RDesc& d, const Team& rod, const RodLane& l, float& x, float& y,
+template <bool SEVERAL, class T>
+__device__ __forceinline__ void cosserat_rod(const RDesc& d, const T& rod, const RodLane& l, float& x, float& y,
                                              float& th, float l0, float ra, float kb, float edg, float2* tab, int S) {
   float2* ex = tab + kThetaChunk * S;
   float* ext = reinterpret_cast<float*>(tab);
@@ -411,8 +435,8 @@ __device__ __forceinline__ void cosserat_rod(const RDesc& d, const Team& rod, co
 // All cycles_per_step iterations at step t of the chain info = (first node, nodes, first edge, first
 // pair).  pos: the rollout's node positions (x, y), updated in place; tab: chain_smem(S) float2 of
 // shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.
-template <bool CHAINED>
-__device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, const Team& tm, float* pos, float2* tab,
+template <bool CHAINED, class T>
+__device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, const T& tm, float* pos, float2* tab,
                                           int S) {
   const int lane = threadIdx.x & 31;
   const int n0 = info.x, nn = info.y, e0 = info.z, b0 = info.w;
@@ -454,7 +478,7 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
   const float edg = ((j < nb) + (j >= 1 && j - 1 < nb)) == 2 ? 0.5f : 1.0f;
   const float ndg = ((j < ne) + (j >= 1 && j - 1 < ne)) == 2 ? 0.5f : 1.0f;
   if (d.solver == 1) {
-    const Team rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
+    const T rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
     if (act && several)
       cosserat_rod<true>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
     else if (act)
