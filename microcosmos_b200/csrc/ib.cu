@@ -308,17 +308,17 @@ __device__ __forceinline__ void sort_regs(int (&k)[R], float (&w)[R]) {
       }
 }
 
-// A head of at most R <= kRunRow contributions: its run in its row, its contributions linked to it; returns
-// the coverage (the weights' sum in order of k).
+// A head of at most R <= kHeadSort contributions (`first`: the first four of its bucket): its run at
+// `start`, its contributions linked to it; returns the coverage (the weights' sum in order of k).
 template <int R>
-__device__ __forceinline__ float head_row(const RDesc& d, int h, int cell, int len, int K2) {
+__device__ __forceinline__ float head_row(const RDesc& d, int h, int cell, int len, int4 first, int start, int K2) {
   int k[R];
   float w[R];
   const int4* bucket = reinterpret_cast<const int4*>(d.ib_bucket + (size_t)cell * d.ib_cap);
 #pragma unroll
   for (int q = 0; q < R; q += 4) {
-    int4 v = make_int4(0, 0, 0, 0);
-    if (q < len) v = bucket[q / 4];
+    int4 v = first;
+    if (q > 0 && q < len) v = bucket[q / 4];
     k[q] = q < len ? v.x : 0x7fffffff;
     k[q + 1] = q + 1 < len ? v.y : 0x7fffffff;
     k[q + 2] = q + 2 < len ? v.z : 0x7fffffff;
@@ -334,7 +334,7 @@ __device__ __forceinline__ float head_row(const RDesc& d, int h, int cell, int l
 #pragma unroll
   for (int q = 1; q < R; ++q)
     if (q < len) cov = cov + w[q];
-  int4* row = reinterpret_cast<int4*>(d.run + (size_t)h * kRunRow);
+  int4* row = reinterpret_cast<int4*>(d.run + start);  // runs start at even entries
 #pragma unroll
   for (int q = 0; q < R; q += 2)
     if (q < len) {
@@ -384,13 +384,13 @@ __device__ const int* sort_warp(int* a, int* b, int n, int lane) {
   return a;
 }
 
-// A head with more contributions than a row holds, by a whole warp: gathered from the bucket and
-// the overflow list into the pool, sorted, and its run written behind them.
+// A head with more contributions than are sorted in registers, by a whole warp: gathered from the bucket
+// and the overflow list, sorted, and its run written behind them.
 __device__ __forceinline__ float head_pool(const RDesc& d, int h, int cell, int len, int K2, int lane, int& start) {
   int base = 0;
   const int pad = (len + 1) & ~1;
   if (lane == 0) base = atomicAdd(d.ib_ctl + 1, 2 * pad);
-  base = d.run_rows * kRunRow + __shfl_sync(0xffffffffu, base, 0);
+  base = __shfl_sync(0xffffffffu, base, 0);
   int2* raw = d.run + base;
   int2* run = raw + pad;
   const int* bucket = d.ib_bucket + (size_t)cell * d.ib_cap;
@@ -418,7 +418,7 @@ __device__ __forceinline__ float head_pool(const RDesc& d, int h, int cell, int 
   return cov;
 }
 
-// The CTA's heads with more contributions than a row holds (deep), a warp each, shared among its warps: the
+// The CTA's heads with more contributions than that (deep), a warp each, shared among its warps: the
 // cells around one spot are neighbours in the list.  Returns the coverage (its bits) and the start of
 // the calling thread's run.
 __device__ __noinline__ int2 deep_heads(const RDesc& d, int h0, int cell, int len, bool deep, int K2) {
@@ -442,13 +442,17 @@ __device__ __noinline__ int2 deep_heads(const RDesc& d, int h0, int cell, int le
 // One thread per touched cell: its contributions ordered by k, the coverage -> 1/max(cov, 1), the
 // macroscopic state pulled from h[parity] (density, clamped velocity), u_corrected = velocity
 // (fluid.py:268-290).  Bound by the latency of its three dependent loads (the cell, its bucket and
-// populations, the weights), with every head's loads in flight at once.
+// populations, the weights), with every head's loads in flight at once.  A CTA's runs lie one behind
+// the other (a scan of their lengths, one atomic per CTA for their place), since every forcing round
+// reads them all: per step at 4096^2 with 307,200 points the rounds' spread halves took 349 us with a
+// row of 16 entries for each cell and 268 packed (and 1 / coverage apart from the macroscopic
+// state), this kernel 154 and 132.
 // Before, one CTA per 16x16 tile counting-sorted the tile's contributions in shared memory, in
 // phases separated by barriers; a tile with more than 2,048 took a sort in global memory, whose
 // tail set the kernel's time on dense rollouts.  Measured (per launch in a step): 1024^2 with
-// 16,384 points 26 -> 11.3 us, a batch of 64 uneven rollouts with 74 k points 225 -> 54 us.  Rows
-// of 8 entries instead of 16 took 46 and 82 us: where rods cross, whole warps of cells then went
-// through the pool.
+// 16,384 points 26 -> 11.3 us, a batch of 64 uneven rollouts with 74 k points 225 -> 54 us.  Sorting
+// up to 8 entries in registers instead of 16 took 46 and 82 us: where rods cross, whole warps of cells
+// then took the path of the longer ones.
 __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restrict__ D, const int* __restrict__ off,
                                                            int n, int parity) {
   const int r = find_rollout(off, n, blockIdx.x);
@@ -461,6 +465,8 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
   const bool on = h < heads;
   const int cell = on ? d.h_new[h] : 0;
   const int len = on ? d.ib_cnt[cell] : 0;
+  int4 first = make_int4(0, 0, 0, 0);
+  if (on) first = *reinterpret_cast<const int4*>(d.ib_bucket + (size_t)cell * d.ib_cap);
   const int lW = d.lW, lH = d.lH, K2 = d.K * d.K;
   const int y = cell / lW, x = cell - y * lW;
   const int xm = x == 0 ? lW - 1 : x - 1, xp = x == lW - 1 ? 0 : x + 1;
@@ -479,12 +485,32 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
   f[6] = rm[6 * HW + xp];
   f[7] = rp[7 * HW + xp];
   f[8] = rp[8 * HW + xm];
+  const int row = min(kHeadSort, d.ib_cap);  // contributions that are sorted in registers and that a bucket holds
+  // places of the runs: a scan over the CTA
+  __shared__ int s_sum[kHeadThreads / 32], s_base;
+  const int lane = threadIdx.x & 31, pad = len <= row ? (len + 1) & ~1 : 0;
+  int start = pad;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, start, o);
+    if (lane >= o) start += v;
+  }
+  if (lane == 31) s_sum[threadIdx.x >> 5] = start;
+  start -= pad;
+  __syncthreads();
+  int all = 0;
+#pragma unroll
+  for (int i = 0; i < kHeadThreads / 32; ++i) {
+    if (i == threadIdx.x >> 5) start += all;
+    all += s_sum[i];
+  }
+  if (threadIdx.x == 0) s_base = atomicAdd(d.ib_ctl + 1, all);
+  const bool deep = __syncthreads_or(len > row);
+  start += s_base;
   float cov = 0.0f;
-  int start = h * kRunRow;
-  if (len > 0 && len <= 8) cov = head_row<8>(d, h, cell, len, K2);
-  const int row = min(kRunRow, d.ib_cap);  // contributions that a run row and a bucket both hold
-  if (len > 8 && len <= row) cov = head_row<kRunRow>(d, h, cell, len, K2);
-  if (__syncthreads_or(len > row)) {
+  if (len > 0 && len <= 8) cov = head_row<8>(d, h, cell, len, first, start, K2);
+  if (len > 8 && len <= row) cov = head_row<kHeadSort>(d, h, cell, len, first, start, K2);
+  if (deep) {
     const int2 long_run = deep_heads(d, h0, cell, len, len > row, K2);
     if (len > row) {
       cov = __int_as_float(long_run.x);
@@ -497,7 +523,8 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
   macroscopic(f, d.vmax, d.vmax_q4, rho, vx, vy);
   d.h_cell[h] = cell;
   d.h_run[h] = make_int2(start, len);
-  d.s_mac[h] = make_float4(rho, vx, vy, 1.0f / max_prop(cov, 1.0f));
+  d.s_mac[h] = make_float4(rho, vx, vy, 0.0f);
+  d.s_inv[h] = 1.0f / max_prop(cov, 1.0f);
   d.s_uc[h] = make_float2(vx, vy);
 }
 
@@ -671,10 +698,12 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
   int2 run = make_int2(0, 0);
   float4 mac;
   float2 u;
+  float inv;
   if (on) {
     run = __ldcg(d.h_run + p);
-    mac = __ldcg(d.s_mac + p);
+    inv = __ldcg(d.s_inv + p);
     u = __ldcg(d.s_uc + p);
+    if (fin) mac = __ldcg(d.s_mac + p);
   }
   RunChunk c;
   c.load(d.run + run.x, run.y, 0);
@@ -687,7 +716,7 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
     c.load(d.run + run.x, run.y, j);
     c.add(run.y, j, d.delta, s);
   }
-  u = make_float2(u.x + s.x * mac.w, u.y + s.y * mac.w);
+  u = make_float2(u.x + s.x * inv, u.y + s.y * inv);
   d.s_uc[p] = u;
   if (fin) d.s_f[p] = head_force(d, mac, u);
 }
@@ -777,7 +806,7 @@ __device__ __forceinline__ void ib_iterations(const RDesc& d, int t0, int stride
             dy = dy + v[q].y * __int_as_float(e[q].y);
           }
       }
-      const float inv = d.s_mac[p].w;
+      const float inv = d.s_inv[p];
       const float2 u = __ldcg(d.s_uc + p);
       d.s_uc[p] = make_float2(u.x + dx * inv, u.y + dy * inv);
     }

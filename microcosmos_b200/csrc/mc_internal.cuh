@@ -26,7 +26,7 @@ constexpr int kStageCells = 1024;  // staged dense pass: lattice cells per item 
 constexpr int kStagedThreads = 256;  // ... and threads per CTA (4 cells each)
 constexpr int kConvTile = 32;     // steric direct convolution: 32 x 32 outputs per CTA
 constexpr int kConvMaxR = 24;     // largest tap radius of the direct convolution
-constexpr int kRunRow = 16;        // entries of a touched cell's run row (k_ib_heads sorts as many in registers)
+constexpr int kHeadSort = 16;        // contributions of a touched cell that k_ib_heads sorts in registers
 constexpr int kCicCap = 512;       // minimum CIC bin capacity per tile
 constexpr int kMaxBinCap = 8192;   // largest bin capacity (the tile sort keeps 4 x cap words in shared memory)
 constexpr int kFftMaxN = 4096;     // largest FFT length (shared memory)
@@ -121,8 +121,7 @@ struct RDesc {
   // IB contributions k = point*K*K + entry.  Each is appended to its cell's bucket
   // (ib_bucket[cell * ib_cap ...], an atomic on ib_cnt picks the place); beyond ib_cap it goes to
   // the cell's overflow list (ib_ovf_head, ib_ovf_next, ib_ovf).  The first one of a cell makes it
-  // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of the run pool, ctl[2] =
-  // heads, ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
+  // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of `run`, ctl[2] = heads, ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
   // ctl[5] = the head count saved for k_collide_heads.
   int ib_cap;
   float* ib_w;      // (M) normalised stencil weight
@@ -133,15 +132,15 @@ struct RDesc {
   int* ib_ovf_next;  // (M)
   int* ib_ovf;      // (M) their contributions
   int* ib_ctl;      // (8)
-  // runs: per head the (point, weight) pairs of its contributions in order of k, in its row
-  // [h * kRunRow ...] or, when longer, in the pool behind the rows
-  int2* run;        // (run_rows * kRunRow + 3 M)
-  int run_rows;
+  // runs: per head the (point, weight) pairs of its contributions in order of k, from an even entry on
+  // (with the space that the sort of a long one needs: at most 20 entries per 9 contributions)
+  int2* run;        // (5 M / 2)
   // per head, in [0, ctl[2])
   int* h_new;       // cell, as the stencil kernel lists it (while k_collide_heads may still use h_cell)
   int* h_cell;      // cell, from k_ib_heads on
   int2* h_run;      // start and length of its run
-  float4* s_mac;    // density, clamped velocity, 1 / max(coverage, 1)
+  float4* s_mac;    // density, clamped velocity (and a word to fill it up)
+  float* s_inv;     // 1 / max(coverage, 1)
   float2* s_uc;     // corrected velocity
   float2* s_f;      // body force
   // CIC deposit contributions k = corner*N + n (4N)

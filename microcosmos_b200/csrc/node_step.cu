@@ -354,7 +354,7 @@ __device__ __forceinline__ void couple(const RDesc& d, const Smem& m, int* warp_
     macroscopic(f, vmax, q4, rho, vx, vy);
     h_cell[h] = cell;
     const float inv = 1.0f / max_prop(cov, 1.0f);
-    s_mac[h] = make_float4(rho, vx, vy, inv);
+    s_mac[h] = make_float4(rho, vx, vy, 0.0f);
     m.inv()[h] = inv;
     m.uc()[h] = make_float2(vx, vy);
   }

@@ -95,9 +95,8 @@ struct HostRollout {
   int T_r = 0, P_r = 0, T_c = 0, P_c = 0;
   // workspace regions (offsets relative to the workspace base)
   Region r_h0, r_h1, r_dep, r_tmp, r_prev, r_pred, r_predw, r_nvl, r_delta;
-  Region r_ibw, r_ibslot, r_ibcnt, r_ibbucket, r_ibovh, r_ibovn, r_ibovf, r_ibctl, r_run, r_hnew, r_hcell, r_hrun, r_smac, r_suc,
+  Region r_ibw, r_ibslot, r_ibcnt, r_ibbucket, r_ibovh, r_ibovn, r_ibovf, r_ibctl, r_run, r_hnew, r_hcell, r_hrun, r_smac, r_sinv, r_suc,
       r_sf;
-  int run_rows = 0;
   Region r_ccell, r_cw, r_cstore, r_ctc, r_covf, r_cctl, r_chain, r_generic;
   Region r_pairs, r_bpairs, r_compn, r_compe, r_compb, r_epo, r_epi, r_neo, r_nei, r_edeg, r_ndeg;
   Region r_twW, r_twH, r_ptW, r_ptH, r_gW, r_gH, r_flags;
@@ -615,7 +614,6 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.nvl = at<float2>(b, h.r_nvl);
   d.delta = at<float2>(b, h.r_delta);
   d.ib_cap = h.ib_cap;
-  d.run_rows = h.run_rows;
   d.ib_w = at<float>(b, h.r_ibw);
   d.ib_slot = at<int>(b, h.r_ibslot);
   d.ib_cnt = at<int>(b, h.r_ibcnt);
@@ -629,6 +627,7 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.h_cell = at<int>(b, h.r_hcell);
   d.h_run = at<int2>(b, h.r_hrun);
   d.s_mac = at<float4>(b, h.r_smac);
+  d.s_inv = at<float>(b, h.r_sinv);
   d.s_uc = at<float2>(b, h.r_suc);
   d.s_f = at<float2>(b, h.r_sf);
   d.c_cap = h.c_cap;
@@ -1588,12 +1587,11 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     h.c_cap = cap_for(4LL * (long long)N, mc::kCicCap, nt);
     // contributions of a cell that stay in its bucket: where two rods of unit spacing cross a cell
     // collects about 8 with the 4-point kernel, more where rods crowd (mean over all cells above 2).
-    // The buckets are the largest part of the workspace behind the populations (64 of 217 B per cell
+    // The buckets are the largest part of the workspace behind the populations (64 of 185 B per cell
     // at 1024^2 with 16,384 points); plans of the node-step kernel, which uses none and needs them
     // only when another layout of the IB kernels is asked for, keep half as many (256 lattices of
-    // 128^2 with 16 points each 677 -> 543 MB).
+    // 128^2 with 16 points each 675 -> 541 MB).
     h.ib_cap = p->compact_ok ? 8 : (double)Mz < 2.0 * (double)LHW ? 16 : 32;
-    h.run_rows = (int)std::min(Mz, LHW);
     const size_t cells = h.M > 0 ? LHW : 0;
     h.r_ibw = lay.take(Mz * 4);
     h.r_ibslot = lay.take(Mz * 4);
@@ -1603,11 +1601,12 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     h.r_ibovn = lay.take(Mz * 4);
     h.r_ibovf = lay.take(Mz * 4);
     h.r_ibctl = lay.take(8 * 4);
-    h.r_run = lay.take(((size_t)h.run_rows * mc::kRunRow + 3 * Mz) * 8);
+    h.r_run = lay.take((5 * Mz / 2 + 2) * 8);
     h.r_hnew = lay.take(Mz * 4);
     h.r_hcell = lay.take(Mz * 4);
     h.r_hrun = lay.take(Mz * 8);
     h.r_smac = lay.take(Mz * 16);
+    h.r_sinv = lay.take(Mz * 4);
     h.r_suc = lay.take(Mz * 8);
     h.r_sf = lay.take(Mz * 8);
     h.r_ccell = lay.take(4 * N * 4);
