@@ -530,8 +530,18 @@ __global__ void __launch_bounds__(kHeadThreads) k_ib_heads(const RDesc* __restri
 
 // Weighted sum of a head-indexed field over the K*K stencil of one point, in stencil order
 // (the reference's sum over axis 1 of values * weights, fluid.py:90-97).  The slots and weights
-// are read past the L1: a chained kernel reads them before it waits (after_previous).
-template <int K2>
+// are read past the L1: a chained kernel reads them before it waits (after_previous).  FUSED, in a
+// kernel that runs all rounds: they are read through the L1, round after round, and the field, which
+// other SMs write between the rounds, past it.
+template <bool FUSED, typename T>
+__device__ __forceinline__ T constant_load(const T* p) {
+  return FUSED ? *p : __ldcg(p);
+}
+template <bool FUSED, typename T>
+__device__ __forceinline__ T field_load(const T* p) {
+  return FUSED ? __ldcg(p) : *p;
+}
+template <int K2, bool FUSED = false>
 struct Taps {
   int slot[K2];
   float w[K2];
@@ -540,23 +550,23 @@ struct Taps {
     if (K2 % 4 == 0) {
 #pragma unroll
       for (int s = 0; s < K2; s += 4) {
-        const int4 q = __ldcg(reinterpret_cast<const int4*>(d.ib_slot + base + s));
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(d.ib_w + base + s));
+        const int4 q = constant_load<FUSED>(reinterpret_cast<const int4*>(d.ib_slot + base + s));
+        const float4 v = constant_load<FUSED>(reinterpret_cast<const float4*>(d.ib_w + base + s));
         slot[s] = q.x; slot[s + 1] = q.y; slot[s + 2] = q.z; slot[s + 3] = q.w;
         w[s] = v.x; w[s + 1] = v.y; w[s + 2] = v.z; w[s + 3] = v.w;
       }
     } else {
 #pragma unroll
       for (int s = 0; s < K2; ++s) {
-        slot[s] = __ldcg(d.ib_slot + base + s);
-        w[s] = __ldcg(d.ib_w + base + s);
+        slot[s] = constant_load<FUSED>(d.ib_slot + base + s);
+        w[s] = constant_load<FUSED>(d.ib_w + base + s);
       }
     }
   }
   __device__ __forceinline__ float2 sum(const float2* field) const {
     float2 v[K2];
 #pragma unroll
-    for (int s = 0; s < K2; ++s) v[s] = field[slot[s]];
+    for (int s = 0; s < K2; ++s) v[s] = field_load<FUSED>(field + slot[s]);
     float x = 0.0f, y = 0.0f;
 #pragma unroll
     for (int s = 0; s < K2; ++s) {
@@ -566,25 +576,26 @@ struct Taps {
     return make_float2(x, y);
   }
 };
-template <int K2>
+template <int K2, bool FUSED>
 __device__ __forceinline__ float2 stencil_sum(const RDesc& d, int point, const float2* field) {
-  Taps<K2> taps;
+  Taps<K2, FUSED> taps;
   taps.load(d, point);
   return taps.sum(field);
 }
 
+template <bool FUSED = false>
 __device__ __forceinline__ float2 stencil_sum_any(const RDesc& d, int point, const float2* field) {
   switch (d.K) {
-    case 4: return stencil_sum<16>(d, point, field);
-    case 2: return stencil_sum<4>(d, point, field);
-    case 3: return stencil_sum<9>(d, point, field);
+    case 4: return stencil_sum<16, FUSED>(d, point, field);
+    case 2: return stencil_sum<4, FUSED>(d, point, field);
+    case 3: return stencil_sum<9, FUSED>(d, point, field);
     default: break;
   }
   const int K2 = d.K * d.K;
   float x = 0.0f, y = 0.0f;
   for (int s = 0; s < K2; ++s) {
     const int k = point * K2 + s;
-    const float2 v = field[d.ib_slot[k]];
+    const float2 v = field_load<FUSED>(field + d.ib_slot[k]);
     const float w = d.ib_w[k];
     x = x + v.x * w;
     y = y + v.y * w;
@@ -653,19 +664,21 @@ __global__ void __launch_bounds__(256) k_ib_interp(const RDesc* __restrict__ D, 
 
 // In-order sum of correction * weight over a head's run (fluid.py:304-309).  Runs are short: 8
 // entries are fetched at a time (those that exist) so that all their loads are in flight together.
+template <bool FUSED = false>
 struct RunChunk {
   int4 e[4];
   __device__ __forceinline__ void load(const int2* run, int len, int j) {
     const int4* pairs = reinterpret_cast<const int4*>(run);  // runs start at even entries
 #pragma unroll
-    for (int q = 0; q < 4; ++q) e[q] = j + 2 * q < len ? __ldcg(pairs + j / 2 + q) : make_int4(0, 0, 0, 0);
+    for (int q = 0; q < 4; ++q)
+      e[q] = j + 2 * q < len ? constant_load<FUSED>(pairs + j / 2 + q) : make_int4(0, 0, 0, 0);
   }
   __device__ __forceinline__ void add(int len, int j, const float2* delta, float2& sum) const {
     float2 v[8];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      v[2 * q] = j + 2 * q < len ? delta[e[q].x] : make_float2(0.0f, 0.0f);
-      v[2 * q + 1] = j + 2 * q + 1 < len ? delta[e[q].z] : make_float2(0.0f, 0.0f);
+      v[2 * q] = j + 2 * q < len ? field_load<FUSED>(delta + e[q].x) : make_float2(0.0f, 0.0f);
+      v[2 * q + 1] = j + 2 * q + 1 < len ? field_load<FUSED>(delta + e[q].z) : make_float2(0.0f, 0.0f);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -705,7 +718,7 @@ __global__ void __launch_bounds__(256) k_ib_spread(const RDesc* __restrict__ D, 
     u = __ldcg(d.s_uc + p);
     if (fin) mac = __ldcg(d.s_mac + p);
   }
-  RunChunk c;
+  RunChunk<> c;
   c.load(d.run + run.x, run.y, 0);
   after_previous();
   if (fin && p == 0) d.ib_ctl[5] = heads;
@@ -752,63 +765,35 @@ __device__ __forceinline__ void rollout_barrier(int* ctl, int nb, unsigned* flag
 // All ibm_iterations of the multi-direct forcing and the body force of every rollout in one
 // cooperative launch: [interpolate (nodes) | barrier | spread (touched cells) | barrier] x
 // iterations, then the finalize of every touched cell.  Same arithmetic and order as
-// k_ib_interp / k_ib_spread / k_ib_finalize; values written in one phase and read in the
-// next are loaded with __ldcg (L2, not the SM's L1).
+// k_ib_interp / k_ib_spread / k_ib_finalize, and the same loads of whole vectors (with loads of single
+// slots, weights and entries instead: 1024^2 162 us a step, in clusters of 8 CTAs 352; 139 and 213 so);
+// values written in one phase and read in the next are loaded past the SM's L1.
 // The shared body: threads t0, t0 + stride, ... of one rollout; `sync` is the barrier among
 // all of the rollout's threads.
 template <typename Sync>
 __device__ __forceinline__ void ib_iterations(const RDesc& d, int t0, int stride, Sync sync) {
   const int nheads = __ldcg(d.ib_ctl + 2);
-  const int K2 = d.K * d.K;
   for (int it = 0; it < d.ib_iters; ++it) {
     for (int p = t0; p < d.NI; p += stride) {  // IB points
-      float ux = 0.0f, uy = 0.0f;
-      const int base = p * K2;
-      for (int q0 = 0; q0 < K2; q0 += 8) {
-        float2 v[8];
-        float w[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (q0 + q < K2) {
-            v[q] = __ldcg(d.s_uc + d.ib_slot[base + q0 + q]);
-            w[q] = d.ib_w[base + q0 + q];
-          }
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (q0 + q < K2) {
-            ux = ux + v[q].x * w[q];
-            uy = uy + v[q].y * w[q];
-          }
-      }
+      const float2 u = stencil_sum_any<true>(d, p, d.s_uc);
       const float2 nv = d.nvl[p];
-      const float sx = (nv.x - ux) * d.relax;
-      const float sy = (nv.y - uy) * d.relax;
+      const float sx = (nv.x - u.x) * d.relax;
+      const float sy = (nv.y - u.y) * d.relax;
       const float cf = clamp_factor(sx, sy, d.vmax);
       d.delta[p] = make_float2(sx * cf, sy * cf);
     }
     sync();
     for (int p = t0; p < nheads; p += stride) {
       const int2 run = d.h_run[p];
-      float dx = 0.0f, dy = 0.0f;
+      float2 s = make_float2(0.0f, 0.0f);
+      RunChunk<true> c;
       for (int j = 0; j < run.y; j += 8) {
-        int2 e[8];
-        float2 v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (j + q < run.y) {
-            e[q] = d.run[run.x + j + q];
-            v[q] = __ldcg(d.delta + e[q].x);
-          }
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (j + q < run.y) {
-            dx = dx + v[q].x * __int_as_float(e[q].y);
-            dy = dy + v[q].y * __int_as_float(e[q].y);
-          }
+        c.load(d.run + run.x, run.y, j);
+        c.add(run.y, j, d.delta, s);
       }
       const float inv = d.s_inv[p];
       const float2 u = __ldcg(d.s_uc + p);
-      d.s_uc[p] = make_float2(u.x + dx * inv, u.y + dy * inv);
+      d.s_uc[p] = make_float2(u.x + s.x * inv, u.y + s.y * inv);
     }
     sync();
   }
