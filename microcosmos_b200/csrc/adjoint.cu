@@ -300,8 +300,8 @@ __device__ __forceinline__ float2 edge_force(const AD& d, const float2* p, float
 // first; the sines, cosines and (in the reverse pass) everything else that depends on the tape
 // alone is computed for all iterations at once, by all threads; the recurrences that remain are a
 // few operations per iteration.  Same operands and summation order as the general loops below, so
-// the same bits.  Measured (256^2, 8 x 48 nodes, per launch): tape 33.7 -> 21.6 us, reverse 33.9 ->
-// 26.9 us; before, each phase of an iteration went through the tape in global memory.
+// the same bits.  Measured (256^2, 8 x 48 nodes, one launch alone with warm caches): tape 36.6 -> 22.8 us,
+// reverse 38.4 -> 28.6 us; before, each phase of an iteration went through the tape in global memory.
 constexpr int kPbdGather = 4;
 constexpr int kTapeChunk = 20;  // iterations whose angles and rest vectors the tape kernel keeps at a time
 constexpr int kRevChunk = 10;   // iterations whose tables the reverse kernel keeps at a time
