@@ -31,23 +31,21 @@ __host__ __device__ constexpr int chain_smem(int S) { return (kThetaChunk + 2) *
 
 // The threads working on one rod.  All of them call chain_rod together; warps beyond the rod's
 // own (chain_warps) help with the sines and cosines.
-// BAR: the number of the team's first barrier where it is known at compile time, else 0.  A barrier
-// whose number is in a register makes the compiler reserve all 16 of a CTA, so that no more than 4
-// such CTAs fit on an SM (8,000 rods of 32 nodes in the chain kernel: 107 us per launch that way).
+// BAR: the number of the team's barrier where it is known at compile time, else 0.  A barrier whose
+// number is in a register makes the compiler reserve all 16 of a CTA, so that no more than 4 such CTAs
+// fit on an SM (8,000 rods of 32 nodes in the chain kernel: 107 us per launch that way, 78 with 3
+// barriers).
 template <int BAR>
 struct TeamOf {
   int warp, warps;  // this warp's index in the team, and the team's warps
-  int bar;          // the team's named barrier; bar + 1 is that of its first warps, when the rod has fewer:
-                    // its count changes from rod to rod, so the whole team meets at `bar` in between
+  int bar;          // the team's named barrier; bar + 1 is that of a rod's own warps
   __device__ __forceinline__ void sync() const {
     if (warps == 1)
       __syncwarp();
     else if (BAR == 0)
       asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(warps * 32) : "memory");
-    else if (bar == BAR)
-      asm volatile("bar.sync %0, %1;" ::"n"(BAR), "r"(warps * 32) : "memory");
     else
-      asm volatile("bar.sync %0, %1;" ::"n"(BAR + 1), "r"(warps * 32) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"n"(BAR), "r"(warps * 32) : "memory");
   }
   // sync, and whether `p` holds for any thread of the team
   __device__ __forceinline__ bool sync_or(bool p) const {
@@ -60,21 +58,20 @@ struct TeamOf {
           : "=r"(r)
           : "r"((int)p), "r"(bar), "r"(warps * 32)
           : "memory");
-    else if (bar == BAR)
+    else
       asm volatile(
           "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
           "selp.s32 %0, 1, 0, b;\n\t}"
           : "=r"(r)
           : "r"((int)p), "n"(BAR), "r"(warps * 32)
           : "memory");
-    else
-      asm volatile(
-          "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\t"
-          "selp.s32 %0, 1, 0, b;\n\t}"
-          : "=r"(r)
-          : "r"((int)p), "n"(BAR + 1), "r"(warps * 32)
-          : "memory");
     return r != 0;
+  }
+  // The first rw warps, those of a rod.  Their barrier's count changes from rod to rod, so the whole
+  // team meets at its own in between.  (With numbers per team all warps of a team stay with its
+  // barrier, since not every team has two.)
+  __device__ __forceinline__ TeamOf<BAR ? BAR + 1 : 0> rod(int rw) const {
+    return {warp, rw, BAR ? BAR + 1 : rw == warps ? bar : bar + 1};
   }
 };
 using Team = TeamOf<0>;
@@ -262,7 +259,7 @@ __device__ __forceinline__ void pbd_iterations(const F& start, const RDesc& d, c
   const bool act = tm.warp < rw, edge = l.j >= 0 && l.j < l.ne;
   const float Wf = (float)d.W, Hf = (float)d.H, ksh = d.k_shear, kst = d.k_stretch;
   float2* ex = tab + kThetaChunk * S;
-  const T rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
+  const auto rod = tm.rod(rw);
   const int cycles = d.cycles;
   int buf = 0;
   if (cycles <= 0) start();
@@ -478,7 +475,7 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
   const float edg = ((j < nb) + (j >= 1 && j - 1 < nb)) == 2 ? 0.5f : 1.0f;
   const float ndg = ((j < ne) + (j >= 1 && j - 1 < ne)) == 2 ? 0.5f : 1.0f;
   if (d.solver == 1) {
-    const T rod = {tm.warp, rw, rw == tm.warps ? tm.bar : tm.bar + 1};
+    const auto rod = tm.rod(rw);
     if (act && several)
       cosserat_rod<true>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
     else if (act)
