@@ -354,9 +354,7 @@ __global__ void __launch_bounds__(kStagedThreads, 2)
 // The cells touched by IB points this step, one thread each: the TRT + Guo collision with
 // the body force F = (u_corrected - u) rho that k_ib_finalize left per head (fluid.py:327-350),
 // written over the dense pass's force-free result.  The populations are pulled again; the
-// density and clamped velocity are the ones the tile kernel computed from the same values.
-// (Storing the pulled populations per head in the tile kernel instead was measured: the
-// stores cost the tile kernel more than the coalesced reads saved here.)
+// density and clamped velocity are the ones k_ib_heads computed from the same values.
 // The head count is the copy k_ib_finalize saved in ib_ctl[5] (the next step's node
 // pipeline resets ib_ctl[2] while this kernel may still run).
 __global__ void __launch_bounds__(kHeadThreads) k_collide_heads(const RDesc* __restrict__ D, const int* __restrict__ off,

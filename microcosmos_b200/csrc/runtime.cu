@@ -730,14 +730,15 @@ void timed(mc_plan* p, int kind, cudaStream_t s, bool capture, F&& launch) {
   p->ev_pending.push_back({kind, a, b});
 }
 
-// One step (src/microcosmos/simulate.py:37-100) is launched as three pieces:
+// One step (src/microcosmos/simulate.py:37-100) is launched as four pieces:
 //   pipeline(t): predict, CIC deposit, steric filter, rod kernels      (simulate.py:41-84)
-//   ib(t):       IB bins, multi-direct forcing iterations, body force   (fluid.py:268-339)
-//   lbm(t):      the dense stream + collide pass                        (fluid.py:341-357)
+//   ib(t):       touched cells, multi-direct forcing rounds, body force (fluid.py:268-339)
+//   lbm(t):      the dense stream + collide pass, then the touched cells (fluid.py:341-357)
 //   tail(t):     node reaction, wrap, recording, step counter           (fluid.py:359-382)
-// pipeline(t+1) depends only on tail(t), so it runs on a second stream concurrently with
-// lbm(t); ib(t+1) joins both.  Per-step field recording needs lbm(t) before tail(t)'s
+// pipeline(t+1) depends only on tail(t), so it follows on the main stream while lbm(t) runs on its
+// own; ib(t+1) joins both (enqueue_body).  Per-step field recording needs lbm(t) before tail(t)'s
 // field copy and before pipeline(t+1) rewrites the steric field, so it runs sequentially.
+
 // e: values per thread of the register-radix kernels (4, 8 or 16); a side of length N takes
 // them when it is a power of two with E <= N <= 256 E.  tv: values per column-pass CTA.
 StericCtas steric_ctas(const HostRollout& h, int e, int tv) {
