@@ -457,8 +457,8 @@ __global__ void __launch_bounds__(256) k_stream_out(const RDesc* __restrict__ D,
                         (off[r + 1] - off[r]) * 8, threadIdx.x & 31);
 }
 
-// Workspace initialisation: deposit grid = 0, counters = 0.
-__global__ void k_clear_ws(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+// Workspace initialisation: deposit grid = 0, counters = 0, and the rollouts' flags if asked for.
+__global__ void k_clear_ws(const RDesc* __restrict__ D, const int* __restrict__ off, int n, int flags) {
   const int r = find_rollout(off, n, blockIdx.x);
   const RDesc& d = D[r];
   const int lb = blockIdx.x - off[r];
@@ -478,7 +478,7 @@ __global__ void k_clear_ws(const RDesc* __restrict__ D, const int* __restrict__ 
     d.ib_ctl[t0] = 0;
     d.c_ctl[t0] = 0;
   }
-  if (t0 == 0) *d.flags = 0u;
+  if (flags && t0 == 0) *d.flags = 0u;
 }
 
 template <int VEC>
@@ -542,6 +542,6 @@ void launch_unstream(const Launch& L) { k_unstream<<<L.grid, 256, 0, L.s>>>(L.d,
 void launch_stream_out(const Launch& L, int parity, float* dst) {
   k_stream_out<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n, parity, dst);
 }
-void launch_clear_ws(const Launch& L) { k_clear_ws<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n); }
+void launch_clear_ws(const Launch& L, bool flags) { k_clear_ws<<<L.grid, 256, 0, L.s>>>(L.d, L.off, L.n, flags); }
 
 }  // namespace mc

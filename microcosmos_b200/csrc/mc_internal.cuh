@@ -305,7 +305,7 @@ void launch_reaction(const Launch& L, const int* tdev);
 void launch_record_fields(const Launch& L, const int* tdev, int advanced);
 void launch_unstream(const Launch& L);
 void launch_stream_out(const Launch& L, int parity, float* dst = nullptr);
-void launch_clear_ws(const Launch& L);
+void launch_clear_ws(const Launch& L, bool flags);
 void launch_tick(const Launch& L, int* tdev);
 cudaError_t fft_set_smem(size_t rows, size_t cols);
 void launch_fft_rows_p2(const Launch& L, size_t smem);

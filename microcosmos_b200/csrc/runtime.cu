@@ -1948,7 +1948,8 @@ mc_status mc_plan_bind(mc_plan* p, void* workspace, size_t bytes, void* stream) 
       p->lbm_staged_ctas = sms * nl;
     }
   }
-  mc::launch_clear_ws(L(p, K_CELLS, s));
+  mc::launch_clear_ws(L(p, K_CELLS, s), true);
+  p->pending_next = false;
   MC_CUDA(cudaGetLastError());
   destroy_graphs(p);
   if (!p->cap_stream) MC_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
@@ -2010,6 +2011,12 @@ mc_status mc_rollout_begin(mc_plan* p, const mc_state* states, const mc_actuatio
   p->step = 0;
   p->active = true;
   p->last_launches = 0;
+  if (p->pending_next) {
+    // a rollout was left with its next step's pipeline launched: its deposit, bins and buckets go
+    MC_CUDA(cudaMemsetAsync(p->ws + p->r_wl_ctl.off, 0, 4 * sizeof(int), s));
+    mc::launch_clear_ws(L(p, K_CELLS, s), false);
+    p->last_launches += 1;
+  }
   if (p->any_fluid) {
     mc::launch_unstream(L(p, K_SHIFT, s));
     p->last_launches += 1;
