@@ -286,6 +286,50 @@ __global__ void __launch_bounds__(256) k_bin_tiles(const RDesc* __restrict__ D, 
 }
 
 // ---------------------------------------------------------------- touched cells
+// The touched cells listed in the order of the lattice, from the cells' counters: 8 cells per thread,
+// one atomic per CTA.  The stencil kernel's own list follows the points; where these are many and lie
+// in no order of the lattice (short rods, loose nodes), neighbouring cells are then far apart in the
+// list and every kernel of the touched cells fetches the same sectors of the populations again and
+// again, from HBM once they exceed the L2 (the rule: ib_list in runtime.cu).  Bound by HBM: 4 B per
+// cell (35 us at 4096^2, 8 at 2048^2 inside a step's launches).
+__global__ void __launch_bounds__(256) k_ib_list(const RDesc* __restrict__ D, const int* __restrict__ off, int n) {
+  __shared__ int s_sum[8], s_base;
+  const int r = find_rollout(off, n, blockIdx.x);
+  const RDesc& d = D[r];
+  after_previous();
+  const int cells = d.lH * d.lW, c0 = (blockIdx.x - off[r]) * kListCells + threadIdx.x * 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned touched = 0;
+  if (c0 + 8 <= cells) {
+    const int4 a = *reinterpret_cast<const int4*>(d.ib_cnt + c0), b = *reinterpret_cast<const int4*>(d.ib_cnt + c0 + 4);
+    touched = (a.x > 0) | (a.y > 0) << 1 | (a.z > 0) << 2 | (a.w > 0) << 3 | (b.x > 0) << 4 | (b.y > 0) << 5 |
+              (b.z > 0) << 6 | (b.w > 0) << 7;
+  } else {
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < cells && d.ib_cnt[c0 + i] > 0) touched |= 1u << i;
+  }
+  const int mine = __popc(touched);
+  int at = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += v;
+  }
+  if (lane == 31) s_sum[warp] = at;
+  at -= mine;
+  __syncthreads();
+  int all = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (i == warp) at += all;
+    all += s_sum[i];
+  }
+  if (threadIdx.x == 0) s_base = all > 0 ? atomicAdd(d.ib_ctl + 2, all) : 0;
+  __syncthreads();
+  at += s_base;
+  for (; touched; touched &= touched - 1) d.h_new[at++] = c0 + __ffs(touched) - 1;
+}
+
 // Sorts R (key, value) pairs in registers by key.
 template <int R>
 __device__ __forceinline__ void sort_regs(int (&k)[R], float (&w)[R]) {
@@ -980,6 +1024,7 @@ cudaError_t tiles_blocks_per_sm(int threads, int capS, int* out) {
 void launch_bin_tiles(const Launch& L, const int2* wl, int* wl_count, int capS, int threads) {
   launch(L, k_bin_tiles, threads, (size_t)4 * capS * sizeof(unsigned), L.d, wl, wl_count, capS);
 }
+void launch_ib_list(const Launch& L) { launch(L, k_ib_list, kListCells / 8, 0, L.d, L.off, L.n); }
 void launch_ib_heads(const Launch& L, int parity) {
   launch(L, k_ib_heads, kHeadThreads, 0, L.d, L.off, L.n, parity);
 }

@@ -27,6 +27,7 @@ constexpr int kStagedThreads = 256;  // ... and threads per CTA (4 cells each)
 constexpr int kConvTile = 32;     // steric direct convolution: 32 x 32 outputs per CTA
 constexpr int kConvMaxR = 24;     // largest tap radius of the direct convolution
 constexpr int kHeadSort = 16;        // contributions of a touched cell that k_ib_heads sorts in registers
+constexpr int kListCells = 2048;   // cells per CTA of k_ib_list
 constexpr int kCicCap = 512;       // minimum CIC bin capacity per tile
 constexpr int kMaxBinCap = 8192;   // largest bin capacity (the tile sort keeps 4 x cap words in shared memory)
 constexpr int kFftMaxN = 4096;     // largest FFT length (shared memory)
@@ -124,6 +125,7 @@ struct RDesc {
   // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of `run`, ctl[2] = heads, ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
   // ctl[5] = the head count saved for k_collide_heads.
   int ib_cap;
+  int ib_list;      // the touched cells are listed by k_ib_list and not by the stencil kernel
   float* ib_w;      // (M) normalised stencil weight
   int* ib_slot;     // (M) contribution -> head of its cell
   int* ib_cnt;      // (lH lW) contributions of the cell, zero between steps
@@ -136,7 +138,7 @@ struct RDesc {
   // (with the space that the sort of a long one needs: at most 20 entries per 9 contributions)
   int2* run;        // (5 M / 2)
   // per head, in [0, ctl[2])
-  int* h_new;       // cell, as the stencil kernel lists it (while k_collide_heads may still use h_cell)
+  int* h_new;       // cell, as the stencil kernel or k_ib_list lists it (while k_collide_heads may still use h_cell)
   int* h_cell;      // cell, from k_ib_heads on
   int2* h_run;      // start and length of its run
   float4* s_mac;    // density, clamped velocity (and a word to fill it up)
@@ -281,6 +283,7 @@ void launch_chain(const Launch& L, const int* tdev, int longest);
 void launch_steric(const Launch& L);
 void launch_stencil(const Launch& L);
 void launch_stencil4(const Launch& L);
+void launch_ib_list(const Launch& L);
 void launch_ib_heads(const Launch& L, int parity);
 void launch_ib_interp(const Launch& L, int it);
 void launch_ib_spread(const Launch& L, int it, int fuse_finalize);

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) k_stencil(const RDesc* __restrict__ D, co
         if (b < K) {
           const int k = p * K2 + a * K + b, cell = cy[b] * d.lW + cx[a];
           d.ib_w[k] = (wx[a] * wy[b]) / den;
-          if (ib_append(d, cell, k)) d.h_new[atomicAdd(d.ib_ctl + 2, 1)] = cell;
+          if (ib_append(d, cell, k) && !d.ib_list) d.h_new[atomicAdd(d.ib_ctl + 2, 1)] = cell;
         }
       }
     }
@@ -268,21 +268,25 @@ __global__ void __launch_bounds__(128) k_stencil4(const RDesc* __restrict__ D, c
 #pragma unroll
   for (int b = 0; b < 4; ++b)
     if (mine && b < K) d.ib_w[k0 + b] = w[b] / den;
-  int fresh = 0;
+  if (!d.ib_list) {
+    int fresh = 0;
 #pragma unroll
-  for (int b = 0; b < 4; ++b) fresh += pos[b] == 0 ? 1 : 0;
-  int before = fresh;
+    for (int b = 0; b < 4; ++b) fresh += pos[b] == 0 ? 1 : 0;
+    int before = fresh;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(full, before, o);
-    if (lane >= o) before += v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(full, before, o);
+      if (lane >= o) before += v;
+    }
+    int base = 0;
+    if (lane == 31 && before > 0) base = atomicAdd(d.ib_ctl + 2, before);
+    base = __shfl_sync(full, base, 31) + before - fresh;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (pos[b] == 0) d.h_new[base++] = cell[b];
   }
-  int base = 0;
-  if (lane == 31 && before > 0) base = atomicAdd(d.ib_ctl + 2, before);
-  base = __shfl_sync(full, base, 31) + before - fresh;
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
-    if (pos[b] == 0) d.h_new[base++] = cell[b];
     if (pos[b] >= 0 && pos[b] < d.ib_cap) {
       d.ib_bucket[(size_t)cell[b] * d.ib_cap + pos[b]] = k0 + b;
     } else if (pos[b] >= 0) {

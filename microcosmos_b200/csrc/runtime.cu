@@ -44,11 +44,13 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 
 constexpr int kDefaultSortCap = 2048;  // contributions per tile sorted in shared memory by default
+// lattice cells of a plan from which its populations exceed the L2 (72 B of 126 MB each)
+constexpr long long kListMinCells = 1750000;
 constexpr int kNodeStepSmem = 220 * 1024;  // dynamic shared memory of a node-step CTA at most
 // largest plan (IB points over all rollouts) whose body force is computed by the last IB round
 constexpr long long kFuseFinalizeMaxPoints = 65536;
 
-enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES4, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_SHIFT, K_COUNT };
+enum Kind { K_NODES = 0, K_COMP, K_CHAIN, K_IB, K_TILES, K_LBM, K_CELLS, K_FFTR, K_FFTC, K_NODES4, K_IBCOOP, K_FFTR2, K_FFTC2, K_SCONV, K_FR16, K_FC16, K_FR12, K_FC12, K_SHIFT, K_LIST, K_COUNT };
 
 // CTAs of the steric filter kernels for one rollout: the radix-16 register kernels for
 // power-of-two sides >= 16, the mixed-radix Stockham kernels for the other FFT sides, or
@@ -90,6 +92,7 @@ struct HostRollout {
   Region r_cgW, r_cgH;
   int M = 0, ntx = 0, nty = 0, lbm_tx = 0, lbm_ty = 0, vec = 4, lbm_th = 4;
   int lH = 0, lW = 0;      // the fluid lattice (= dims.H, dims.W unless dims.fluid_H/W are set)
+  int ib_list = 0;            // touched cells listed from the cells' counters (k_ib_list)
   int ib_cap = 0, c_cap = 0;  // capacities of a cell's bucket (IB) and of a tile's bin (CIC), powers of two
   int logW = -1, logH = -1;   // log2 of power-of-two grid sides (-1: mixed radix path)
   int T_r = 0, P_r = 0, T_c = 0, P_c = 0;
@@ -614,6 +617,7 @@ void fill_desc(mc_plan* p, int i, const mc_state* st, const mc_actuation* act, c
   d.nvl = at<float2>(b, h.r_nvl);
   d.delta = at<float2>(b, h.r_delta);
   d.ib_cap = h.ib_cap;
+  d.ib_list = h.ib_list;
   d.ib_w = at<float>(b, h.r_ibw);
   d.ib_slot = at<int>(b, h.r_ibslot);
   d.ib_cnt = at<int>(b, h.r_ibcnt);
@@ -698,7 +702,7 @@ const char* const kProfNames[] = {"predict", "cic_bins",  "fft_rows",    "fft_co
                                    "node",    "ib_bins",   "ib_interp",   "ib_spread", "ib_finalize",
                                    "lbm",     "reaction",  "record_fields", "tick",    "steric",
                                    "stencil", "ib_fused", "steric_conv", "collide_heads", "ib_cluster",
-                                   "node_step"};
+                                   "node_step", "ib_list"};
 constexpr int kNumProf = sizeof(kProfNames) / sizeof(kProfNames[0]);
 
 cudaEvent_t take_event(mc_plan* p) {
@@ -928,6 +932,10 @@ int64_t enqueue_pipeline(mc_plan* p, bool tick, cudaStream_t s, bool chained, bo
       timed(p, 15, s, capture, [&] { mc::launch_stencil4(L(p, K_NODES4, s, on)); });
     else
       timed(p, 15, s, capture, [&] { mc::launch_stencil(L(p, K_NODES, s, on)); });
+    ++k;
+  }
+  if (p->grid[K_LIST]) {
+    timed(p, 21, s, capture, [&] { mc::launch_ib_list(L(p, K_LIST, s, on)); });
     ++k;
   }
   return k;
@@ -1554,6 +1562,8 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     }
   }
   p->compact_ok = compact_shape(p->R, &p->ns);
+  long long plan_cells = 0;
+  for (const auto& h : p->R) plan_cells += (long long)h.lH * h.lW;
   for (int i = 0; i < n; ++i) {
     HostRollout& h = p->R[i];
     const mc_dims& D = h.dims;
@@ -1593,6 +1603,13 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     // only when another layout of the IB kernels is asked for, keep half as many (256 lattices of
     // 128^2 with 16 points each 675 -> 541 MB).
     h.ib_cap = p->compact_ok ? 8 : (double)Mz < 2.0 * (double)LHW ? 16 : 32;
+    // Touched cells listed in the order of the lattice where the plan's populations exceed the L2 and
+    // the contributions are a third of the cells or more.  us per step, listed by the points and by the
+    // lattice: 500,000 loose nodes on 4096^2 4,855 and 3,512, 20,000 rods of 20 on 2048^2 with the 3-point
+    // kernel 1,029 and 843, 1,600 rods of 64 there (0.39 of the cells) 430 and 404, 160 rollouts of 1,600
+    // nodes on 128^2 740 and 742.  Below a third long rods keep their cells together and the list over
+    // all cells is paid for nothing; with populations in the L2 (1.75 M cells) the order hardly counts.
+    h.ib_list = plan_cells >= kListMinCells && 3 * Mz >= LHW;
     const size_t cells = h.M > 0 ? LHW : 0;
     h.r_ibw = lay.take(Mz * 4);
     h.r_ibslot = lay.take(Mz * 4);
@@ -1658,8 +1675,6 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
   // default dense-pass tile: 4 cells per lane x 16 rows for plans of >= 4 M lattice cells
   // (measured best at 2048^2 and on the 25 M-cell batch: 0.78 / 0.91 of HBM), 2 x 4 below
   // (best at 1024^2: 20.8 us vs 22.9 us for 4 x 16); narrower when the widths need it
-  long long plan_cells = 0;
-  for (const auto& h : p->R) plan_cells += (long long)h.lH * h.lW;
   const bool big_plan = plan_cells >= (4LL << 20);
   if (!big_plan && vec_all == 4) vec_all = 2;
   p->lbm_vec = vec_all;
@@ -1700,6 +1715,7 @@ mc_status mc_plan_create(int32_t n, const mc_dims* dims, const mc_config* cfg, c
     cnt[K_TILES] = h.ntx * h.nty;
     cnt[K_LBM] = c.enable_fluid ? h.lbm_tx * h.lbm_ty : 0;
     cnt[K_CELLS] = std::min(div_up(HW, 256), 1024);
+    cnt[K_LIST] = h.ib_list ? div_up((long long)h.lH * h.lW, mc::kListCells) : 0;
     cnt[K_SHIFT] = std::min(div_up((long long)h.lH * div_up(h.lW, 128), 8), 2048);  // 8 warps, 128 cells each
     // every length goes through the multi-transform kernels (the one-transform-per-CTA
     // kernels serve the allocation-free entry point)
