@@ -221,7 +221,8 @@ mc_status mc_rollout(mc_plan* plan, const mc_state* states, int32_t num_steps,
  * (last != 0: the final one of them writes fields.fluid_velocity and the call returns with
  * that step complete -- none of the next step is started -- so the caller may change the
  * state's positions, velocities, rest lengths or rest angles before a further advance; the
- * advance before end must pass last != 0); end: write fields.f_grid back.
+ * advance before end must pass last != 0); end: write fields.f_grid back.  A begin without an
+ * end before it drops the rollout that was in progress.
  * mc_rollout(...) == begin + advance(num_steps, last=1) + end. */
 mc_status mc_rollout_begin(mc_plan* plan, const mc_state* states, const mc_actuation* const* act,
                            const mc_record* const* rec, void* stream);

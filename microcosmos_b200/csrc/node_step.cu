@@ -471,10 +471,14 @@ __global__ void __launch_bounds__(kNodeStepMaxThreads, 1)
     // ---- rods: teams of the same number of warps, one rod at a time each
     {
       const int tw = shape.rod_warps, team = warp / tw;
+      const Team tm = {warp - team * tw, tw, 1 + shape.bars * team};
       if (team < shape.teams)
-        for (int c = team; c < d.nchain; c += shape.teams)
-          chain_rod<false>(d, d.chain_info[c], t, Team{warp - team * tw, tw, 1 + shape.bars * team}, m.pos(),
-                    m.tab() + (size_t)team * chain_smem(shape.longest), shape.longest);
+        for (int c = team; c < d.nchain; c += shape.teams) {
+          // all warps of the team, those that the rod before did not use too
+          if (c != team && d.solver == 1) tm.sync();
+          chain_rod<false>(d, d.chain_info[c], t, tm, m.pos(), m.tab() + (size_t)team * chain_smem(shape.longest),
+                           shape.longest);
+        }
     }
     __syncthreads();
     // ---- velocity, IB points and their stencils: 4 lanes per IB point, lane a column a of the

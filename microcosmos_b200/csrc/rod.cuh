@@ -431,7 +431,9 @@ __device__ __forceinline__ void cosserat_rod(const RDesc& d, const T& rod, const
 
 // All cycles_per_step iterations at step t of the chain info = (first node, nodes, first edge, first
 // pair).  pos: the rollout's node positions (x, y), updated in place; tab: chain_smem(S) float2 of
-// shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.
+// shared memory, S >= the rod's nodes.  Every warp of the team calls it with the same arguments.  A PBD
+// rod ends with a barrier of the whole team, a Cosserat rod does not: its exchange buffers and its own
+// warps' barrier are free for another rod of the team only after one (k_node_step).
 template <bool CHAINED, class T>
 __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, const T& tm, float* pos, float2* tab,
                                           int S) {
@@ -480,10 +482,6 @@ __device__ __forceinline__ void chain_rod(const RDesc& d, int4 info, int t, cons
       cosserat_rod<true>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
     else if (act)
       cosserat_rod<false>(d, rod, l, x, y, th, l0, ra, kb, edg, tab, S);
-    // All warps of the team, those the rod does not use too: its exchange buffers and its barrier
-    // (bar + 1, with this rod's warps) are free for the team's next rod.  A PBD rod ends with such
-    // a barrier in pbd_iterations.  (A team of the chain kernel has one rod.)
-    if (!CHAINED) tm.sync();
   }
   else if (several)
     pbd_iterations<true>(late, d, tm, rw, l, e0, x, y, th, l0, ra, kb, edg, ndg, tab, S);
