@@ -122,8 +122,9 @@ struct RDesc {
   // IB contributions k = point*K*K + entry.  Each is appended to its cell's bucket
   // (ib_bucket[cell * ib_cap ...], an atomic on ib_cnt picks the place); beyond ib_cap it goes to
   // the cell's overflow list (ib_ovf_head, ib_ovf_next, ib_ovf).  The first one of a cell makes it
-  // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of `run`, ctl[2] = heads, ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier,
-  // ctl[5] = the head count saved for k_collide_heads.
+  // a touched cell ("head").  ctl[0] = overflow entries, ctl[1] = use of `run`, ctl[2] = heads,
+  // ctl[3], ctl[4] = arrival count and generation of the fused IB kernel's barrier, ctl[5] = the
+  // head count saved for k_collide_heads.
   int ib_cap;
   int ib_list;      // the touched cells are listed by k_ib_list and not by the stencil kernel
   float* ib_w;      // (M) normalised stencil weight
