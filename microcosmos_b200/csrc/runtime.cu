@@ -1011,10 +1011,10 @@ int64_t enqueue_tail(mc_plan* p, int rec_fields, bool has_next, cudaStream_t s, 
 // Whether a step's kernels are launched chained.  Not while kernels are timed one at a time, and not
 // where the node grid is more than half of what a B200 holds at once (148 SMs x 16 CTAs of 128
 // threads): the CTAs that wait then take the slots the dense pass beside them would run in.  us per
-// step without and with, by node CTAs: one lattice of 1024^2 (128) 126 and 114; uneven rollouts 931:
-// 751 and 726, 1,295: 1,004 and 1,037, 1,578: 1,199 and 1,242, 2,091: 1,557 and 1,657, 2,344: 1,947 and
-// 2,068.  Equal rollouts, whose CTAs all end together, gain beyond the line too, but less and less
-// (1,024: 472 and 449, 1,536: 672 and 650, 2,048: 897 and 878); uneven ones are what is batched.
+// step without and with, by node CTAs: one lattice of 1024^2 (128) 122 and 111; uneven rollouts 931:
+// 720 and 693, 1,295: 954 and 970, 1,578: 1,144 and 1,170, 2,091: 1,487 and 1,539, 2,344: 1,860 and
+// 1,936.  Equal rollouts, whose CTAs all end together, gain beyond the line too, but less and less
+// (1,024: 424 and 400, 1,536: 599 and 573, 2,048: 807 and 781); uneven ones are what is batched.
 bool chain_launches(const mc_plan* p) { return !p->profiling && p->grid[K_NODES] <= 8 * 148; }
 
 // Everything of step t after its pipeline, plus pipeline(t+1) when has_next; with `first` the
@@ -1183,11 +1183,11 @@ void destroy_graphs(mc_plan* p) {
 // and 1,400 with the 2-point one.  One CTA's time grows with the points; the separate launches of a few
 // rollouts cost about 55 us a step whatever their size, those of many rollouts grow with all points.
 // Measured, us per step in the node-step kernel and in separate launches (128^2 or 64^2 lattices):
-//   one rollout, 4-point: 32 points 36 and 54; 128: 46 and 55; 192: 55 and 54; 256: 64 and 55;
-//     384: 82 and 57;  3-point: 128: 39 and 54; 256: 51 and 54; 384: 60 and 56; 640: 91 and 57;
-//     2-point: 128: 43 and 52; 384: 53 and 54; 640: 71 and 54; 1,280: 123 and 55;
-//   384 points, 4-point: 8 rollouts 80 and 65; 32: 85 and 88; 64: 86 and 124; 148: 107 and 233;
-//     1,024: 809 and 1,641.  16 points: 256 rollouts 121 and 157; 1,024: 218 and 248.
+//   one rollout, 4-point: 32 points 35 and 52; 128: 45 and 54; 192: 55 and 54; 256: 63 and 55;
+//     384: 81 and 57;  3-point: 128: 39 and 53; 256: 50 and 54; 384: 60 and 55; 640: 91 and 56;
+//     2-point: 128: 42 and 52; 384: 51 and 53; 640: 72 and 53; 1,280: 123 and 55;
+//   384 points, 4-point: 8 rollouts 80 and 63; 32: 85 and 85; 64: 87 and 108; 148: 107 and 192;
+//     1,024: 810 and 1,312.  16 points: 256 rollouts 121 and 157; 1,024: 218 and 236.
 // So for fewer than some 30 rollouts the line lies too high (it was set when the separate launches
 // were not chained and took 90 us at 384 points); below about 190, 320 and 400 points, and for
 // more rollouts at every size, the kernel is the faster form.
